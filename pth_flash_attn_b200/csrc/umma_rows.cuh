@@ -1,18 +1,31 @@
-// Building blocks of the row-major tcgen05 attention kernel (head size 128): query
-// rows on the MMA M dimension, as a prefill or a wide verification step wants them.
+// Building blocks of the row-major tcgen05 attention kernels (query rows on the MMA M
+// dimension, as a prefill or a wide verification step wants them).
 //
 //   S[row, key] = sum_d   Q[row, d] * K[key, d]     A = Q image (K-major), B = K tile (K-major)
 //   O[row, d]  += sum_key P[row, key] * V[key, d]   A = P in TMEM,         B = V tile (MN-major)
 //
-// K and V tiles are the widened bf16 images of umma_tile.cuh (chunk c of 8 d, key t at
-// c * kChunkStride + t * 16), which serve as B operands unchanged: for K (N = keys,
-// K-major) LBO = chunk stride, SBO = 128; for V (N = d, MN-major) LBO = 128 (next 8
-// keys), SBO = chunk stride (next 8 d).  The Q image has the same form with rows in
-// place of keys.  P never touches shared memory: the softmax thread of a row writes
-// its probabilities as packed bf16 pairs into TMEM (lane = row, 32-bit column j =
-// keys 2j, 2j + 1) and the PV MMA reads its A operand from there.
+// K and V tiles are widened images (chunk c of 8 d, key t at c * kChunkStride + t * 16), which
+// serve as B operands unchanged: for K (N = keys, K-major) LBO = chunk stride, SBO = 128; for V
+// (N = d, MN-major) LBO = 128 (next 8 keys), SBO = chunk stride (next 8 d).  The Q image has the
+// same form with rows in place of keys.  P never touches shared memory: the softmax thread of a
+// row writes its probabilities as packed pairs into TMEM (lane = row, 32-bit column j = keys
+// 2j, 2j + 1) and the PV MMA reads its A operand from there.
+//
+// Every operand is fp16, whatever the queries are (both operands of an MMA have one format):
+//   K, V   int8 is exact in fp16, and its widening costs 1.25 instructions per value; to bf16,
+//          whose 8 bits hold no biased int8, it takes 2;
+//   Q      fp16 as it is; bf16 times the power of two that puts the largest query value of the
+//          CTA into [2^14, 2^15): exact down to 2^-31 of that value, and the inverse is folded
+//          into the keys' score factor;
+//   P      exp2(score + log2(v_scale) - reference): the key's v_scale sits in the exponent, so
+//          V needs no multiplication, the 11 bits of P are relative to the largest weighted
+//          probability of the row (fp16's range is that of one row, not of the cache), and the
+//          row sum takes P / v_scale back in fp32.
 #pragma once
 
+#include <cuda_fp16.h>
+
+#include "params.cuh"
 #include "umma_tile.cuh"
 
 namespace pthb200 {
@@ -119,7 +132,7 @@ __device__ __forceinline__ void mma_ts_words(uint32_t d_tmem, uint32_t a_tmem, u
 }
 // q = rows_desc(Q image, kChunkStride, 128), k = rows_desc(K image, kChunkStride, 128)
 __device__ __forceinline__ void issue_qk_rows_words(uint32_t s_tmem, RowsDesc q, RowsDesc k) {
-  constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kTileKeys, tc::kFmtBF16, tc::kFmtBF16, 0, 0);
+  constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kTileKeys, tc::kFmtF16, tc::kFmtF16, 0, 0);
   constexpr uint32_t step = (2 * kChunkStride) >> 4;
   mma_ss_words<false>(s_tmem, q.lo, q.hi, k.lo, k.hi, idesc);
 #pragma unroll
@@ -128,7 +141,7 @@ __device__ __forceinline__ void issue_qk_rows_words(uint32_t s_tmem, RowsDesc q,
 }
 // v = rows_desc(V image, 128, kChunkStride)
 __device__ __forceinline__ void issue_pv_rows_words(uint32_t o_tmem, uint32_t p_tmem, RowsDesc v, bool accumulate) {
-  constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kHeadDim, tc::kFmtBF16, tc::kFmtBF16, 0, 1);
+  constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kHeadDim, tc::kFmtF16, tc::kFmtF16, 0, 1);
 #pragma unroll
   for (int kk = 0; kk < kTileKeys / 16; ++kk)
     mma_ts_words(o_tmem, p_tmem + kk * 8, v.lo + kk * (256 >> 4), v.hi, idesc, accumulate || kk > 0);
@@ -137,13 +150,161 @@ __device__ __forceinline__ void issue_pv_rows_words(uint32_t o_tmem, uint32_t p_
 // PV of one tile as two chains: keys 0-63 (P columns 0-31 of the S buffer, V rows 0-63) into the
 // accumulator at o_tmem, keys 64-127 (P columns 64-95, V rows 64-127) into the one at o_tmem + 128.
 __device__ __forceinline__ void issue_pv_halves_words(uint32_t o_tmem, uint32_t s_tmem, RowsDesc v, bool accumulate) {
-  constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kHeadDim, tc::kFmtBF16, tc::kFmtBF16, 0, 1);
+  constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kHeadDim, tc::kFmtF16, tc::kFmtF16, 0, 1);
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
     for (int kk = 0; kk < kTileKeys / 32; ++kk)
       mma_ts_words(o_tmem + h * 128, s_tmem + h * 64 + kk * 8, v.lo + (h * 4 + kk) * (256 >> 4), v.hi, idesc,
                    accumulate || kk > 0);
+}
+
+// 4 int8 (one 32-bit word) -> 4 fp16, exactly: with the sign bit flipped a byte is x + 128, the
+// fp16 bit pattern 0x6400 | (x + 128) is the integer 1152 + x.
+__device__ __forceinline__ void widen4_f16(uint32_t w, uint32_t& out01, uint32_t& out23) {
+  const uint32_t b = w ^ 0x80808080u;
+  const uint32_t a01 = __byte_perm(b, 0x64646464u, 0x5140);
+  const uint32_t a23 = __byte_perm(b, 0x64646464u, 0x7362);
+  const __half2 off = __half2half2(__ushort_as_half(0x6480));  // 1152
+  const __half2 r01 = __hsub2(*reinterpret_cast<const __half2*>(&a01), off);
+  const __half2 r23 = __hsub2(*reinterpret_cast<const __half2*>(&a23), off);
+  out01 = *reinterpret_cast<const uint32_t*>(&r01);
+  out23 = *reinterpret_cast<const uint32_t*>(&r23);
+}
+__device__ __forceinline__ uint4 widen8_f16(uint2 raw) {
+  uint4 r;
+  widen4_f16(raw.x, r.x, r.y);
+  widen4_f16(raw.y, r.z, r.w);
+  return r;
+}
+__device__ __forceinline__ uint32_t pack_f16(float a, float b) {
+  const __half2 v = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ float ex2f(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// ---- queries ----
+// Largest magnitude of 8 bf16 values, as fp32 bits (which order like the values).
+__device__ __forceinline__ uint32_t amax_bits_bf16(uint4 v, uint32_t m) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) m = max(m, max((w[e] << 16) & 0x7fffffffu, w[e] & 0x7fff0000u));
+  return m;
+}
+// The power of two that moves a value of these bits into [2^14, 2^15) (1 for zero).
+__device__ __forceinline__ float query_scale(uint32_t amax_bits) {
+  if (amax_bits == 0u) return 1.0f;
+  const int e = min((int)(amax_bits >> 23) - 127, 127);  // (subnormal: -127)
+  return __uint_as_float((uint32_t)(min(14 - e, 126) + 127) << 23);
+}
+// 8 bf16 queries times a power of two -> fp16.
+__device__ __forceinline__ uint4 queries_to_f16(uint4 v, float scale) {
+  auto two = [&](uint32_t w) { return pack_f16(__uint_as_float(w << 16) * scale, __uint_as_float(w & 0xffff0000u) * scale); };
+  return make_uint4(two(v.x), two(v.y), two(v.z), two(v.w));
+}
+
+// ---- the softmax's two fp32 lanes per instruction ----
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpair(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// What the softmax needs of a key, one vector of N floats each: the score factor k_scale *
+// softmax_scale * log2 e / query scale, log2(v_scale) and 1 / v_scale.
+template <int N>
+struct KeyScales {
+  float score[N], lv[N], iv[N];
+};
+// v_scale as the softmax uses it: a scale of zero (or one too small to matter) must not turn
+// into 0 * infinity in the row sum.
+__device__ __forceinline__ float usable_v_scale(float v) { return v >= 7.9e-31f ? v : 7.9e-31f; }
+
+// Pass 1 of the softmax over N scores of a row (r: bits of S, replaced by score + log2(v_scale) in log2
+// units); returns their maximum.  visible(n): whether the row sees the key of column n.
+template <int N, bool kMask, class Wait, class Visible>
+__device__ __forceinline__ float softmax_pass1(uint32_t (&r)[N], const float* score, const float* lv, Wait half_ready,
+                                               Visible visible) {
+  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int n4 = 0; n4 < N / 4; ++n4) {
+    if (n4 == N / 8) half_ready();
+    const float4 k4 = reinterpret_cast<const float4*>(score)[n4], l4 = reinterpret_cast<const float4*>(lv)[n4];
+    const f32x2 a = fma2(pair(__uint_as_float(r[4 * n4]), __uint_as_float(r[4 * n4 + 1])), pair(k4.x, k4.y), pair(l4.x, l4.y));
+    const f32x2 b = fma2(pair(__uint_as_float(r[4 * n4 + 2]), __uint_as_float(r[4 * n4 + 3])), pair(k4.z, k4.w), pair(l4.z, l4.w));
+    float t[4];
+    unpair(a, t[0], t[1]);
+    unpair(b, t[2], t[3]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if constexpr (kMask) t[e] = visible(4 * n4 + e) ? t[e] : -INFINITY;
+      r[4 * n4 + e] = __float_as_uint(t[e]);
+      mx[e] = fmaxf(mx[e], t[e]);
+    }
+  }
+  return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+}
+// Pass 2: probabilities of 32 of the scores as packed fp16 (a masked score is -inf: exp2 gives 0); adds
+// p / v_scale to the two pairs of partial row sums.
+__device__ __forceinline__ void softmax_pass2(const uint32_t* r, const float* iv, float m_use, f32x2 (&ls)[2], uint32_t (&pk)[16]) {
+  const f32x2 neg_m = pair(-m_use, -m_use);
+#pragma unroll
+  for (int n4 = 0; n4 < 8; ++n4) {
+    const float4 i4 = reinterpret_cast<const float4*>(iv)[n4];
+    float x[4];
+    unpair(add2(pair(__uint_as_float(r[4 * n4]), __uint_as_float(r[4 * n4 + 1])), neg_m), x[0], x[1]);
+    unpair(add2(pair(__uint_as_float(r[4 * n4 + 2]), __uint_as_float(r[4 * n4 + 3])), neg_m), x[2], x[3]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x[e] = ex2f(x[e]);
+    ls[0] = fma2(pair(x[0], x[1]), pair(i4.x, i4.y), ls[0]);
+    ls[1] = fma2(pair(x[2], x[3]), pair(i4.z, i4.w), ls[1]);
+    pk[2 * n4] = pack_f16(x[0], x[1]);
+    pk[2 * n4 + 1] = pack_f16(x[2], x[3]);
+  }
+}
+__device__ __forceinline__ float sum_pairs(const f32x2 (&ls)[2]) {
+  float a, b, c, d;
+  unpair(ls[0], a, b);
+  unpair(ls[1], c, d);
+  return (a + b) + (c + d);
+}
+
+// 32 consecutive dims of an output row (16-byte aligned) in the caller's type, as 16-byte stores.
+__device__ __forceinline__ void store_out32(uint8_t* dst, int dtype, const float (&o)[32]) {
+  if (dtype == PTH_ATTN_F32) {
+#pragma unroll
+    for (int n = 0; n < 32; n += 4) *reinterpret_cast<float4*>(dst + n * 4) = make_float4(o[n], o[n + 1], o[n + 2], o[n + 3]);
+  } else if (dtype == PTH_ATTN_BF16) {
+#pragma unroll
+    for (int n = 0; n < 32; n += 8)
+      *reinterpret_cast<uint4*>(dst + n * 2) = make_uint4(pack_bf16(o[n], o[n + 1]), pack_bf16(o[n + 2], o[n + 3]),
+                                                          pack_bf16(o[n + 4], o[n + 5]), pack_bf16(o[n + 6], o[n + 7]));
+  } else {
+#pragma unroll
+    for (int n = 0; n < 32; n += 8)
+      *reinterpret_cast<uint4*>(dst + n * 2) = make_uint4(pack_f16(o[n], o[n + 1]), pack_f16(o[n + 2], o[n + 3]),
+                                                          pack_f16(o[n + 4], o[n + 5]), pack_f16(o[n + 6], o[n + 7]));
+  }
 }
 
 }  // namespace pthb200

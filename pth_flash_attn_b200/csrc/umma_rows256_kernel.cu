@@ -1,19 +1,19 @@
 // Row-major tcgen05 attention kernel for head size 256: query rows on the MMA M dimension,
 // KV tiles of 64 keys.
 //
-// The 128-dim row-major kernel (umma_rows_kernel.cu) does not stretch to 256 dims: its bf16 K
+// The 128-dim row-major kernel (umma_rows_kernel.cu) does not stretch to 256 dims: its 16-bit K
 // and V images of 128 keys would take 4 x 66 KB.  This kernel keeps the same roles and the
-// same exact int8 -> bf16 widening, with other shapes:
+// same exact widening, with other shapes:
 //   tile       128 query rows x 64 keys; the split partition stays in units of 128 keys, a
 //              CTA walks its range in steps of 64;
 //   TMEM       S0 S1 (64 columns each: tile i uses buffer i % 2, so S(i + 1) is computed while
 //              the softmax warps work on tile i), ONE accumulator O of 256 columns, and Q (128
-//              columns, two bf16 per column): Q is the A operand of QK from TMEM like P is of
+//              columns, two fp16 per column): Q is the A operand of QK from TMEM like P is of
 //              PV, which takes its 64 KB image out of shared memory;
 //   MMAs       S = Q K^T: M 128, N 64, sixteen steps of 16 dims; O += P V: M 128, N 256, four
 //              steps of 16 keys;
 //   producers  thread (key, half) of the K set / V set widens 128 of the key's 256 dims; the
-//              threads of the upper halves also carry the key's scale;
+//              K threads of the upper halves also publish the key's scales;
 //   softmax    two groups of 4 warps; group g owns keys 32 g .. 32 g + 31 of EVERY tile and
 //              columns 128 g .. 128 g + 127 of O.  The two threads of a row agree on the row's
 //              reference maximum tile by tile (through shared memory and one named barrier), which
@@ -37,14 +37,14 @@ namespace {
 
 constexpr int kWDim = 256;                          // head size
 constexpr int kWKeys = 64;                          // keys of a tile
-constexpr int kWChunks = kWDim / 8;                 // 16-byte column blocks of a widened row: 8 bf16 each
+constexpr int kWChunks = kWDim / 8;                 // 16-byte column blocks of a widened row: 8 fp16 each
 constexpr int kWChunkStride = kWKeys * 16 + 16;     // 1,040 B: one column block of all keys, padded
 constexpr int kWImage = kWChunks * kWChunkStride;   // 33,280 B: widened K or V of a tile
 constexpr int kWRawRow = raw_row_for(kWDim);        // 528 B
 constexpr int kWRawUnit = kWKeys * kWRawRow;        // 33,792 B: raw cells of a tile
-constexpr int kWVStage = kWImage + kWKeys * 4;      // V image + v_scale[64]
+constexpr int kWVStage = kWImage;                   // V image
 constexpr int kWNK = 2, kWNS = 2, kWNR = 2;         // K images, V stages, raw units
-constexpr int kWKsRing = 4;                         // tiles of scaled k_scale vectors kept
+constexpr int kWKsRing = 4;                         // tiles of key scales kept
 constexpr int kWGroup = 128;                        // threads of one softmax group = rows of a tile
 constexpr int kWSoftmax = 2 * kWGroup;              // warps 0-3, 4-7
 constexpr int kWGroupKeys = kWKeys / 2;             // 32 keys of a tile per group
@@ -52,6 +52,7 @@ constexpr int kWGroupDims = kWDim / 2;              // 128 columns of O per grou
 constexpr int kWProducers = 256;                    // warps 8-11 (K set) and 12-15 (V set)
 constexpr int kWMmaWarp = 16, kWLoadWarp = 17;
 constexpr int kWThreads = 576;
+constexpr int kWQBarrier = kWSoftmax + kWProducers / 2 + 32;  // Q in TMEM: softmax, K set, MMA issuer
 constexpr int kWProducerRegs = 72, kWSoftmaxRegs = 120;  // of the 96 per thread the CTA starts with
 constexpr int kWSCol = 0, kWOCol = 128, kWQCol = 384;    // TMEM columns: S buffers at 0 and 64, O, Q
 constexpr float kWRescaleGap = 8.0f;                // log2 units a row maximum may outgrow its reference
@@ -60,8 +61,8 @@ struct WLayout {
   static constexpr int kimg = 0;
   static constexpr int vst = kimg + kWNK * kWImage;
   static constexpr int raw = (vst + kWNS * kWVStage + 127) / 128 * 128;
-  static constexpr int ksc = raw + kWNR * kWRawUnit;                 // float [kWKsRing][64]: k_scale * scale * log2 e
-  static constexpr int tile_max = ksc + kWKsRing * kWKeys * 4;       // float [2 tiles][2 groups][128 rows]
+  static constexpr int ksc = raw + kWNR * kWRawUnit;                 // KeyScales<64> [kWKsRing]
+  static constexpr int tile_max = ksc + kWKsRing * (int)sizeof(KeyScales<kWKeys>);  // float [2 tiles][2 groups][128 rows]
   static constexpr int half_sum = tile_max + 2 * 2 * kWGroup * 4;    // float [2 groups][128 rows]
   static constexpr int bars = half_sum + 2 * kWGroup * 4;            // uint64 [...]
   static constexpr int n_bars = kWNS * 2 + 2 * kWNK + 6 + 2 * kWNR;
@@ -84,19 +85,9 @@ struct WBars {
 // Key of a tile held by row `r` of its images: with contiguous cells the even keys, then the odd ones.
 __device__ __forceinline__ int tile_key_w(int raw_mode, int r) { return raw_mode == 2 ? 2 * (r & 31) + (r >> 5) : r; }
 
-__device__ __forceinline__ uint32_t pack_bf16_w(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-__device__ __forceinline__ float ex2f_w(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // S(buffer) = Q K^T with Q in TMEM: 16 steps of 16 dims = two column blocks of the K image each.
 __device__ __forceinline__ void issue_qk_w(uint32_t s_tmem, uint32_t q_tmem, RowsDesc k) {
-  constexpr uint32_t idesc = tc::instr_desc(128, kWKeys, tc::kFmtBF16, tc::kFmtBF16, 0, 0);
+  constexpr uint32_t idesc = tc::instr_desc(128, kWKeys, tc::kFmtF16, tc::kFmtF16, 0, 0);
   constexpr uint32_t step = (2 * kWChunkStride) >> 4;
 #pragma unroll
   for (int kk = 0; kk < kWDim / 16; ++kk) mma_ts_words(s_tmem, q_tmem + kk * 8, k.lo + kk * step, k.hi, idesc, kk > 0);
@@ -104,7 +95,7 @@ __device__ __forceinline__ void issue_qk_w(uint32_t s_tmem, uint32_t q_tmem, Row
 // O += P V: P in two pieces (keys 0-31 in columns 0-15 of the S buffer, keys 32-63 in columns
 // 32-47: each softmax group writes P over its own half of S), four steps of 16 keys.
 __device__ __forceinline__ void issue_pv_w(uint32_t o_tmem, uint32_t s_tmem, RowsDesc v, bool accumulate) {
-  constexpr uint32_t idesc = tc::instr_desc(128, kWDim, tc::kFmtBF16, tc::kFmtBF16, 0, 1);
+  constexpr uint32_t idesc = tc::instr_desc(128, kWDim, tc::kFmtF16, tc::kFmtF16, 0, 1);
 #pragma unroll
   for (int g = 0; g < 2; ++g)
 #pragma unroll
@@ -126,6 +117,9 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::bars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
+  uint32_t* qmax_s = reinterpret_cast<uint32_t*>(smem + L::misc + 24);           // bits of the largest query value
+  volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
+  KeyScales<kWKeys>* key_scales = reinterpret_cast<KeyScales<kWKeys>*>(smem + L::ksc);
 
   const int kvh = blockIdx.y, split = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -243,6 +237,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       tc::mbar_init(&bars[B::raw_free + s], kWProducers);             // every producer thread reads every unit
     }
     *abort_flag = 0;
+    *qmax_s = 0u;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -261,8 +256,8 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kWProducerRegs));
     // Warps 8-11 widen K, warps 12-15 V.  Thread pt of a set owns key pt % 64 and dims
     // 128 (pt / 64) .. + 127 of it: 128 bytes of the raw cell, which start 0 or 8 (K) or 4 or
-    // 12 (V) bytes after a 16-byte boundary; the threads of the upper halves find the key's
-    // scale right behind their bytes.
+    // 12 (V) bytes after a 16-byte boundary; the K threads of the upper halves find k_scale
+    // right behind their bytes.
     const int pt = tid & 127;
     const bool v_part = warp >= 12;
     // Contiguous cells (raw_mode 2) alternate between the two 8-byte alignments: a warp takes
@@ -279,6 +274,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     // first byte of this thread's 128 bytes inside a raw unit
     const uint32_t piece = my_page * bs * kWRawRow + my_slot * row_pitch + delta + (v_part ? kWDim + 4 : 0) + upper * 128;
     const int wo = (int)((piece & 15u) >> 2);  // first word of the piece in the 16-byte chunks read: 0 / 2 (K), 1 / 3 (V)
+    float score_mul = 0.f;  // softmax_scale * log2 e / query scale
 #pragma unroll 1
     for (int j = 0; j < n_tiles; ++j) {
       const int rs = j % kWNR;
@@ -301,6 +297,11 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
 #pragma unroll
         for (int c = 0; c < 36; ++c) w[c] = 0u;
       }
+      // (the v_scale of the key, for the threads that publish its scales)
+      float v_scale = 1.f;
+      if (!v_part && upper && valid)
+        v_scale = *reinterpret_cast<const float*>(smem + L::raw + rs * kWRawUnit + my_page * bs * kWRawRow + my_slot * row_pitch +
+                                                  delta + 2 * kWDim + 4);
       mbar_arrive(&bars[B::raw_free + rs]);  // the bytes are in registers: the unit may be refilled
       uint8_t* dst;
       if (!v_part) {
@@ -317,19 +318,23 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
         constexpr int kW0 = decltype(first_word)::value;
 #pragma unroll
         for (int c = 0; c < 16; ++c)
-          *reinterpret_cast<uint4*>(out16 + c * kWChunkStride) = widen8_bf16(make_uint2(w[kW0 + 2 * c], w[kW0 + 2 * c + 1]));
+          *reinterpret_cast<uint4*>(out16 + c * kWChunkStride) = widen8_f16(make_uint2(w[kW0 + 2 * c], w[kW0 + 2 * c + 1]));
         scale_bits = w[kW0 + 32];
       };
       if (wo == 0) widen_piece(std::integral_constant<int, 0>{});
       else if (wo == 1) widen_piece(std::integral_constant<int, 1>{});
       else if (wo == 2) widen_piece(std::integral_constant<int, 2>{});
       else widen_piece(std::integral_constant<int, 3>{});
-      if (upper) {
-        if (!v_part) {
-          reinterpret_cast<float*>(smem + L::ksc)[(j % kWKsRing) * kWKeys + img_row] = __uint_as_float(scale_bits) * p.scale_log2;
-        } else {
-          *reinterpret_cast<uint32_t*>(dst + kWImage + img_row * 4) = scale_bits;
-        }
+      if (!v_part && j == 0) {  // the query scale is known once Q is complete
+        named_barrier(5, kWQBarrier);
+        score_mul = p.scale_log2 * *qinv_s;
+      }
+      if (upper && !v_part) {
+        KeyScales<kWKeys>& ks = key_scales[j % kWKsRing];
+        const float vs = usable_v_scale(v_scale);
+        ks.score[img_row] = __uint_as_float(scale_bits) * score_mul;
+        ks.lv[img_row] = __log2f(vs);
+        ks.iv[img_row] = __fdividef(1.0f, vs);
       }
       tc::fence_async_smem();
       mbar_arrive(&bars[(v_part ? B::vfull + j % kWNS : B::kfull + j % kWNK)]);
@@ -388,7 +393,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     // ONE elected lane issues every tcgen05.mma of the CTA in one fixed order: QK(0), QK(1),
     // then PV(i), QK(i + 2).  QK(i + 2) overwrites the S buffer P(i) was written over: it
     // waits for PV(i) to have finished reading it, a whole tile of softmax after it is issued.
-    named_barrier(5, kWSoftmax + 32);  // wait for Q in TMEM
+    named_barrier(5, kWQBarrier);  // wait for Q in TMEM
     tc::fence_after_sync();
     {
       const RowsDesc kd = rows_desc(kimg_s, kWChunkStride, 128);
@@ -436,18 +441,32 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     const uint32_t s_part = tmem_base + kWSCol + g * kWGroupKeys + lane_addr;   // this group's columns of S buffer 0
     const uint32_t o_part = tmem_base + kWOCol + g * kWGroupDims + lane_addr;   // this group's columns of O
 
-    // ---- Q into TMEM: thread (row, g) stores dims 128 g .. 128 g + 127 of its row, two bf16 per column ----
+    // ---- Q into TMEM: thread (row, g) stores dims 128 g .. 128 g + 127 of its row, two fp16 per column ----
     {
       int token, head;
       row_target(p, t, kvh, row, &token, &head);
       const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
                                                         (int64_t)head * p.q_stride_head) + g * (kWGroupDims / 8);
+      auto load_q = [&](int c) { return row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u); };
+      const bool from_bf16 = p.q_dtype == PTH_ATTN_BF16;
+      float qscale = 1.0f;
+      if (from_bf16) {  // one power of two for all rows of the CTA
+        uint32_t m = 0u;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) m = amax_bits_bf16(load_q(c), m);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) atomicMax(qmax_s, m);
+        named_barrier(4, kWSoftmax);
+        qscale = query_scale(*reinterpret_cast<volatile uint32_t*>(qmax_s));
+      }
+      if (tid == 0) *qinv_s = 1.0f / qscale;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint32_t qw[32];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          const uint4 v = row < rows ? __ldg(src + h * 8 + c) : make_uint4(0u, 0u, 0u, 0u);
+          uint4 v = load_q(h * 8 + c);
+          if (from_bf16) v = queries_to_f16(v, qscale);
           qw[4 * c] = v.x;
           qw[4 * c + 1] = v.y;
           qw[4 * c + 2] = v.z;
@@ -458,7 +477,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       tc::tmem_st_wait();
     }
     tc::fence_before_sync();
-    named_barrier(5, kWSoftmax + 32);  // Q complete; the QK issuer may start
+    named_barrier(5, kWQBarrier);  // Q complete; the QK issuer may start
 
     int rlo = 0, rhi = -1;  // visible keys of this row (none for a padding row)
     if (row < rows) visible_range(p, t, t.first_idx + row / p.group, &rlo, &rhi);
@@ -466,11 +485,10 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     visible_range(p, t, t.first_idx + t.ntok - 1, &mask_lo, &tmp);
     visible_range(p, t, t.first_idx, &tmp, &mask_hi);
     float m_ref = -INFINITY;  // reference maximum of the row's exponentials (log2 units)
-    float l = 0.f;            // sum of exp2(score - m_ref) over this group's keys
+    float l = 0.f;            // sum of exp2(score - m_ref) over this group's keys, without v_scale
 #pragma unroll 1
     for (int i = 0; i < n_tiles; ++i) {
-      const float* ksp = reinterpret_cast<const float*>(smem + L::ksc) + (i % kWKsRing) * kWKeys + g * kWGroupKeys;
-      const float* vsp = reinterpret_cast<const float*>(smem + L::vst + (i % kWNS) * kWVStage + kWImage) + g * kWGroupKeys;
+      const KeyScales<kWKeys>& ks = key_scales[i % kWKsRing];
       const uint32_t s_tmem = s_part + (i & 1) * kWKeys;
       const int pos0 = key_begin + i * kWKeys;
       const bool interior = pos0 >= mask_lo && pos0 + (kWKeys - 1) <= mask_hi;
@@ -480,30 +498,14 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       tc::tmem_ld32(s_tmem, r);
       tc::tmem_ld_wait();
 
-      // ---- pass 1: scores in log2 units (kept in the registers) and their maximum ----
-      float m_t;
-      auto pass1 = [&](auto masked) {
-        constexpr bool kMask = decltype(masked)::value;
-        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int n4 = 0; n4 < kWGroupKeys / 4; ++n4) {
-          const float4 ks4 = reinterpret_cast<const float4*>(ksp)[n4];  // k_scale * scale * log2 e
-          const float kk[4] = {ks4.x, ks4.y, ks4.z, ks4.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int n = n4 * 4 + e;
-            float sc = __uint_as_float(r[n]) * kk[e];
-            if constexpr (kMask) {
-              const int pos = pos0 + tile_key_w(p.raw_mode, g * kWGroupKeys + n);  // key held by this column
-              sc = (pos >= rlo && pos <= rhi) ? sc : -INFINITY;
-            }
-            r[n] = __float_as_uint(sc);
-            mx[e] = fmaxf(mx[e], sc);
-          }
-        }
-        m_t = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      };
-      if (interior) pass1(std::false_type{}); else pass1(std::true_type{});
+      // ---- pass 1: weighted scores in log2 units (kept in the registers) and their maximum ----
+      auto all_ready = [] {};
+      const int k0 = g * kWGroupKeys;
+      float m_t = interior ? softmax_pass1<kWGroupKeys, false>(r, ks.score + k0, ks.lv + k0, all_ready, [](int) { return true; })
+                           : softmax_pass1<kWGroupKeys, true>(r, ks.score + k0, ks.lv + k0, all_ready, [&](int n) {
+                               const int pos = pos0 + tile_key_w(p.raw_mode, k0 + n);  // key held by this column
+                               return pos >= rlo && pos <= rhi;
+                             });
       // ---- the row's maximum over the whole tile: the other group has the other keys ----
       float* tm = tile_max + (i & 1) * 2 * kWGroup + row;
       tm[g * kWGroup] = m_t;
@@ -518,7 +520,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
         // O must be at rest: the PV of the previous tile has completed
         ok &= wait_or_abort(&bars[B::pv_done + ((i - 1) & 1)], ((i - 1) >> 1) & 1, abort_flag);
         tc::fence_after_sync();
-        const float alpha = need ? ex2f_w(m_ref - m_new) : 1.0f;  // 0 when m_ref was -inf
+        const float alpha = need ? ex2f(m_ref - m_new) : 1.0f;  // 0 when m_ref was -inf
 #pragma unroll 1
         for (int j = 0; j < kWGroupDims / 16; ++j) {
           uint32_t o[16];
@@ -534,27 +536,12 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       }
       const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
 
-      // ---- pass 2: p * v_scale as packed bf16 over the first columns of this part of S ----
-      // (a masked score is -inf: its p is exp2(-inf) = 0)
-      ok &= wait_or_abort(&bars[B::vfull + i % kWNS], (i / kWNS) & 1, abort_flag);  // v_scale of tile i
-      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+      // ---- pass 2: P as packed fp16 over the first columns of this part of S ----
+      f32x2 ls[2] = {0ull, 0ull};
       uint32_t pk[16];
-#pragma unroll
-      for (int n4 = 0; n4 < 8; ++n4) {
-        const float4 vs4 = reinterpret_cast<const float4*>(vsp)[n4];
-        const float vv[4] = {vs4.x, vs4.y, vs4.z, vs4.w};
-        float pv[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float pr = ex2f_w(__uint_as_float(r[n4 * 4 + e]) - m_use);
-          ls[e] += pr;
-          pv[e] = pr * vv[e];
-        }
-        pk[n4 * 2] = pack_bf16_w(pv[0], pv[1]);
-        pk[n4 * 2 + 1] = pack_bf16_w(pv[2], pv[3]);
-      }
+      softmax_pass2(r, ks.iv + k0, m_use, ls, pk);
       tc::tmem_st16(s_tmem, pk);
-      l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+      l += sum_pairs(ls);
       tc::tmem_st_wait();
       tc::fence_before_sync();
       mbar_arrive(&bars[B::p_ready + (i & 1)]);  // this group's part of P(i) is complete
@@ -584,18 +571,9 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       const int d0 = g * kWGroupDims + j * 32;
       if (row < rows) {
         if (p.num_splits > 1) {
-#pragma unroll
-          for (int n = 0; n < 32; n += 4)
-            *reinterpret_cast<float4*>(ws_row + d0 + n) = make_float4(o[n], o[n + 1], o[n + 2], o[n + 3]);
-        } else if (p.out_dtype == PTH_ATTN_BF16) {
-#pragma unroll
-          for (int n = 0; n < 32; n += 8)
-            *reinterpret_cast<uint4*>(out_row + (d0 + n) * 2) =
-                make_uint4(pack_bf16_w(o[n], o[n + 1]), pack_bf16_w(o[n + 2], o[n + 3]), pack_bf16_w(o[n + 4], o[n + 5]),
-                           pack_bf16_w(o[n + 6], o[n + 7]));
+          store_out32(reinterpret_cast<uint8_t*>(ws_row + d0), PTH_ATTN_F32, o);
         } else {
-#pragma unroll
-          for (int n = 0; n < 32; ++n) store_out_elem(out_row, d0 + n, p.out_dtype, o[n]);
+          store_out32(out_row + d0 * (p.out_dtype == PTH_ATTN_F32 ? 4 : 2), p.out_dtype, o);
         }
       }
     }

@@ -3,7 +3,7 @@
 // the accumulators and the contraction steps over the head are half as large.)
 //
 // In the one-tile kernel (umma_rows_kernel.cu) every row tile of 128 rows widens the int8 keys
-// and values of its whole context to bf16 for itself, and that widening and the shared-memory
+// and values of its whole context for itself, and that widening and the shared-memory
 // traffic around it - not the tensor core, not the softmax - take most of a tile's time.
 // Here a CTA owns 256 rows (two MMA row tiles) and 64-key tiles:
 //   TMEM       S(rt, b): 64 columns for row tile rt and buffer b = tile % 2 (256 columns), O(rt):
@@ -11,10 +11,8 @@
 //   MMAs       per KV tile two QK (M 128, N 64, eight steps of 16 dims, Q images in shared
 //              memory) on ONE K image and two PV (M 128, N 128, four steps of 16 keys, P from
 //              TMEM) on ONE V stage;
-//   producers  thread (key, half) of the K set / V set widens 64 of the key's 128 dims; the K
-//              set's upper halves carry k_scale to the softmax, the V set multiplies its rows
-//              by v_scale as it widens them (x * v_scale rounded once to bf16), so P is the
-//              bare probability and the softmax spends nothing on v_scale;
+//   producers  thread (key, half) of the K set / V set widens 64 of the key's 128 dims to fp16;
+//              the K set's upper halves carry both scales of the key to the softmax;
 //   softmax    256 threads, one per row: the row's maximum, sum and reference never leave the
 //              thread, and there is nothing to merge at the end.
 // Raw ring: four units of 64 keys x 272 bytes.  Every mbarrier wait is bounded (page_copy.cuh).
@@ -41,8 +39,8 @@ constexpr int kXQStride = 128 * 16 + 16;            // 2,064 B: one column block
 template <int HD>
 struct XG {
   static_assert(HD == 64 || HD == 128, "head size");
-  static constexpr int chunks = HD / 8;                    // 16-byte column blocks of a widened row: 8 bf16 each
-  static constexpr int image = chunks * kXChunkStride;     // 16,640 B: widened K or V of a tile (V rows times v_scale)
+  static constexpr int chunks = HD / 8;                    // 16-byte column blocks of a widened row: 8 fp16 each
+  static constexpr int image = chunks * kXChunkStride;     // 16,640 B: widened K or V of a tile
   static constexpr int qimage = chunks * kXQStride;        // 33,024 B
   static constexpr int raw_row = raw_row_for(HD);          // 272 B
   static constexpr int raw_unit = kXKeys * raw_row;        // 17,408 B: raw cells of a tile
@@ -51,14 +49,15 @@ struct XG {
   static constexpr int load_chunks = piece / 16 + 1;       // 16-byte chunks it reads: the piece, its misalignment, the scale
 };
 constexpr int kXNK = 2, kXNS = 2, kXNR = 4;         // K images, V stages, raw units
-constexpr int kXKsRing = 4;                         // tiles of scaled k_scale vectors kept
+constexpr int kXKsRing = 4;                         // tiles of key scales kept
 constexpr int kXSoftmax = 256;                      // warps 0-3 (row tile 0), 4-7 (row tile 1)
 constexpr int kXProducers = 256;                    // warps 8-11 (K set) and 12-15 (V set)
 constexpr int kXMmaWarp = 16, kXLoadWarp = 17;
 constexpr int kXThreads = 576;
+constexpr int kXQBarrier = kXSoftmax + kXProducers / 2 + 32;  // Q images complete: softmax, K set, MMA issuer
 constexpr int kXProducerRegs = 72, kXSoftmaxRegs = 120;  // of the 96 per thread the CTA starts with
 constexpr int kXOCol = 256;                         // TMEM columns: S(rt, b) at (2 rt + b) 64, O(rt) at 256 + 128 rt
-constexpr float kXRescaleGap = 8.0f;                // log2 units a row maximum may outgrow its reference
+constexpr float kXRescaleGap = 8.0f;                // log2 units a row maximum may outgrow its reference (P stays below 2^8)
 
 template <int HD>
 struct XLayout {
@@ -67,8 +66,8 @@ struct XLayout {
   static constexpr int vst = kimg + kXNK * G::image;
   static constexpr int qimg = vst + kXNS * G::image;                 // [2 row tiles] Q images
   static constexpr int raw = (qimg + 2 * G::qimage + 127) / 128 * 128;
-  static constexpr int ksc = raw + kXNR * G::raw_unit;               // float [kXKsRing][64]: k_scale * scale * log2 e
-  static constexpr int bars = ksc + kXKsRing * kXKeys * 4;           // uint64 [...]
+  static constexpr int ksc = raw + kXNR * G::raw_unit;               // KeyScales<64> [kXKsRing]
+  static constexpr int bars = ksc + kXKsRing * (int)sizeof(KeyScales<kXKeys>);  // uint64 [...]
   static constexpr int n_bars = 2 * kXNS + 2 * kXNK + 12 + 2 * kXNR;
   static constexpr int misc = bars + n_bars * 8;
   static constexpr int total = misc + 32;
@@ -86,31 +85,22 @@ struct XBars {
   static constexpr int raw_free = raw_full + kXNR;     // [NR] producers -> loader
 };
 
-__device__ __forceinline__ uint32_t pack_bf16_x(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-__device__ __forceinline__ float ex2f_x(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // Key of a tile held by row `r` of its images: with contiguous cells the even keys, then the odd ones.
 __device__ __forceinline__ int tile_key_x(int raw_mode, int r) { return raw_mode == 2 ? 2 * (r & 31) + (r >> 5) : r; }
 
 // S = Q K^T for one row tile: HD / 16 steps of 16 dims = two column blocks of either image each.
 template <int HD>
 __device__ __forceinline__ void issue_qk_x(uint32_t s_tmem, RowsDesc q, RowsDesc k) {
-  constexpr uint32_t idesc = tc::instr_desc(128, kXKeys, tc::kFmtBF16, tc::kFmtBF16, 0, 0);
+  constexpr uint32_t idesc = tc::instr_desc(128, kXKeys, tc::kFmtF16, tc::kFmtF16, 0, 0);
   constexpr uint32_t qstep = (2 * kXQStride) >> 4, kstep = (2 * kXChunkStride) >> 4;
   mma_ss_words<false>(s_tmem, q.lo, q.hi, k.lo, k.hi, idesc);
 #pragma unroll
   for (int kk = 1; kk < HD / 16; ++kk) mma_ss_words<true>(s_tmem, q.lo + kk * qstep, q.hi, k.lo + kk * kstep, k.hi, idesc);
 }
-// O += P V for one row tile: P (64 keys, two bf16 per column) in the first 32 columns of its S buffer.
+// O += P V for one row tile: P (64 keys, two fp16 per column) in the first 32 columns of its S buffer.
 template <int HD>
 __device__ __forceinline__ void issue_pv_x(uint32_t o_tmem, uint32_t p_tmem, RowsDesc v, bool accumulate) {
-  constexpr uint32_t idesc = tc::instr_desc(128, HD, tc::kFmtBF16, tc::kFmtBF16, 0, 1);
+  constexpr uint32_t idesc = tc::instr_desc(128, HD, tc::kFmtF16, tc::kFmtF16, 0, 1);
 #pragma unroll
   for (int kk = 0; kk < kXKeys / 16; ++kk) mma_ts_words(o_tmem, p_tmem + kk * 8, v.lo + kk * (256 >> 4), v.hi, idesc, accumulate || kk > 0);
 }
@@ -132,6 +122,9 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::bars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
+  uint32_t* qmax_s = reinterpret_cast<uint32_t*>(smem + L::misc + 24);           // bits of the largest query value
+  volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
+  KeyScales<kXKeys>* key_scales = reinterpret_cast<KeyScales<kXKeys>*>(smem + L::ksc);
 
   const int kvh = blockIdx.y, split = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -252,6 +245,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       tc::mbar_init(&bars[B::raw_free + s], kXProducers);             // every producer thread reads every unit
     }
     *abort_flag = 0;
+    *qmax_s = 0u;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -270,8 +264,8 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kXProducerRegs));
     // Warps 8-11 widen K, warps 12-15 V.  Thread pt of a set owns row pt % 64 of the images and
     // half of its key's dims (the lower or the upper): HD / 2 bytes of the raw cell, which start 0 or 8 (K) or
-    // 4 or 12 (V) bytes after a 16-byte boundary; the threads of the upper halves find the key's
-    // scale right behind their bytes.  Contiguous cells (raw_mode 2) alternate between the two
+    // 4 or 12 (V) bytes after a 16-byte boundary; the K threads of the upper halves find k_scale
+    // right behind their bytes.  Contiguous cells (raw_mode 2) alternate between the two
     // 8-byte alignments: a warp takes the even keys or the odd ones (one widening path per warp),
     // so the images hold a tile's even keys, then its odd ones; the softmax masks by that key.
     const int pt = tid & 127;
@@ -286,6 +280,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     // first byte of this thread's bytes inside a raw unit
     const uint32_t piece = my_page * bs * kXRawRow + my_slot * row_pitch + delta + (v_part ? kXDim + 4 : 0) + upper * G::piece;
     const int wo = (int)((piece & 15u) >> 2);  // first word of the piece in the 16-byte chunks read: 0 / 2 (K), 1 / 3 (V)
+    float score_mul = 0.f;  // softmax_scale * log2 e / query scale
 #pragma unroll 1
     for (int j = 0; j < n_tiles; ++j) {
       const int rs = j % kXNR;
@@ -308,10 +303,9 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
 #pragma unroll
         for (int c = 0; c < 4 * G::load_chunks; ++c) w[c] = 0u;
       }
-      // The V set multiplies its row by the key's v_scale as it widens it (below): the scale word
-      // sits behind the upper half of V, which only half of the threads of a key have read.
-      float v_scale = 0.f;
-      if (v_part && valid)
+      // (the v_scale of the key, for the threads that publish its scales)
+      float v_scale = 1.f;
+      if (!v_part && upper && valid)
         v_scale = *reinterpret_cast<const float*>(smem + L::raw + rs * kXRawUnit + my_page * bs * kXRawRow + my_slot * row_pitch +
                                                   delta + 2 * kXDim + 4);
       mbar_arrive(&bars[B::raw_free + rs]);  // the bytes are in registers: the unit may be refilled
@@ -326,23 +320,11 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       uint8_t* out16 = dst + (upper * G::piece_chunks) * kXChunkStride + img_row * 16;  // this half's column blocks
       uint32_t scale_bits;
       // (one instance per alignment: the words of w must be compile-time indices)
-      // v_scale as the sum of two bf16 (hi + lo carries 16 bits of it): x * lo rounds a term 2^-9
-      // of the product, the fused multiply-add then rounds x * v_scale once
-      const __nv_bfloat16 vs_hi = __float2bfloat16_rn(v_scale);
-      const __nv_bfloat162 hi2 = __bfloat162bfloat162(vs_hi);
-      const __nv_bfloat162 lo2 = __bfloat162bfloat162(__float2bfloat16_rn(v_scale - __bfloat162float(vs_hi)));
-      auto scale2 = [&](uint32_t x) -> uint32_t {
-        const __nv_bfloat162 xv = *reinterpret_cast<const __nv_bfloat162*>(&x);
-        const __nv_bfloat162 y = __hfma2(xv, hi2, __hmul2(xv, lo2));
-        return *reinterpret_cast<const uint32_t*>(&y);
-      };
       auto widen_piece = [&](auto first_word) {
         constexpr int kW0 = decltype(first_word)::value;
 #pragma unroll
         for (int c = 0; c < G::piece_chunks; ++c) {
-          uint4 x = widen8_bf16(make_uint2(w[kW0 + 2 * c], w[kW0 + 2 * c + 1]));
-          if (v_part) x = make_uint4(scale2(x.x), scale2(x.y), scale2(x.z), scale2(x.w));
-          *reinterpret_cast<uint4*>(out16 + c * kXChunkStride) = x;
+          *reinterpret_cast<uint4*>(out16 + c * kXChunkStride) = widen8_f16(make_uint2(w[kW0 + 2 * c], w[kW0 + 2 * c + 1]));
         }
         scale_bits = w[kW0 + G::piece / 4];
       };
@@ -350,8 +332,17 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       else if (wo == 1) widen_piece(std::integral_constant<int, 1>{});
       else if (wo == 2) widen_piece(std::integral_constant<int, 2>{});
       else widen_piece(std::integral_constant<int, 3>{});
-      if (upper && !v_part)
-        reinterpret_cast<float*>(smem + L::ksc)[(j % kXKsRing) * kXKeys + img_row] = __uint_as_float(scale_bits) * p.scale_log2;
+      if (!v_part && j == 0) {  // the query scale is known once the Q images are complete
+        named_barrier(5, kXQBarrier);
+        score_mul = p.scale_log2 * *qinv_s;
+      }
+      if (upper && !v_part) {
+        KeyScales<kXKeys>& ks = key_scales[j % kXKsRing];
+        const float vs = usable_v_scale(v_scale);
+        ks.score[img_row] = __uint_as_float(scale_bits) * score_mul;
+        ks.lv[img_row] = __log2f(vs);
+        ks.iv[img_row] = __fdividef(1.0f, vs);
+      }
       tc::fence_async_smem();
       mbar_arrive(&bars[(v_part ? B::vfull + j % kXNS : B::kfull + j % kXNK)]);
     }
@@ -410,7 +401,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     // tiles 0 and 1, then for every tile i the two PV(i) and the two QK(i + 2).  Row tile rt's
     // QK(i + 2) overwrites the S buffer its P(i) was written over: it waits for its PV(i) to have
     // finished reading it, a whole tile of softmax after it is issued.
-    named_barrier(5, kXSoftmax + 32);  // wait for the Q images
+    named_barrier(5, kXQBarrier);  // wait for the Q images
     // (one instance per number of live row tiles: the loops over them unroll as constants)
     auto issue_all = [&](auto live_row_tiles) {
       constexpr int kRowTiles = decltype(live_row_tiles)::value;
@@ -468,21 +459,34 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     const uint32_t s_rt = tmem_base + 2 * rt * kXKeys + lane_addr;          // S(rt, 0)
     const uint32_t o_tmem = tmem_base + kXOCol + rt * kXDim + lane_addr;    // O(rt)
 
-    // ---- Q image of this row tile: thread copies its row, 16 column blocks of 8 dims ----
+    // ---- Q image of this row tile: thread converts its row, 16 column blocks of 8 dims ----
     {
       int token, head;
       row_target(p, t, kvh, row, &token, &head);
       const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
                                                         (int64_t)head * p.q_stride_head);
       uint8_t* qrow = smem + L::qimg + rt * kXQImage + (tid & 127) * 16;
+      auto load_q = [&](int c) { return row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u); };
+      const bool from_bf16 = p.q_dtype == PTH_ATTN_BF16;
+      float qscale = 1.0f;
+      if (from_bf16) {  // one power of two for all rows of the CTA
+        uint32_t m = 0u;
+#pragma unroll
+        for (int c = 0; c < kXChunks; ++c) m = amax_bits_bf16(load_q(c), m);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) atomicMax(qmax_s, m);
+        named_barrier(6, kXSoftmax);
+        qscale = query_scale(*reinterpret_cast<volatile uint32_t*>(qmax_s));
+      }
+      if (tid == 0) *qinv_s = 1.0f / qscale;
 #pragma unroll
       for (int c = 0; c < kXChunks; ++c) {
-        const uint4 v = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(qrow + c * kXQStride) = v;
+        const uint4 v = load_q(c);
+        *reinterpret_cast<uint4*>(qrow + c * kXQStride) = from_bf16 ? queries_to_f16(v, qscale) : v;
       }
     }
     tc::fence_async_smem();
-    named_barrier(5, kXSoftmax + 32);  // Q images complete; the QK issuer may start
+    named_barrier(5, kXQBarrier);  // Q images complete; the QK issuer may start
 
     int rlo = 0, rhi = -1;  // visible keys of this row (none for a padding row)
     if (row < rows) visible_range(p, t, t.first_idx + row / p.group, &rlo, &rhi);
@@ -490,7 +494,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     visible_range(p, t, t.first_idx + t.ntok - 1, &mask_lo, &tmp);
     visible_range(p, t, t.first_idx, &tmp, &mask_hi);
     float m_ref = -INFINITY;  // reference maximum of the row's exponentials (log2 units)
-    float l = 0.f;            // sum of exp2(score - m_ref)
+    float l = 0.f;            // sum of exp2(score - m_ref), without v_scale
     // A warp whose 32 rows are all padding (the last row tile of a chunk, a short request inside
     // a prefill launch) leaves the issue slots to the others; its rows end as rows without keys
     // (m = -inf, l = 0), which the epilogue never writes.
@@ -510,7 +514,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
 #pragma unroll 1
     for (int i = 0; i < n_tiles; ++i) {
       const int b = i & 1;
-      const float* ksp = reinterpret_cast<const float*>(smem + L::ksc) + (i % kXKsRing) * kXKeys;
+      const KeyScales<kXKeys>& ks = key_scales[i % kXKsRing];
       const uint32_t s_tmem = s_rt + b * kXKeys;
       const int pos0 = key_begin + i * kXKeys;
       const bool interior = pos0 >= mask_lo && pos0 + (kXKeys - 1) <= mask_hi;
@@ -521,31 +525,14 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       tc::tmem_ld_wait();
       tc::tmem_ld32(s_tmem + 32, r + 32);
 
-      // ---- pass 1: scores in log2 units (kept in the registers) and their maximum ----
-      float m_t;
-      auto pass1 = [&](auto masked) {
-        constexpr bool kMask = decltype(masked)::value;
-        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int n4 = 0; n4 < kXKeys / 4; ++n4) {
-          if (n4 == kXKeys / 8) tc::tmem_ld_wait();
-          const float4 ks4 = reinterpret_cast<const float4*>(ksp)[n4];  // k_scale * scale * log2 e
-          const float kk[4] = {ks4.x, ks4.y, ks4.z, ks4.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int n = n4 * 4 + e;
-            float sc = __uint_as_float(r[n]) * kk[e];
-            if constexpr (kMask) {
-              const int pos = pos0 + tile_key_x(p.raw_mode, n);  // key held by this column
-              sc = (pos >= rlo && pos <= rhi) ? sc : -INFINITY;
-            }
-            r[n] = __float_as_uint(sc);
-            mx[e] = fmaxf(mx[e], sc);
-          }
-        }
-        m_t = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      };
-      if (interior) pass1(std::false_type{}); else pass1(std::true_type{});
+      // ---- pass 1: weighted scores in log2 units (kept in the registers) and their maximum ----
+      auto half_ready = [] { tc::tmem_ld_wait(); };
+      const float m_t =
+          interior ? softmax_pass1<kXKeys, false>(r, ks.score, ks.lv, half_ready, [](int) { return true; })
+                   : softmax_pass1<kXKeys, true>(r, ks.score, ks.lv, half_ready, [&](int n) {
+                       const int pos = pos0 + tile_key_x(p.raw_mode, n);  // key held by this column
+                       return pos >= rlo && pos <= rhi;
+                     });
       // ---- move the reference maximum if the row has outgrown it ----
       const float m_new = fmaxf(m_ref, m_t);
       const bool need = m_t > m_ref + kXRescaleGap;  // also true when m_ref is still -inf
@@ -555,7 +542,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
         // O(rt) must be at rest: this row tile's PV of the previous tile has completed
         ok &= wait_or_abort(&bars[B::pv_done + 2 * rt + ((i - 1) & 1)], ((i - 1) >> 1) & 1, abort_flag);
         tc::fence_after_sync();
-        const float alpha = need ? ex2f_x(m_ref - m_new) : 1.0f;  // 0 when m_ref was -inf
+        const float alpha = need ? ex2f(m_ref - m_new) : 1.0f;  // 0 when m_ref was -inf
 #pragma unroll 1
         for (int j = 0; j < kXDim / 16; ++j) {
           uint32_t o[16];
@@ -571,26 +558,15 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       }
       const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
 
-      // ---- pass 2: p as packed bf16 over the first 32 columns of S (the V image carries v_scale) ----
-      // (a masked score is -inf: its p is exp2(-inf) = 0)
-      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+      // ---- pass 2: P as packed fp16 over the first 32 columns of S ----
+      f32x2 ls[2] = {0ull, 0ull};
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         uint32_t pk[16];
-#pragma unroll
-        for (int n4 = 0; n4 < 8; ++n4) {
-          float pv[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            pv[e] = ex2f_x(__uint_as_float(r[j * 32 + n4 * 4 + e]) - m_use);
-            ls[e] += pv[e];
-          }
-          pk[n4 * 2] = pack_bf16_x(pv[0], pv[1]);
-          pk[n4 * 2 + 1] = pack_bf16_x(pv[2], pv[3]);
-        }
+        softmax_pass2(r + j * 32, ks.iv + j * 32, m_use, ls, pk);
         tc::tmem_st16(s_tmem + j * 16, pk);
       }
-      l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+      l += sum_pairs(ls);
       tc::tmem_st_wait();
       tc::fence_before_sync();
       mbar_arrive(&bars[B::p_ready + 2 * rt + b]);  // P(rt, i) is complete
@@ -617,18 +593,9 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       const int d0 = j * 32;
       if (row < rows) {
         if (p.num_splits > 1) {
-#pragma unroll
-          for (int n = 0; n < 32; n += 4)
-            *reinterpret_cast<float4*>(ws_row + d0 + n) = make_float4(o[n], o[n + 1], o[n + 2], o[n + 3]);
-        } else if (p.out_dtype == PTH_ATTN_BF16) {
-#pragma unroll
-          for (int n = 0; n < 32; n += 8)
-            *reinterpret_cast<uint4*>(out_row + (d0 + n) * 2) =
-                make_uint4(pack_bf16_x(o[n], o[n + 1]), pack_bf16_x(o[n + 2], o[n + 3]), pack_bf16_x(o[n + 4], o[n + 5]),
-                           pack_bf16_x(o[n + 6], o[n + 7]));
+          store_out32(reinterpret_cast<uint8_t*>(ws_row + d0), PTH_ATTN_F32, o);
         } else {
-#pragma unroll
-          for (int n = 0; n < 32; ++n) store_out_elem(out_row, d0 + n, p.out_dtype, o[n]);
+          store_out32(out_row + d0 * (p.out_dtype == PTH_ATTN_F32 ? 4 : 2), p.out_dtype, o);
         }
       }
     }

@@ -8,9 +8,8 @@
 //   loader     (1 warp)   TMA page copies of the raw cache cells into a ring of raw half
 //                         stages of 64 keys (same scheme as the integer kernel);
 //   producers  (8 warps)  thread t of the K set / V set widens key t's int8 K / V bytes
-//                         exactly to bf16 into the K image / the V stage (canonical
-//                         no-swizzle layout), with k_scale * softmax_scale * log2 e and
-//                         v_scale of the key;
+//                         exactly to fp16 into the K image / the V stage (canonical
+//                         no-swizzle layout); the K set publishes both scales of the key;
 //   MMA issuer (1 warp, one elected lane) S = Q K^T (M = 128 rows, N = 128 keys, fp32 in
 //                         TMEM, two buffers: tile i uses buffer i % 2, so S(i + 1) is computed
 //                         while the softmax warps work on tile i) and O(g) += P V for each
@@ -18,9 +17,9 @@
 //                         the V stage as an MN-major B operand;
 //   softmax    (2 groups of 4 warps; group g owns keys 64 g .. 64 g + 63 of EVERY tile)
 //                         thread r reads the 64 scores of row r and its half once, pass 1
-//                         turns them into log2 units (score = S * k_scale * softmax_scale *
-//                         log2 e) and finds their maximum, pass 2 writes p * v_scale as
-//                         packed bf16 into TMEM over the columns of S it has read.  The
+//                         turns them into log2 units (S * k_scale * softmax_scale * log2 e +
+//                         log2 v_scale) and finds their maximum, pass 2 writes P as packed
+//                         fp16 into TMEM over the columns of S it has read.  The
 //                         reference maximum of a (row, half) moves only when the running
 //                         maximum outgrows it by 2^8; then the thread rescales its row of
 //                         O(g) in TMEM.  In steady state O is never touched by the softmax.
@@ -48,11 +47,12 @@ constexpr int kRSoftmax = 2 * kRGroup;   // warps 0-3, 4-7
 constexpr int kRProducers = 256;         // warps 8-11 (K half) and 12-15 (V half)
 constexpr int kRMmaWarp = 16, kRLoadWarp = 17;
 constexpr int kRThreads = 576;
-constexpr int kRNS = 2;                  // V stages (V image + v_scale)
+constexpr int kRNS = 2;                  // V stages
 constexpr int kHalfKeys = 64;            // keys of one raw half stage
 constexpr int kRawHalfBytes = kHalfKeys * kRawRow;   // 17,408 B
-constexpr int kRVStage = kWideBytes + kTileKeys * 4;  // V image + v_scale[128]
-constexpr int kRKsRing = 4;                          // tiles of scaled k_scale vectors kept
+constexpr int kRVStage = kWideBytes;                 // V image
+constexpr int kRKsRing = 4;                          // tiles of key scales kept
+constexpr int kRQBarrier = kRSoftmax + kRProducers / 2 + 32;  // Q image complete: softmax, K set, MMA issuer
 // Registers: the CTA starts with 96 per thread (18 warps: five on two of the SM's four schedulers, whose
 // 16,384 registers that fills).  The two producer warpgroups hand 16 per thread to the two softmax
 // warpgroups, which keep the 64 scores of a row and half tile in registers between the two passes;
@@ -66,8 +66,8 @@ struct RLayout {
   static constexpr int vst = kimg + kRNK * kWideBytes;
   static constexpr int qimg = vst + kRNS * kRVStage;
   static constexpr int raw = qimg + kQImageBytes;
-  static constexpr int ksc = raw + kRNR * kRawHalfBytes;       // float [kRKsRing][128]: k_scale * scale * log2 e
-  static constexpr int park_m = ksc + kRKsRing * kTileKeys * 4; // float [128]
+  static constexpr int ksc = raw + kRNR * kRawHalfBytes;       // KeyScales<128> [kRKsRing]
+  static constexpr int park_m = ksc + kRKsRing * (int)sizeof(KeyScales<kTileKeys>); // float [128]
   static constexpr int park_l = park_m + kRGroup * 4;          // float [128]
   static constexpr int bars = park_l + kRGroup * 4;            // uint64 [...]
   static constexpr int n_bars = kRNS * 2 + 2 * kRNK + 6 + 2 * kRNR;
@@ -94,16 +94,6 @@ __device__ __forceinline__ int tile_key_rows(int raw_mode, int r) {
   return raw_mode == 2 ? (r & 64) + 2 * (r & 31) + ((r >> 5) & 1) : r;
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-__device__ __forceinline__ float ex2f(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 template <int kRNK, int kRNR>
 __global__ void __launch_bounds__(kRThreads, 1)
 umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_constant__ CUtensorMap tmap) {
@@ -118,6 +108,9 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::bars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
+  uint32_t* qmax_s = reinterpret_cast<uint32_t*>(smem + L::misc + 24);           // bits of the largest query value
+  volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
+  KeyScales<kTileKeys>* key_scales = reinterpret_cast<KeyScales<kTileKeys>*>(smem + L::ksc);
 
   const int kvh = blockIdx.y, split = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -231,6 +224,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       tc::mbar_init(&bars[B::raw_free + s], kRProducers / 2);             // 64 K-set + 64 V-set threads
     }
     *abort_flag = 0;
+    *qmax_s = 0u;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -247,8 +241,8 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   if (warp >= 8 && warp < kRMmaWarp) {
     // =========================== producers ====================================
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRProducerRegs));
-    // Warps 8-11 widen the K half of the raw cells into the K image, warps 12-15 the V half
-    // (and both scales) into the V stage; thread pt of either set owns key pt of the tile.
+    // Warps 8-11 widen the K half of the raw cells into the K image and publish both scales,
+    // warps 12-15 the V half into the V stage; thread pt of either set owns key pt of the tile.
     const int pt = tid & 127;
     const bool v_part = warp >= 12;
     const int bs = p.copy_slots;  // slots of one page copy
@@ -266,6 +260,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     const int my_page = (key & (kHalfKeys - 1)) >> p.copy_shift, my_slot = key & (bs - 1);
     const uint32_t cell_off = my_page * bs * kRawRow + my_slot * row_pitch + delta;  // inside a half stage
     const bool odd = (cell_off & 8u) != 0;
+    float score_mul = 0.f;  // softmax_scale * log2 e / query scale
 #pragma unroll 1
     for (int j = 0; j < n_tiles; ++j) {
       const int u = 2 * j + half;
@@ -297,23 +292,35 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
 #pragma unroll
         for (int c = 0; c < 36; ++c) w[c] = 0u;
       }
+      float v_scale = 1.f;
+      if (!v_part && valid)
+        v_scale = *reinterpret_cast<const float*>(smem + L::raw + rs * kRawHalfBytes + cell_off + 2 * kHeadDim + 4);
       mbar_arrive(&bars[B::raw_free + rs]);  // the half row is in registers: the stage may be refilled
       const int st = j % kRNS;
       if (!v_part) {
         uint8_t* kdst = smem + L::kimg + (j % kRNK) * kWideBytes + pt * 16;
         if (j >= kRNK) ok &= wait_or_abort(&bars[B::kempty + j % kRNK], ((j / kRNK) - 1) & 1, abort_flag);
-        float* ksc = reinterpret_cast<float*>(smem + L::ksc) + (j % kRKsRing) * kTileKeys;
+        float k_scale;
         if (!odd) {
 #pragma unroll
           for (int c = 0; c < kChunks; ++c)
-            *reinterpret_cast<uint4*>(kdst + c * kChunkStride) = widen8_bf16(make_uint2(w[2 * c], w[2 * c + 1]));
-          ksc[pt] = __uint_as_float(w[32]) * p.scale_log2;
+            *reinterpret_cast<uint4*>(kdst + c * kChunkStride) = widen8_f16(make_uint2(w[2 * c], w[2 * c + 1]));
+          k_scale = __uint_as_float(w[32]);
         } else {
 #pragma unroll
           for (int c = 0; c < kChunks; ++c)
-            *reinterpret_cast<uint4*>(kdst + c * kChunkStride) = widen8_bf16(make_uint2(w[2 + 2 * c], w[3 + 2 * c]));
-          ksc[pt] = __uint_as_float(w[34]) * p.scale_log2;
+            *reinterpret_cast<uint4*>(kdst + c * kChunkStride) = widen8_f16(make_uint2(w[2 + 2 * c], w[3 + 2 * c]));
+          k_scale = __uint_as_float(w[34]);
         }
+        if (j == 0) {  // the query scale is known once the Q image is complete
+          named_barrier(5, kRQBarrier);
+          score_mul = p.scale_log2 * *qinv_s;
+        }
+        KeyScales<kTileKeys>& ks = key_scales[j % kRKsRing];
+        const float vs = usable_v_scale(v_scale);
+        ks.score[pt] = k_scale * score_mul;
+        ks.lv[pt] = __log2f(vs);
+        ks.iv[pt] = __fdividef(1.0f, vs);
         tc::fence_async_smem();
         mbar_arrive(&bars[B::kfull + j % kRNK]);
       } else {
@@ -323,13 +330,11 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
         if (!odd) {
 #pragma unroll
           for (int c = 0; c < kChunks; ++c)
-            *reinterpret_cast<uint4*>(vdst + c * kChunkStride) = widen8_bf16(make_uint2(w[1 + 2 * c], w[2 + 2 * c]));
-          *reinterpret_cast<uint32_t*>(vstage + kWideBytes + pt * 4) = w[33];
+            *reinterpret_cast<uint4*>(vdst + c * kChunkStride) = widen8_f16(make_uint2(w[1 + 2 * c], w[2 + 2 * c]));
         } else {
 #pragma unroll
           for (int c = 0; c < kChunks; ++c)
-            *reinterpret_cast<uint4*>(vdst + c * kChunkStride) = widen8_bf16(make_uint2(w[3 + 2 * c], w[4 + 2 * c]));
-          *reinterpret_cast<uint32_t*>(vstage + kWideBytes + pt * 4) = w[35];
+            *reinterpret_cast<uint4*>(vdst + c * kChunkStride) = widen8_f16(make_uint2(w[3 + 2 * c], w[4 + 2 * c]));
         }
         tc::fence_async_smem();
         mbar_arrive(&bars[B::vfull + st]);
@@ -400,7 +405,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     // produced results that varied from run to run; a version that polled the barriers and
     // issued whatever was ready first was slower.)  Operand descriptors are kept as register
     // word pairs.
-    named_barrier(5, kRSoftmax + 32);  // wait for the Q image
+    named_barrier(5, kRQBarrier);  // wait for the Q image
     {
       const RowsDesc qd = rows_desc(tc::smem_u32(qimg), kChunkStride, 128);
       const RowsDesc kd = rows_desc(kimg_s, kChunkStride, 128);
@@ -451,22 +456,34 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     const uint32_t s_half = tmem_base + g * 64 + lane_addr;         // this group's columns of S buffer 0
     const uint32_t o_tmem = tmem_base + 256 + g * 128 + lane_addr;  // O(g)
 
-    // ---- Q image: thread (row, half) copies 8 of the 16 d-chunks of its row ----
+    // ---- Q image: thread (row, half) converts 8 of the 16 d-chunks of its row ----
     {
       const int half = tid >> 7;
       int token, head;
       row_target(p, t, kvh, row, &token, &head);
       const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
-                                                        (int64_t)head * p.q_stride_head);
+                                                        (int64_t)head * p.q_stride_head) + half * 8;
+      uint4 qv[8];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const int cc = half * 8 + c;
-        const uint4 v = row < rows ? __ldg(src + cc) : make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(qimg + cc * kChunkStride + row * 16) = v;
+      for (int c = 0; c < 8; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
+      float qscale = 1.0f;
+      if (p.q_dtype == PTH_ATTN_BF16) {  // one power of two for all rows of the CTA
+        uint32_t m = 0u;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) m = amax_bits_bf16(qv[c], m);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) atomicMax(qmax_s, m);
+        named_barrier(4, kRSoftmax);
+        qscale = query_scale(*reinterpret_cast<volatile uint32_t*>(qmax_s));
+#pragma unroll
+        for (int c = 0; c < 8; ++c) qv[c] = queries_to_f16(qv[c], qscale);
       }
+      if (tid == 0) *qinv_s = 1.0f / qscale;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(qimg + (half * 8 + c) * kChunkStride + row * 16) = qv[c];
     }
     tc::fence_async_smem();
-    named_barrier(5, kRSoftmax + 32);  // Q image complete; the QK issuer may start
+    named_barrier(5, kRQBarrier);  // Q image complete; the QK issuer may start
 
     int rlo = 0, rhi = -1;  // visible keys of this row (none for a padding row)
     if (row < rows) visible_range(p, t, t.first_idx + row / p.group, &rlo, &rhi);
@@ -474,7 +491,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     visible_range(p, t, t.first_idx + t.ntok - 1, &mask_lo, &tmp);
     visible_range(p, t, t.first_idx, &tmp, &mask_hi);
     float m_ref = -INFINITY;  // reference maximum of the row's exponentials (log2 units)
-    float l = 0.f;            // sum of exp2(score - m_ref)
+    float l = 0.f;            // sum of exp2(score - m_ref), without v_scale
     // A warp whose 32 rows are all padding (a drafter step fills 64 of the 128 rows, a wide
     // verification step 32) leaves the issue slots to the others; its rows end as rows without
     // keys (m = -inf, l = 0), which the epilogue never writes.
@@ -490,8 +507,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     } else {  // warps with live rows (the loop keeps its indentation)
 #pragma unroll 1
     for (int i = 0; i < n_tiles; ++i) {
-      const float* ksp = reinterpret_cast<const float*>(smem + L::ksc) + (i % kRKsRing) * kTileKeys + g * 64;
-      const float* vsp = reinterpret_cast<const float*>(smem + L::vst + (i % kRNS) * kRVStage + kWideBytes) + g * 64;
+      const KeyScales<kTileKeys>& ks = key_scales[i % kRKsRing];
       const uint32_t s_tmem = s_half + (i & 1) * 128;
       const int pos0 = (tile_begin + i) * kTileKeys;
       const bool interior = pos0 >= mask_lo && pos0 + (kTileKeys - 1) <= mask_hi;
@@ -503,31 +519,15 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       tc::tmem_ld32(s_tmem + 32, r + 32);
       tc::tmem_ld_wait();
 
-      // ---- pass 1: scores in log2 units (kept in the registers) and their maximum ----
+      // ---- pass 1: weighted scores in log2 units (kept in the registers) and their maximum ----
       // (two instances: interior tiles, which every live row sees whole, skip the mask)
-      float m_t;
-      auto pass1 = [&](auto masked) {
-        constexpr bool kMask = decltype(masked)::value;
-        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int n4 = 0; n4 < 16; ++n4) {
-          const float4 ks4 = reinterpret_cast<const float4*>(ksp)[n4];  // k_scale * scale * log2 e
-          const float kk[4] = {ks4.x, ks4.y, ks4.z, ks4.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int n = n4 * 4 + e;
-            float sc = __uint_as_float(r[n]) * kk[e];
-            if constexpr (kMask) {
-              const int pos = pos0 + tile_key_rows(p.raw_mode, g * 64 + n);  // key held by column g 64 + n
-              sc = (pos >= rlo && pos <= rhi) ? sc : -INFINITY;
-            }
-            r[n] = __float_as_uint(sc);
-            mx[e] = fmaxf(mx[e], sc);
-          }
-        }
-        m_t = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      };
-      if (interior) pass1(std::false_type{}); else pass1(std::true_type{});
+      auto all_ready = [] {};
+      const float m_t =
+          interior ? softmax_pass1<64, false>(r, ks.score + g * 64, ks.lv + g * 64, all_ready, [](int) { return true; })
+                   : softmax_pass1<64, true>(r, ks.score + g * 64, ks.lv + g * 64, all_ready, [&](int n) {
+                       const int pos = pos0 + tile_key_rows(p.raw_mode, g * 64 + n);  // key held by column g 64 + n
+                       return pos >= rlo && pos <= rhi;
+                     });
       // ---- move the reference maximum if the row has outgrown it ----
       const float m_new = fmaxf(m_ref, m_t);
       const bool need = m_t > m_ref + kRescaleGap;  // also true when m_ref is still -inf
@@ -553,30 +553,15 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       }
       const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
 
-      // ---- pass 2: p * v_scale as packed bf16 over the first columns of this half of S ----
-      // (a masked score is -inf: its p is exp2(-inf) = 0)
-      ok &= wait_or_abort(&bars[B::vfull + i % kRNS], (i / kRNS) & 1, abort_flag);  // v_scale (and V) of tile i
-      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+      // ---- pass 2: P as packed fp16 over the first columns of this half of S ----
+      f32x2 ls[2] = {0ull, 0ull};
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         uint32_t pk[16];
-#pragma unroll
-        for (int n4 = 0; n4 < 8; ++n4) {
-          const float4 vs4 = reinterpret_cast<const float4*>(vsp)[j * 8 + n4];
-          const float vv[4] = {vs4.x, vs4.y, vs4.z, vs4.w};
-          float pv[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float pr = ex2f(__uint_as_float(r[j * 32 + n4 * 4 + e]) - m_use);
-            ls[e] += pr;
-            pv[e] = pr * vv[e];
-          }
-          pk[n4 * 2] = pack_bf16(pv[0], pv[1]);
-          pk[n4 * 2 + 1] = pack_bf16(pv[2], pv[3]);
-        }
+        softmax_pass2(r + j * 32, ks.iv + g * 64 + j * 32, m_use, ls, pk);
         tc::tmem_st16(s_tmem + j * 16, pk);
       }
-      l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+      l += sum_pairs(ls);
       tc::tmem_st_wait();
       tc::fence_before_sync();
       mbar_arrive(&bars[B::p_ready + (i & 1)]);  // this group's half of P(i) is complete
@@ -639,18 +624,9 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
         }
         if (row < rows) {
           if (p.num_splits > 1) {
-#pragma unroll
-            for (int n = 0; n < 32; n += 4)
-              *reinterpret_cast<float4*>(ws_row + j * 32 + n) = make_float4(o[n], o[n + 1], o[n + 2], o[n + 3]);
-          } else if (p.out_dtype == PTH_ATTN_BF16) {
-#pragma unroll
-            for (int n = 0; n < 32; n += 8)
-              *reinterpret_cast<uint4*>(out_row + (j * 32 + n) * 2) =
-                  make_uint4(pack_bf16(o[n], o[n + 1]), pack_bf16(o[n + 2], o[n + 3]), pack_bf16(o[n + 4], o[n + 5]),
-                             pack_bf16(o[n + 6], o[n + 7]));
+            store_out32(reinterpret_cast<uint8_t*>(ws_row + j * 32), PTH_ATTN_F32, o);
           } else {
-#pragma unroll
-            for (int n = 0; n < 32; ++n) store_out_elem(out_row, j * 32 + n, p.out_dtype, o[n]);
+            store_out32(out_row + (j * 32) * (p.out_dtype == PTH_ATTN_F32 ? 4 : 2), p.out_dtype, o);
           }
         }
       }
@@ -677,14 +653,10 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
 }  // namespace
 
 // The row-major kernel reads the cache like the integer kernel (packed cells through TMA
-// page copies) and takes bf16 queries.
+// page copies).
 bool umma_rows_supports(const KernelParams& p, const char** why) {
   if (!umma_i8_supports(p, why)) return false;
   // (this file: 128 dims; 256 dims: umma_rows256_kernel.cu; 64 dims: umma_rows2_kernel.cu)
-  if (p.q_dtype != PTH_ATTN_BF16) {
-    *why = "q is not bf16";  // the Q image is the query bits as they are, and K / V are widened to bf16
-    return false;
-  }
   return true;
 }
 
