@@ -14,13 +14,15 @@
 // Every operand is fp16, whatever the queries are (both operands of an MMA have one format):
 //   K, V   int8 is exact in fp16, and its widening costs 1.25 instructions per value; to bf16,
 //          whose 8 bits hold no biased int8, it takes 2;
-//   Q      fp16 as it is; bf16 times the power of two that puts the largest query value of the
-//          CTA into [2^14, 2^15): exact down to 2^-31 of that value, and the inverse is folded
+//   Q      fp16 as it is; bf16 times the power of two that puts the largest finite query value of
+//          the CTA into [2^14, 2^15): exact down to 2^-31 of that value, and the inverse is folded
 //          into the keys' score factor;
-//   P      exp2(score + log2(v_scale) - reference): the key's v_scale sits in the exponent, so
-//          V needs no multiplication, the 11 bits of P are relative to the largest weighted
-//          probability of the row (fp16's range is that of one row, not of the cache), and the
-//          row sum takes P / v_scale back in fp32.
+//   P      2^7 exp2(score + log2(v_scale) - reference): the key's v_scale sits in the exponent, so
+//          V needs no multiplication and fp16's range is that of one row, not of the cache.  A
+//          weighted score exceeds its reference by at most 8, so P stays at or below 2^15, and
+//          the factor of 2^7 puts what fp16 drops below 2^-32 of the reference: a long context
+//          whose mass sits in many small probabilities beside one large one keeps it.  The row
+//          sum takes P / v_scale back in fp32.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -192,11 +194,13 @@ __device__ __forceinline__ float ex2f(float x) {
 }
 
 // ---- queries ----
-// Largest magnitude of 8 bf16 values, as fp32 bits (which order like the values).
+// Largest finite magnitude of 8 bf16 values, as fp32 bits (which order like the values).  An infinity or
+// a NaN makes its own row what it makes it anywhere; it must not choose the scale of the CTA's other rows.
 __device__ __forceinline__ uint32_t amax_bits_bf16(uint4 v, uint32_t m) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  auto finite = [](uint32_t bits) { return bits < 0x7f800000u ? bits : 0u; };
 #pragma unroll
-  for (int e = 0; e < 4; ++e) m = max(m, max((w[e] << 16) & 0x7fffffffu, w[e] & 0x7fff0000u));
+  for (int e = 0; e < 4; ++e) m = max(m, max(finite((w[e] << 16) & 0x7fffffffu), finite(w[e] & 0x7fff0000u)));
   return m;
 }
 // The power of two that moves a value of these bits into [2^14, 2^15) (1 for zero).
@@ -236,9 +240,11 @@ template <int N>
 struct KeyScales {
   float score[N], lv[N], iv[N];
 };
-// v_scale as the softmax uses it: a scale of zero (or one too small to matter) must not turn
-// into 0 * infinity in the row sum.
-__device__ __forceinline__ float usable_v_scale(float v) { return v >= 7.9e-31f ? v : 7.9e-31f; }
+// log2 of what P is multiplied by (see the head of this file).
+constexpr float kPGain = 7.0f;
+// v_scale as the softmax uses it: a scale of zero (or one below 2^-90, too small to matter) must not
+// turn into 0 * infinity in the row sum, nor the sum of 2^15 / v_scale over a long row into infinity.
+__device__ __forceinline__ float usable_v_scale(float v) { return v < 8.1e-28f ? 8.1e-28f : v; }
 
 // Pass 1 of the softmax over N scores of a row (r: bits of S, replaced by score + log2(v_scale) in log2
 // units); returns their maximum.  visible(n): whether the row sees the key of column n.

@@ -485,7 +485,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     visible_range(p, t, t.first_idx + t.ntok - 1, &mask_lo, &tmp);
     visible_range(p, t, t.first_idx, &tmp, &mask_hi);
     float m_ref = -INFINITY;  // reference maximum of the row's exponentials (log2 units)
-    float l = 0.f;            // sum of exp2(score - m_ref) over this group's keys, without v_scale
+    float l = 0.f;            // 2^kPGain times the sum of exp2(score - m_ref) over this group's keys, without v_scale
 #pragma unroll 1
     for (int i = 0; i < n_tiles; ++i) {
       const KeyScales<kWKeys>& ks = key_scales[i % kWKsRing];
@@ -534,7 +534,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
         l *= alpha;
         if (need) m_ref = m_new;
       }
-      const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+      const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref - kPGain;
 
       // ---- pass 2: P as packed fp16 over the first columns of this part of S ----
       f32x2 ls[2] = {0ull, 0ull};
@@ -578,7 +578,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       }
     }
     if (g == 0 && row < rows) {
-      const float lse2 = lsum > 0.f ? m_ref + log2f(lsum) : -INFINITY;
+      const float lse2 = lsum > 0.f ? m_ref - kPGain + log2f(lsum) : -INFINITY;
       if (p.num_splits > 1) {
         *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
                                   (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = lse2;

@@ -57,7 +57,7 @@ constexpr int kXThreads = 576;
 constexpr int kXQBarrier = kXSoftmax + kXProducers / 2 + 32;  // Q images complete: softmax, K set, MMA issuer
 constexpr int kXProducerRegs = 72, kXSoftmaxRegs = 120;  // of the 96 per thread the CTA starts with
 constexpr int kXOCol = 256;                         // TMEM columns: S(rt, b) at (2 rt + b) 64, O(rt) at 256 + 128 rt
-constexpr float kXRescaleGap = 8.0f;                // log2 units a row maximum may outgrow its reference (P stays below 2^8)
+constexpr float kXRescaleGap = 8.0f;                // log2 units a row maximum may outgrow its reference (P stays at or below 2^15)
 
 template <int HD>
 struct XLayout {
@@ -494,7 +494,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     visible_range(p, t, t.first_idx + t.ntok - 1, &mask_lo, &tmp);
     visible_range(p, t, t.first_idx, &tmp, &mask_hi);
     float m_ref = -INFINITY;  // reference maximum of the row's exponentials (log2 units)
-    float l = 0.f;            // sum of exp2(score - m_ref), without v_scale
+    float l = 0.f;            // 2^kPGain times the sum of exp2(score - m_ref), without v_scale
     // A warp whose 32 rows are all padding (the last row tile of a chunk, a short request inside
     // a prefill launch) leaves the issue slots to the others; its rows end as rows without keys
     // (m = -inf, l = 0), which the epilogue never writes.
@@ -556,7 +556,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
         l *= alpha;
         if (need) m_ref = m_new;
       }
-      const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+      const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref - kPGain;
 
       // ---- pass 2: P as packed fp16 over the first 32 columns of S ----
       f32x2 ls[2] = {0ull, 0ull};
@@ -600,7 +600,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       }
     }
     if (row < rows) {
-      const float lse2 = l > 0.f ? m_ref + log2f(l) : -INFINITY;
+      const float lse2 = l > 0.f ? m_ref - kPGain + log2f(l) : -INFINITY;
       if (p.num_splits > 1) {
         *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
                                   (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = lse2;

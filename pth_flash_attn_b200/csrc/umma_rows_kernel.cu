@@ -491,7 +491,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     visible_range(p, t, t.first_idx + t.ntok - 1, &mask_lo, &tmp);
     visible_range(p, t, t.first_idx, &tmp, &mask_hi);
     float m_ref = -INFINITY;  // reference maximum of the row's exponentials (log2 units)
-    float l = 0.f;            // sum of exp2(score - m_ref), without v_scale
+    float l = 0.f;            // 2^kPGain times the sum of exp2(score - m_ref), without v_scale
     // A warp whose 32 rows are all padding (a drafter step fills 64 of the 128 rows, a wide
     // verification step 32) leaves the issue slots to the others; its rows end as rows without
     // keys (m = -inf, l = 0), which the epilogue never writes.
@@ -551,7 +551,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
         l *= alpha;
         if (need) m_ref = m_new;
       }
-      const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+      const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref - kPGain;
 
       // ---- pass 2: P as packed fp16 over the first columns of this half of S ----
       f32x2 ls[2] = {0ull, 0ull};
@@ -631,7 +631,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
         }
       }
       if (row < rows) {
-        const float lse2 = lsum > 0.f ? m + log2f(lsum) : -INFINITY;
+        const float lse2 = lsum > 0.f ? m - kPGain + log2f(lsum) : -INFINITY;
         if (p.num_splits > 1) {
           *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
                                     (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = lse2;
