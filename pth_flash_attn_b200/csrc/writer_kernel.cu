@@ -9,9 +9,14 @@
 // attention op reads (K bytes, V bytes, K scales, V scales), at the slot slot_mapping names:
 // block = slot / block_size, position = slot % block_size; a negative slot skips the token.
 //
-// One warp per row: lane l owns D / 32 consecutive elements, the row maximum is a warp
-// reduction, and a row's bytes leave as one coalesced store.  The kernel is bound by HBM
-// (it reads 2 T Hkv D source elements and writes T Hkv (2 D + 8) bytes).
+// A cell (token, KV head) belongs to one warp: its first 16 lanes take the K row, the others the V
+// row.  A row is read 64 elements at a time, four per lane, so that a load is 8 bytes of a 16-bit
+// source, the 16 lanes' words leave as one run of 64 bytes whatever the 4-byte alignment of the
+// cell, and the row maximum is a reduction over 16 lanes.  The kernel is bound by HBM (it reads
+// 2 T Hkv D source elements and writes T Hkv (2 D + 8) bytes) as long as enough loads are in flight:
+// a warp issues those of two to four cells before it uses any.
+#include <type_traits>
+
 #include "params.cuh"
 
 namespace pthb200 {
@@ -28,70 +33,107 @@ struct WriterParams {
   int32_t src_dtype, block_size, num_kv_heads, num_tokens;
 };
 
-template <int EPL>  // elements per lane = D / 32
-__device__ __forceinline__ void load_row(const uint8_t* row, int lane, int dtype, float (&x)[EPL]) {
-  if (dtype == PTH_ATTN_F32) {
-    const float* p = reinterpret_cast<const float*>(row) + lane * EPL;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) x[e] = p[e];
-  } else if (dtype == PTH_ATTN_BF16) {
-    const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(row) + lane * EPL;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) x[e] = __bfloat162float(p[e]);
-  } else {
-    const __half* p = reinterpret_cast<const __half*>(row) + lane * EPL;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) x[e] = __half2float(p[e]);
-  }
-}
+constexpr int kRowLanes = 16;
+// Cells a warp has in flight: 2 KB of a 16-bit source up to 128 dims.
+__host__ __device__ constexpr int cells_in_flight(int head_size) { return head_size == 256 ? 2 : 4; }
 
-template <int EPL>
-__global__ void __launch_bounds__(kWriterThreads) kv_writer_kernel(const WriterParams p) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * kWriterThreads + threadIdx.x) >> 5;
-  const int64_t warps = ((int64_t)gridDim.x * kWriterThreads) >> 5;
-  const int64_t rows = 2ll * p.num_tokens * p.num_kv_heads;  // K rows, then V rows
-  for (int64_t r = warp; r < rows; r += warps) {
-    const bool is_v = r >= rows / 2;
-    const int64_t tr = is_v ? r - rows / 2 : r;
-    const int token = (int)(tr / p.num_kv_heads), head = (int)(tr % p.num_kv_heads);
-    const int64_t slot = p.slot_mapping[token];
-    if (slot < 0) continue;  // padding token
-    const int64_t block = slot / p.block_size, pos = slot % p.block_size;
-    const uint8_t* src = is_v ? p.value + token * p.value_stride_token + head * p.value_stride_head
-                              : p.key + token * p.key_stride_token + head * p.key_stride_head;
-    float x[EPL];
-    load_row<EPL>(src, lane, p.src_dtype, x);
-    float amax = 0.f;
+// Four consecutive elements of a source row, as they are in memory.  kVector: 16-bit elements whose rows
+// are 8-byte aligned, two per word; otherwise loaded element by element.
+template <bool kVector>
+struct Four {
+  uint32_t w[kVector ? 2 : 4];
+  __device__ __forceinline__ void load(const uint8_t* row, int e0, int dtype) {
+    if constexpr (kVector) {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(row + e0 * 2));
+      w[0] = v.x;
+      w[1] = v.y;
+    } else if (dtype == PTH_ATTN_F32) {
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) amax = fmaxf(amax, fabsf(x[e]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float scale = fmaxf(__fdiv_rn(amax, 127.0f), 1e-6f);
-    const float inv = __fdiv_rn(1.0f, scale);
-    uint8_t q[EPL];
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-      float v = __fmul_rn(x[e], inv);
-      v = v >= 0.f ? __fadd_rn(v, 0.5f) : __fadd_rn(v, -0.5f);
-      v = fminf(fmaxf(v, -128.0f), 127.0f);
-      q[e] = (uint8_t)(int8_t)(int)truncf(v);
-    }
-    const StreamParams& rows_s = is_v ? p.v : p.k;
-    const StreamParams& scale_s = is_v ? p.vs : p.ks;
-    uint8_t* dst = const_cast<uint8_t*>(rows_s.data) + block * rows_s.stride_block + pos * rows_s.stride_slot +
-                   head * rows_s.stride_head + lane * EPL;
-    if constexpr (EPL == 2) {
-      *reinterpret_cast<uint16_t*>(dst) = (uint16_t)(q[0] | (q[1] << 8));
+      for (int e = 0; e < 4; ++e) w[e] = __ldg(reinterpret_cast<const uint32_t*>(row) + e0 + e);
     } else {
 #pragma unroll
-      for (int w = 0; w < EPL / 4; ++w)
-        reinterpret_cast<uint32_t*>(dst)[w] = (uint32_t)q[4 * w] | ((uint32_t)q[4 * w + 1] << 8) |
-                                              ((uint32_t)q[4 * w + 2] << 16) | ((uint32_t)q[4 * w + 3] << 24);
+      for (int e = 0; e < 4; ++e) w[e] = __ldg(reinterpret_cast<const unsigned short*>(row) + e0 + e);
     }
-    if (lane == 0) {
-      *reinterpret_cast<float*>(const_cast<uint8_t*>(scale_s.data) + block * scale_s.stride_block +
-                                pos * scale_s.stride_slot + head * scale_s.stride_head) = scale;
+  }
+  __device__ __forceinline__ float get(int e, int dtype) const {
+    if (!kVector && dtype == PTH_ATTN_F32) return __uint_as_float(w[e]);
+    const uint32_t bits = kVector ? (e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu) : w[e];
+    return dtype == PTH_ATTN_BF16 ? __uint_as_float(bits << 16) : __half2float(__ushort_as_half((unsigned short)bits));
+  }
+};
+
+template <int D, bool kVector>
+__global__ void __launch_bounds__(kWriterThreads) kv_writer_kernel(const WriterParams p) {
+  constexpr int kCells = cells_in_flight(D);
+  constexpr int kRuns = D / (4 * kRowLanes);  // runs of 64 elements per row
+  const int lane = threadIdx.x & 31, rl = lane & (kRowLanes - 1);
+  const bool is_v = lane >= kRowLanes;
+  const int64_t warp = ((int64_t)blockIdx.x * kWriterThreads + threadIdx.x) >> 5;
+  const int64_t warps = ((int64_t)gridDim.x * kWriterThreads) >> 5;
+  const int64_t cells = (int64_t)p.num_tokens * p.num_kv_heads;
+  const uint8_t* src0 = is_v ? p.value : p.key;
+  const int64_t src_token = is_v ? p.value_stride_token : p.key_stride_token;
+  const int64_t src_head = is_v ? p.value_stride_head : p.key_stride_head;
+  const StreamParams& rows = is_v ? p.v : p.k;
+  const StreamParams& scales = is_v ? p.vs : p.ks;
+  for (int64_t cell0 = warp * kCells; cell0 < cells; cell0 += warps * kCells) {
+    int64_t slot[kCells];
+    int head[kCells];
+    Four<kVector> x[kCells][kRuns];
+#pragma unroll
+    for (int c = 0; c < kCells; ++c) {
+      slot[c] = -1;  // (past the end: treated like a padding token)
+      head[c] = 0;
+      if (cell0 + c < cells) {
+        const int token = cells <= 0x7fffffff ? (int)((uint32_t)(cell0 + c) / (uint32_t)p.num_kv_heads)
+                                              : (int)((cell0 + c) / p.num_kv_heads);
+        head[c] = (int)(cell0 + c - (int64_t)token * p.num_kv_heads);
+        slot[c] = __ldg(p.slot_mapping + token);
+        const uint8_t* row = src0 + token * src_token + head[c] * src_head;
+#pragma unroll
+        for (int r = 0; r < kRuns; ++r) x[c][r].load(row, r * 64 + rl * 4, p.src_dtype);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < kCells; ++c) {
+      if (slot[c] < 0) continue;  // (the same for all lanes)
+      float f[kRuns][4], amax = 0.f;
+#pragma unroll
+      for (int r = 0; r < kRuns; ++r)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          f[r][e] = x[c][r].get(e, p.src_dtype);
+          amax = fmaxf(amax, fabsf(f[r][e]));
+        }
+#pragma unroll
+      for (int o = kRowLanes / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      const float scale = fmaxf(__fdiv_rn(amax, 127.0f), 1e-6f);
+      const float inv = __fdiv_rn(1.0f, scale);
+      int64_t block, pos;
+      if (slot[c] <= 0x7fffffff) {
+        block = (uint32_t)slot[c] / (uint32_t)p.block_size;
+        pos = (uint32_t)slot[c] - (uint32_t)block * (uint32_t)p.block_size;
+      } else {
+        block = slot[c] / p.block_size;
+        pos = slot[c] - block * p.block_size;
+      }
+      uint8_t* dst = const_cast<uint8_t*>(rows.data) + block * rows.stride_block + pos * rows.stride_slot + head[c] * rows.stride_head;
+#pragma unroll
+      for (int r = 0; r < kRuns; ++r) {
+        uint32_t word = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float v = __fmul_rn(f[r][e], inv);
+          v = v >= 0.f ? __fadd_rn(v, 0.5f) : __fadd_rn(v, -0.5f);
+          v = fminf(fmaxf(v, -128.0f), 127.0f);
+          word |= (uint32_t)(uint8_t)(int8_t)(int)truncf(v) << (8 * e);
+        }
+        reinterpret_cast<uint32_t*>(dst)[r * kRowLanes + rl] = word;
+      }
+      if (rl == 0) {
+        *reinterpret_cast<float*>(const_cast<uint8_t*>(scales.data) + block * scales.stride_block +
+                                  pos * scales.stride_slot + head[c] * scales.stride_head) = scale;
+      }
     }
   }
 }
@@ -118,18 +160,27 @@ cudaError_t launch_kv_writer(const PthB200WriteArgs& a, cudaStream_t stream) {
   p.block_size = a.block_size;
   p.num_kv_heads = a.num_kv_heads;
   p.num_tokens = a.num_tokens;
-  const int64_t rows = 2ll * a.num_tokens * a.num_kv_heads;
-  const int64_t want = (rows + kWriterThreads / 32 - 1) / (kWriterThreads / 32);
-  const unsigned grid = (unsigned)(want < 1 ? 1 : (want > 148 * 8 ? 148 * 8 : want));  // a few CTAs per SM, grid-stride
+  const int64_t cells = (int64_t)a.num_tokens * a.num_kv_heads, per_cta = kWriterThreads / 32 * cells_in_flight(a.head_size);
+  const int64_t want = (cells + per_cta - 1) / per_cta;
+  const unsigned grid = (unsigned)(want > (1 << 30) ? (1 << 30) : want);
+  // 8-byte loads need 16-bit rows that start on 8-byte boundaries (D is a multiple of 64)
+  auto on8 = [](const void* ptr, int64_t st, int64_t sh) { return (reinterpret_cast<uintptr_t>(ptr) | (uint64_t)st | (uint64_t)sh) % 8 == 0; };
+  const bool vector = a.src_dtype != PTH_ATTN_F32 && on8(a.key, a.key_stride_token, a.key_stride_head) &&
+                      on8(a.value, a.value_stride_token, a.value_stride_head);
+  auto launch = [&](auto head_size) {
+    constexpr int D = decltype(head_size)::value;
+    if (vector) kv_writer_kernel<D, true><<<grid, kWriterThreads, 0, stream>>>(p);
+    else kv_writer_kernel<D, false><<<grid, kWriterThreads, 0, stream>>>(p);
+  };
   switch (a.head_size) {
     case 64:
-      kv_writer_kernel<2><<<grid, kWriterThreads, 0, stream>>>(p);
+      launch(std::integral_constant<int, 64>{});
       break;
     case 128:
-      kv_writer_kernel<4><<<grid, kWriterThreads, 0, stream>>>(p);
+      launch(std::integral_constant<int, 128>{});
       break;
     default:
-      kv_writer_kernel<8><<<grid, kWriterThreads, 0, stream>>>(p);
+      launch(std::integral_constant<int, 256>{});
       break;
   }
   return cudaGetLastError();
