@@ -193,6 +193,19 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// The loaded registers are written between the load and the wait, but the compiler takes them for written by
+// the load: arithmetic on them that touches no memory it may move above a wait that does not name them.
+// These do (the empty statements stay behind the wait, and what uses the registers behind them).
+template <int N>
+__device__ __forceinline__ void tmem_landed(uint32_t* r) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
+}
+template <int N>
+__device__ __forceinline__ void tmem_ld_wait(uint32_t* r) {
+  tmem_ld_wait();
+  tmem_landed<N>(r);
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 }  // namespace tc

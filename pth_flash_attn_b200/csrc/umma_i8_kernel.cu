@@ -816,6 +816,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
 #pragma unroll
               for (int k = 0; k < PD; ++k) tmem_ld4(o_tmem + h * (PD * NPAD) + k * NPAD + (qb + c) * 4, d[c][k]);
             tc::tmem_ld_wait();
+            tc::tmem_landed<FB * PD * 4>(&d[0][0][0]);
 #pragma unroll
             for (int c = 0; c < FB; ++c) {
 #pragma unroll
@@ -868,6 +869,8 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
             tmem_ld4(s_tmem + NPAD + (qb + c) * 4, lo[c]);
           }
           tc::tmem_ld_wait();
+          tc::tmem_landed<QB * 4>(&hi[0][0]);
+          tc::tmem_landed<QB * 4>(&lo[0][0]);
 #pragma unroll
           for (int c = 0; c < QB; ++c) {
 #pragma unroll

@@ -292,7 +292,7 @@ umma_attention_kernel(const __grid_constant__ KernelParams p) {
 #pragma unroll
     for (int g = 0; g < NPAD / 16; ++g)
       if (g * 16 < rows) tc::tmem_ld16(s_tmem + lane_addr + g * 16, sr + g * 16);
-    tc::tmem_ld_wait();
+    tc::tmem_ld_wait<NPAD>(sr);
     const int pos = tile * kTileKeys + tid;
     const bool interior = tile * kTileKeys >= mask_lo && tile * kTileKeys + (kTileKeys - 1) <= mask_hi;
     const float mult = ks_cur * p.scale_log2;
@@ -345,7 +345,7 @@ umma_attention_kernel(const __grid_constant__ KernelParams p) {
         if (g * 16 < rows) {
           uint32_t o[16];
           tc::tmem_ld16(o_tmem + lane_addr + g * 16, o);
-          tc::tmem_ld_wait();
+          tc::tmem_ld_wait<16>(o);
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             const int n = g * 16 + e;
@@ -395,7 +395,7 @@ umma_attention_kernel(const __grid_constant__ KernelParams p) {
 #pragma unroll
   for (int g = 0; g < NPAD / 16; ++g)
     if (g * 16 < rows) tc::tmem_ld16(o_tmem + lane_addr + g * 16, ot + g * 16);
-  tc::tmem_ld_wait();
+  tc::tmem_ld_wait<NPAD>(ot);
 #pragma unroll
   for (int n = 0; n < NPAD; ++n) {
     if (n < rows) {

@@ -496,7 +496,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       tc::fence_after_sync();
       uint32_t r[kWGroupKeys];  // the scores of this row and part, read once
       tc::tmem_ld32(s_tmem, r);
-      tc::tmem_ld_wait();
+      tc::tmem_ld_wait<kWGroupKeys>(r);
 
       // ---- pass 1: weighted scores in log2 units (kept in the registers) and their maximum ----
       auto all_ready = [] {};
@@ -525,7 +525,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
         for (int j = 0; j < kWGroupDims / 16; ++j) {
           uint32_t o[16];
           tc::tmem_ld16(o_part + j * 16, o);
-          tc::tmem_ld_wait();
+          tc::tmem_ld_wait<16>(o);
 #pragma unroll
           for (int n = 0; n < 16; ++n) o[n] = __float_as_uint(__uint_as_float(o[n]) * alpha);
           tc::tmem_st16(o_part + j * 16, o);
@@ -564,7 +564,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     for (int j = 0; j < kWGroupDims / 32; ++j) {
       uint32_t r[32];
       tc::tmem_ld32(o_part + j * 32, r);
-      tc::tmem_ld_wait();
+      tc::tmem_ld_wait<32>(r);
       float o[32];
 #pragma unroll
       for (int n = 0; n < 32; ++n) o[n] = __uint_as_float(r[n]) * inv;

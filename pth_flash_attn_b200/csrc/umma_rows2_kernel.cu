@@ -522,11 +522,11 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       tc::fence_after_sync();
       uint32_t r[kXKeys];  // the row's scores of this tile, read once: the second half arrives while
       tc::tmem_ld32(s_tmem, r);  // pass 1 works on the first
-      tc::tmem_ld_wait();
+      tc::tmem_ld_wait<32>(r);
       tc::tmem_ld32(s_tmem + 32, r + 32);
 
       // ---- pass 1: weighted scores in log2 units (kept in the registers) and their maximum ----
-      auto half_ready = [] { tc::tmem_ld_wait(); };
+      auto half_ready = [&] { tc::tmem_ld_wait<32>(r + 32); };
       const float m_t =
           interior ? softmax_pass1<kXKeys, false>(r, ks.score, ks.lv, half_ready, [](int) { return true; })
                    : softmax_pass1<kXKeys, true>(r, ks.score, ks.lv, half_ready, [&](int n) {
@@ -547,7 +547,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
         for (int j = 0; j < kXDim / 16; ++j) {
           uint32_t o[16];
           tc::tmem_ld16(o_tmem + j * 16, o);
-          tc::tmem_ld_wait();
+          tc::tmem_ld_wait<16>(o);
 #pragma unroll
           for (int n = 0; n < 16; ++n) o[n] = __float_as_uint(__uint_as_float(o[n]) * alpha);
           tc::tmem_st16(o_tmem + j * 16, o);
@@ -586,7 +586,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     for (int j = 0; j < kXDim / 32; ++j) {
       uint32_t r[32];
       tc::tmem_ld32(o_tmem + j * 32, r);
-      tc::tmem_ld_wait();
+      tc::tmem_ld_wait<32>(r);
       float o[32];
 #pragma unroll
       for (int n = 0; n < 32; ++n) o[n] = __uint_as_float(r[n]) * inv;

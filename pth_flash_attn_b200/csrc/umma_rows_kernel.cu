@@ -517,7 +517,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       uint32_t r[64];
       tc::tmem_ld32(s_tmem, r);
       tc::tmem_ld32(s_tmem + 32, r + 32);
-      tc::tmem_ld_wait();
+      tc::tmem_ld_wait<64>(r);
 
       // ---- pass 1: weighted scores in log2 units (kept in the registers) and their maximum ----
       // (two instances: interior tiles, which every live row sees whole, skip the mask)
@@ -542,7 +542,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
         for (int j = 0; j < 8; ++j) {
           uint32_t o[16];
           tc::tmem_ld16(o_tmem + j * 16, o);
-          tc::tmem_ld_wait();
+          tc::tmem_ld_wait<16>(o);
 #pragma unroll
           for (int n = 0; n < 16; ++n) o[n] = __float_as_uint(__uint_as_float(o[n]) * alpha);
           tc::tmem_st16(o_tmem + j * 16, o);
@@ -593,7 +593,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       for (int j = 0; j < 4; ++j) {
         uint32_t r[32];
         tc::tmem_ld32(o_tmem + j * 32, r);
-        tc::tmem_ld_wait();
+        tc::tmem_ld_wait<32>(r);
 #pragma unroll
         for (int n = 0; n < 32; ++n) park[(j * 32 + n) * kRGroup + row] = __uint_as_float(r[n]);
       }
@@ -615,7 +615,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       for (int j = 0; j < 4; ++j) {
         uint32_t r[32];
         tc::tmem_ld32(o_tmem + j * 32, r);
-        tc::tmem_ld_wait();
+        tc::tmem_ld_wait<32>(r);
         float o[32];
 #pragma unroll
         for (int n = 0; n < 32; ++n) {
