@@ -42,13 +42,6 @@ struct I8Geom {
   static constexpr int halves = HD > 128 ? 2 : 1;              // O^T accumulators of 128 dims (MMA M = 128)
 };
 
-// Order-preserving map float -> int, so an integer warp reduction finds a float maximum.
-__device__ __forceinline__ int float_key(float f) {
-  const int i = __float_as_int(f);
-  return i ^ ((i >> 31) & 0x7fffffff);
-}
-__device__ __forceinline__ float key_float(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
-
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

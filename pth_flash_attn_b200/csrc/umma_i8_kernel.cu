@@ -51,6 +51,12 @@
 //              accumulator (acc = acc * alpha + O^T * u), so TMEM never holds a value
 //              that needs rescaling.  Per-row factors live in lanes and travel by
 //              shuffle.  The two groups' states are merged at the end of every item.
+// What bounds it: HBM at four rows of 128 dims (5.4 TB/s), with more rows or fewer dims the softmax
+// warps' instructions.  At 16 rows they were 75 per row and thread, 5,450 warp instructions per
+// tile; row factors, masks and maxima fetched and stored four rows at a time, the maximum by
+// redux.f32, the two integer accumulators joined before their conversion and the digits cut out of
+// two rows at once brought verification of 4 tokens (32 requests x 16 to 32 K keys) from 495 to
+// 406 us, decode at 64 dims from 199 to 193, at 256 dims from 151 to 146.
 // Every mbarrier wait is bounded: a wait that gives up raises a CTA-wide abort
 // flag (all later waits return at once), sets bit 2 of the status word, and the
 // CTA still finishes and frees its TMEM.
@@ -87,7 +93,7 @@ struct ItemDesc {
   int32_t pad;
 };
 
-template <int HD, int NPAD, int PD, int NS, int NK, int NR, int SB>
+template <int HD, int NPAD, int PD, int NS, int NK, int NR, int SB, int RQ>
 struct Layout {
   using G = I8Geom<HD>;
   static constexpr int img_bytes = G::img_bytes;
@@ -104,12 +110,16 @@ struct Layout {
   static constexpr int unit_keys = kKeys / raw_units;
   static constexpr int unit_bytes = unit_keys * G::raw_row;
   static constexpr int raw = (pimg + pimg_bytes + 127) / 128 * 128; // [NR] raw units (TMA destinations: 128-byte aligned)
-  static constexpr int wred = raw + NR * unit_bytes;                // float [2 groups][2][4][NPAD + 1]
-  static constexpr int mrun = wred + 2 * 2 * 4 * (NPAD + 1) * 4;    // float [2 groups][2 NPAD], first NPAD used
+  static constexpr int wred_row = NPAD + 4;                         // a warp's maxima (or sums) of the rows, then of v_scale
+  static constexpr int wred = raw + NR * unit_bytes;                // float [2 groups][2][4][wred_row]
+  static constexpr int mrun = wred + 2 * 2 * 4 * wred_row * 4;      // float [2 groups][2 NPAD], first NPAD used
   static constexpr int sq = mrun + 2 * 2 * NPAD * 4;                // float [slots][NPAD]
   static constexpr int rlo = sq + kItemSlots * NPAD * 4;            // int [slots][NPAD]
   static constexpr int rhi = rlo + kItemSlots * NPAD * 4;           // int [slots][NPAD]
-  static constexpr int desc = (rhi + kItemSlots * NPAD * 4 + 15) / 16 * 16;  // ItemDesc [slots]
+  // row factors of the latest tile, for the warps to fetch four rows at a time: float [8 warps][4][rows]
+  static constexpr int factor_rows = NPAD <= 32 ? 4 * RQ : 0;
+  static constexpr int factors = rhi + kItemSlots * NPAD * 4;
+  static constexpr int desc = (factors + 8 * 4 * factor_rows * 4 + 15) / 16 * 16;  // ItemDesc [slots]
   static constexpr int bars = desc + kItemSlots * (int)sizeof(ItemDesc);
   static constexpr int n_bars = 2 * NS + 14 + 2 * NR + 2 * kItemSlots;
   static constexpr int misc = bars + n_bars * 8;                    // abort flag, TMEM slot, total work
@@ -149,6 +159,26 @@ __device__ __forceinline__ int tile_key(const KernelParams& p, int r) {
   return p.raw_mode == 2 ? 2 * (r & 63) + (r >> 6) : r;
 }
 
+// Maximum over a converged warp.
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+// Digits of four rows' fixed-point values, each the low 21 bits of a word: byte e of dig[k] gets bits
+// 7 k .. 7 k + 6 of x[e].  Two rows share the halves of a word, so a digit of a row costs 7 / 6 instructions.
+template <int PD>
+__device__ __forceinline__ void digits_of_four(const uint32_t (&x)[4], uint32_t (&dig)[PD]) {
+  static_assert(PD == 2 || PD == 3, "digits");
+  const uint32_t w01 = __byte_perm(x[0], x[1], 0x5410), w23 = __byte_perm(x[2], x[3], 0x5410);  // bits 0 .. 15
+  dig[0] = __byte_perm(w01, w23, 0x6420) & 0x7f7f7f7fu;
+  dig[1] = __byte_perm(w01 >> 7, w23 >> 7, 0x6420) & 0x7f7f7f7fu;
+  if constexpr (PD == 3) {
+    const uint32_t u01 = __byte_perm(x[0], x[1], 0x6521), u23 = __byte_perm(x[2], x[3], 0x6521);  // bits 8 .. 23
+    dig[2] = __byte_perm(u01 >> 6, u23 >> 6, 0x6420) & 0x7f7f7f7fu;
+  }
+}
+
 // Barrier over `count` threads that also ORs a predicate over them (uniform result).
 __device__ __forceinline__ bool named_barrier_or(int id, int count, bool pred) {
   uint32_t r;
@@ -168,16 +198,19 @@ __device__ __forceinline__ bool named_barrier_or(int id, int count, bool pred) {
 template <int HD, int NPAD, int PD, int NS, int NK, int NR, int SB, int RQ, int NP>
 __global__ void __launch_bounds__(threads_for(NP), 1)
 umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_constant__ CUtensorMap tmap) {
-  using L = Layout<HD, NPAD, PD, NS, NK, NR, SB>;
+  using L = Layout<HD, NPAD, PD, NS, NK, NR, SB, RQ>;
   using B = Bars<NS, NR>;
   using G = I8Geom<HD>;
+  constexpr int WP = L::wred_row;
   constexpr int kRawRowHD = G::raw_row, kRawStageHD = L::unit_bytes, kImgHD = G::img_bytes;
   constexpr int RU = L::raw_units, kUnitKeys = L::unit_keys;  // raw units per tile, keys per unit
   // QK runs LA tiles ahead of PV: two when there is a V stage for it, else one
   constexpr int LA = NS >= 3 ? 2 : 1;
   constexpr int kVStageHD = L::vstage_bytes, kHalves = G::halves;
   constexpr int kRawStages = NR;
-  constexpr int XMAX = (1 << (7 * PD)) - 1;
+  // Largest value of P's digits.  A product that reaches it in exact arithmetic may come out 2^-21 of itself
+  // above (exp2, the division, two roundings) and still has to fit 7 PD bits: nothing clamps it.
+  constexpr float kTop = PD == 3 ? (float)((1 << 21) - 3) : (float)((1 << 14) - 1) - 0.25f;
   constexpr int kThreads = threads_for(NP);
   constexpr int kMmaWarp = 8 + 4 * NP;     // lane 0 issues every MMA
   constexpr int kLoadWarp = kMmaWarp + 1;  // issues the page copies
@@ -759,7 +792,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     const int gw = warp & 3;           // warp inside the group = TMEM lane quadrant
     const uint32_t lane_addr = (uint32_t)(gw * 32) << 16;
     uint8_t* pimg_g = pimg + g * (PD * NPAD * kKeys);
-    float* wred_g = wred + g * (2 * 4 * (NPAD + 1));   // [2][4][NPAD + 1]
+    float* wred_g = wred + g * (2 * 4 * WP);   // [2][4][NPAD + 1]
     float* mrun_g = mrun + g * (2 * NPAD);             // [2][NPAD]
     constexpr int NROW = 4 * RQ;  // rows this instance computes (live rows rounded up to four)
     constexpr int RL = (NPAD + 31) / 32;
@@ -786,9 +819,10 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         for (int h = 0; h < kHalves; ++h) acc[h][n] = 0.f;
         l_part[n] = 0.f;
       }
-      // Per-row softmax state lives in LANES, not in shared memory: lane l of every warp holds,
-      // for row l + 32 j, the running maximum and the factors of the latest tile (every warp
-      // computes the same values), and the row loops fetch them with warp shuffles.
+      // Per-row softmax state lives in LANES: lane l of every warp holds, for row l + 32 j, the
+      // running maximum and the factors of the latest tile (every warp computes the same
+      // values).  The row loops fetch the factors four rows at a time, from the warp's own copy in
+      // shared memory, or with warp shuffles where there is no room for one.
       float m_run[RL], a_l[RL], unit_l[RL], muse_l[RL], invu_l[RL];
 #pragma unroll
       for (int j = 0; j < RL; ++j) {
@@ -798,6 +832,16 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         muse_l[j] = 0.f;
         invu_l[j] = 0.f;
       }
+
+      float* my_factors = reinterpret_cast<float*>(smem + L::factors) + warp * (4 * L::factor_rows);
+      auto factor4 = [&](int which, const float (&in_lanes)[RL], int n) -> float4 {  // rows n .. n + 3
+        if constexpr (L::factor_rows > 0) return *reinterpret_cast<const float4*>(my_factors + which * L::factor_rows + n);
+        else
+          return make_float4(__shfl_sync(0xffffffffu, in_lanes[n >> 5], n & 31), __shfl_sync(0xffffffffu, in_lanes[n >> 5], (n + 1) & 31),
+                             __shfl_sync(0xffffffffu, in_lanes[n >> 5], (n + 2) & 31),
+                             __shfl_sync(0xffffffffu, in_lanes[n >> 5], (n + 3) & 31));
+      };
+      constexpr int kAlpha = 0, kUnit = 1, kMax = 2, kInvUnit = 3;
 
       // Folds O^T of the tile with running count q (this group's TMEM buffer) into the register
       // accumulator, with the rescale factor and digit unit of that tile (still in a_l / unit_l).
@@ -819,15 +863,15 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
             tc::tmem_landed<FB * PD * 4>(&d[0][0][0]);
 #pragma unroll
             for (int c = 0; c < FB; ++c) {
+              const int n0 = (qb + c) * 4;
+              const float4 alpha4 = factor4(kAlpha, a_l, n0), unit4 = factor4(kUnit, unit_l, n0);
+              const float alpha[4] = {alpha4.x, alpha4.y, alpha4.z, alpha4.w}, unit[4] = {unit4.x, unit4.y, unit4.z, unit4.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const int n = (qb + c) * 4 + e;
-                const float alpha_n = __shfl_sync(0xffffffffu, a_l[n >> 5], n & 31);
-                const float unit_n = __shfl_sync(0xffffffffu, unit_l[n >> 5], n & 31);
-                float o = int_to_float(d[c][PD - 1][e]);
-#pragma unroll
-                for (int k = PD - 2; k >= 0; --k) o = fmaf(o, 128.f, int_to_float(d[c][k][e]));
-                acc[h][n] = fmaf(acc[h][n], alpha_n, o * unit_n);
+                // (the upper two digits together stay below 2^29)
+                float o = __int2float_rn((int)d[c][PD - 1][e] * 128 + (int)d[c][PD - 2][e]);
+                if constexpr (PD == 3) o = fmaf(o, 128.f, int_to_float(d[c][0][e]));
+                acc[h][n0 + e] = fmaf(acc[h][n0 + e], alpha[e], o * unit[e]);
               }
             }
           }
@@ -843,7 +887,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         const int q = g0 + j;     // running tile count
         const int it = q >> 1;    // running count of this group's tiles; buffers alternate with it
         const int b = it & 1;
-        float* wred_i = wred_g + b * 4 * (NPAD + 1);
+        float* wred_i = wred_g + b * 4 * WP;
         const uint8_t* scales = smem + L::vstages + (q % NS) * kVStageHD + kImgHD;
         const int sb = it % SB;
         ok &= wait_or_abort(&bars[B::s_ready + 2 * g + sb], (it / SB) & 1, abort_flag);
@@ -855,9 +899,6 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         const bool interior = (tile_begin + j) * kKeys >= mask_lo && (tile_begin + j) * kKeys + (kKeys - 1) <= mask_hi;
         const float mult = ks_cur * p.scale_log2;
         float s[NROW];
-        int mykey[RL];  // warp maximum of row lane + 32 j, as an ordered integer key
-#pragma unroll
-        for (int jj = 0; jj < RL; ++jj) mykey[jj] = float_key(-INFINITY);
         // up to sixteen rows per round trip to TMEM (one wait for the batch)
         constexpr int QB = RQ < 4 ? RQ : 4;
 #pragma unroll
@@ -873,47 +914,58 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
           tc::tmem_landed<QB * 4>(&lo[0][0]);
 #pragma unroll
           for (int c = 0; c < QB; ++c) {
+            const int n0 = (qb + c) * 4;
+            const float4 sq4 = *reinterpret_cast<const float4*>(sq + n0);
+            const float sqv[4] = {sq4.x, sq4.y, sq4.z, sq4.w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int n = (qb + c) * 4 + e;
-              const float sv = fmaf(int_to_float(hi[c][e]), 256.f, int_to_float(lo[c][e])) * (sq[n] * mult);
-              const bool vis = interior || (pos >= rlo[n] && pos <= rhi[n]);
-              s[n] = vis ? sv : -INFINITY;
-              const int key = __reduce_max_sync(0xffffffffu, float_key(s[n]));
-              if (lane == (n & 31)) mykey[n >> 5] = key;
+            for (int e = 0; e < 4; ++e)  // (256 hi + lo stays below 2^30)
+              s[n0 + e] = __int2float_rn((int)hi[c][e] * 256 + (int)lo[c][e]) * (sqv[e] * mult);
+            if (!interior) {
+              const int4 lo4 = *reinterpret_cast<const int4*>(rlo + n0), hi4 = *reinterpret_cast<const int4*>(rhi + n0);
+              const int first[4] = {lo4.x, lo4.y, lo4.z, lo4.w}, last[4] = {hi4.x, hi4.y, hi4.z, hi4.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) s[n0 + e] = pos >= first[e] && pos <= last[e] ? s[n0 + e] : -INFINITY;
             }
+            const float4 mx = make_float4(warp_max(s[n0]), warp_max(s[n0 + 1]), warp_max(s[n0 + 2]), warp_max(s[n0 + 3]));
+            if (lane == 0) *reinterpret_cast<float4*>(wred_i + gw * WP + n0) = mx;
           }
         }
-#pragma unroll
-        for (int jj = 0; jj < RL; ++jj)
-          if (lane + 32 * jj < NPAD) wred_i[gw * (NPAD + 1) + lane + 32 * jj] = key_float(mykey[jj]);
         tc::fence_before_sync();
         mbar_arrive(&bars[B::s_free + 2 * g + sb]);  // this S^T buffer may be overwritten by a later QK
         {
-          const int key = __reduce_max_sync(0xffffffffu, float_key(vs_cur));
-          if (lane == 0) wred_i[gw * (NPAD + 1) + NPAD] = key_float(key);
+          const float mx = warp_max(vs_cur);
+          if (lane == 0) wred_i[gw * WP + NPAD] = mx;
         }
         // O^T of this group's previous tile of the item; afterwards its P image is free.
         if (lit > 0) fold_o(q - 2);
         named_barrier(1 + g, kGroupThreads);  // per-warp maxima of the tile visible to the whole group
-        const float vs_max = fmaxf(fmaxf(wred_i[NPAD], wred_i[(NPAD + 1) + NPAD]),
-                                   fmaxf(wred_i[2 * (NPAD + 1) + NPAD], wred_i[3 * (NPAD + 1) + NPAD]));
+        const float vs_max = fmaxf(fmaxf(wred_i[NPAD], wred_i[WP + NPAD]),
+                                   fmaxf(wred_i[2 * WP + NPAD], wred_i[3 * WP + NPAD]));
 #pragma unroll
         for (int jj = 0; jj < RL; ++jj) {
           const int r = (lane + 32 * jj) & (NPAD - 1);
-          const float m_tile = fmaxf(fmaxf(wred_i[r], wred_i[(NPAD + 1) + r]),
-                                     fmaxf(wred_i[2 * (NPAD + 1) + r], wred_i[3 * (NPAD + 1) + r]));
+          const float m_tile = fmaxf(fmaxf(wred_i[r], wred_i[WP + r]),
+                                     fmaxf(wred_i[2 * WP + r], wred_i[3 * WP + r]));
           const float m_old = m_run[jj];
           const float m_new = fmaxf(m_old, m_tile);
           const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
           a_l[jj] = fast_exp2(m_old - m_use);
           // largest p * v_scale of the tile bounds the fixed-point range of its digits
           const float bound = vs_max * fast_exp2(m_tile - m_use);
-          invu_l[jj] = bound > 0.f ? __fdividef((float)XMAX, bound) : 0.f;
-          unit_l[jj] = bound * (1.0f / (float)XMAX);
+          invu_l[jj] = bound > 0.f ? __fdividef(kTop, bound) : 0.f;
+          unit_l[jj] = bound * (1.0f / kTop);
           muse_l[jj] = m_use;
           m_run[jj] = m_new;
+          if constexpr (L::factor_rows > 0) {
+            if (r < L::factor_rows) {
+              my_factors[kAlpha * L::factor_rows + r] = a_l[jj];
+              my_factors[kUnit * L::factor_rows + r] = unit_l[jj];
+              my_factors[kMax * L::factor_rows + r] = m_use;
+              my_factors[kInvUnit * L::factor_rows + r] = invu_l[jj];
+            }
+          }
         }
+        __syncwarp();
 #pragma unroll
         for (int q16 = 0; q16 < NPAD / 16; ++q16) {
           if (q16 * 4 < RQ) {
@@ -924,19 +976,20 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
               // and their columns of O^T are never read): no branch per row, so the four
               // dependency chains overlap.
               if (q16 * 4 + q4 < RQ) {
+                const int n0 = q16 * 16 + q4 * 4;
+                const float4 m4 = factor4(kMax, muse_l, n0), a4 = factor4(kAlpha, a_l, n0), u4 = factor4(kInvUnit, invu_l, n0);
+                const float m_use[4] = {m4.x, m4.y, m4.z, m4.w}, alpha[4] = {a4.x, a4.y, a4.z, a4.w};
+                const float inv_u[4] = {u4.x, u4.y, u4.z, u4.w};
+                uint32_t x[4], dg[PD];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                  const int n = q16 * 16 + q4 * 4 + e;
-                  const float m_use = __shfl_sync(0xffffffffu, muse_l[n >> 5], n & 31);
-                  const float a = __shfl_sync(0xffffffffu, a_l[n >> 5], n & 31);
-                  const float inv_u = __shfl_sync(0xffffffffu, invu_l[n >> 5], n & 31);
-                  const float pr = fast_exp2(s[n] - m_use);
-                  l_part[n] = fmaf(l_part[n], a, pr);
-                  int x = __float2int_rn(pr * vs_cur * inv_u);
-                  x = min(x, XMAX);
-#pragma unroll
-                  for (int k = 0; k < PD; ++k) dig[k][q4] |= (uint32_t)((x >> (7 * k)) & 127) << (8 * e);
+                  const float pr = fast_exp2(s[n0 + e] - m_use[e]);
+                  l_part[n0 + e] = fmaf(l_part[n0 + e], alpha[e], pr);
+                  x[e] = __float_as_uint(fmaf(pr * vs_cur, inv_u[e], 12582912.0f));  // rounded into the low 22 bits
                 }
+                digits_of_four<PD>(x, dg);
+#pragma unroll
+                for (int k = 0; k < PD; ++k) dig[k][q4] = dg[k];
               }
             }
 #pragma unroll
@@ -966,7 +1019,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
           float v = l_part[n];
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == (n & 31)) wsum[gw * (NPAD + 1) + n] = v;
+          if (lane == (n & 31)) wsum[gw * WP + n] = v;
         }
       }
       // The P images hold 128 dims of a parked accumulator ([row][128] fp32): a head of 256 dims
@@ -984,14 +1037,14 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         const int d = h * kKeys + gt;       // output column of this thread in this round
         if (g == 0) {
           const float* w0 = wred;
-          const float* w1 = wred + 2 * 4 * (NPAD + 1);
+          const float* w1 = wred + 2 * 4 * WP;
           const float* m0p = mrun;             // running maxima published by the two groups
           const float* m1p = mrun + 2 * NPAD;
 #pragma unroll
           for (int n = 0; n < NROW; ++n) {
             if (n < rows) {
-              const float l0 = w0[n] + w0[(NPAD + 1) + n] + w0[2 * (NPAD + 1) + n] + w0[3 * (NPAD + 1) + n];
-              const float l1 = w1[n] + w1[(NPAD + 1) + n] + w1[2 * (NPAD + 1) + n] + w1[3 * (NPAD + 1) + n];
+              const float l0 = w0[n] + w0[WP + n] + w0[2 * WP + n] + w0[3 * WP + n];
+              const float l1 = w1[n] + w1[WP + n] + w1[2 * WP + n] + w1[3 * WP + n];
               const float m0 = m0p[n], m1 = m1p[n];
               const float m = fmaxf(m0, m1);
               const float c0 = m0 == -INFINITY ? 0.f : fast_exp2(m0 - m);
@@ -1043,12 +1096,12 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
 
 template <int HD, int NPAD, int PD, int NS, int NK, int NR, int SB, int RQ, int NP>
 cudaError_t launch_cfg(const KernelParams& p, const CUtensorMap& map, int num_ctas, cudaStream_t stream) {
-  constexpr int smem = Layout<HD, NPAD, PD, NS, NK, NR, SB>::total;
+  constexpr int smem = Layout<HD, NPAD, PD, NS, NK, NR, SB, RQ>::total;
   static_assert(smem <= 227 * 1024, "shared memory of one CTA");
-  static_assert(Layout<HD, NPAD, PD, NS, NK, NR, SB>::tmem_need <= 512, "TMEM columns");
+  static_assert(Layout<HD, NPAD, PD, NS, NK, NR, SB, RQ>::tmem_need <= 512, "TMEM columns");
   // a head of 64 dims makes the PV instruction read 64 image "rows" past the V image: they
   // must still be shared memory of this CTA
-  static_assert(HD >= 128 || Layout<HD, NPAD, PD, NS, NK, NR, SB>::vstages + NS * Layout<HD, NPAD, PD, NS, NK, NR, SB>::vstage_bytes +
+  static_assert(HD >= 128 || Layout<HD, NPAD, PD, NS, NK, NR, SB, RQ>::vstages + NS * Layout<HD, NPAD, PD, NS, NK, NR, SB, RQ>::vstage_bytes +
                                      8 * kImgChunk <= smem, "reads past the last V image stay inside the CTA's shared memory");
   static bool configured[64] = {};
   int dev = 0;
