@@ -210,7 +210,8 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   constexpr int kRawStages = NR;
   // Largest value of P's digits.  A product that reaches it in exact arithmetic may come out 2^-21 of itself
   // above (exp2, the division, two roundings) and still has to fit 7 PD bits: nothing clamps it.
-  constexpr float kTop = PD == 3 ? (float)((1 << 21) - 3) : (float)((1 << 14) - 1) - 0.25f;
+  // (A whole number, so that the largest probability of a tile is exact.)
+  constexpr float kTop = PD == 3 ? (float)((1 << 21) - 3) : (float)((1 << 14) - 2);
   constexpr int kThreads = threads_for(NP);
   constexpr int kMmaWarp = 8 + 4 * NP;     // lane 0 issues every MMA
   constexpr int kLoadWarp = kMmaWarp + 1;  // issues the page copies
