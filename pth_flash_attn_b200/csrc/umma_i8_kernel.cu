@@ -26,7 +26,7 @@
 //              without keys, and for every other item publishes a descriptor together
 //              with the item's Q digit image, row scales and row masks (two slots, so the
 //              next item is staged while the current one runs);
-//   loader     (1 warp)  lane `c` issues page copy c of a tile - a [copy_slots slots] x
+//   loaders    (2 warps) lane l of warp w issues page copy c = 2 l + w of a tile - a [copy_slots slots] x
 //              [raw row] box of a tiled tensor map (raw row = the 16-byte aligned bytes
 //              that cover a cell: 144 / 272 / 528 for head sizes 64 / 128 / 256), or a bulk
 //              copy when the cells of a page are contiguous - into a ring of NR raw stages;
@@ -78,8 +78,8 @@ constexpr int kSoftmaxThreads = 2 * kGroupThreads;      // warps 0-3 and 4-7
 constexpr int kProducerThreads = 128;                   // one producer group: one thread per key of a tile
 constexpr int kItemSlots = 2;                           // item descriptors (and Q images) in flight
 // Warps after the softmax groups: NP producer groups of four warps, then the MMA issuer,
-// the loader and the scheduler.
-__host__ __device__ constexpr int threads_for(int np) { return kSoftmaxThreads + np * kProducerThreads + 96; }
+// two loaders and the scheduler.
+__host__ __device__ constexpr int threads_for(int np) { return kSoftmaxThreads + np * kProducerThreads + 128; }
 constexpr int kStageScales = 2 * kKeys * 4;                 // k_scale[128], v_scale[128]
 
 // What the scheduler publishes for one item (shared memory, one per slot).
@@ -214,10 +214,10 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   constexpr float kTop = PD == 3 ? (float)((1 << 21) - 3) : (float)((1 << 14) - 2);
   constexpr int kThreads = threads_for(NP);
   constexpr int kMmaWarp = 8 + 4 * NP;     // lane 0 issues every MMA
-  constexpr int kLoadWarp = kMmaWarp + 1;  // issues the page copies
-  constexpr int kSchedWarp = kMmaWarp + 2; // finds and stages the items
-  // arrivals that free an item slot: every softmax and producer thread, the issuer, the loader
-  constexpr int kItemReaders = kSoftmaxThreads + NP * kProducerThreads + 2;
+  constexpr int kLoadWarp = kMmaWarp + 1;  // this warp and the next issue the page copies
+  constexpr int kSchedWarp = kMmaWarp + 3; // finds and stages the items
+  // arrivals that free an item slot: every softmax and producer thread, the issuer, the loaders
+  constexpr int kItemReaders = kSoftmaxThreads + NP * kProducerThreads + 3;
   static_assert(RQ >= 1 && 4 * RQ <= NPAD, "RQ = groups of four rows the softmax handles (rows <= 4 RQ)");
   // QK(i + LA) is issued before PV(i) (see the issuer) and needs the V stage of tile i + LA
   // filled: with LA + 1 stages or more that is never the one PV(i) has yet to free.
@@ -490,10 +490,10 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
       __syncwarp();
       mbar_arrive(&bars[B::item_full + slot]);
     }
-  } else if (warp == kLoadWarp) {
+  } else if (warp == kLoadWarp || warp == kLoadWarp + 1) {
     // =========================== loader =======================================
     // The raw bytes of a tile arrive PAGE BY PAGE through TMA: one copy per KV page and head,
-    // issued by lane `page` of this warp, completing on the raw stage's mbarrier.
+    // issued by one lane of a loader warp, completing on the raw stage's mbarrier.
     //   raw_mode 1 (slot stride a multiple of 16, e.g. NHD with several heads): a tiled
     //     tensor-map copy of a [block_size slots] x [272 bytes] box whose inner start is the
     //     cell address rounded down to 16 bytes;
@@ -504,6 +504,8 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     // before waiting for the raw stage, so the block-table latency is off the refill path.
     const int pages_per_unit = kUnitKeys >> p.copy_shift;  // page copies of a raw unit (a tile, or half of one)
     const int bs = p.copy_slots;                            // slots of one copy
+    // (copies are issued one lane after another: with eight of 16 slots a tile, one warp took as long as the tile)
+    const int copy = 2 * lane + (warp - kLoadWarp);         // this lane's copy of every unit
     const uint32_t raw_s = tc::smem_u32(smem + L::raw);
     int g0 = 0;  // running tile count at the start of the item
 #pragma unroll 1
@@ -513,7 +515,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
       if (!ok) break;
       const int n_tiles = descs[slot].n_tiles;
       if (n_tiles == 0) break;
-      if (lane < pages_per_unit) {
+      if (copy < pages_per_unit) {
         const int tile_begin = descs[slot].tile_begin, range_begin = descs[slot].range_begin,
                   range_end = descs[slot].range_end;
         const int n_units = n_tiles * RU;
@@ -526,7 +528,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
                                  (reinterpret_cast<uintptr_t>(p.k.data) & ~(uintptr_t)15)) >> 2);
         // block id of this lane's copy of unit v of the item, -1 if no key of the copy is in range
         auto page_block = [&](int v) -> int {
-          const int pos0 = tile_begin * kKeys + v * kUnitKeys + lane * bs;
+          const int pos0 = tile_begin * kKeys + v * kUnitKeys + copy * bs;
           if (v >= n_units || pos0 >= range_end || pos0 + bs <= range_begin) return -1;
           int page, slot;
           page_and_slot(p, pos0, &page, &slot);
@@ -535,7 +537,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         // first slot, inside its page, of this lane's copy of unit v
         auto first_slot = [&](int v) -> int {
           int page, slot;
-          page_and_slot(p, tile_begin * kKeys + v * kUnitKeys + lane * bs, &page, &slot);
+          page_and_slot(p, tile_begin * kKeys + v * kUnitKeys + copy * bs, &page, &slot);
           return slot;
         };
         int blk = page_block(0);
@@ -546,7 +548,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
           if (u >= kRawStages) ok &= wait_or_abort(&bars[B::raw_free + rs], ((u / kRawStages) - 1) & 1, abort_flag);
           uint64_t* bar = &bars[B::raw_full + rs];
           if (blk >= 0 && ok) {
-            const uint32_t dst = raw_s + rs * kRawStageHD + lane * bs * kRawRowHD;
+            const uint32_t dst = raw_s + rs * kRawStageHD + copy * bs * kRawRowHD;
             if (p.raw_mode == 1) {
               mbar_arrive_expect_tx(bar, bs * kRawRowHD);
               tma_load_3d(dst, &tmap, tma_x, first_slot(v), blk, bar);
