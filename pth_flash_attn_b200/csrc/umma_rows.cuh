@@ -246,12 +246,18 @@ constexpr float kPGain = 7.0f;
 // turn into 0 * infinity in the row sum, nor the sum of 2^15 / v_scale over a long row into infinity.
 __device__ __forceinline__ float usable_v_scale(float v) { return v < 8.1e-28f ? 8.1e-28f : v; }
 
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 // Pass 1 of the softmax over N scores of a row (r: bits of S, replaced by score + log2(v_scale) in log2
 // units); returns their maximum.  visible(n): whether the row sees the key of column n.
 template <int N, bool kMask, class Wait, class Visible>
 __device__ __forceinline__ float softmax_pass1(uint32_t (&r)[N], const float* score, const float* lv, Wait half_ready,
                                                Visible visible) {
-  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
   for (int n4 = 0; n4 < N / 4; ++n4) {
     if (n4 == N / 8) half_ready();
@@ -265,10 +271,11 @@ __device__ __forceinline__ float softmax_pass1(uint32_t (&r)[N], const float* sc
     for (int e = 0; e < 4; ++e) {
       if constexpr (kMask) t[e] = visible(4 * n4 + e) ? t[e] : -INFINITY;
       r[4 * n4 + e] = __float_as_uint(t[e]);
-      mx[e] = fmaxf(mx[e], t[e]);
     }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) mx[e] = max3(mx[e], t[2 * e], t[2 * e + 1]);
   }
-  return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+  return fmaxf(mx[0], mx[1]);
 }
 // Pass 2: probabilities of 32 of the scores as packed fp16 (a masked score is -inf: exp2 gives 0); adds
 // p / v_scale to the two pairs of partial row sums.

@@ -53,7 +53,7 @@ constexpr int kWProducers = 256;                    // warps 8-11 (K set) and 12
 constexpr int kWMmaWarp = 16, kWLoadWarp = 17;
 constexpr int kWThreads = 576;
 constexpr int kWQBarrier = kWSoftmax + kWProducers / 2 + 32;  // Q in TMEM: softmax, K set, MMA issuer
-constexpr int kWProducerRegs = 72, kWSoftmaxRegs = 120;  // of the 96 per thread the CTA starts with
+constexpr int kWProducerRegs = 64, kWSoftmaxRegs = 128;  // of the 96 per thread the CTA starts with
 constexpr int kWSCol = 0, kWOCol = 128, kWQCol = 384;    // TMEM columns: S buffers at 0 and 64, O, Q
 constexpr float kWRescaleGap = 8.0f;                // log2 units a row maximum may outgrow its reference
 

@@ -57,7 +57,7 @@ constexpr int kRQBarrier = kRSoftmax + kRProducers / 2 + 32;  // Q image complet
 // 16,384 registers that fills).  The two producer warpgroups hand 16 per thread to the two softmax
 // warpgroups, which keep the 64 scores of a row and half tile in registers between the two passes;
 // every scheduler has two warps of either kind.
-constexpr int kRProducerRegs = 72, kRSoftmaxRegs = 120;
+constexpr int kRProducerRegs = 64, kRSoftmaxRegs = 128;
 constexpr float kRescaleGap = 8.0f;      // log2 units a row maximum may outgrow its reference
 
 template <int kRNK, int kRNR>  // K images, raw HALF stages (64 keys each)
