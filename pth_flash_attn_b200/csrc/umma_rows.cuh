@@ -193,6 +193,17 @@ __device__ __forceinline__ float ex2f(float x) {
   return y;
 }
 
+// KV head and row tile of a CTA: the heads of a row tile side by side, the last row tile of the launch first.
+// CTAs start in index order and one fits an SM, so what starts last decides how long the SMs wait for one
+// another: under a causal mask those are then the first tiles of the first request, its shortest.  (Row tiles
+// in ascending order, head by head: twelve new prompts of 37 to 2,500 tokens ended on the longest tiles of the
+// last of them.)
+__device__ __forceinline__ void rows_cta(const KernelParams& p, int* kvh, int* tile_index) {
+  const uint32_t t = blockIdx.x / (uint32_t)p.num_kv_heads;
+  *kvh = (int)(blockIdx.x - t * (uint32_t)p.num_kv_heads);
+  *tile_index = p.num_q_tiles - 1 - (int)t;
+}
+
 // ---- queries ----
 // Largest finite magnitude of 8 bf16 values, as fp32 bits (which order like the values).  An infinity or
 // a NaN makes its own row what it makes it anywhere; it must not choose the scale of the CTA's other rows.

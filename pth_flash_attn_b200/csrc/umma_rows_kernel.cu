@@ -112,7 +112,9 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
   KeyScales<kTileKeys>* key_scales = reinterpret_cast<KeyScales<kTileKeys>*>(smem + L::ksc);
 
-  const int kvh = blockIdx.y, split = blockIdx.z;
+  int kvh, tile_index;
+  rows_cta(p, &kvh, &tile_index);
+  const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // Row tile of this CTA: bisect a shared-memory copy of query_start_loc when it fits.
   constexpr int kQslCache = 4096;
@@ -126,10 +128,10 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       if (i < p.num_reqs) len_s[i] = __ldg(p.seq_lens + i);
     }
     __syncthreads();
-    t = resolve_row_tile_with(p, blockIdx.x, [&](int i) { return qsl_s[i]; }, [&](int r) { return len_s[r]; });
+    t = resolve_row_tile_with(p, tile_index, [&](int i) { return qsl_s[i]; }, [&](int r) { return len_s[r]; });
     __syncthreads();
   } else {
-    t = resolve_row_tile(p, blockIdx.x);
+    t = resolve_row_tile(p, tile_index);
   }
   if (t.req < 0) return;
   const int rows = t.ntok * p.group;  // <= 128 by construction of bq
@@ -704,7 +706,9 @@ cudaError_t launch_umma_rows_attention(const KernelParams& p_in, cudaStream_t st
   // their K operand from the same shared-memory addresses: with a single K image that the
   // producers rewrote between two QKs, results varied from run to run although every
   // producer / consumer edge was ordered by an mbarrier and a proxy fence.
-  const dim3 grid(p.num_q_tiles, p.num_kv_heads, p.num_splits);
+  const int64_t ctas = (int64_t)p.num_q_tiles * p.num_kv_heads;
+  if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
+  const dim3 grid((unsigned)ctas, p.num_splits);
   return launch_rows<2, 3>(p, map, grid, stream);
 }
 
