@@ -15,8 +15,8 @@
 // cell, and the row maximum is a reduction over 16 lanes.  The kernel is bound by HBM (it reads
 // 2 T Hkv D source elements and writes T Hkv (2 D + 8) bytes) as long as enough loads are in flight:
 // a warp issues those of two to four cells before it uses any.
-// 8,192 tokens of 8 KV heads x 128 dims in bf16 (51 MB): 14 us in a graph, 3.7 TB/s; 20 us a call, of which the
-// caller's side is 13 (one warp per row with 2-byte loads, fourteen rows after another: 43 us a call).
+// 8,192 tokens of 8 KV heads x 128 dims in bf16 (51 MB): 14 us in a graph, 3.7 TB/s; 19 us a call, of which the
+// caller's side is 11 (one warp per row with 2-byte loads, fourteen rows after another: 43 us a call).
 #include <type_traits>
 
 #include "params.cuh"

@@ -10,12 +10,15 @@ synchronise.
 from __future__ import annotations
 
 import ctypes
+import struct
 from dataclasses import dataclass
 
 import torch
 
 from . import capi
 
+_WRITE_ARGS = struct.Struct("@iiPPiqqqq" + "Pqqq" * 4 + "iiiiiP")   # capi.PthB200WriteArgs, in native alignment
+assert _WRITE_ARGS.size == ctypes.sizeof(capi.PthB200WriteArgs)
 _DTYPE_CODE = {torch.float32: capi.F32, torch.float16: capi.F16, torch.bfloat16: capi.BF16}
 
 
@@ -147,20 +150,18 @@ def write_kv(key, value, cache: CacheViews, slot_mapping, *, lib: capi.B200Lib |
     """Quantise ``key`` / ``value`` ``[T, Hkv, D]`` into the cache at ``slot_mapping`` (int64 ``[T]``;
     negative = skip) on the current stream, exactly as the cache format's own writer does."""
     lib = lib or capi.load_library()
-    a = capi.new_write_args()
     es = key.element_size()
-    a.key, a.value, a.src_dtype = key.data_ptr(), value.data_ptr(), _DTYPE_CODE[key.dtype]
-    a.key_stride_token, a.key_stride_head = key.stride(0) * es, key.stride(1) * es
-    a.value_stride_token, a.value_stride_head = value.stride(0) * es, value.stride(1) * es
-    _set_stream(a.k_cache, cache.k)
-    _set_stream(a.v_cache, cache.v)
-    _set_stream(a.k_scale, cache.ks)
-    _set_stream(a.v_scale, cache.vs)
-    a.num_blocks, a.block_size = cache.num_blocks, cache.block_size
-    a.num_kv_heads, a.head_size = cache.num_kv_heads, cache.head_size
-    a.num_tokens = key.shape[0]
-    a.slot_mapping = slot_mapping.data_ptr()
-    with torch.cuda.device(key.device):
-        rc = lib.write_kv(a, stream=torch.cuda.current_stream(key.device).cuda_stream)
+    ks, vs, device = key.stride(), value.stride(), key.device
+    # (packed in one go, in the order of the fields, and the device switched only if it is another: a decode
+    # step's call takes longer here than on the device)
+    a = capi.PthB200WriteArgs.from_buffer_copy(_WRITE_ARGS.pack(
+        capi.ABI_VERSION, _WRITE_ARGS.size, key.data_ptr(), value.data_ptr(), _DTYPE_CODE[key.dtype],
+        ks[0] * es, ks[1] * es, vs[0] * es, vs[1] * es, *cache.k, *cache.v, *cache.ks, *cache.vs,
+        cache.num_blocks, cache.block_size, cache.num_kv_heads, cache.head_size, key.shape[0], slot_mapping.data_ptr()))
+    if device.type == "cuda" and device.index == torch.cuda.current_device():
+        rc = lib.write_kv(a, stream=torch.cuda.current_stream(device).cuda_stream)
+    else:
+        with torch.cuda.device(device):
+            rc = lib.write_kv(a, stream=torch.cuda.current_stream(device).cuda_stream)
     if rc != capi.OK:
         raise RuntimeError(f"pthb200_write_kv: {lib.last_error()} (code {rc})")
