@@ -23,6 +23,9 @@
 //          the factor of 2^7 puts what fp16 drops below 2^-32 of the reference: a long context
 //          whose mass sits in many small probabilities beside one large one keeps it.  The row
 //          sum takes P / v_scale back in fp32.
+// Measured against bf16 operands (same launches, one box): 4 x 2,048 tokens over 30,720 keys 10.05 -> 9.80 ms,
+// at 256 dims 4.43 -> 3.6 ms, a drafter step 126.5 -> 117.9 us; fp16 queries, which bf16 operands could not
+// take, leave the integer kernel's 64-row instance: twelve prompts of 37 to 2,500 tokens 5,754 -> 453 us.
 #pragma once
 
 #include <cuda_fp16.h>
