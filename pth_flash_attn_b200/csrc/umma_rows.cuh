@@ -30,7 +30,6 @@
 
 #include <cuda_fp16.h>
 
-#include "page_copy.cuh"
 #include "params.cuh"
 #include "umma_tile.cuh"
 
@@ -209,46 +208,20 @@ __device__ __forceinline__ void rows_cta(const KernelParams& p, int* kvh, int* t
 }
 
 // ---- queries ----
+// Largest finite magnitude of 8 bf16 values, as fp32 bits (which order like the values).  An infinity or
+// a NaN makes its own row what it makes it anywhere; it must not choose the scale of the CTA's other rows.
+__device__ __forceinline__ uint32_t amax_bits_bf16(uint4 v, uint32_t m) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  auto finite = [](uint32_t bits) { return bits < 0x7f800000u ? bits : 0u; };
+#pragma unroll
+  for (int e = 0; e < 4; ++e) m = max(m, max(finite((w[e] << 16) & 0x7fffffffu), finite(w[e] & 0x7fff0000u)));
+  return m;
+}
 // The power of two that moves a value of these bits into [2^14, 2^15) (1 for zero).
 __device__ __forceinline__ float query_scale(uint32_t amax_bits) {
   if (amax_bits == 0u) return 1.0f;
   const int e = min((int)(amax_bits >> 23) - 127, 127);  // (subnormal: -127)
   return __uint_as_float((uint32_t)(min(14 - e, 126) + 127) << 23);
-}
-// The power of two for the bf16 queries of a CTA, of which this thread holds N x 8: that of the largest finite
-// magnitude among all of them.  An infinity or a NaN makes its own row what it makes it anywhere; it must not
-// choose the scale of the others, so where one turns up the maximum is taken again without them.
-// (Two queries per instruction: with four of its own for each, and the queries loaded again for the
-// conversion, a short prompt's launch, which is mostly set-up, took 2 to 4 us longer.)
-template <int N>
-__device__ __forceinline__ float query_scale_of(const uint4 (&q)[N], uint32_t* any_s, uint32_t* finite_s, int barrier, int threads) {
-  uint32_t m = 0u;
-#pragma unroll
-  for (int c = 0; c < N; ++c) {
-    m = __vimax3_u16x2(m, q[c].x & 0x7fff7fffu, q[c].y & 0x7fff7fffu);
-    m = __vimax3_u16x2(m, q[c].z & 0x7fff7fffu, q[c].w & 0x7fff7fffu);
-  }
-  m = __reduce_max_sync(0xffffffffu, max(m & 0xffffu, m >> 16));
-  if ((threadIdx.x & 31) == 0) atomicMax(any_s, m);
-  named_barrier(barrier, threads);
-  uint32_t top = *reinterpret_cast<volatile uint32_t*>(any_s);
-  if (top >= 0x7f80u) {  // (the same for all of the CTA's softmax threads)
-    m = 0u;
-#pragma unroll
-    for (int c = 0; c < N; ++c) {
-      const uint32_t w[4] = {q[c].x, q[c].y, q[c].z, q[c].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const uint32_t lo = w[e] & 0x7fffu, hi = (w[e] >> 16) & 0x7fffu;
-        m = max(m, max(lo < 0x7f80u ? lo : 0u, hi < 0x7f80u ? hi : 0u));
-      }
-    }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(finite_s, m);
-    named_barrier(barrier, threads);
-    top = *reinterpret_cast<volatile uint32_t*>(finite_s);
-  }
-  return query_scale(top << 16);
 }
 // 8 bf16 queries times a power of two -> fp16.
 __device__ __forceinline__ uint4 queries_to_f16(uint4 v, float scale) {

@@ -118,7 +118,6 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
   uint32_t* qmax_s = reinterpret_cast<uint32_t*>(smem + L::misc + 24);           // bits of the largest query value
-  uint32_t* qfinite_s = reinterpret_cast<uint32_t*>(smem + L::misc + 12);        // of the largest finite one, if they differ
   volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
   KeyScales<kWKeys>* key_scales = reinterpret_cast<KeyScales<kWKeys>*>(smem + L::ksc);
 
@@ -241,7 +240,6 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     }
     *abort_flag = 0;
     *qmax_s = 0u;
-    *qfinite_s = 0u;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -451,14 +449,17 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       row_target(p, t, kvh, row, &token, &head);
       const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
                                                         (int64_t)head * p.q_stride_head) + g * (kWGroupDims / 8);
-      uint4 qv[16];
-#pragma unroll
-      for (int c = 0; c < 16; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
+      auto load_q = [&](int c) { return row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u); };
+      const bool from_bf16 = p.q_dtype == PTH_ATTN_BF16;
       float qscale = 1.0f;
-      if (p.q_dtype == PTH_ATTN_BF16) {  // one power of two for all rows of the CTA
-        qscale = query_scale_of(qv, qmax_s, qfinite_s, 4, kWSoftmax);
+      if (from_bf16) {  // one power of two for all rows of the CTA
+        uint32_t m = 0u;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) qv[c] = queries_to_f16(qv[c], qscale);
+        for (int c = 0; c < 16; ++c) m = amax_bits_bf16(load_q(c), m);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) atomicMax(qmax_s, m);
+        named_barrier(4, kWSoftmax);
+        qscale = query_scale(*reinterpret_cast<volatile uint32_t*>(qmax_s));
       }
       if (tid == 0) *qinv_s = 1.0f / qscale;
 #pragma unroll
@@ -466,7 +467,8 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
         uint32_t qw[32];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          const uint4 v = qv[h * 8 + c];
+          uint4 v = load_q(h * 8 + c);
+          if (from_bf16) v = queries_to_f16(v, qscale);
           qw[4 * c] = v.x;
           qw[4 * c + 1] = v.y;
           qw[4 * c + 2] = v.z;

@@ -129,7 +129,6 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
   uint32_t* qmax_s = reinterpret_cast<uint32_t*>(smem + L::misc + 24);           // bits of the largest query value
-  uint32_t* qfinite_s = reinterpret_cast<uint32_t*>(smem + L::misc + 12);        // of the largest finite one, if they differ
   volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
   KeyScales<kXKeys>* key_scales = reinterpret_cast<KeyScales<kXKeys>*>(smem + L::ksc);
 
@@ -255,7 +254,6 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     }
     *abort_flag = 0;
     *qmax_s = 0u;
-    *qfinite_s = 0u;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -476,18 +474,24 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
                                                         (int64_t)head * p.q_stride_head);
       uint8_t* qrow = smem + L::qimg + rt * kXQImage + (tid & 127) * 16;
-      uint4 qv[kXChunks];
-#pragma unroll
-      for (int c = 0; c < kXChunks; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
+      auto load_q = [&](int c) { return row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u); };
+      const bool from_bf16 = p.q_dtype == PTH_ATTN_BF16;
       float qscale = 1.0f;
-      if (p.q_dtype == PTH_ATTN_BF16) {  // one power of two for all rows of the CTA
-        qscale = query_scale_of(qv, qmax_s, qfinite_s, 6, kXSoftmax);
+      if (from_bf16) {  // one power of two for all rows of the CTA
+        uint32_t m = 0u;
 #pragma unroll
-        for (int c = 0; c < kXChunks; ++c) qv[c] = queries_to_f16(qv[c], qscale);
+        for (int c = 0; c < kXChunks; ++c) m = amax_bits_bf16(load_q(c), m);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) atomicMax(qmax_s, m);
+        named_barrier(6, kXSoftmax);
+        qscale = query_scale(*reinterpret_cast<volatile uint32_t*>(qmax_s));
       }
       if (tid == 0) *qinv_s = 1.0f / qscale;
 #pragma unroll
-      for (int c = 0; c < kXChunks; ++c) *reinterpret_cast<uint4*>(qrow + c * kXQStride) = qv[c];
+      for (int c = 0; c < kXChunks; ++c) {
+        const uint4 v = load_q(c);
+        *reinterpret_cast<uint4*>(qrow + c * kXQStride) = from_bf16 ? queries_to_f16(v, qscale) : v;
+      }
     }
     tc::fence_async_smem();
     named_barrier(5, kXQBarrier);  // Q images complete; the QK issuer may start

@@ -109,7 +109,6 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
   uint32_t* qmax_s = reinterpret_cast<uint32_t*>(smem + L::misc + 24);           // bits of the largest query value
-  uint32_t* qfinite_s = reinterpret_cast<uint32_t*>(smem + L::misc + 12);        // of the largest finite one, if they differ
   volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
   KeyScales<kTileKeys>* key_scales = reinterpret_cast<KeyScales<kTileKeys>*>(smem + L::ksc);
 
@@ -228,7 +227,6 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     }
     *abort_flag = 0;
     *qmax_s = 0u;
-    *qfinite_s = 0u;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -472,7 +470,13 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       for (int c = 0; c < 8; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
       float qscale = 1.0f;
       if (p.q_dtype == PTH_ATTN_BF16) {  // one power of two for all rows of the CTA
-        qscale = query_scale_of(qv, qmax_s, qfinite_s, 4, kRSoftmax);
+        uint32_t m = 0u;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) m = amax_bits_bf16(qv[c], m);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) atomicMax(qmax_s, m);
+        named_barrier(4, kRSoftmax);
+        qscale = query_scale(*reinterpret_cast<volatile uint32_t*>(qmax_s));
 #pragma unroll
         for (int c = 0; c < 8; ++c) qv[c] = queries_to_f16(qv[c], qscale);
       }
