@@ -248,11 +248,16 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   // (the loads of the total-work pass below are issued first: their latency hides behind the
   // barrier initialisation and the TMEM allocation)
   unsigned long long work = 0;
+  bool served = false;
   for (int r = tid; r < p.num_reqs; r += kThreads) {
     const int q0 = __ldg(p.query_start_loc + r), q1 = __ldg(p.query_start_loc + r + 1);
     const int len = __ldg(p.seq_lens + r);
-    work += (unsigned long long)req_row_tiles(shape, q1 - q0) * (unsigned long long)req_kv_tiles(shape, q1 - q0, len);
+    const int row_tiles = req_row_tiles(shape, q1 - q0);
+    work += (unsigned long long)row_tiles * (unsigned long long)req_kv_tiles(shape, q1 - q0, len);
+    served |= row_tiles > 0;
   }
+  // A prefill launch whose requests are all tall has nothing for this kernel: its CTAs leave before any set-up.
+  if (p.row_class == 1 && !__syncthreads_or(served)) return;
   if (tid == 0) {
     for (int s = 0; s < NS; ++s) {
       tc::mbar_init(&bars[B::full + s], kProducerThreads);
