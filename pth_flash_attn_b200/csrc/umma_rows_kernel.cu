@@ -77,12 +77,12 @@ struct RLayout {
 
 template <int kRNK, int kRNR>
 struct RBars {
-  static constexpr int vfull = 0;                      // [NS] V producers -> softmax (pass 2), 128 arrivals
+  static constexpr int vfull = 0;                      // [NS] V producers -> PV, 128 arrivals
   static constexpr int vempty = kRNS;                  // [NS] PV commit -> V producers
   static constexpr int kempty = 2 * kRNS;              // [NK] QK commit -> K producers
   static constexpr int kfull = 2 * kRNS + kRNK;        // [NK] K producers -> QK, 128 arrivals
   static constexpr int s_ready = 2 * kRNS + 2 * kRNK;  // [2] QK commit -> softmax
-  static constexpr int p_ready = s_ready + 2;          // [2] softmax -> PV, 128 arrivals
+  static constexpr int p_ready = s_ready + 2;          // [2] softmax -> PV, 256 arrivals
   static constexpr int pv_done = p_ready + 2;          // [2] PV commit -> QK, softmax
   static constexpr int raw_full = pv_done + 2;         // [NR]
   static constexpr int raw_free = raw_full + kRNR;     // [NR] producers -> loader, 128 arrivals
@@ -430,6 +430,8 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       for (int i = 0; i < n_tiles && ok; ++i) {
         const int sb = i & 1;
         ok &= wait_or_abort(&bars[B::p_ready + sb], (i >> 1) & 1, abort_flag);
+        // (P says nothing about V: the softmax reads the keys' scales, which the K set publishes)
+        ok &= wait_or_abort(&bars[B::vfull + i % kRNS], (i / kRNS) & 1, abort_flag);
         if (ok && elect_one()) {
           tc::fence_after_sync();
           RowsDesc v = vd;

@@ -1,0 +1,44 @@
+"""Barrier edges of the row-major kernels, read off their sources.
+
+A wait that is missing between two roles of a CTA shows on the GPU only when the late role is
+late, and running such a kernel there is a data race.  So the edges are checked in the text: in
+the MMA issuer's part every QK stands behind a wait for its K image, and every PV behind the waits
+for its P and for its V image.
+"""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "pth_flash_attn_b200" / "csrc"
+KERNELS = ["umma_rows_kernel.cu", "umma_rows2_kernel.cu", "umma_rows256_kernel.cu"]
+WAIT = re.compile(r"wait_or_abort\w*\(&bars\[B::(\w+)")
+
+
+def _code(name):
+    text = (CSRC / name).read_text()
+    text = re.sub(r"//[^\n]*", "", text)
+    return text[text.index("__global__"):text.index("cudaError_t launch")]
+
+
+def _issuer(code):
+    """The text of the MMA issuer's role: from its branch to the next one."""
+    start = re.search(r"else if \(warp == k\w*MmaWarp\)", code).start()
+    return code[start:code.index("else if (warp", start + 10)]
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_every_mma_stands_behind_the_waits_for_its_operands(name):
+    issuer = _issuer(_code(name))
+    needs = {"issue_qk": {"kfull"}, "issue_pv": {"p_ready", "vfull"}}
+    seen = set()
+    waited = set()
+    for token in re.finditer(WAIT.pattern + r"|\b(issue_qk|issue_pv)(?:_rows|_halves|_x|_w)\w*(?:<\w+>)?\(", issuer):
+        barrier, issue = token.groups()
+        if barrier:
+            waited.add(barrier)
+            continue
+        seen.add(issue)
+        assert needs[issue] <= waited, f"{name}: {issue} is issued without a wait for {sorted(needs[issue] - waited)}"
+        waited -= needs[issue]
+    assert seen == set(needs)
