@@ -117,6 +117,19 @@ __device__ __forceinline__ bool wait_or_abort_spin_s(uint32_t bar_s, uint32_t pa
   return false;
 }
 
+// What a lane of a loader waits for before it copies into a raw stage again: every reader's arrive on
+// raw_free.  The readers' loads go through the generic proxy and the copy's writes through the async proxy, and an
+// mbarrier alone does not keep the one in front of the other: that takes a proxy fence between the wait and the copy.
+// (Without it, now and then, the v_scale that a row-major kernel reads last before its arrive was the next
+// tile's: in one launch of 500 at 256 dims, of 800 to 50,000 at 64 and 128, on the first tile of a piece, whose stage is
+// refilled while the keys wait for the queries.  A fence of the generic proxy on the readers' side changed nothing;
+// a proxy fence there does as well as here, but in the readers' chain: decode at 256 dims 141.5 -> 145.4 us.)
+__device__ __forceinline__ bool wait_raw_free(uint64_t* raw_free, uint32_t parity, volatile int* abort_flag) {
+  const bool ok = wait_or_abort(raw_free, parity, abort_flag);
+  tc::fence_async_smem();
+  return ok;
+}
+
 // True in exactly one lane of a converged warp (elect.sync): the form in which the compiler
 // knows that a single thread issues what follows.
 __device__ __forceinline__ bool elect_one() {

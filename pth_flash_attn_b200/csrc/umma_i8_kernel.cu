@@ -550,7 +550,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         for (int v = 0; v < n_units; ++v) {
           const int blk_next = page_block(v + 1);
           const int u = g0 * RU + v, rs = u % kRawStages;  // running unit count, ring slot
-          if (u >= kRawStages) ok &= wait_or_abort(&bars[B::raw_free + rs], ((u / kRawStages) - 1) & 1, abort_flag);
+          if (u >= kRawStages) ok &= wait_raw_free(&bars[B::raw_free + rs], ((u / kRawStages) - 1) & 1, abort_flag);
           uint64_t* bar = &bars[B::raw_full + rs];
           if (blk >= 0 && ok) {
             const uint32_t dst = raw_s + rs * kRawStageHD + copy * bs * kRawRowHD;
@@ -649,8 +649,8 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         load_part(row, kw);
         if constexpr (!kTwoPhase) {
           load_part(row + NCH, vw);
-          // this thread's row is in registers (the arrive orders the loads before it): once all
-          // producers of the tile have arrived the loader may refill the raw stage
+          // this thread's row is in registers: once all producers of the tile have arrived the loader
+          // may refill the raw stage
           mbar_arrive(&bars[B::raw_free + rs]);
         }
         const int st = g % NS;

@@ -71,7 +71,7 @@ struct WLayout {
 };
 
 struct WBars {
-  static constexpr int vfull = 0;                      // [NS] V producers -> softmax (pass 2) and PV
+  static constexpr int vfull = 0;                      // [NS] V producers -> PV
   static constexpr int vempty = kWNS;                  // [NS] PV commit -> V producers
   static constexpr int kempty = 2 * kWNS;              // [NK] QK commit -> K producers
   static constexpr int kfull = 2 * kWNS + kWNK;        // [NK] K producers -> QK
@@ -372,7 +372,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       for (int j = 0; j < n_tiles; ++j) {
         const int blk_next = page_block(j + 1);
         const int rs = j % kWNR;
-        if (j >= kWNR) ok &= wait_or_abort(&bars[B::raw_free + rs], ((j / kWNR) - 1) & 1, abort_flag);
+        if (j >= kWNR) ok &= wait_raw_free(&bars[B::raw_free + rs], ((j / kWNR) - 1) & 1, abort_flag);
         uint64_t* bar = &bars[B::raw_full + rs];
         if (blk >= 0 && ok) {
           const uint32_t dst = raw_s + rs * kWRawUnit + lane * bs * kWRawRow;

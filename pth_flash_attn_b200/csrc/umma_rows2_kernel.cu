@@ -386,7 +386,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       for (int j = 0; j < n_tiles; ++j) {
         const int blk_next = page_block(j + 1);
         const int rs = j % kXNR;
-        if (j >= kXNR) ok &= wait_or_abort(&bars[B::raw_free + rs], ((j / kXNR) - 1) & 1, abort_flag);
+        if (j >= kXNR) ok &= wait_raw_free(&bars[B::raw_free + rs], ((j / kXNR) - 1) & 1, abort_flag);
         uint64_t* bar = &bars[B::raw_full + rs];
         if (blk >= 0 && ok) {
           const uint32_t dst = raw_s + rs * kXRawUnit + lane * bs * kXRawRow;

@@ -376,7 +376,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       for (int u = 0; u < n_halves; ++u) {
         const int blk_next = page_block(u + 1);
         const int rs = u % kRNR;
-        if (u >= kRNR) ok &= wait_or_abort(&bars[B::raw_free + rs], ((u / kRNR) - 1) & 1, abort_flag);
+        if (u >= kRNR) ok &= wait_raw_free(&bars[B::raw_free + rs], ((u / kRNR) - 1) & 1, abort_flag);
         uint64_t* bar = &bars[B::raw_full + rs];
         if (blk >= 0 && ok) {
           const uint32_t dst = raw_s + rs * kRawHalfBytes + lane * bs * kRawRow;

@@ -1,8 +1,9 @@
 """Run-to-run determinism: the same launch repeated must give the same bytes.
 
-The kernels have no atomics and a fixed reduction order, so any difference between
-two runs is a synchronisation bug (one was found this way: two threads issuing
-tcgen05.mma concurrently in the row-major kernel)."""
+The kernels' reductions have a fixed order (their atomics add whole numbers or take maxima), so any
+difference between two runs is a synchronisation bug (two were found this way: two threads issuing
+tcgen05.mma concurrently in the row-major kernel, and page copies without a proxy fence behind the
+reads of the stage they overwrite)."""
 import numpy as np
 import pytest
 import torch
@@ -17,16 +18,16 @@ pytestmark = pytest.mark.gpu
 # 128 dims), drafter / wide-verification sizes (the one-tile kernel, whose raw ring is shared by two
 # producer halves), and the kernels of the other head sizes.
 LONG_CASES = [
-    (capi.KERNEL_UMMA_ROWS, [4096, 700], [2048, 40], 16, 2, 8, 1, 300, 128),
-    (capi.KERNEL_UMMA_ROWS, [6000, 3000], [300, 16], 32, 8, 16, 3, 300, 128),
-    (capi.KERNEL_UMMA_ROWS, [9000, 5000, 700], [16, 16, 40], 32, 8, 16, 2, 300, 128),
-    (capi.KERNEL_UMMA, [20000, 9000, 300, 4100], [1, 1, 1, 1], 32, 8, 1, 4, 300, 128),
-    (capi.KERNEL_UMMA, [9000, 2500], [4, 4], 32, 8, 4, 2, 300, 128),
-    (capi.KERNEL_AUTO, [9000, 700, 3000, 64], [1, 300, 4, 1], 16, 2, 8, 2, 300, 128),
-    (capi.KERNEL_UMMA_ROWS, [4096, 700], [1024, 40], 12, 2, 10, 2, 200, 256),
-    (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 2, 1], 12, 2, 2, 3, 200, 256),
-    (capi.KERNEL_UMMA_ROWS, [4096, 700], [1024, 40], 16, 4, 16, 1, 200, 64),
-    (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 4, 1], 16, 4, 4, 3, 200, 64),
+    (capi.KERNEL_UMMA_ROWS, [4096, 700], [2048, 40], 16, 2, 8, 1, 5000, 128),
+    (capi.KERNEL_UMMA_ROWS, [6000, 3000], [300, 16], 32, 8, 16, 3, 5000, 128),
+    (capi.KERNEL_UMMA_ROWS, [9000, 5000, 700], [16, 16, 40], 32, 8, 16, 2, 5000, 128),
+    (capi.KERNEL_UMMA, [20000, 9000, 300, 4100], [1, 1, 1, 1], 32, 8, 1, 4, 5000, 128),
+    (capi.KERNEL_UMMA, [9000, 2500], [4, 4], 32, 8, 4, 2, 5000, 128),
+    (capi.KERNEL_AUTO, [9000, 700, 3000, 64], [1, 300, 4, 1], 16, 2, 8, 2, 5000, 128),
+    (capi.KERNEL_UMMA_ROWS, [4096, 700], [1024, 40], 12, 2, 10, 2, 5000, 256),
+    (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 2, 1], 12, 2, 2, 3, 5000, 256),
+    (capi.KERNEL_UMMA_ROWS, [4096, 700], [1024, 40], 16, 4, 16, 1, 5000, 64),
+    (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 4, 1], 16, 4, 4, 3, 5000, 64),
 ]
 
 CASES = [
@@ -68,9 +69,10 @@ def test_repeated_launches_are_identical(kernel, lens, qlens, Hq, Hkv, bq, S):
 
 @pytest.mark.parametrize("kernel,lens,qlens,Hq,Hkv,bq,S,repeats,D", LONG_CASES)
 def test_many_repeats_on_cold_and_warm_caches(kernel, lens, qlens, Hq, Hkv, bq, S, repeats, D):
-    """A rare ordering bug shows as one launch in a hundred: repeat each launch 300 times, with
-    a buffer larger than L2 written between some of them (so that page copies arrive in other
-    orders), and compare every result with the first on the device."""
+    """A rare ordering bug shows as one launch in several hundred (a raw stage refilled around its last
+    read: 12 of 5,686 launches at 256 dims) or fewer: repeat each launch 5,000 times, with a buffer
+    larger than L2 written between some of them (so that page copies arrive in other orders), and
+    compare every result with the first on the device."""
     from tests.gpu_util import cache_to_device, q_to_device
 
     c = orc.make_paged_cache(lens, Hkv, D, 16, seed=41)

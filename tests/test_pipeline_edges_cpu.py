@@ -1,9 +1,11 @@
-"""Barrier edges of the row-major kernels, read off their sources.
+"""Barrier edges of the tensor-core kernels, read off their sources.
 
 A wait that is missing between two roles of a CTA shows on the GPU only when the late role is
 late, and running such a kernel there is a data race.  So the edges are checked in the text: in
-the MMA issuer's part every QK stands behind a wait for its K image, and every PV behind the waits
-for its P and for its V image.
+the row-major kernels' MMA issuers every QK stands behind a wait for its K image, and every PV behind the
+waits for its P and for its V image; in every loader a proxy fence stands between the wait for
+a raw stage's readers, which read through the generic proxy, and the page copies, which write through
+the async proxy.
 """
 import re
 from pathlib import Path
@@ -21,15 +23,15 @@ def _code(name):
     return text[text.index("__global__"):text.index("cudaError_t launch")]
 
 
-def _issuer(code):
-    """The text of the MMA issuer's role: from its branch to the next one."""
-    start = re.search(r"else if \(warp == k\w*MmaWarp\)", code).start()
+def _role(code, warp):
+    """The text of a role: from its branch to the next one."""
+    start = re.search(rf"else if \(warp == k\w*{warp}\b", code).start()
     return code[start:code.index("else if (warp", start + 10)]
 
 
 @pytest.mark.parametrize("name", KERNELS)
 def test_every_mma_stands_behind_the_waits_for_its_operands(name):
-    issuer = _issuer(_code(name))
+    issuer = _role(_code(name), "MmaWarp")
     needs = {"issue_qk": {"kfull"}, "issue_pv": {"p_ready", "vfull"}}
     seen = set()
     waited = set()
@@ -42,3 +44,16 @@ def test_every_mma_stands_behind_the_waits_for_its_operands(name):
         assert needs[issue] <= waited, f"{name}: {issue} is issued without a wait for {sorted(needs[issue] - waited)}"
         waited -= needs[issue]
     assert seen == set(needs)
+
+
+@pytest.mark.parametrize("name", KERNELS + ["umma_i8_kernel.cu"])
+def test_page_copies_stand_behind_a_proxy_fence(name):
+    loader = _role(_code(name), "LoadWarp")
+    for copy in ("tma_load_3d(", "bulk_copy_g2s("):
+        wait = re.search(r"(\w+)\(&bars\[B::raw_free", loader)
+        assert wait and wait.start() < loader.index(copy)
+        assert wait.group(1) == "wait_raw_free", f"{name}: {copy}) behind {wait.group(1)}"
+    shared = (CSRC / "page_copy.cuh").read_text()
+    body = shared[shared.index("bool wait_raw_free("):]
+    body = body[:body.index("\n}")]
+    assert body.index("wait_or_abort(") < body.index("fence_async_smem();") < body.index("return")
