@@ -14,9 +14,15 @@
 // Every operand is fp16, whatever the queries are (both operands of an MMA have one format):
 //   K, V   int8 is exact in fp16, and its widening costs 1.25 instructions per value; to bf16,
 //          whose 8 bits hold no biased int8, it takes 2;
-//   Q      fp16 as it is; bf16 times the power of two that puts the largest finite query value of
-//          the CTA into [2^14, 2^15): exact down to 2^-31 of that value, and the inverse is folded
-//          into the keys' score factor;
+//   Q      fp16 as it is; bf16 times a power of two that depends on the row alone: 2^7 where the row's
+//          largest finite value is in [2^-4, 2^8), and the keys' score factor takes that back, else the one
+//          that puts it into [2^14, 2^15), and the row's scores are multiplied by the rest (one
+//          more multiplication per score, for warps that hold such a row).  A value is exact down to
+//          2^-17 (2^-20 of the row's largest, 2^-31 of it with a power of its own) and off by
+//          2^-25 (2^-28 of the largest) at most below.  (One power for the whole CTA let a huge query of one
+//          row take the others' bits, and the keys' scales had to wait for it: one bf16 prompt of 100 tokens
+//          took 24.3 us against 21.3, two of 1,000 59.5 against 55.1; long chunks, whose loop now has two
+//          instances, 2 x 2,048 tokens over 14,336 keys 2,375 against 2,402.)
 //   P      2^7 exp2(score + log2(v_scale) - reference): the key's v_scale sits in the exponent, so
 //          V needs no multiplication and fp16's range is that of one row, not of the cache.  A
 //          weighted score exceeds its reference by at most 8, so P stays at or below 2^15, and
@@ -208,20 +214,51 @@ __device__ __forceinline__ void rows_cta(const KernelParams& p, int* kvh, int* t
 }
 
 // ---- queries ----
-// Largest finite magnitude of 8 bf16 values, as fp32 bits (which order like the values).  An infinity or
-// a NaN makes its own row what it makes it anywhere; it must not choose the scale of the CTA's other rows.
-__device__ __forceinline__ uint32_t amax_bits_bf16(uint4 v, uint32_t m) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  auto finite = [](uint32_t bits) { return bits < 0x7f800000u ? bits : 0u; };
+constexpr float kQueryGain = 128.0f;
+// What the keys' score factor takes back of the queries' power of two.
+__device__ __forceinline__ float query_ungain(int q_dtype) { return q_dtype == PTH_ATTN_BF16 ? 1.0f / kQueryGain : 1.0f; }
+// Bits of the largest finite magnitude among 8 N bf16 values.  An infinity or a NaN makes its row what it
+// makes it anywhere; where one turns up the maximum is taken again without them.
+template <int N>
+__device__ __forceinline__ uint32_t finite_amax_bf16(const uint4 (&q)[N]) {
+  uint32_t m = 0u;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) m = max(m, max(finite((w[e] << 16) & 0x7fffffffu), finite(w[e] & 0x7fff0000u)));
+  for (int c = 0; c < N; ++c) {
+    m = __vimax3_u16x2(m, q[c].x & 0x7fff7fffu, q[c].y & 0x7fff7fffu);
+    m = __vimax3_u16x2(m, q[c].z & 0x7fff7fffu, q[c].w & 0x7fff7fffu);
+  }
+  m = max(m & 0xffffu, m >> 16);
+  if (m >= 0x7f80u) {
+    m = 0u;
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+      const uint32_t w[4] = {q[c].x, q[c].y, q[c].z, q[c].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t lo = w[e] & 0x7fffu, hi = (w[e] >> 16) & 0x7fffu;
+        m = max(m, max(lo < 0x7f80u ? lo : 0u, hi < 0x7f80u ? hi : 0u));
+      }
+    }
+  }
   return m;
 }
-// The power of two that moves a value of these bits into [2^14, 2^15) (1 for zero).
-__device__ __forceinline__ float query_scale(uint32_t amax_bits) {
-  if (amax_bits == 0u) return 1.0f;
-  const int e = min((int)(amax_bits >> 23) - 127, 127);  // (subnormal: -127)
-  return __uint_as_float((uint32_t)(min(14 - e, 126) + 127) << 23);
+// The power of two of a row, and what its scores are multiplied by besides the keys' factor.
+struct QueryScale {
+  float scale, fix;
+};
+__device__ __forceinline__ QueryScale query_scale(uint32_t amax_bits) {
+  const int e = (int)(amax_bits >> 7) - 127;  // (zero and subnormals: -127)
+  if (amax_bits == 0u || (e >= -4 && e < 8)) return QueryScale{kQueryGain, 1.0f};
+  const int s = min(14 - e, 126);             // -113 .. 126
+  return QueryScale{__uint_as_float((uint32_t)(127 + s) << 23), __uint_as_float((uint32_t)(127 + 7 - s) << 23)};
+}
+// N scores of a row times what its own power of two leaves.  (In an instance of the tile loop of its own: the
+// same multiplications behind a branch cost warps without such a row 1 to 4 %, a rolled loop over
+// the scores in TMEM in front of the loads 3 to 5 % at 128 dims.)
+template <int N>
+__device__ __forceinline__ void scale_scores(uint32_t* r, float fix) {
+#pragma unroll
+  for (int n = 0; n < N; ++n) r[n] = __float_as_uint(__uint_as_float(r[n]) * fix);
 }
 // 8 bf16 queries times a power of two -> fp16.
 __device__ __forceinline__ uint4 queries_to_f16(uint4 v, float scale) {
@@ -249,7 +286,7 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
 }
 
 // What the softmax needs of a key, one vector of N floats each: the score factor k_scale *
-// softmax_scale * log2 e / query scale, log2(v_scale) and 1 / v_scale.
+// softmax_scale * log2 e (/ 2^7 for bf16 queries), log2(v_scale) and 1 / v_scale.
 template <int N>
 struct KeyScales {
   float score[N], lv[N], iv[N];

@@ -52,7 +52,7 @@ constexpr int kWGroupDims = kWDim / 2;              // 128 columns of O per grou
 constexpr int kWProducers = 256;                    // warps 8-11 (K set) and 12-15 (V set)
 constexpr int kWMmaWarp = 16, kWLoadWarp = 17;
 constexpr int kWThreads = 576;
-constexpr int kWQBarrier = kWSoftmax + kWProducers / 2 + 32;  // Q in TMEM: softmax, K set, MMA issuer
+constexpr int kWQBarrier = kWSoftmax + 32;  // Q in TMEM: softmax, MMA issuer
 constexpr int kWProducerRegs = 64, kWSoftmaxRegs = 128;  // of the 96 per thread the CTA starts with
 constexpr int kWSCol = 0, kWOCol = 128, kWQCol = 384;    // TMEM columns: S buffers at 0 and 64, O, Q
 constexpr float kWRescaleGap = 8.0f;                // log2 units a row maximum may outgrow its reference
@@ -117,8 +117,6 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::bars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
-  uint32_t* qmax_s = reinterpret_cast<uint32_t*>(smem + L::misc + 24);           // bits of the largest query value
-  volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
   KeyScales<kWKeys>* key_scales = reinterpret_cast<KeyScales<kWKeys>*>(smem + L::ksc);
 
   int kvh, tile_index;
@@ -239,7 +237,6 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       tc::mbar_init(&bars[B::raw_free + s], kWProducers);             // every producer thread reads every unit
     }
     *abort_flag = 0;
-    *qmax_s = 0u;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -276,7 +273,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     // first byte of this thread's 128 bytes inside a raw unit
     const uint32_t piece = my_page * bs * kWRawRow + my_slot * row_pitch + delta + (v_part ? kWDim + 4 : 0) + upper * 128;
     const int wo = (int)((piece & 15u) >> 2);  // first word of the piece in the 16-byte chunks read: 0 / 2 (K), 1 / 3 (V)
-    float score_mul = 0.f;  // softmax_scale * log2 e / query scale
+    const float score_mul = p.scale_log2 * query_ungain(p.q_dtype);
 #pragma unroll 1
     for (int j = 0; j < n_tiles; ++j) {
       const int rs = j % kWNR;
@@ -327,10 +324,6 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       else if (wo == 1) widen_piece(std::integral_constant<int, 1>{});
       else if (wo == 2) widen_piece(std::integral_constant<int, 2>{});
       else widen_piece(std::integral_constant<int, 3>{});
-      if (!v_part && j == 0) {  // the query scale is known once Q is complete
-        named_barrier(5, kWQBarrier);
-        score_mul = p.scale_log2 * *qinv_s;
-      }
       if (upper && !v_part) {
         KeyScales<kWKeys>& ks = key_scales[j % kWKsRing];
         const float vs = usable_v_scale(v_scale);
@@ -444,31 +437,31 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     const uint32_t o_part = tmem_base + kWOCol + g * kWGroupDims + lane_addr;   // this group's columns of O
 
     // ---- Q into TMEM: thread (row, g) stores dims 128 g .. 128 g + 127 of its row, two fp16 per column ----
+    float q_fix = 1.0f;  // what the row's scores are multiplied by (QueryScale)
     {
       int token, head;
       row_target(p, t, kvh, row, &token, &head);
       const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
                                                         (int64_t)head * p.q_stride_head) + g * (kWGroupDims / 8);
-      auto load_q = [&](int c) { return row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u); };
-      const bool from_bf16 = p.q_dtype == PTH_ATTN_BF16;
-      float qscale = 1.0f;
-      if (from_bf16) {  // one power of two for all rows of the CTA
-        uint32_t m = 0u;
+      uint4 qv[16];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) m = amax_bits_bf16(load_q(c), m);
-        m = __reduce_max_sync(0xffffffffu, m);
-        if (lane == 0) atomicMax(qmax_s, m);
+      for (int c = 0; c < 16; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
+      if (p.q_dtype == PTH_ATTN_BF16) {
+        uint32_t* part = reinterpret_cast<uint32_t*>(tile_max);  // [2 groups][128 rows] (idle until the first tile)
+        const uint32_t mine = finite_amax_bf16(qv);
+        part[g * kWGroup + row] = mine;
         named_barrier(4, kWSoftmax);
-        qscale = query_scale(*reinterpret_cast<volatile uint32_t*>(qmax_s));
+        const QueryScale qs = query_scale(max(mine, part[(g ^ 1) * kWGroup + row]));
+        q_fix = qs.fix;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) qv[c] = queries_to_f16(qv[c], qs.scale);
       }
-      if (tid == 0) *qinv_s = 1.0f / qscale;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint32_t qw[32];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          uint4 v = load_q(h * 8 + c);
-          if (from_bf16) v = queries_to_f16(v, qscale);
+          const uint4 v = qv[h * 8 + c];
           qw[4 * c] = v.x;
           qw[4 * c + 1] = v.y;
           qw[4 * c + 2] = v.z;
@@ -488,6 +481,8 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     visible_range(p, t, t.first_idx, &tmp, &mask_hi);
     float m_ref = -INFINITY;  // reference maximum of the row's exponentials (log2 units)
     float l = 0.f;            // 2^kPGain times the sum of exp2(score - m_ref) over this group's keys, without v_scale
+    auto walk_tiles = [&](auto own_power) {  // (one instance for warps without a row of its own power of two)
+      constexpr bool kOwnPower = decltype(own_power)::value;
 #pragma unroll 1
     for (int i = 0; i < n_tiles; ++i) {
       const KeyScales<kWKeys>& ks = key_scales[i % kWKsRing];
@@ -499,6 +494,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       uint32_t r[kWGroupKeys];  // the scores of this row and part, read once
       tc::tmem_ld32(s_tmem, r);
       tc::tmem_ld_wait<kWGroupKeys>(r);
+      if constexpr (kOwnPower) scale_scores<kWGroupKeys>(r, q_fix);
 
       // ---- pass 1: weighted scores in log2 units (kept in the registers) and their maximum ----
       auto all_ready = [] {};
@@ -548,6 +544,8 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       tc::fence_before_sync();
       mbar_arrive(&bars[B::p_ready + (i & 1)]);  // this group's part of P(i) is complete
     }
+    };
+    if (__any_sync(0xffffffffu, q_fix != 1.0f)) walk_tiles(std::true_type{}); else walk_tiles(std::false_type{});
 
     // ---- epilogue: the row's sum is the two groups' sums; each group writes its half of the dims ----
     // (the commit after the last PV covers every MMA issued before it)

@@ -58,7 +58,7 @@ constexpr int kXSoftmax = 256;                      // warps 0-3 (row tile 0), 4
 constexpr int kXProducers = 256;                    // warps 8-11 (K set) and 12-15 (V set)
 constexpr int kXMmaWarp = 16, kXLoadWarp = 17;
 constexpr int kXThreads = 576;
-constexpr int kXQBarrier = kXSoftmax + kXProducers / 2 + 32;  // Q images complete: softmax, K set, MMA issuer
+constexpr int kXQBarrier = kXSoftmax + 32;  // Q images complete: softmax, MMA issuer
 // Registers per thread, of the 96 the CTA starts with.  The softmax, which bounds the kernel by its instructions,
 // keeps more of a tile's scales in flight with 136 than with 120; a producer's words fit 56.  (4 x 2,048 tokens
 // over 14,336 keys at 64 dims: 2,052 us, with 128 registers 2,085.)
@@ -81,7 +81,7 @@ struct XLayout {
 };
 
 struct XBars {
-  static constexpr int vfull = 0;                      // [NS] V producers -> softmax (pass 2) and PV
+  static constexpr int vfull = 0;                      // [NS] V producers -> PV
   static constexpr int vempty = kXNS;                  // [NS] PV commit -> V producers
   static constexpr int kempty = 2 * kXNS;              // [NK] QK commit -> K producers
   static constexpr int kfull = 2 * kXNS + kXNK;        // [NK] K producers -> QK
@@ -129,8 +129,6 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::bars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
-  uint32_t* qmax_s = reinterpret_cast<uint32_t*>(smem + L::misc + 24);           // bits of the largest query value
-  volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
   KeyScales<kXKeys>* key_scales = reinterpret_cast<KeyScales<kXKeys>*>(smem + L::ksc);
 
   int kvh, tile_index;
@@ -254,7 +252,6 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       tc::mbar_init(&bars[B::raw_free + s], kXProducers);             // every producer thread reads every unit
     }
     *abort_flag = 0;
-    *qmax_s = 0u;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -289,7 +286,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     // first byte of this thread's bytes inside a raw unit
     const uint32_t piece = my_page * bs * kXRawRow + my_slot * row_pitch + delta + (v_part ? kXDim + 4 : 0) + upper * G::piece;
     const int wo = (int)((piece & 15u) >> 2);  // first word of the piece in the 16-byte chunks read: 0 / 2 (K), 1 / 3 (V)
-    float score_mul = 0.f;  // softmax_scale * log2 e / query scale
+    const float score_mul = p.scale_log2 * query_ungain(p.q_dtype);
 #pragma unroll 1
     for (int j = 0; j < n_tiles; ++j) {
       const int rs = j % kXNR;
@@ -341,10 +338,6 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       else if (wo == 1) widen_piece(std::integral_constant<int, 1>{});
       else if (wo == 2) widen_piece(std::integral_constant<int, 2>{});
       else widen_piece(std::integral_constant<int, 3>{});
-      if (!v_part && j == 0) {  // the query scale is known once the Q images are complete
-        named_barrier(5, kXQBarrier);
-        score_mul = p.scale_log2 * *qinv_s;
-      }
       if (upper && !v_part) {
         KeyScales<kXKeys>& ks = key_scales[j % kXKsRing];
         const float vs = usable_v_scale(v_scale);
@@ -469,30 +462,24 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     const uint32_t o_tmem = tmem_base + kXOCol + rt * kXDim + lane_addr;    // O(rt)
 
     // ---- Q image of this row tile: thread converts its row, 16 column blocks of 8 dims ----
+    float q_fix = 1.0f;  // what the row's scores are multiplied by (QueryScale)
     {
       int token, head;
       row_target(p, t, kvh, row, &token, &head);
       const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
                                                         (int64_t)head * p.q_stride_head);
       uint8_t* qrow = smem + L::qimg + rt * kXQImage + (tid & 127) * 16;
-      auto load_q = [&](int c) { return row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u); };
-      const bool from_bf16 = p.q_dtype == PTH_ATTN_BF16;
-      float qscale = 1.0f;
-      if (from_bf16) {  // one power of two for all rows of the CTA
-        uint32_t m = 0u;
+      uint4 qv[kXChunks];
 #pragma unroll
-        for (int c = 0; c < kXChunks; ++c) m = amax_bits_bf16(load_q(c), m);
-        m = __reduce_max_sync(0xffffffffu, m);
-        if (lane == 0) atomicMax(qmax_s, m);
-        named_barrier(6, kXSoftmax);
-        qscale = query_scale(*reinterpret_cast<volatile uint32_t*>(qmax_s));
-      }
-      if (tid == 0) *qinv_s = 1.0f / qscale;
+      for (int c = 0; c < kXChunks; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
+      if (p.q_dtype == PTH_ATTN_BF16) {
+        const QueryScale qs = query_scale(finite_amax_bf16(qv));
+        q_fix = qs.fix;
 #pragma unroll
-      for (int c = 0; c < kXChunks; ++c) {
-        const uint4 v = load_q(c);
-        *reinterpret_cast<uint4*>(qrow + c * kXQStride) = from_bf16 ? queries_to_f16(v, qscale) : v;
+        for (int c = 0; c < kXChunks; ++c) qv[c] = queries_to_f16(qv[c], qs.scale);
       }
+#pragma unroll
+      for (int c = 0; c < kXChunks; ++c) *reinterpret_cast<uint4*>(qrow + c * kXQStride) = qv[c];
     }
     tc::fence_async_smem();
     named_barrier(5, kXQBarrier);  // Q images complete; the QK issuer may start
@@ -520,6 +507,8 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
         }
       }
     } else {  // warps with live rows (the loop keeps its indentation)
+    auto walk_tiles = [&](auto own_power) {  // (one instance for warps without a row of its own power of two)
+      constexpr bool kOwnPower = decltype(own_power)::value;
 #pragma unroll 1
     for (int i = 0; i < n_tiles; ++i) {
       const int b = i & 1;
@@ -533,9 +522,13 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       tc::tmem_ld32(s_tmem, r);  // pass 1 works on the first
       tc::tmem_ld_wait<32>(r);
       tc::tmem_ld32(s_tmem + 32, r + 32);
+      if constexpr (kOwnPower) scale_scores<32>(r, q_fix);
 
       // ---- pass 1: weighted scores in log2 units (kept in the registers) and their maximum ----
-      auto half_ready = [&] { tc::tmem_ld_wait<32>(r + 32); };
+      auto half_ready = [&] {
+        tc::tmem_ld_wait<32>(r + 32);
+        if constexpr (kOwnPower) scale_scores<32>(r + 32, q_fix);
+      };
       const float m_t =
           interior ? softmax_pass1<kXKeys, false>(r, ks.score, ks.lv, half_ready, [](int) { return true; })
                    : softmax_pass1<kXKeys, true>(r, ks.score, ks.lv, half_ready, [&](int n) {
@@ -580,6 +573,8 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       tc::fence_before_sync();
       mbar_arrive(&bars[B::p_ready + 2 * rt + b]);  // P(rt, i) is complete
     }
+    };
+    if (__any_sync(0xffffffffu, q_fix != 1.0f)) walk_tiles(std::true_type{}); else walk_tiles(std::false_type{});
     }  // warps with live rows
 
     // ---- epilogue: the row's output (the commit after the last PV covers every MMA issued before it) ----

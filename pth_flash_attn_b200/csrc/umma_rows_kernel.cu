@@ -52,7 +52,7 @@ constexpr int kHalfKeys = 64;            // keys of one raw half stage
 constexpr int kRawHalfBytes = kHalfKeys * kRawRow;   // 17,408 B
 constexpr int kRVStage = kWideBytes;                 // V image
 constexpr int kRKsRing = 4;                          // tiles of key scales kept
-constexpr int kRQBarrier = kRSoftmax + kRProducers / 2 + 32;  // Q image complete: softmax, K set, MMA issuer
+constexpr int kRQBarrier = kRSoftmax + 32;  // Q image complete: softmax, MMA issuer
 // Registers: the CTA starts with 96 per thread (18 warps: five on two of the SM's four schedulers, whose
 // 16,384 registers that fills).  The two producer warpgroups hand 16 per thread to the two softmax
 // warpgroups, which keep the 64 scores of a row and half tile in registers between the two passes;
@@ -108,8 +108,6 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::bars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
-  uint32_t* qmax_s = reinterpret_cast<uint32_t*>(smem + L::misc + 24);           // bits of the largest query value
-  volatile float* qinv_s = reinterpret_cast<volatile float*>(smem + L::misc + 28);  // 1 / query scale
   KeyScales<kTileKeys>* key_scales = reinterpret_cast<KeyScales<kTileKeys>*>(smem + L::ksc);
 
   int kvh, tile_index;
@@ -226,7 +224,6 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       tc::mbar_init(&bars[B::raw_free + s], kRProducers / 2);             // 64 K-set + 64 V-set threads
     }
     *abort_flag = 0;
-    *qmax_s = 0u;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -262,7 +259,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     const int my_page = (key & (kHalfKeys - 1)) >> p.copy_shift, my_slot = key & (bs - 1);
     const uint32_t cell_off = my_page * bs * kRawRow + my_slot * row_pitch + delta;  // inside a half stage
     const bool odd = (cell_off & 8u) != 0;
-    float score_mul = 0.f;  // softmax_scale * log2 e / query scale
+    const float score_mul = p.scale_log2 * query_ungain(p.q_dtype);
 #pragma unroll 1
     for (int j = 0; j < n_tiles; ++j) {
       const int u = 2 * j + half;
@@ -313,10 +310,6 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
           for (int c = 0; c < kChunks; ++c)
             *reinterpret_cast<uint4*>(kdst + c * kChunkStride) = widen8_f16(make_uint2(w[2 + 2 * c], w[3 + 2 * c]));
           k_scale = __uint_as_float(w[34]);
-        }
-        if (j == 0) {  // the query scale is known once the Q image is complete
-          named_barrier(5, kRQBarrier);
-          score_mul = p.scale_log2 * *qinv_s;
         }
         KeyScales<kTileKeys>& ks = key_scales[j % kRKsRing];
         const float vs = usable_v_scale(v_scale);
@@ -461,6 +454,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     const uint32_t o_tmem = tmem_base + 256 + g * 128 + lane_addr;  // O(g)
 
     // ---- Q image: thread (row, half) converts 8 of the 16 d-chunks of its row ----
+    float q_fix = 1.0f;  // what the row's scores are multiplied by (QueryScale)
     {
       const int half = tid >> 7;
       int token, head;
@@ -470,19 +464,16 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       uint4 qv[8];
 #pragma unroll
       for (int c = 0; c < 8; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
-      float qscale = 1.0f;
-      if (p.q_dtype == PTH_ATTN_BF16) {  // one power of two for all rows of the CTA
-        uint32_t m = 0u;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) m = amax_bits_bf16(qv[c], m);
-        m = __reduce_max_sync(0xffffffffu, m);
-        if (lane == 0) atomicMax(qmax_s, m);
+      if (p.q_dtype == PTH_ATTN_BF16) {
+        uint32_t* part = reinterpret_cast<uint32_t*>(half == 0 ? park_m : park_l);  // (idle until the epilogue)
+        const uint32_t mine = finite_amax_bf16(qv);
+        part[row] = mine;
         named_barrier(4, kRSoftmax);
-        qscale = query_scale(*reinterpret_cast<volatile uint32_t*>(qmax_s));
+        const QueryScale qs = query_scale(max(mine, reinterpret_cast<const uint32_t*>(half == 0 ? park_l : park_m)[row]));
+        q_fix = qs.fix;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) qv[c] = queries_to_f16(qv[c], qscale);
+        for (int c = 0; c < 8; ++c) qv[c] = queries_to_f16(qv[c], qs.scale);
       }
-      if (tid == 0) *qinv_s = 1.0f / qscale;
 #pragma unroll
       for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(qimg + (half * 8 + c) * kChunkStride + row * 16) = qv[c];
     }
@@ -509,6 +500,8 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
         mbar_arrive(&bars[B::p_ready + (i & 1)]);
       }
     } else {  // warps with live rows (the loop keeps its indentation)
+    auto walk_tiles = [&](auto own_power) {  // (one instance for warps without a row of its own power of two)
+      constexpr bool kOwnPower = decltype(own_power)::value;
 #pragma unroll 1
     for (int i = 0; i < n_tiles; ++i) {
       const KeyScales<kTileKeys>& ks = key_scales[i % kRKsRing];
@@ -522,6 +515,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       tc::tmem_ld32(s_tmem, r);
       tc::tmem_ld32(s_tmem + 32, r + 32);
       tc::tmem_ld_wait<64>(r);
+      if constexpr (kOwnPower) scale_scores<64>(r, q_fix);
 
       // ---- pass 1: weighted scores in log2 units (kept in the registers) and their maximum ----
       // (two instances: interior tiles, which every live row sees whole, skip the mask)
@@ -570,6 +564,8 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       tc::fence_before_sync();
       mbar_arrive(&bars[B::p_ready + (i & 1)]);  // this group's half of P(i) is complete
     }
+    };
+    if (__any_sync(0xffffffffu, q_fix != 1.0f)) walk_tiles(std::true_type{}); else walk_tiles(std::false_type{});
     }  // warps with live rows
 
     // ---- epilogue: merge the two groups' (m, l, O) and write the rows ----

@@ -60,6 +60,46 @@ def test_a_row_of_infinities_leaves_the_other_rows_alone(D, qlen):
     assert not np.isfinite(dirty["out"].reshape(qlen, 8, D)[3, 2]).any()
 
 
+@pytest.mark.parametrize("D,qlen", SHAPES)
+def test_a_huge_finite_row_leaves_the_other_rows_alone(D, qlen):
+    """The power of two of bf16 queries is the row's own: beside a row near the type's largest value and one near
+    its smallest, the ordinary rows keep every bit."""
+    c = orc.make_paged_cache([300], 2, D, 16, seed=9)
+    rng = np.random.default_rng(10)
+    q = orc.round_to_bf16(rng.standard_normal((qlen, 8, D), dtype=np.float32))
+    qsl = np.array([0, qlen])
+    clean = _run(c, q, qsl, D, 16, out_dtype=torch.float32)
+    q[3, 2] = np.where(rng.random(D) < 0.5, 3e38, -3e38)
+    q[4, 5] *= np.float32(2.0 ** -120)
+    dirty = _run(c, q, qsl, D, 16, out_dtype=torch.float32)
+    others = np.ones((qlen, 8), dtype=bool)
+    others[3, 2] = others[4, 5] = False
+    out = lambda r: r["out"].reshape(qlen, 8, D)  # noqa: E731
+    assert np.array_equal(out(dirty)[others], out(clean)[others])
+    assert np.array_equal(dirty["lse"][others], clean["lse"][others])
+    ref = orc.ref_attention_paged(q, c, qsl, D ** -0.5)
+    others[4, 5] = True   # (a row of tiny queries weighs its keys alike)
+    check_out(out(dirty)[others], ref.out.reshape(qlen, 8, D)[others], max_tol=8 * 2.0 ** -11, mean_tol=2.0 ** -11)
+    check_lse(dirty["lse"][others], ref.lse.reshape(qlen, 8)[others])
+
+
+@pytest.mark.parametrize("D,qlen", SHAPES)
+def test_every_row_with_a_power_of_two_of_its_own(D, qlen):
+    """Rows on both sides of the limits between which the common power serves (largest value in [2^-4, 2^8)), mixed
+    in every warp, against the oracle: the scaling is exact, so only the scores' own rounding may show."""
+    c = orc.make_paged_cache([200], 2, D, 16, seed=17)
+    rng = np.random.default_rng(18)
+    q = orc.round_to_bf16(rng.standard_normal((qlen, 8, D), dtype=np.float32))
+    q /= np.abs(q).max(axis=-1, keepdims=True)          # largest magnitude of every row: one
+    top = np.exp2(rng.integers(-6, 9, (qlen, 8, 1)).astype(np.float32)) * rng.choice([1.0, 0.99609375], (qlen, 8, 1))
+    q = orc.round_to_bf16((q * top).astype(np.float32))
+    qsl = np.array([0, qlen])
+    ref = orc.ref_attention_paged(q, c, qsl, D ** -0.5)
+    res = _run(c, q, qsl, D, 16, out_dtype=torch.float32)
+    # scores reach 2^8 * 4 * sqrt(D) / ln 2 < 2^15 and are held to 2^-24 of that: P within 2^-9, |out| < 8
+    check_out(res["out"], ref.out, max_tol=8 * 2.0 ** -8, mean_tol=2.0 ** -10)
+
+
 @pytest.mark.parametrize("exponent", [-90, 100])
 @pytest.mark.parametrize("D,qlen", SHAPES)
 def test_bf16_queries_beyond_the_range_of_fp16(D, qlen, exponent):
