@@ -136,6 +136,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     }
     __syncthreads();
     t = resolve_row_tile_with(p, tile_index, [&](int i) { return qsl_s[i]; }, [&](int r) { return len_s[r]; });
+    tc::fence_async_smem();  // (page copies write here next, through the other proxy)
     __syncthreads();
   } else {
     t = resolve_row_tile(p, tile_index);

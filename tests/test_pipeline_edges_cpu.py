@@ -57,3 +57,12 @@ def test_page_copies_stand_behind_a_proxy_fence(name):
     body = shared[shared.index("bool wait_raw_free("):]
     body = body[:body.index("\n}")]
     assert body.index("wait_or_abort(") < body.index("fence_async_smem();") < body.index("return")
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_the_scratch_copies_in_the_raw_ring_are_fenced(name):
+    """query_start_loc and seq_lens are copied into the raw ring by plain stores before the first page copy."""
+    code = _code(name)
+    scratch = code[code.index("int* qsl_s = reinterpret_cast<int*>(smem + L::raw)"):code.index("resolve_row_tile(p, tile_index)")]
+    last = scratch.rindex("__syncthreads();")
+    assert scratch.index("resolve_row_tile_with(") < scratch.index("fence_async_smem();") < last
