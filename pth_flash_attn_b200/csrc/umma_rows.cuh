@@ -46,18 +46,6 @@ constexpr int kQImageBytes = kChunks * kChunkStride;    // 33,024 B
 
 namespace tc {
 
-// D[tmem] (+)= A[tmem] * B[smem]; issued by ONE thread.
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
-      : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -82,29 +70,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
 
 }  // namespace tc
 
-// S = Q K^T over the full head dimension: 8 MMAs of K = 16, N = 128 keys.  One thread.
-__device__ __forceinline__ void issue_qk_rows(uint32_t s_tmem, uint32_t q_saddr, uint32_t kw_saddr) {
-  constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kTileKeys, tc::kFmtBF16, tc::kFmtBF16, 0, 0);
-#pragma unroll
-  for (int kk = 0; kk < kHeadDim / 16; ++kk) {
-    const uint64_t a = tc::smem_desc(q_saddr + kk * 2 * kChunkStride, kChunkStride, 128);
-    const uint64_t b = tc::smem_desc(kw_saddr + kk * 2 * kChunkStride, kChunkStride, 128);
-    tc::mma_ss(s_tmem, a, b, idesc, kk > 0);
-  }
-}
-
-// O (+)= P V over the 128 keys of the tile: 8 MMAs of K = 16 keys, N = 128 (d).  P is read
-// from TMEM: 16 keys = 8 columns per step.  One thread.
-__device__ __forceinline__ void issue_pv_rows(uint32_t o_tmem, uint32_t p_tmem, uint32_t vw_saddr, bool accumulate) {
-  constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kHeadDim, tc::kFmtBF16, tc::kFmtBF16, 0, 1);
-#pragma unroll
-  for (int kk = 0; kk < kTileKeys / 16; ++kk) {
-    const uint64_t b = tc::smem_desc(vw_saddr + kk * 256, 128, kChunkStride);
-    tc::mma_ts(o_tmem, p_tmem + kk * 8, b, idesc, accumulate || kk > 0);
-  }
-}
-
-// ---- the same chains for an issuing thread that keeps its descriptors in registers ----
+// ---- MMA chains, for an issuing thread that keeps its descriptors in registers ----
 // (low word = start address in 16-byte units: moving an operand by `bytes` adds bytes / 16)
 struct RowsDesc {
   uint32_t lo, hi;
@@ -150,15 +116,7 @@ __device__ __forceinline__ void issue_qk_rows_words(uint32_t s_tmem, RowsDesc q,
   for (int kk = 1; kk < kHeadDim / 16; ++kk)
     mma_ss_words<true>(s_tmem, q.lo + kk * step, q.hi, k.lo + kk * step, k.hi, idesc);
 }
-// v = rows_desc(V image, 128, kChunkStride)
-__device__ __forceinline__ void issue_pv_rows_words(uint32_t o_tmem, uint32_t p_tmem, RowsDesc v, bool accumulate) {
-  constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kHeadDim, tc::kFmtF16, tc::kFmtF16, 0, 1);
-#pragma unroll
-  for (int kk = 0; kk < kTileKeys / 16; ++kk)
-    mma_ts_words(o_tmem, p_tmem + kk * 8, v.lo + kk * (256 >> 4), v.hi, idesc, accumulate || kk > 0);
-}
-
-// PV of one tile as two chains: keys 0-63 (P columns 0-31 of the S buffer, V rows 0-63) into the
+// v = rows_desc(V image, 128, kChunkStride).  PV of one tile as two chains: keys 0-63 (P columns 0-31 of the S buffer, V rows 0-63) into the
 // accumulator at o_tmem, keys 64-127 (P columns 64-95, V rows 64-127) into the one at o_tmem + 128.
 __device__ __forceinline__ void issue_pv_halves_words(uint32_t o_tmem, uint32_t s_tmem, RowsDesc v, bool accumulate) {
   constexpr uint32_t idesc = tc::instr_desc(kRowsPerTile, kHeadDim, tc::kFmtF16, tc::kFmtF16, 0, 1);

@@ -59,17 +59,17 @@ def test_umma_tile_int8():
 
 
 def test_umma_tile_rows():
-    """Row-major building blocks: S = Q K^T (rows on M) and O = P V with P read from TMEM."""
+    """Row-major building blocks in fp16: S = Q K^T (rows on M) and O = P V, P read from TMEM in two halves."""
     lib = capi.load_library()
     rng = np.random.default_rng(21)
     k = rng.integers(-128, 128, size=(128, 128), dtype=np.int8)
     v = rng.integers(-128, 128, size=(128, 128), dtype=np.int8)
-    q = orc.round_to_bf16(rng.standard_normal((128, 128), dtype=np.float32))
-    pm = orc.round_to_bf16(rng.random((128, 128), dtype=np.float32))
+    k[0, :4] = [-128, 127, 0, -1]
+    q = rng.standard_normal((128, 128), dtype=np.float32).astype(np.float16)   # (products are exact in fp32 below)
+    pm = rng.random((128, 128), dtype=np.float32).astype(np.float16)
     dev = "cuda"
     kt, vt = torch.from_numpy(k).to(dev), torch.from_numpy(v).to(dev)
-    qt = torch.from_numpy(q).to(dev).to(torch.bfloat16)
-    pt = torch.from_numpy(pm).to(dev).to(torch.bfloat16)
+    qt, pt = torch.from_numpy(q).to(dev), torch.from_numpy(pm).to(dev)
     s_out = torch.full((128, 128), float("nan"), dtype=torch.float32, device=dev)
     o_out = torch.full((128, 128), float("nan"), dtype=torch.float32, device=dev)
     rc = lib.lib.pthb200_test_tile_rows(kt.data_ptr(), qt.data_ptr(), vt.data_ptr(), pt.data_ptr(),
