@@ -23,11 +23,13 @@
 //          row take the others' bits, and the keys' scales had to wait for it: one bf16 prompt of 100 tokens
 //          took 24.3 us against 21.3, two of 1,000 59.5 against 55.1; long chunks, whose loop now has two
 //          instances, 2 x 2,048 tokens over 14,336 keys 2,375 against 2,402.)
-//   P      2^7 exp2(score + log2(v_scale) - reference): the key's v_scale sits in the exponent, so
+//   P      2^11 exp2(score + log2(v_scale) - reference): the key's v_scale sits in the exponent, so
 //          V needs no multiplication and fp16's range is that of one row, not of the cache.  A
-//          weighted score exceeds its reference by at most 8, so P stays at or below 2^15, and
-//          the factor of 2^7 puts what fp16 drops below 2^-32 of the reference: a long context
-//          whose mass sits in many small probabilities beside one large one keeps it.  The row
+//          weighted score exceeds its reference by at most 4, so P stays at or below 2^15, and
+//          with the factor of 2^11 P keeps eight bits (bf16's) down to 2^-28 of the reference and is off by at
+//          most 2^-36 of it below: a long context whose mass sits in many small probabilities beside
+//          one large one keeps it.  (A reference that scores may exceed by 8, with four bits less below, measured
+//          the same within 0.5 %: 3,574 us at 256 dims, 10.21 against 10.26 ms at 128.)  The row
 //          sum takes P / v_scale back in fp32.
 // Measured against bf16 operands (same launches, one box): 4 x 2,048 tokens over 30,720 keys 10.05 -> 9.80 ms,
 // at 256 dims 4.43 -> 3.6 ms, a drafter step 126.5 -> 117.9 us; fp16 queries, which bf16 operands could not
@@ -250,7 +252,7 @@ struct KeyScales {
   float score[N], lv[N], iv[N];
 };
 // log2 of what P is multiplied by (see the head of this file).
-constexpr float kPGain = 7.0f;
+constexpr float kPGain = 11.0f;
 // v_scale as the softmax uses it: a scale of zero (or one below 2^-90, too small to matter) must not
 // turn into 0 * infinity in the row sum, nor the sum of 2^15 / v_scale over a long row into infinity.
 __device__ __forceinline__ float usable_v_scale(float v) { return v < 8.1e-28f ? 8.1e-28f : v; }

@@ -55,7 +55,7 @@ constexpr int kWThreads = 576;
 constexpr int kWQBarrier = kWSoftmax + 32;  // Q in TMEM: softmax, MMA issuer
 constexpr int kWProducerRegs = 64, kWSoftmaxRegs = 128;  // of the 96 per thread the CTA starts with
 constexpr int kWSCol = 0, kWOCol = 128, kWQCol = 384;    // TMEM columns: S buffers at 0 and 64, O, Q
-constexpr float kWRescaleGap = 8.0f;                // log2 units a row maximum may outgrow its reference
+constexpr float kWRescaleGap = 4.0f;                // log2 units a row maximum may outgrow its reference
 
 struct WLayout {
   static constexpr int kimg = 0;

@@ -64,7 +64,7 @@ constexpr int kXQBarrier = kXSoftmax + 32;  // Q images complete: softmax, MMA i
 // over 14,336 keys at 64 dims: 2,052 us, with 128 registers 2,085.)
 constexpr int kXProducerRegs = 56, kXSoftmaxRegs = 136;
 constexpr int kXOCol = 256;                         // TMEM columns: S(rt, b) at (2 rt + b) 64, O(rt) at 256 + 128 rt
-constexpr float kXRescaleGap = 8.0f;                // log2 units a row maximum may outgrow its reference (P stays at or below 2^15)
+constexpr float kXRescaleGap = 4.0f;                // log2 units a row maximum may outgrow its reference (P stays at or below 2^15)
 
 template <int HD>
 struct XLayout {

@@ -21,7 +21,7 @@
 //                         log2 v_scale) and finds their maximum, pass 2 writes P as packed
 //                         fp16 into TMEM over the columns of S it has read.  The
 //                         reference maximum of a (row, half) moves only when the running
-//                         maximum outgrows it by 2^8; then the thread rescales its row of
+//                         maximum outgrows it by 2^4; then the thread rescales its row of
 //                         O(g) in TMEM.  In steady state O is never touched by the softmax.
 // The two groups' (m, l, O) are merged in the epilogue.  TMEM: S0 S1 O0 O1, 128 columns
 // each.  The CTA starts with 96 registers per thread; the producer warpgroups hand part of
@@ -58,7 +58,7 @@ constexpr int kRQBarrier = kRSoftmax + 32;  // Q image complete: softmax, MMA is
 // warpgroups, which keep the 64 scores of a row and half tile in registers between the two passes;
 // every scheduler has two warps of either kind.
 constexpr int kRProducerRegs = 64, kRSoftmaxRegs = 128;
-constexpr float kRescaleGap = 8.0f;      // log2 units a row maximum may outgrow its reference
+constexpr float kRescaleGap = 4.0f;      // log2 units a row maximum may outgrow its reference
 
 template <int kRNK, int kRNR>  // K images, raw HALF stages (64 keys each)
 struct RLayout {

@@ -139,6 +139,24 @@ def test_small_probabilities_beside_a_large_one(D, qlen, q_dtype):
     check_lse(res["lse"][rows], ref.lse.reshape(2, 4))
 
 
+@pytest.mark.parametrize("q_dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D,qlen", SHAPES)
+def test_small_probabilities_keep_eight_bits(D, qlen, q_dtype):
+    """The same with no allowance for P's steps: at 2^-25.5 of the reference P is 2^-14.5 and a step 2^-24, so the
+    outputs are within half of bf16's step of 2^-8 (2^-10.5 of P, 2^-10 of the scores' last digits)."""
+    n, gap = 1 << 15, 25.5
+    k = np.zeros((n, 1, D), dtype=np.float32)
+    k[5] = gap / (2.0 * np.log2(np.e) * D ** 0.5)   # queries are all 2
+    v = np.ones((n, 1, D), dtype=np.float32)
+    v[5, 0, 1::2] = 0.0
+    c = orc.make_paged_cache([n], 1, D, 64, sources=[(k, v)], seed=13)
+    q = np.full((qlen, 4, D), 2.0, dtype=np.float32)
+    ref = orc.ref_attention_paged(q[:1], c, np.array([0, 1]), D ** -0.5, causal=False)
+    res = _run(c, q, np.array([0, qlen]), D, 16, q_dtype=q_dtype, out_dtype=torch.float32, causal=False)
+    got, want = res["out"].reshape(qlen, 4, D)[:, :, 1::2], ref.out.reshape(1, 4, D)[:, :, 1::2]
+    np.testing.assert_allclose(got, np.broadcast_to(want, got.shape), rtol=2.0 ** -9)
+
+
 @pytest.mark.parametrize("D,qlen", SHAPES)
 def test_values_of_scale_zero_and_of_very_different_scales(D, qlen):
     c = orc.make_paged_cache([500], 2, D, 16, seed=14)
