@@ -1,12 +1,12 @@
 // Paged-copy ceiling: a kernel that fetches exactly the cache bytes the integer attention
-// kernel fetches, in the same way, and throws them away.
+// kernel fetches, page copy by page copy, and throws them away.
 //
 // It is the measuring stick for the attention kernel's memory side (the counterpart of the
 // reference's copy-ceiling program, bench/sol_copy.cu:424-512, whose ratio eta_mem = T_copy /
 // T_kernel the reference reports for its decode shapes): same persistent CTAs (one per SM),
 // same work-item schedule (sched.cuh), same TMA page copies (one [block_size slots] x
-// [272 bytes] box of the page tensor map, or one bulk copy of a contiguous page run) into
-// the same ring of three 34,816-byte raw stages in shared memory.  What is missing is
+// [272 bytes] box of the page tensor map, or one bulk copy of a contiguous page run; issued by
+// one warp, where the attention kernel has two) into a ring of three 34,816-byte raw stages in shared memory.  What is missing is
 // everything after the copy: a stage is handed back as soon as its bytes have landed.  The
 // time of this kernel on a launch is therefore the least the attention kernel could need
 // for that launch with this access pattern and this many bytes in flight.

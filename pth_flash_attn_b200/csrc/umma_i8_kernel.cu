@@ -800,7 +800,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     const int gw = warp & 3;           // warp inside the group = TMEM lane quadrant
     const uint32_t lane_addr = (uint32_t)(gw * 32) << 16;
     uint8_t* pimg_g = pimg + g * (PD * NPAD * kKeys);
-    float* wred_g = wred + g * (2 * 4 * WP);   // [2][4][NPAD + 1]
+    float* wred_g = wred + g * (2 * 4 * WP);   // [2][4][wred_row]
     float* mrun_g = mrun + g * (2 * NPAD);             // [2][NPAD]
     constexpr int NROW = 4 * RQ;  // rows this instance computes (live rows rounded up to four)
     constexpr int RL = (NPAD + 31) / 32;
@@ -1015,7 +1015,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
       // Every PV of the item has been folded by now, so the P images of both groups are idle:
       // group 1 parks its accumulator there ([row][d] fp32) for group 0 to pick up.
       named_barrier(4, kSoftmaxThreads);  // both groups have left their last tile
-      float* wsum = wred_g;  // [4][NPAD + 1]
+      float* wsum = wred_g;  // [4][wred_row]
       if (gw == 0) {
 #pragma unroll
         for (int jj = 0; jj < RL; ++jj)
