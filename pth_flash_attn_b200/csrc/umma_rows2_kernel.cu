@@ -60,8 +60,9 @@ constexpr int kXMmaWarp = 16, kXLoadWarp = 17;
 constexpr int kXThreads = 576;
 constexpr int kXQBarrier = kXSoftmax + 32;  // Q images complete: softmax, MMA issuer
 // Registers per thread, of the 96 the CTA starts with.  The softmax, which bounds the kernel by its instructions,
-// keeps more of a tile's scales in flight with 136 than with 120; a producer's words fit 56.  (4 x 2,048 tokens
-// over 14,336 keys at 64 dims: 2,052 us, with 128 registers 2,085.)
+// keeps more of a tile's scales in flight with 136 than with 120; a producer's words fit 56 but for a few.  (Against
+// 128 and 64: 4 x 2,048 tokens over 14,336 keys at 64 dims 2,052 us and 2,085; at 128 dims 4 x 2,048 over 30,720
+// 9,606 and 9,652, 2 x 1,000 new tokens 54.3 and 55.2, twelve prompts of 37 to 2,500 430 and 434.)
 constexpr int kXProducerRegs = 56, kXSoftmaxRegs = 136;
 constexpr int kXOCol = 256;                         // TMEM columns: S(rt, b) at (2 rt + b) 64, O(rt) at 256 + 128 rt
 constexpr float kXRescaleGap = 4.0f;                // log2 units a row maximum may outgrow its reference (P stays at or below 2^15)
