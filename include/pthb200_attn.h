@@ -324,6 +324,12 @@ int32_t pthb200_test_schedule(const int32_t* query_start_loc, const int32_t* seq
                               int32_t group, int32_t num_kv_heads, int32_t bq, int32_t num_splits,
                               int32_t window, int32_t causal, int32_t row_class, int32_t class_rows,
                               int32_t num_ctas, int32_t* out, int32_t max_items);
+/* The same for a launch that the kernel deals out in ranges of the sequence of all KV tiles
+ * (enough work, a large enough num_splits); returns 0 for a launch it would not. */
+int32_t pthb200_test_range_schedule(const int32_t* query_start_loc, const int32_t* seq_lens, int32_t num_reqs,
+                                    int32_t group, int32_t num_kv_heads, int32_t bq, int32_t num_splits,
+                                    int32_t window, int32_t causal, int32_t row_class, int32_t class_rows,
+                                    int32_t num_ctas, int32_t* out, int32_t max_items);
 /* Synchronises the device, returns and clears the status word in which a
  * kernel records a bounded wait that gave up (0 = none). */
 int32_t pthb200_device_status(int32_t* status);

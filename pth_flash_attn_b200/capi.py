@@ -158,6 +158,7 @@ EXPORTED_SYMBOLS = (
     "pthb200_check_call",
     "pthb200_launch_count",
     "pthb200_test_schedule",
+    "pthb200_test_range_schedule",
     "pthb200_test_tile",
     "pthb200_test_tile_i8",
     "pthb200_test_tile_rows",
@@ -213,9 +214,9 @@ class B200Lib:
         lib.pthb200_write_args_bytes.argtypes = []
         lib.pthb200_write_kv.restype = ctypes.c_int32
         lib.pthb200_write_kv.argtypes = [ctypes.POINTER(PthB200WriteArgs), ctypes.c_void_p]
-        lib.pthb200_test_schedule.restype = ctypes.c_int32
-        lib.pthb200_test_schedule.argtypes = ([ctypes.c_void_p] * 2 + [ctypes.c_int32] * 10
-                                              + [ctypes.c_void_p, ctypes.c_int32])
+        for fn in (lib.pthb200_test_schedule, lib.pthb200_test_range_schedule):
+            fn.restype = ctypes.c_int32
+            fn.argtypes = [ctypes.c_void_p] * 2 + [ctypes.c_int32] * 10 + [ctypes.c_void_p, ctypes.c_int32]
         lib.pthb200_test_tile.restype = ctypes.c_int32
         lib.pthb200_test_tile.argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_int32, ctypes.c_void_p]
         lib.pthb200_test_tile_i8.restype = ctypes.c_int32
@@ -282,11 +283,12 @@ class B200Lib:
 
     def schedule(self, query_start_loc, seq_lens, *, group: int, num_kv_heads: int, bq: int,
                  num_splits: int, num_ctas: int, window: int = 0, causal: bool = True,
-                 row_class: int = 0, class_rows: int = 0):
+                 row_class: int = 0, class_rows: int = 0, ranges: bool = False):
         """The persistent kernel's work-item schedule, computed on the host (no device access).
 
         Returns an int32 array ``[items, 8]`` of ``(cta, request, row tile, KV head, split,
         splits of the request, first KV tile, end KV tile)`` in the order the CTAs run them.
+        With ``ranges`` the one that deals the launch out in ranges: empty if it does not apply.
         """
         import numpy as np
 
@@ -294,12 +296,13 @@ class B200Lib:
         lens = np.ascontiguousarray(seq_lens, dtype=np.int32)
         args = (qsl.ctypes.data, lens.ctypes.data, len(lens), group, num_kv_heads, bq, num_splits, window,
                 int(causal), row_class, class_rows, num_ctas)
+        fn = self.lib.pthb200_test_range_schedule if ranges else self.lib.pthb200_test_schedule
         probe = np.zeros((1, 8), dtype=np.int32)
-        n = int(self.lib.pthb200_test_schedule(*args, probe.ctypes.data, 0))
+        n = int(fn(*args, probe.ctypes.data, 0))
         if n < 0:
             raise RuntimeError(self.last_error())
         out = np.zeros((max(n, 1), 8), dtype=np.int32)
-        self.lib.pthb200_test_schedule(*args, out.ctypes.data, n)
+        fn(*args, out.ctypes.data, n)
         return out[:n]
 
     def launch_count(self, args: PthAttnArgs) -> tuple[int, int]:

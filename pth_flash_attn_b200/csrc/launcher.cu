@@ -461,6 +461,72 @@ int32_t pthb200_test_schedule(const int32_t* query_start_loc, const int32_t* seq
   return count;
 }
 
+// The same for a launch that is dealt out in ranges (sched.cuh); 0 items if this one would not be.
+int32_t pthb200_test_range_schedule(const int32_t* query_start_loc, const int32_t* seq_lens, int32_t num_reqs,
+                                    int32_t group, int32_t num_kv_heads, int32_t bq, int32_t num_splits, int32_t window,
+                                    int32_t causal, int32_t row_class, int32_t class_rows, int32_t num_ctas, int32_t* out,
+                                    int32_t max_items) {
+  using namespace pthb200;
+  g_last_error.clear();
+  PTHB_REQUIRE(query_start_loc != nullptr && seq_lens != nullptr && out != nullptr, "NULL argument");
+  PTHB_REQUIRE(num_reqs >= 1 && group >= 1 && num_kv_heads >= 1 && bq >= 1 && num_splits >= 1 && num_ctas >= 1 &&
+                   max_items >= 0,
+               "counts must be >= 1");
+  SchedShape sh{group, num_kv_heads, bq, num_splits, window, causal, row_class, class_rows};
+  unsigned long long total = 0;
+  int longest = 0;
+  for (int r = 0; r < num_reqs; ++r) {
+    const int q_len = query_start_loc[r + 1] - query_start_loc[r];
+    const int rt = req_row_tiles(sh, q_len), tiles = req_kv_tiles(sh, q_len, seq_lens[r]);
+    total += (unsigned long long)rt * (unsigned long long)tiles;
+    if (rt > 0) longest = sched_max(longest, tiles > 0 ? tiles : 0x7fffffff);
+  }
+  const RangeSched ranges = range_sched(total, longest, num_kv_heads, num_ctas, num_splits);
+  if (ranges.work == 0) return 0;
+  int32_t count = 0;
+  for (int cta = 0; cta < num_ctas; ++cta) {
+    const int g = sched_min(cta / num_kv_heads, ranges.full);
+    const uint32_t lo = range_cut(ranges, g), hi = range_cut(ranges, g + 1);
+    for (int head = cta - g * num_kv_heads; head < num_kv_heads; head += g < ranges.full ? num_kv_heads : ranges.tail) {
+      uint32_t start = 0;
+      for (int r = 0; r < num_reqs; ++r) {
+        const int q_len = query_start_loc[r + 1] - query_start_loc[r];
+        const int rts = req_row_tiles(sh, q_len), n = req_kv_tiles(sh, q_len, seq_lens[r]);
+        for (int rt = 0; rt < rts; ++rt, start += (uint32_t)n) {
+          if (start + (uint32_t)n <= lo || start >= hi) continue;
+          int b, e;
+          if (!range_part(ranges, start, n, lo, hi, &b, &e)) continue;
+          int split = 0, splits = 1;
+          for (int k = 1; k < range_groups(ranges); ++k) {
+            const uint32_t cut = range_cut(ranges, k);
+            if (!range_divides(ranges, start, n, cut)) continue;
+            ++splits;
+            if (cut <= start + (uint32_t)b) ++split;
+          }
+          const int first_idx = rt * bq, ntok = sched_min(bq, q_len - first_idx);
+          int lo0, hi0, lo1, hi1;
+          visible_bounds(window, causal, seq_lens[r], q_len, first_idx, &lo0, &hi0);
+          visible_bounds(window, causal, seq_lens[r], q_len, first_idx + ntok - 1, &lo1, &hi1);
+          const int end = sched_max(hi0, hi1) + 1, t0 = lo0 / kKvTile, t1 = end > lo0 ? (end + kKvTile - 1) / kKvTile : t0;
+          if (count < max_items) {
+            int32_t* o = out + (int64_t)count * 8;
+            o[0] = cta;
+            o[1] = r;
+            o[2] = rt;
+            o[3] = head;
+            o[4] = split;
+            o[5] = splits;
+            o[6] = sched_min(t0 + b, t1);
+            o[7] = sched_min(t0 + e, t1);
+          }
+          ++count;
+        }
+      }
+    }
+  }
+  return count;
+}
+
 }  // extern "C"
 
 // ---- split attention without a caller workspace ---------------------------------

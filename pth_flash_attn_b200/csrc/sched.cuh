@@ -20,6 +20,16 @@
 //                 one page set) run at the same time on neighbouring CTAs, which lets the
 //                 boundary sectors of neighbouring 264-byte cells be served from L2.
 //
+// That schedule leaves CTAs idle in the last round (mean over longest CTA: 0.83 for a mixed batch of 48
+// decode requests, 0.87 for 64 requests of two KV heads, 0.5 - 0.8 for short ragged contexts).  A launch with enough
+// work whose caller allows enough pieces (range_sched) is dealt out in RANGES instead: the KV tiles of all
+// served row tiles form one sequence, which is cut into equal runs, one for every group of Hkv CTAs; CTA h of a group
+// reads KV head h, so the heads of a page are still read at the same time.  The CTAs left over when Hkv does not
+// divide their number form a last, smaller group, whose CTAs take several heads one after the other and whose run is
+// as much shorter.  A cut closer than `snap` tiles to an end of a row tile moves to that end.
+// Measured (equal pieces -> ranges): 32 requests x 4 tokens x 16 to 32 K keys 414 -> 383 us, decode at 64 dims over
+// 4 to 12 K keys 184 -> 170, 64 x 8,192 keys 212 -> 205, mixed batch 3,350 -> 3,120.
+//
 // Splits s >= S(r) of a request hold no keys: their log-sum-exp is set to -inf by the CTA
 // that runs split 0 of the same rows, and the combine skips them.
 //
@@ -85,21 +95,23 @@ PTHB_HD int req_kv_tiles(const SchedShape& s, int q_len, int seq_len) {
 
 // t*: KV tiles an item should hold, from the total work and the number of CTAs.
 PTHB_HD int item_tiles(unsigned long long total_tiles, int num_ctas) {
-  const unsigned long long ctas = num_ctas > 0 ? (unsigned long long)num_ctas : 1ull;
-  const unsigned long long per_cta = (total_tiles + ctas - 1) / ctas;
-  unsigned long long m = per_cta / kItemTilesTarget;
+  // (divisions of 64-bit numbers are slow, and the first item waits for them)
+  const unsigned ctas = num_ctas > 0 ? (unsigned)num_ctas : 1u;
+  const unsigned long long per = total_tiles < (1ull << 31) ? ((unsigned)total_tiles + ctas - 1) / ctas : (total_tiles + ctas - 1) / ctas;
+  const unsigned per_cta = per > (1ull << 31) ? 1u << 31 : (unsigned)per;  // (far more than a cache holds)
+  unsigned m = per_cta / kItemTilesTarget;
   if (m < 1) m = 1;
-  if (m > kItemsPerCtaMax) m = kItemsPerCtaMax;
-  unsigned long long t = (per_cta + m - 1) / m;
-  if (t < kItemTilesMin) t = kItemTilesMin;
-  if (t > (1ull << 30)) t = 1ull << 30;
+  if (m > (unsigned)kItemsPerCtaMax) m = kItemsPerCtaMax;
+  unsigned t = (per_cta + m - 1) / m;
+  if (t < (unsigned)kItemTilesMin) t = kItemTilesMin;
+  if (t > (1u << 30)) t = 1u << 30;
   return (int)t;
 }
 
 // S(r): splits of a request whose rows touch kv_tiles KV tiles.
 PTHB_HD int req_splits(int kv_tiles, int t_star, int num_splits) {
-  const int64_t s = ((int64_t)kv_tiles + t_star / 2) / t_star;
-  return s < 1 ? 1 : (s > num_splits ? num_splits : (int)s);
+  const unsigned s = ((unsigned)kv_tiles + (unsigned)t_star / 2) / (unsigned)t_star;
+  return s < 1 ? 1 : (s > (unsigned)num_splits ? num_splits : (int)s);
 }
 
 // Items of a request, and the coordinates of its item `local`.
@@ -130,6 +142,72 @@ PTHB_HD void split_tile_span(int range_begin, int range_end, int split, int spli
   const int64_t n = t1 - t0;
   *tile_begin = t0 + (int)((int64_t)split * n / splits);
   *tile_end = t0 + (int)((int64_t)(split + 1) * n / splits);
+}
+
+// ---- ranges ----
+// KV tiles per CTA from which a launch is dealt out in ranges.  Below, a CTA's share is a few short pieces, whose ends
+// cost more than the balance gives: 8 x 8,192 keys of 8 heads (27 tiles per CTA) 46.1 us in ranges, 45.1 in equal
+// pieces; 60 x U[1, 988] (14 tiles) 55.3 and 51.3; 64 x U[1, 4096] (60 tiles) 89.7 and 96.8.
+constexpr int kRangeTilesMin = 32;
+constexpr int kRangeGroupsMax = 160;   // groups a scheduler warp holds the cuts of
+
+struct RangeSched {
+  uint32_t work;         // KV tiles of one head; 0: the launch is not dealt out in ranges
+  int32_t full;          // groups of num_kv_heads CTAs
+  int32_t tail;          // CTAs of the last, smaller group (0: there is none)
+  int32_t tail_passes;   // heads each of its CTAs takes one after the other
+  int32_t snap;
+};
+
+// The run of a group of `tail_passes` times the tail group's length, or a rounding of it: the cut in front of group g
+// is at ceil(work * g * passes / (full * passes + 1)) (without a tail group: ceil(work * g / full)).
+PTHB_HD int range_groups(const RangeSched& r) { return r.full + (r.tail > 0 ? 1 : 0); }
+PTHB_HD uint32_t range_cut(const RangeSched& r, int g) {
+  const uint32_t per = r.tail > 0 ? (uint32_t)r.tail_passes : 1u, whole = (uint32_t)r.full * per + (r.tail > 0 ? 1u : 0u);
+  if (g >= range_groups(r)) return r.work;
+  const unsigned long long num = (unsigned long long)r.work * ((uint32_t)g * per) + (whole - 1);
+  if (num <= 0xffffffffull) return (uint32_t)num / whole;
+  return (uint32_t)(num / whole);
+}
+// work: KV tiles of one head over the row tiles of all served requests; longest: of one row tile at most.
+PTHB_HD RangeSched range_sched(unsigned long long work, int longest, int num_kv_heads, int num_ctas, int num_splits) {
+  RangeSched r;
+  r.work = 0;
+  r.full = r.tail = r.tail_passes = 0;
+  r.snap = 1;
+  if (num_splits < 2 || work > (1ull << 30) || work * (unsigned long long)num_kv_heads < (unsigned long long)num_ctas * kRangeTilesMin)
+    return r;
+  r.full = num_ctas / num_kv_heads;
+  r.tail = num_ctas % num_kv_heads;
+  r.tail_passes = r.tail > 0 ? (num_kv_heads + r.tail - 1) / r.tail : 0;
+  if (range_groups(r) > kRangeGroupsMax) return r;
+  const uint32_t per = r.tail > 0 ? (uint32_t)r.tail_passes : 1u, whole = (uint32_t)r.full * per + (r.tail > 0 ? 1u : 0u);
+  // the shortest distance of two cuts inside a row tile: a whole group's run
+  const unsigned long long run = work * per / whole;
+  if (r.full < 1 || run < 4) return r;
+  // a row tile of n tiles holds at most ceil((n - 1) / run) cuts, and one piece more than cuts
+  const unsigned long long cuts = longest > 1 ? ((unsigned long long)longest - 1 + run - 1) / run : 0;
+  if (cuts + 1 > (unsigned long long)num_splits) return r;
+  r.snap = run >= 32 ? 2 : 1;
+  r.work = (uint32_t)work;
+  return r;
+}
+// Part [*begin, *end) of a row tile that starts at `start` of the sequence and has n KV tiles which belongs to the
+// run [lo, hi) of a group; false if there is none.
+PTHB_HD bool range_part(const RangeSched& r, uint32_t start, int n, uint32_t lo, uint32_t hi, int* begin, int* end) {
+  int b = lo > start ? (int)(lo - start) : 0;
+  int e = hi - start < (uint32_t)n ? (int)(hi - start) : n;
+  if (b > 0 && b <= r.snap) b = 0;
+  else if (b > 0 && n - b <= r.snap) b = n;
+  if (e < n && e <= r.snap) e = 0;
+  else if (e < n && n - e <= r.snap) e = n;
+  *begin = b;
+  *end = e;
+  return b < e;
+}
+// Whether a cut of the sequence divides a row tile (rather than moving to one of its ends).
+PTHB_HD bool range_divides(const RangeSched& r, uint32_t start, int n, uint32_t cut) {
+  return cut > start + (uint32_t)r.snap && cut + (uint32_t)r.snap < start + (uint32_t)n;
 }
 
 }  // namespace pthb200

@@ -232,6 +232,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
   unsigned long long* total_s = reinterpret_cast<unsigned long long*>(smem + L::misc + 16);
+  int* longest_s = reinterpret_cast<int*>(smem + L::misc + 24);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   SchedShape shape;
@@ -248,12 +249,16 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   // (the loads of the total-work pass below are issued first: their latency hides behind the
   // barrier initialisation and the TMEM allocation)
   unsigned long long work = 0;
+  int longest = 0;
   bool served = false;
   for (int r = tid; r < p.num_reqs; r += kThreads) {
     const int q0 = __ldg(p.query_start_loc + r), q1 = __ldg(p.query_start_loc + r + 1);
     const int len = __ldg(p.seq_lens + r);
     const int row_tiles = req_row_tiles(shape, q1 - q0);
-    work += (unsigned long long)row_tiles * (unsigned long long)req_kv_tiles(shape, q1 - q0, len);
+    const int kv_tiles = req_kv_tiles(shape, q1 - q0, len);
+    work += (unsigned long long)row_tiles * (unsigned long long)kv_tiles;
+    // (a request without keys has a result but no tiles: such a launch is not dealt out in ranges)
+    if (row_tiles > 0) longest = max(longest, kv_tiles > 0 ? kv_tiles : 0x7fffffff);
     served |= row_tiles > 0;
   }
   // A prefill launch whose requests are all tall has nothing for this kernel: its CTAs leave before any set-up.
@@ -282,6 +287,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     }
     *abort_flag = 0;
     *total_s = 0ull;
+    *longest_s = 0;
     tc::mbar_init_fence();
   }
   if (warp == 0) {
@@ -294,14 +300,17 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     unsigned long long w = work;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-    if (lane == 0 && w != 0) atomicAdd(total_s, w);
+    const int n = __reduce_max_sync(0xffffffffu, longest);
+    if (lane == 0) {
+      if (w != 0) atomicAdd(total_s, w);
+      if (n != 0) atomicMax(longest_s, n);
+    }
   }
   tc::fence_before_sync();
   tc::fence_async_smem();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tslot;
-  const int t_star = item_tiles(*total_s * (unsigned long long)p.num_kv_heads, (int)gridDim.x);
   const uint32_t kstage0 = tc::smem_u32(smem + L::kstages), vstage0 = tc::smem_u32(smem + L::vstages);
   bool ok = true;
 
@@ -310,22 +319,27 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     // Walks the requests in blocks of 32 (lane l holds request base + l and the items of the
     // requests before it), so this CTA's items c, c + CTAs, ... are found in one pass.
     const int S = p.num_splits, hkv = p.num_kv_heads;
+    const RangeSched ranges = range_sched(*total_s, *longest_s, hkv, (int)gridDim.x, S);
+    const bool ranged = ranges.work != 0;
+    const int t_star = item_tiles(*total_s * (unsigned long long)hkv, (int)gridDim.x);
     int base = 0;
     long long blk_first = 0;
     int blk_total = 0;
-    int my_q0 = 0, my_qlen = 0, my_len = 0, my_splits = 1, my_n = 0, my_excl = 0;
+    int my_q0 = 0, my_qlen = 0, my_len = 0, my_splits = 1, my_n = 0, my_excl = 0, my_tiles = 0;
+    // (my_n: items of the request, or the KV tiles of its row tiles when the launch is dealt out in ranges)
     auto load_block = [&](int b) {
       const int r = b + lane;
       my_n = 0;
-      my_q0 = my_qlen = my_len = 0;
+      my_q0 = my_qlen = my_len = my_tiles = 0;
       my_splits = 1;
       if (r < p.num_reqs) {
         my_q0 = __ldg(p.query_start_loc + r);
         my_qlen = __ldg(p.query_start_loc + r + 1) - my_q0;
         my_len = __ldg(p.seq_lens + r);
         const int rt = req_row_tiles(shape, my_qlen);
-        my_splits = req_splits(req_kv_tiles(shape, my_qlen, my_len), t_star, S);
-        my_n = (int)req_items(rt, my_splits, hkv);
+        my_tiles = req_kv_tiles(shape, my_qlen, my_len);
+        my_splits = req_splits(my_tiles, t_star, S);
+        my_n = ranged ? rt * my_tiles : (int)req_items(rt, my_splits, hkv);
       }
       int v = my_n;
 #pragma unroll
@@ -337,26 +351,88 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
       blk_total = __shfl_sync(0xffffffffu, v, 31);
     };
     load_block(0);
+    // Ranges: this CTA's group and run of the sequence, the head it reads (one after the other in the last, smaller
+    // group), and the cuts of the sequence, lane l holding cuts l + 1, l + 33, ...
+    int group_of = 0, range_head = 0;
+    uint32_t run_lo = 0, run_hi = 0, at = 0, cuts[kRangeGroupsMax / 32];
+    if (ranged) {
+      group_of = min((int)blockIdx.x / hkv, ranges.full);
+      range_head = (int)blockIdx.x - group_of * hkv;
+      run_lo = range_cut(ranges, group_of);
+      run_hi = range_cut(ranges, group_of + 1);
+      at = run_lo;
+#pragma unroll
+      for (int k = 0; k < kRangeGroupsMax / 32; ++k) {
+        const int g = 32 * k + lane + 1;
+        cuts[k] = g < range_groups(ranges) ? range_cut(ranges, g) : 0x7fffffffu;  // (past every row tile, and no sum with it overflows)
+      }
+    }
     int pub = 0;  // items published so far
     for (long long idx = blockIdx.x;; idx += gridDim.x) {
-      bool done = false;
-      while (idx >= blk_first + blk_total) {
-        blk_first += blk_total;
-        base += 32;
-        if (base >= p.num_reqs) {
-          done = true;
-          break;
+      int req, q0, q_len, seq_len, splits;
+      ItemCoord c;
+      int part_begin = 0, part_end = 0;
+      if (!ranged) {
+        bool done = false;
+        while (idx >= blk_first + blk_total) {
+          blk_first += blk_total;
+          base += 32;
+          if (base >= p.num_reqs) {
+            done = true;
+            break;
+          }
+          load_block(base);
         }
-        load_block(base);
+        if (done) break;
+        const int rel = (int)(idx - blk_first);
+        const bool mine = rel >= my_excl && rel < my_excl + my_n;
+        const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+        req = base + src;
+        q0 = __shfl_sync(0xffffffffu, my_q0, src);
+        q_len = __shfl_sync(0xffffffffu, my_qlen, src);
+        seq_len = __shfl_sync(0xffffffffu, my_len, src);
+        splits = __shfl_sync(0xffffffffu, my_splits, src);
+        c = item_coord(rel - __shfl_sync(0xffffffffu, my_excl, src), hkv, splits);
+      } else {
+        bool found = false;
+        while (!found) {
+          if (at >= run_hi) {  // the next head of a CTA of the last group, from the start of its run
+            range_head += ranges.tail;
+            if (group_of < ranges.full || range_head >= hkv) break;
+            at = run_lo;
+            base = 0;
+            blk_first = 0;
+            load_block(0);
+          }
+          while (at >= blk_first + blk_total) {  // (the sequence does not end before run_hi)
+            blk_first += blk_total;
+            base += 32;
+            load_block(base);
+          }
+          const int rel = (int)(at - blk_first);
+          const bool mine = rel >= my_excl && rel < my_excl + my_n;
+          const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+          req = base + src;
+          q0 = __shfl_sync(0xffffffffu, my_q0, src);
+          q_len = __shfl_sync(0xffffffffu, my_qlen, src);
+          seq_len = __shfl_sync(0xffffffffu, my_len, src);
+          const int tiles = __shfl_sync(0xffffffffu, my_tiles, src), req_rel = rel - __shfl_sync(0xffffffffu, my_excl, src);
+          c.row_tile = req_rel / tiles;
+          c.kvh = range_head;
+          const uint32_t start = at - (uint32_t)(req_rel - c.row_tile * tiles);
+          found = range_part(ranges, start, tiles, run_lo, run_hi, &part_begin, &part_end);
+          c.split = 0;
+          splits = 1;
+#pragma unroll
+          for (int k = 0; k < kRangeGroupsMax / 32; ++k) {
+            const bool divides = range_divides(ranges, start, tiles, cuts[k]);
+            splits += __popc(__ballot_sync(0xffffffffu, divides));
+            c.split += __popc(__ballot_sync(0xffffffffu, divides && cuts[k] <= start + (uint32_t)part_begin));
+          }
+          at = start + (uint32_t)tiles;
+        }
+        if (!found) break;
       }
-      if (done) break;
-      const int rel = (int)(idx - blk_first);
-      const bool mine = rel >= my_excl && rel < my_excl + my_n;
-      const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
-      const int req = base + src;
-      const int q0 = __shfl_sync(0xffffffffu, my_q0, src), q_len = __shfl_sync(0xffffffffu, my_qlen, src);
-      const int seq_len = __shfl_sync(0xffffffffu, my_len, src), splits = __shfl_sync(0xffffffffu, my_splits, src);
-      const ItemCoord c = item_coord(rel - __shfl_sync(0xffffffffu, my_excl, src), hkv, splits);
       const int first_idx = c.row_tile * p.bq;
       const int ntok = min(p.bq, q_len - first_idx), tok0 = q0 + first_idx;
       const int rows = ntok * p.group;
@@ -365,7 +441,14 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
       visible_bounds(p.window, p.causal, seq_len, q_len, first_idx + ntok - 1, &lo_last, &hi_last);
       const int range_begin = lo_first, range_end = max(hi_first, hi_last) + 1;  // lo and hi grow with the token
       int tile_begin, tile_end;
-      split_tile_span(range_begin, range_end, c.split, splits, &tile_begin, &tile_end);
+      if (ranged) {
+        // (a row tile of several may touch fewer tiles than the request's rows together)
+        const int t0 = range_begin / kKeys, t1 = range_end > range_begin ? (range_end + kKeys - 1) / kKeys : t0;
+        tile_begin = min(t0 + part_begin, t1);
+        tile_end = min(t0 + part_end, t1);
+      } else {
+        split_tile_span(range_begin, range_end, c.split, splits, &tile_begin, &tile_end);
+      }
       auto lse_slot = [&](int s, int n) -> float* {
         const int token = tok0 + n / p.group, head = c.kvh * p.group + n % p.group;
         return reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)s * p.ws_lse_stride_split +
