@@ -62,6 +62,8 @@
 // CTA still finishes and frees its TMEM.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "params.cuh"
 #include "sched.cuh"
 #include "umma_i8.cuh"
@@ -76,6 +78,10 @@ namespace {
 constexpr int kGroupThreads = 128;                      // one softmax warpgroup
 constexpr int kSoftmaxThreads = 2 * kGroupThreads;      // warps 0-3 and 4-7
 constexpr int kProducerThreads = 128;                   // one producer group: one thread per key of a tile
+// Registers per thread of the instances with one producer group up to 128 dims, which start with 128: the softmax loops of 8 and more
+// rows want more, and the others need at least this.  (48 decode requests of 4 to 128 K keys at 8 rows: 1,455 us with
+// 144 / 112, 1,300 with 152 / 104, 1,515 with 160 / 96, whose producers spill.)
+constexpr int kSoftmaxRegs = 152, kProducerRegs = 104, kOtherRegs = 104;
 constexpr int kItemSlots = 2;                           // item descriptors (and Q images) in flight
 // Warps after the softmax groups: NP producer groups of four warps, then the MMA issuer,
 // two loaders and the scheduler.
@@ -112,14 +118,15 @@ struct Layout {
   static constexpr int raw = (pimg + pimg_bytes + 127) / 128 * 128; // [NR] raw units (TMA destinations: 128-byte aligned)
   static constexpr int wred_row = NPAD + 4;                         // a warp's maxima (or sums) of the rows, then of v_scale
   static constexpr int wred = raw + NR * unit_bytes;                // float [2 groups][2][4][wred_row]
-  static constexpr int mrun = wred + 2 * 2 * 4 * wred_row * 4;      // float [2 groups][2 NPAD], first NPAD used
-  static constexpr int sq = mrun + 2 * 2 * NPAD * 4;                // float [slots][NPAD]
+  static constexpr int mrun = wred + 2 * 2 * 4 * wred_row * 4;      // float [2 groups][NPAD]
+  static constexpr int sq = mrun + 2 * NPAD * 4;                    // float [slots][NPAD]
   static constexpr int rlo = sq + kItemSlots * NPAD * 4;            // int [slots][NPAD]
   static constexpr int rhi = rlo + kItemSlots * NPAD * 4;           // int [slots][NPAD]
   // row factors of the latest tile, for the warps to fetch four rows at a time: float [8 warps][4][rows]
   static constexpr int factor_rows = NPAD <= 32 ? 4 * RQ : 0;
   static constexpr int factors = rhi + kItemSlots * NPAD * 4;
-  static constexpr int desc = (factors + 8 * 4 * factor_rows * 4 + 15) / 16 * 16;  // ItemDesc [slots]
+  static constexpr int rowid = (factors + 8 * 4 * factor_rows * 4 + 15) / 16 * 16;   // uint16 [slots][NPAD], see the scheduler
+  static constexpr int desc = rowid + kItemSlots * 2 * NPAD;                         // ItemDesc [slots]
   static constexpr int bars = desc + kItemSlots * (int)sizeof(ItemDesc);
   static constexpr int n_bars = 2 * NS + 14 + 2 * NR + 2 * kItemSlots;
   static constexpr int misc = bars + n_bars * 8;                    // abort flag, TMEM slot, total work
@@ -314,6 +321,12 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   const uint32_t kstage0 = tc::smem_u32(smem + L::kstages), vstage0 = tc::smem_u32(smem + L::vstages);
   bool ok = true;
 
+  // (setmaxnreg is for whole warpgroups: the issuer, the loaders and the scheduler are one)
+  if constexpr (NP == 1 && HD < 256) {  // (256 dims: 125.6 us without, 128.1 with)
+    if (warp < 8) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+    else if (warp < kMmaWarp) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kProducerRegs));
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+  }
   if (warp == kSchedWarp) {
     // =========================== scheduler ====================================
     // Walks the requests in blocks of 32 (lane l holds request base + l and the items of the
@@ -506,9 +519,16 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         int* rlo = reinterpret_cast<int*>(smem + L::rlo) + slot * NPAD;
         int* rhi = reinterpret_cast<int*>(smem + L::rhi) + slot * NPAD;
         uint8_t* qimg = smem + L::qimg + slot * L::qimg_bytes;
+        // Token of the tile (low byte) and head of the group of every row.  (Worked out here, ahead of time: the threads
+        // that write an item's rows took thousands of cycles for the divisions.)
+        uint16_t* rowid = reinterpret_cast<uint16_t*>(smem + L::rowid) + slot * NPAD;
         for (int n = lane; n < NPAD; n += 32) {
           int lo = 0, hi = -1;
-          if (n < rows) visible_bounds(p.window, p.causal, seq_len, q_len, first_idx + n / p.group, &lo, &hi);
+          if (n < rows) {
+            const int tok = n / p.group;
+            visible_bounds(p.window, p.causal, seq_len, q_len, first_idx + tok, &lo, &hi);
+            rowid[n] = (uint16_t)(tok | (n - tok * p.group) << 8);
+          }
           rlo[n] = lo;
           rhi[n] = hi;
         }
@@ -884,10 +904,10 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     const uint32_t lane_addr = (uint32_t)(gw * 32) << 16;
     uint8_t* pimg_g = pimg + g * (PD * NPAD * kKeys);
     float* wred_g = wred + g * (2 * 4 * WP);   // [2][4][wred_row]
-    float* mrun_g = mrun + g * (2 * NPAD);             // [2][NPAD]
-    constexpr int NROW = 4 * RQ;  // rows this instance computes (live rows rounded up to four)
+    float* mrun_g = mrun + g * NPAD;
     constexpr int RL = (NPAD + 31) / 32;
     const int my_key = tile_key(p, gt);
+    const bool S1 = p.num_splits == 1;
 
     int g0 = 0, item = 0;
     ok &= wait_or_abort(&bars[B::item_full + 0], 0, abort_flag);
@@ -896,16 +916,20 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     while (!stop) {
       const int slot = item % kItemSlots;
       const int n_tiles = descs[slot].n_tiles, tile_begin = descs[slot].tile_begin;
-      const int kvh = descs[slot].kvh, split = descs[slot].split, tok0 = descs[slot].tok0;
-      const int rows = descs[slot].ntok * p.group;  // <= NROW by construction of bq
+      const int split = descs[slot].split, tok0 = descs[slot].tok0, head0 = descs[slot].kvh * p.group;
+      const int rows = descs[slot].ntok * p.group;  // <= 4 RQ by construction of bq
       const int mask_lo = descs[slot].mask_lo, mask_hi = descs[slot].mask_hi;
       const float* sq = reinterpret_cast<const float*>(smem + L::sq) + slot * NPAD;
       const int* rlo = reinterpret_cast<const int*>(smem + L::rlo) + slot * NPAD;
       const int* rhi = reinterpret_cast<const int*>(smem + L::rhi) + slot * NPAD;
 
-      float acc[kHalves][NROW], l_part[NROW];  // thread t accumulates output columns t (and t + 128)
+      // (One instance per number of row groups: a launch whose row tiles may hold 16 rows also serves decode requests of
+      // 4 or 8: with 8 rows of 12 requests x 4 to 128 K keys computed as 16, 351 us; as 8, 295.)
+      auto run_item = [&](auto row_groups) {
+      constexpr int RQI = decltype(row_groups)::value, NROWI = 4 * RQI;
+      float acc[kHalves][NROWI], l_part[NROWI];  // thread t accumulates output columns t (and t + 128)
 #pragma unroll
-      for (int n = 0; n < NROW; ++n) {
+      for (int n = 0; n < NROWI; ++n) {
 #pragma unroll
         for (int h = 0; h < kHalves; ++h) acc[h][n] = 0.f;
         l_part[n] = 0.f;
@@ -940,11 +964,11 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         ok &= wait_or_abort(&bars[B::o_ready + g], (q >> 1) & 1, abort_flag);
         tc::fence_after_sync();
         const uint32_t o_tmem = tmem_base + L::s_total + g * L::o_cols + lane_addr;
-        constexpr int FB = RQ < 2 ? RQ : 2;  // eight rows per round trip to TMEM
+        constexpr int FB = RQI < 2 ? RQI : 2;  // eight rows per round trip to TMEM
 #pragma unroll
         for (int h = 0; h < kHalves; ++h) {
 #pragma unroll
-          for (int qb = 0; qb < RQ; qb += FB) {
+          for (int qb = 0; qb < RQI; qb += FB) {
             uint32_t d[FB][PD][4];
 #pragma unroll
             for (int c = 0; c < FB; ++c)
@@ -989,11 +1013,11 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         const int pos = (tile_begin + j) * kKeys + my_key;
         const bool interior = (tile_begin + j) * kKeys >= mask_lo && (tile_begin + j) * kKeys + (kKeys - 1) <= mask_hi;
         const float mult = ks_cur * p.scale_log2;
-        float s[NROW];
+        float s[NROWI];
         // up to sixteen rows per round trip to TMEM (one wait for the batch)
-        constexpr int QB = RQ < 4 ? RQ : 4;
+        constexpr int QB = RQI < 4 ? RQI : 4;
 #pragma unroll
-        for (int qb = 0; qb < RQ; qb += QB) {
+        for (int qb = 0; qb < RQI; qb += QB) {
           uint32_t hi[QB][4], lo[QB][4];
 #pragma unroll
           for (int c = 0; c < QB; ++c) {
@@ -1059,14 +1083,14 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         __syncwarp();
 #pragma unroll
         for (int q16 = 0; q16 < NPAD / 16; ++q16) {
-          if (q16 * 4 < RQ) {
+          if (q16 * 4 < RQI) {
             uint32_t dig[PD][4] = {};
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
               // Whole groups of four rows, padded rows included (their scores are finite
               // and their columns of O^T are never read): no branch per row, so the four
               // dependency chains overlap.
-              if (q16 * 4 + q4 < RQ) {
+              if (q16 * 4 + q4 < RQI) {
                 const int n0 = q16 * 16 + q4 * 4;
                 const float4 m4 = factor4(kMax, muse_l, n0), a4 = factor4(kAlpha, a_l, n0), u4 = factor4(kInvUnit, invu_l, n0);
                 const float m_use[4] = {m4.x, m4.y, m4.z, m4.w}, alpha[4] = {a4.x, a4.y, a4.z, a4.w};
@@ -1104,68 +1128,96 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         for (int jj = 0; jj < RL; ++jj)
           if (lane + 32 * jj < NPAD) mrun_g[lane + 32 * jj] = m_run[jj];
       }
+      // Sums of four rows over a warp in six shuffles: halves of the lanes go on with two rows each, quarters with one.
 #pragma unroll
-      for (int n = 0; n < NROW; ++n) {
-        if (n < rows) {
-          float v = l_part[n];
+      for (int qb = 0; qb < RQI; ++qb) {
+        if (4 * qb < rows) {
+          const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
+          const float* lp = l_part + 4 * qb;
+          const float a0 = (up16 ? lp[2] : lp[0]) + __shfl_xor_sync(0xffffffffu, up16 ? lp[0] : lp[2], 16);
+          const float a1 = (up16 ? lp[3] : lp[1]) + __shfl_xor_sync(0xffffffffu, up16 ? lp[1] : lp[3], 16);
+          float v = (up8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up8 ? a0 : a1, 8);
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == (n & 31)) wsum[gw * WP + n] = v;
+          for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if ((lane & 7) == 0) wsum[gw * WP + 4 * qb + (up16 ? 2 : 0) + (up8 ? 1 : 0)] = v;
         }
       }
-      // The P images hold 128 dims of a parked accumulator ([row][128] fp32): a head of 256 dims
-      // goes through them in two rounds.
+      // The even rows are finished and written by group 0, the odd ones by group 1; each parks its accumulator of the
+      // other's rows.  The P images hold 128 dims of it ([row][128] fp32): a head of 256 dims goes through them in
+      // two rounds.  What a row needs comes out of one lane (the factors of the two accumulators) and from the
+      // scheduler: the end of an item is not overlapped with anything.  (All rows by one group, each thread
+      // working out every row's factors, token and head: 4,200 cycles at 4 rows, 8,000 to 12,000 at 8.)
       float* park = reinterpret_cast<float*>(pimg);
+      const uint16_t* rowid = reinterpret_cast<const uint16_t*>(smem + L::rowid) + slot * NPAD;
+      uint8_t* const o_item = S1 ? p.out + (int64_t)tok0 * p.out_stride_token + (int64_t)head0 * p.out_stride_head
+                                 : reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
+                                       (int64_t)tok0 * p.ws_o_stride_token + (int64_t)head0 * p.ws_o_stride_head;
+      const int64_t o_token = S1 ? p.out_stride_token : p.ws_o_stride_token, o_head = S1 ? p.out_stride_head : p.ws_o_stride_head;
+      float f0[RL], f1[RL];
 #pragma unroll
       for (int h = 0; h < kHalves; ++h) {
         if (h > 0) named_barrier(4, kSoftmaxThreads);  // the previous round's parked values have been read
-        if (g == 1) {
 #pragma unroll
-          for (int n = 0; n < NROW; ++n)
-            if (n < rows) park[n * kKeys + gt] = acc[h][n];
+        for (int n2 = 0; n2 < NROWI / 2; ++n2) {
+          const int n = 2 * n2 + (g ^ 1);
+          if (n < rows) park[n * kKeys + gt] = g ? acc[h][2 * n2] : acc[h][2 * n2 + 1];
         }
-        named_barrier(4, kSoftmaxThreads);  // sums, maxima and the parked accumulator visible
+        named_barrier(4, kSoftmaxThreads);  // sums, maxima and the parked accumulators visible
         const int d = h * kKeys + gt;       // output column of this thread in this round
-        if (g == 0) {
+        if (h == 0) {
           const float* w0 = wred;
           const float* w1 = wred + 2 * 4 * WP;
-          const float* m0p = mrun;             // running maxima published by the two groups
-          const float* m1p = mrun + 2 * NPAD;
 #pragma unroll
-          for (int n = 0; n < NROW; ++n) {
-            if (n < rows) {
-              const float l0 = w0[n] + w0[WP + n] + w0[2 * WP + n] + w0[3 * WP + n];
-              const float l1 = w1[n] + w1[WP + n] + w1[2 * WP + n] + w1[3 * WP + n];
-              const float m0 = m0p[n], m1 = m1p[n];
+          for (int jj = 0; jj < RL; ++jj) {
+            const int r = lane + 32 * jj;
+            f0[jj] = f1[jj] = 0.f;
+            if (r < rows) {
+              const float l0 = w0[r] + w0[WP + r] + w0[2 * WP + r] + w0[3 * WP + r];
+              const float l1 = w1[r] + w1[WP + r] + w1[2 * WP + r] + w1[3 * WP + r];
+              const float m0 = mrun[r], m1 = mrun[NPAD + r];  // running maxima published by the two groups
               const float m = fmaxf(m0, m1);
               const float c0 = m0 == -INFINITY ? 0.f : fast_exp2(m0 - m);
               const float c1 = m1 == -INFINITY ? 0.f : fast_exp2(m1 - m);
               const float l = l0 * c0 + l1 * c1;
-              const float o = acc[h][n] * c0 + (c1 > 0.f ? park[n * kKeys + gt] * c1 : 0.f);
-              const float val = l > 0.f ? o / l : 0.f;
-              const int token = tok0 + n / p.group, head = kvh * p.group + n % p.group;
-              if (d < HD) {  // (a head of 64 dims uses half of the group's threads)
-                if (p.num_splits == 1) {
-                  store_out_elem(p.out + (int64_t)token * p.out_stride_token + (int64_t)head * p.out_stride_head, d,
-                                 p.out_dtype, val);
-                } else {
-                  reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
-                                           (int64_t)token * p.ws_o_stride_token + (int64_t)head * p.ws_o_stride_head)[d] = val;
-                }
-              }
-              if (h == 0 && gt == n) {
+              const float inv = l > 0.f ? 1.0f / l : 0.f;
+              f0[jj] = c0 * inv;
+              f1[jj] = c1 * inv;
+              if (warp == 0) {
                 const float lse2 = l > 0.f ? m + log2f(l) : -INFINITY;
-                if (p.num_splits > 1) {
-                  *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
-                                            (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = lse2;
+                const int64_t token = tok0 + (rowid[r] & 255), head = head0 + (rowid[r] >> 8);
+                if (!S1) {
+                  *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + split * p.ws_lse_stride_split +
+                                            token * p.ws_lse_stride_token + head * p.ws_lse_stride_head) = lse2;
                 } else if (p.lse_out != nullptr) {
-                  *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) + (int64_t)token * p.lse_stride_token +
-                                            (int64_t)head * p.lse_stride_head) = lse2 * kLn2;
+                  *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) + token * p.lse_stride_token +
+                                            head * p.lse_stride_head) = lse2 * kLn2;
                 }
               }
             }
           }
         }
+#pragma unroll
+        for (int n2 = 0; n2 < NROWI / 2; ++n2) {
+          const int n = 2 * n2 + g;
+          const float x0 = __shfl_sync(0xffffffffu, f0[(2 * n2) >> 5], n & 31), x1 = __shfl_sync(0xffffffffu, f1[(2 * n2) >> 5], n & 31);
+          if (n < rows && d < HD) {  // (a head of 64 dims uses half of the group's threads)
+            const float mine = g ? acc[h][2 * n2 + 1] : acc[h][2 * n2], other = park[n * kKeys + gt];
+            const float a0 = g ? other : mine, a1 = g ? mine : other;
+            const float val = fmaf(a0, x0, x1 > 0.f ? a1 * x1 : 0.f);
+            const uint32_t id = rowid[n];
+            uint8_t* const row = o_item + (int64_t)(id & 255u) * o_token + (int64_t)(id >> 8) * o_head;
+            if (!S1) reinterpret_cast<float*>(row)[d] = val;
+            else store_out_elem(row, d, p.out_dtype, val);
+          }
+        }
+      }
+      };
+      if constexpr (RQ == 4) {
+        if (rows <= 4) run_item(std::integral_constant<int, 1>{});
+        else if (rows <= 8) run_item(std::integral_constant<int, 2>{});
+        else run_item(std::integral_constant<int, 4>{});
+      } else {
+        run_item(std::integral_constant<int, RQ>{});
       }
       // ---- next item: the slot is released, and the barrier that protects the buffers of the
       // merge also makes "no more items" one decision of all 256 threads ----
