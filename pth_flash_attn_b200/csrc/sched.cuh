@@ -139,9 +139,14 @@ PTHB_HD void split_tile_span(int range_begin, int range_end, int split, int spli
   }
   const int t0 = range_begin / kKvTile;
   const int t1 = (range_end + kKvTile - 1) / kKvTile;
-  const int64_t n = t1 - t0;
-  *tile_begin = t0 + (int)((int64_t)split * n / splits);
-  *tile_end = t0 + (int)((int64_t)(split + 1) * n / splits);
+  const int n = t1 - t0;
+  if (n < (1 << 15) && split < (1 << 16)) {  // (the products fit 32 bits, whose divisions are much faster)
+    *tile_begin = t0 + (int)((uint32_t)split * (uint32_t)n / (uint32_t)splits);
+    *tile_end = t0 + (int)((uint32_t)(split + 1) * (uint32_t)n / (uint32_t)splits);
+  } else {
+    *tile_begin = t0 + (int)((int64_t)split * n / splits);
+    *tile_end = t0 + (int)((int64_t)(split + 1) * n / splits);
+  }
 }
 
 // ---- ranges ----

@@ -128,7 +128,7 @@ struct Layout {
   static constexpr int rowid = (factors + 8 * 4 * factor_rows * 4 + 15) / 16 * 16;   // uint16 [slots][NPAD], see the scheduler
   static constexpr int desc = rowid + kItemSlots * 2 * NPAD;                         // ItemDesc [slots]
   static constexpr int bars = desc + kItemSlots * (int)sizeof(ItemDesc);
-  static constexpr int n_bars = 2 * NS + 14 + 2 * NR + 2 * kItemSlots;
+  static constexpr int n_bars = 2 * NS + 14 + 2 * NR + 3 * kItemSlots;
   static constexpr int misc = bars + n_bars * 8;                    // abort flag, TMEM slot, total work
   static constexpr int total = misc + 32;
   static constexpr int s_cols = 2 * NPAD;
@@ -157,8 +157,9 @@ struct Bars {
   static constexpr int p_ready = 2 * NS + 12; // [2] softmax -> MMA, 128 arrivals
   static constexpr int raw_full = 2 * NS + 14;// [NR] page copies -> producers
   static constexpr int raw_free = 2 * NS + 14 + NR;  // [NR] producers -> loader, 128 arrivals
-  static constexpr int item_full = 2 * NS + 14 + 2 * NR;               // [slots] scheduler -> every other role
+  static constexpr int item_full = 2 * NS + 14 + 2 * NR;               // [slots] scheduler -> issuer, softmax: descriptor and queries
   static constexpr int item_empty = 2 * NS + 14 + 2 * NR + kItemSlots; // [slots] every other role -> scheduler
+  static constexpr int item_desc = 2 * NS + 14 + 2 * NR + 2 * kItemSlots;  // [slots] scheduler -> loaders, producers: descriptor
 };
 
 // Key of a tile held by row `r` of its operand images (see the producers).
@@ -238,8 +239,10 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   volatile ItemDesc* descs = reinterpret_cast<volatile ItemDesc*>(smem + L::desc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
-  unsigned long long* total_s = reinterpret_cast<unsigned long long*>(smem + L::misc + 16);
-  int* longest_s = reinterpret_cast<int*>(smem + L::misc + 24);
+  // (each warp's part of the launch's work and its longest row tile, in the softmax's scratch until the roles begin)
+  unsigned long long* work_s = reinterpret_cast<unsigned long long*>(smem + L::wred);
+  int* longest_s = reinterpret_cast<int*>(smem + L::wred + 8 * 32);
+  static_assert(2 * 2 * 4 * L::wred_row * 4 >= 12 * 32, "room for the parts of every warp");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   SchedShape shape;
@@ -253,8 +256,18 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   shape.class_rows = p.class_rows;
 
   // ---- set-up by all threads -------------------------------------------------
-  // (the loads of the total-work pass below are issued first: their latency hides behind the
-  // barrier initialisation and the TMEM allocation)
+  // The first copies wait for all of this, so it is one pass: the warps that hold requests load them while others
+  // initialise the barriers and allocate TMEM, and there is one barrier of the CTA.  (With a second one behind an
+  // atomic sum, and the copies waiting for the queries' digits, the first copy of a launch of 8 x U[1, 4096] keys left
+  // 14,000 cycles after the kernel's start; now @@.)
+  if (warp == kLoadWarp && lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
+  // (the scheduler's first 32 requests)
+  int pre_q0 = 0, pre_q1 = 0, pre_len = 0;
+  if (warp == kSchedWarp && lane < p.num_reqs) {
+    pre_q0 = __ldg(p.query_start_loc + lane);
+    pre_q1 = __ldg(p.query_start_loc + lane + 1);
+    pre_len = __ldg(p.seq_lens + lane);
+  }
   unsigned long long work = 0;
   int longest = 0;
   bool served = false;
@@ -270,7 +283,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   }
   // A prefill launch whose requests are all tall has nothing for this kernel: its CTAs leave before any set-up.
   if (p.row_class == 1 && !__syncthreads_or(served)) return;
-  if (tid == 0) {
+  if (warp == kMmaWarp && lane == 0) {
     for (int s = 0; s < NS; ++s) {
       tc::mbar_init(&bars[B::full + s], kProducerThreads);
       tc::mbar_init(&bars[B::empty + s], 1);
@@ -290,27 +303,24 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     }
     for (int s = 0; s < kItemSlots; ++s) {
       tc::mbar_init(&bars[B::item_full + s], 32);
+      tc::mbar_init(&bars[B::item_desc + s], 1);
       tc::mbar_init(&bars[B::item_empty + s], kItemReaders);
     }
     *abort_flag = 0;
-    *total_s = 0ull;
-    *longest_s = 0;
     tc::mbar_init_fence();
   }
-  if (warp == 0) {
+  if (warp == kLoadWarp + 1) {
     tc::tmem_alloc(tslot, L::tmem_alloc);
     tc::tmem_relinquish();
   }
-  __syncthreads();
   {
-    // total work of the launch in KV tiles (every CTA computes the same number)
     unsigned long long w = work;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
     const int n = __reduce_max_sync(0xffffffffu, longest);
     if (lane == 0) {
-      if (w != 0) atomicAdd(total_s, w);
-      if (n != 0) atomicMax(longest_s, n);
+      work_s[warp] = w;
+      longest_s[warp] = n;
     }
   }
   tc::fence_before_sync();
@@ -332,9 +342,13 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     // Walks the requests in blocks of 32 (lane l holds request base + l and the items of the
     // requests before it), so this CTA's items c, c + CTAs, ... are found in one pass.
     const int S = p.num_splits, hkv = p.num_kv_heads;
-    const RangeSched ranges = range_sched(*total_s, *longest_s, hkv, (int)gridDim.x, S);
+    unsigned long long total = lane < kThreads / 32 ? work_s[lane] : 0ull;  // (every CTA computes the same number)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    const int row_tile_max = __reduce_max_sync(0xffffffffu, lane < kThreads / 32 ? longest_s[lane] : 0);
+    const RangeSched ranges = range_sched(total, row_tile_max, hkv, (int)gridDim.x, S);
     const bool ranged = ranges.work != 0;
-    const int t_star = item_tiles(*total_s * (unsigned long long)hkv, (int)gridDim.x);
+    const int t_star = ranged ? 1 : item_tiles(total * (unsigned long long)hkv, (int)gridDim.x);
     int base = 0;
     long long blk_first = 0;
     int blk_total = 0;
@@ -346,9 +360,9 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
       my_q0 = my_qlen = my_len = my_tiles = 0;
       my_splits = 1;
       if (r < p.num_reqs) {
-        my_q0 = __ldg(p.query_start_loc + r);
-        my_qlen = __ldg(p.query_start_loc + r + 1) - my_q0;
-        my_len = __ldg(p.seq_lens + r);
+        my_q0 = b == 0 ? pre_q0 : __ldg(p.query_start_loc + r);
+        my_qlen = (b == 0 ? pre_q1 : __ldg(p.query_start_loc + r + 1)) - my_q0;
+        my_len = b == 0 ? pre_len : __ldg(p.seq_lens + r);
         const int rt = req_row_tiles(shape, my_qlen);
         my_tiles = req_kv_tiles(shape, my_qlen, my_len);
         my_splits = req_splits(my_tiles, t_star, S);
@@ -513,36 +527,61 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         d->range_end = range_end;
         d->mask_lo = lo_last;
         d->mask_hi = hi_first;
+        mbar_arrive(&bars[B::item_desc + slot]);  // the copies of the item's first tiles can leave
       }
       {
+        // Q digits: HD / 16 lanes per row, 16 elements each (32 / (HD / 16) rows per pass); the loads of up to four
+        // passes first.  Rows past the live ones of the last pass are left as they are: whole numbers whose scores
+        // are multiplied by a row scale of zero, in rows that nothing reads.
+        constexpr int kQLanes = G::chunks, kQRows = 32 / kQLanes;
+        constexpr int kAllPasses = (4 * RQ + kQRows - 1) / kQRows, kPasses = kAllPasses < 4 ? kAllPasses : 4;
         float* sq = reinterpret_cast<float*>(smem + L::sq) + slot * NPAD;
         int* rlo = reinterpret_cast<int*>(smem + L::rlo) + slot * NPAD;
         int* rhi = reinterpret_cast<int*>(smem + L::rhi) + slot * NPAD;
+        uint16_t* rowid = reinterpret_cast<uint16_t*>(smem + L::rowid) + slot * NPAD;
         uint8_t* qimg = smem + L::qimg + slot * L::qimg_bytes;
+        const float inv_group = 1.0f / (float)p.group;
+        const int part = lane % kQLanes;
+        // token of the tile that row n (below 64) belongs to: n + 1/2 keeps a distance of 1 / 128 from every multiple
+        auto token_of = [&](int n) { return (int)(((float)n + 0.5f) * inv_group); };
+        uint4 qa[kPasses], qb[kPasses];
+        auto load_rows = [&](int nb) {
+#pragma unroll
+          for (int k = 0; k < kPasses; ++k) {
+            const int n = nb + k * kQRows + lane / kQLanes;
+            qa[k] = qb[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (n < rows) {
+              const int tok = token_of(n);
+              const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)(tok0 + tok) * p.q_stride_token +
+                                                                (int64_t)(c.kvh * p.group + (n - tok * p.group)) * p.q_stride_head + part * 32);
+              qa[k] = __ldg(src);
+              qb[k] = __ldg(src + 1);
+            }
+          }
+        };
+        load_rows(0);
         // Token of the tile (low byte) and head of the group of every row.  (Worked out here, ahead of time: the threads
         // that write an item's rows took thousands of cycles for the divisions.)
-        uint16_t* rowid = reinterpret_cast<uint16_t*>(smem + L::rowid) + slot * NPAD;
         for (int n = lane; n < NPAD; n += 32) {
           int lo = 0, hi = -1;
           if (n < rows) {
-            const int tok = n / p.group;
+            const int tok = token_of(n);
             visible_bounds(p.window, p.causal, seq_len, q_len, first_idx + tok, &lo, &hi);
             rowid[n] = (uint16_t)(tok | (n - tok * p.group) << 8);
           }
           rlo[n] = lo;
           rhi[n] = hi;
+          if (n >= rows) sq[n] = 0.f;
         }
-        // Q digits: HD / 16 lanes per row, 16 elements each (32 / (HD / 16) rows per pass).
-        constexpr int kQLanes = G::chunks, kQRows = 32 / kQLanes;
-        for (int nb = 0; nb < NPAD; nb += kQRows) {
-          const int n = nb + lane / kQLanes, part = lane % kQLanes;
-          float v[16];
-          if (n < rows) {
-            const int token = tok0 + n / p.group, head = c.kvh * p.group + n % p.group;
-            const uint4* srcq = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
-                                                               (int64_t)head * p.q_stride_head + part * 32);
-            const uint4 a = __ldg(srcq), b = __ldg(srcq + 1);
-            const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll 1
+        for (int nb = 0; nb < rows; nb += kPasses * kQRows) {
+          if (nb > 0) load_rows(nb);
+#pragma unroll
+          for (int k = 0; k < kPasses; ++k) {
+            if (nb + k * kQRows >= rows) break;
+            const int n = nb + k * kQRows + lane / kQLanes;
+            const uint32_t w[8] = {qa[k].x, qa[k].y, qa[k].z, qa[k].w, qb[k].x, qb[k].y, qb[k].z, qb[k].w};
+            float v[16];
             if (p.q_dtype == PTH_ATTN_BF16) {
 #pragma unroll
               for (int e = 0; e < 8; ++e) {
@@ -557,32 +596,29 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
                 v[2 * e + 1] = f.y;
               }
             }
-          } else {
+            float amax = 0.f;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) v[e] = 0.f;
+            for (int e = 0; e < 16; ++e) amax = fmaxf(amax, fabsf(v[e]));
+#pragma unroll
+            for (int o = 1; o < kQLanes; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            const bool finite_row = amax > 0.f && amax < INFINITY;
+            const float inv = finite_row ? 32512.f / amax : 0.f;
+            uint32_t hi_w[4] = {0, 0, 0, 0}, lo_w[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              int qi = __float2int_rn(v[e] * inv);
+              qi = max(-32512, min(32512, qi));
+              const int qh = (qi + 128) >> 8;
+              const int ql = qi - (qh << 8);
+              hi_w[e >> 2] |= (uint32_t)(qh & 0xff) << (8 * (e & 3));
+              lo_w[e >> 2] |= (uint32_t)(ql & 0xff) << (8 * (e & 3));
+            }
+            // image row of (digit, n) is digit * NPAD + n; 16-byte column block `part`
+            *reinterpret_cast<uint4*>(qimg + part * (2 * NPAD * 16) + n * 16) = make_uint4(hi_w[0], hi_w[1], hi_w[2], hi_w[3]);
+            *reinterpret_cast<uint4*>(qimg + part * (2 * NPAD * 16) + (NPAD + n) * 16) =
+                make_uint4(lo_w[0], lo_w[1], lo_w[2], lo_w[3]);
+            if (part == 0 && n < rows) sq[n] = finite_row ? amax / 32512.f : 0.f;
           }
-          float amax = 0.f;
-#pragma unroll
-          for (int e = 0; e < 16; ++e) amax = fmaxf(amax, fabsf(v[e]));
-#pragma unroll
-          for (int o = 1; o < kQLanes; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-          const bool finite_row = amax > 0.f && amax < INFINITY;
-          const float inv = finite_row ? 32512.f / amax : 0.f;
-          uint32_t hi_w[4] = {0, 0, 0, 0}, lo_w[4] = {0, 0, 0, 0};
-#pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            int qi = __float2int_rn(v[e] * inv);
-            qi = max(-32512, min(32512, qi));
-            const int qh = (qi + 128) >> 8;
-            const int ql = qi - (qh << 8);
-            hi_w[e >> 2] |= (uint32_t)(qh & 0xff) << (8 * (e & 3));
-            lo_w[e >> 2] |= (uint32_t)(ql & 0xff) << (8 * (e & 3));
-          }
-          // image row of (digit, n) is digit * NPAD + n; 16-byte column block `part`
-          *reinterpret_cast<uint4*>(qimg + part * (2 * NPAD * 16) + n * 16) = make_uint4(hi_w[0], hi_w[1], hi_w[2], hi_w[3]);
-          *reinterpret_cast<uint4*>(qimg + part * (2 * NPAD * 16) + (NPAD + n) * 16) =
-              make_uint4(lo_w[0], lo_w[1], lo_w[2], lo_w[3]);
-          if (part == 0) sq[n] = finite_row ? amax / 32512.f : 0.f;
         }
       }
       tc::fence_async_smem();
@@ -594,7 +630,10 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     {
       const int slot = pub % kItemSlots;
       if (pub >= kItemSlots && ok) ok &= wait_or_abort(&bars[B::item_empty + slot], ((pub / kItemSlots) - 1) & 1, abort_flag);
-      if (lane == 0) descs[slot].n_tiles = 0;
+      if (lane == 0) {
+        descs[slot].n_tiles = 0;
+        mbar_arrive(&bars[B::item_desc + slot]);
+      }
       __syncwarp();
       mbar_arrive(&bars[B::item_full + slot]);
     }
@@ -619,7 +658,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
 #pragma unroll 1
     for (int item = 0;; ++item) {
       const int slot = item % kItemSlots;
-      ok &= wait_or_abort(&bars[B::item_full + slot], (item / kItemSlots) & 1, abort_flag);
+      ok &= wait_or_abort(&bars[B::item_desc + slot], (item / kItemSlots) & 1, abort_flag);
       if (!ok) break;
       const int n_tiles = descs[slot].n_tiles;
       if (n_tiles == 0) break;
@@ -698,7 +737,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
 #pragma unroll 1
     for (int item = 0;; ++item) {
       const int slot = item % kItemSlots;
-      ok &= wait_or_abort(&bars[B::item_full + slot], (item / kItemSlots) & 1, abort_flag);
+      ok &= wait_or_abort(&bars[B::item_desc + slot], (item / kItemSlots) & 1, abort_flag);
       if (!ok) break;
       const int n_tiles = descs[slot].n_tiles;
       if (n_tiles == 0) break;
@@ -1232,7 +1271,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
 
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem_base, L::tmem_alloc);
+  if (warp == kLoadWarp + 1) tc::tmem_dealloc(tmem_base, L::tmem_alloc);
   if (tid == 0 && *abort_flag) atomicOr(&g_i8_status, 4u);
   (void)ok;
 }
