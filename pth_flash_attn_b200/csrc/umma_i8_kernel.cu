@@ -23,9 +23,9 @@
 // while the last tiles of the current item are still being computed:
 //   scheduler  (1 warp)  walks the requests, finds this CTA's next item, writes -inf
 //              markers for splits a request does not use and the result of an item
-//              without keys, and for every other item publishes a descriptor together
-//              with the item's Q digit image, row scales and row masks (two slots, so the
-//              next item is staged while the current one runs);
+//              without keys, and for every other item publishes a descriptor, for which the
+//              copies wait, and then the item's Q digit image, row scales and row masks (two
+//              slots, so the next item is staged while the current one runs);
 //   loaders    (2 warps) lane l of warp w issues page copy c = 2 l + w of a tile - a [copy_slots slots] x
 //              [raw row] box of a tiled tensor map (raw row = the 16-byte aligned bytes
 //              that cover a cell: 144 / 272 / 528 for head sizes 64 / 128 / 256), or a bulk
@@ -40,9 +40,9 @@
 //              V and the two scale vectors into a ring of NS V stages.  A cell is only
 //              8-byte aligned and V starts D + 4 bytes into it, which is why the bytes
 //              pass through registers once (a 256-dim row in two halves);
-//   MMA issuer (1 thread) per item, in a fixed order: QK(0), QK(1), then QK(i + 2), PV(i);
-//              S^T of a tile lands in one of SB buffers of the tile's softmax group, O^T in
-//              the group's O^T buffer; its commits signal the softmax and free the images;
+//   MMA issuer (1 thread) QK tile by tile; S^T of a tile lands in one of SB buffers of the tile's
+//              softmax group, O^T (PV, issued by the softmax up to 8 rows, else here in a fixed
+//              order) in the group's O^T buffer; the commits signal the softmax and free the images;
 //   softmax    (2 groups of 4 warps; group g owns the tiles whose running count is g mod 2,
 //              with its own running maximum, sum and accumulator) thread t owns key t of
 //              S^T (scores -> tile maximum -> probabilities -> digits of P) and output
@@ -128,7 +128,7 @@ struct Layout {
   static constexpr int rowid = (factors + 8 * 4 * factor_rows * 4 + 15) / 16 * 16;   // uint16 [slots][NPAD], see the scheduler
   static constexpr int desc = rowid + kItemSlots * 2 * NPAD;                         // ItemDesc [slots]
   static constexpr int bars = desc + kItemSlots * (int)sizeof(ItemDesc);
-  static constexpr int n_bars = 2 * NS + 14 + 2 * NR + 3 * kItemSlots;
+  static constexpr int n_bars = 2 * NS + 12 + 2 * NR + 3 * kItemSlots;
   static constexpr int misc = bars + n_bars * 8;                    // abort flag, TMEM slot, total work
   static constexpr int total = misc + 32;
   static constexpr int s_cols = 2 * NPAD;
@@ -153,13 +153,12 @@ struct Bars {
   static constexpr int s_ready = 2 * NS;      // [2 groups][2] MMA -> softmax (and producers: K image free)
   static constexpr int s_free = 2 * NS + 4;   // [2 groups][2] softmax -> MMA, 128 arrivals
   static constexpr int o_ready = 2 * NS + 8;  // [2] MMA -> softmax
-  static constexpr int o_free = 2 * NS + 10;  // [2] softmax -> MMA, 128 arrivals
-  static constexpr int p_ready = 2 * NS + 12; // [2] softmax -> MMA, 128 arrivals
-  static constexpr int raw_full = 2 * NS + 14;// [NR] page copies -> producers
-  static constexpr int raw_free = 2 * NS + 14 + NR;  // [NR] producers -> loader, 128 arrivals
-  static constexpr int item_full = 2 * NS + 14 + 2 * NR;               // [slots] scheduler -> issuer, softmax: descriptor and queries
-  static constexpr int item_empty = 2 * NS + 14 + 2 * NR + kItemSlots; // [slots] every other role -> scheduler
-  static constexpr int item_desc = 2 * NS + 14 + 2 * NR + 2 * kItemSlots;  // [slots] scheduler -> loaders, producers: descriptor
+  static constexpr int p_ready = 2 * NS + 10; // [2] softmax -> MMA, 128 arrivals (where the MMA issuer issues PV)
+  static constexpr int raw_full = 2 * NS + 12;// [NR] page copies -> producers
+  static constexpr int raw_free = 2 * NS + 12 + NR;  // [NR] producers -> loader, 128 arrivals
+  static constexpr int item_full = 2 * NS + 12 + 2 * NR;               // [slots] scheduler -> issuer, softmax: descriptor and queries
+  static constexpr int item_empty = 2 * NS + 12 + 2 * NR + kItemSlots; // [slots] every other role -> scheduler
+  static constexpr int item_desc = 2 * NS + 12 + 2 * NR + 2 * kItemSlots;  // [slots] scheduler -> loaders, producers: descriptor
 };
 
 // Key of a tile held by row `r` of its operand images (see the producers).
@@ -212,8 +211,6 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   constexpr int WP = L::wred_row;
   constexpr int kRawRowHD = G::raw_row, kRawStageHD = L::unit_bytes, kImgHD = G::img_bytes;
   constexpr int RU = L::raw_units, kUnitKeys = L::unit_keys;  // raw units per tile, keys per unit
-  // QK runs LA tiles ahead of PV: two when there is a V stage for it, else one
-  constexpr int LA = NS >= 3 ? 2 : 1;
   constexpr int kVStageHD = L::vstage_bytes, kHalves = G::halves;
   constexpr int kRawStages = NR;
   // Largest value of P's digits.  A product that reaches it in exact arithmetic may come out 2^-21 of itself
@@ -221,15 +218,18 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   // (A whole number, so that the largest probability of a tile is exact.)
   constexpr float kTop = PD == 3 ? (float)((1 << 21) - 3) : (float)((1 << 14) - 2);
   constexpr int kThreads = threads_for(NP);
-  constexpr int kMmaWarp = 8 + 4 * NP;     // lane 0 issues every MMA
+  // Who issues PV: up to 8 rows a warp of the softmax group whose P it is, in turn, so that P does not go by way of an
+  // mbarrier and the warp that issues QK, which looks at four barriers kept busy for all of a 64-dim tile's 1,185
+  // cycles (decode at 64 dims 159.8 -> 156.4 us, 256 dims 118.9 -> 116.5, 8 x 8,192 keys 40.9 -> 39.6).  At 16 rows the
+  // softmax is the longest of a tile's stages (verification of 4 tokens 373.8 -> 377 us, 48 decode requests of 4 to
+  // 128 K keys in a 16-row launch 1,320 -> 1,371).
+  constexpr bool kSoftmaxIssuesPV = RQ <= 2;
+  constexpr int kMmaWarp = 8 + 4 * NP;     // issues QK, and PV where the softmax does not
   constexpr int kLoadWarp = kMmaWarp + 1;  // this warp and the next issue the page copies
   constexpr int kSchedWarp = kMmaWarp + 3; // finds and stages the items
   // arrivals that free an item slot: every softmax and producer thread, the issuer, the loaders
   constexpr int kItemReaders = kSoftmaxThreads + NP * kProducerThreads + 3;
   static_assert(RQ >= 1 && 4 * RQ <= NPAD, "RQ = groups of four rows the softmax handles (rows <= 4 RQ)");
-  // QK(i + LA) is issued before PV(i) (see the issuer) and needs the V stage of tile i + LA
-  // filled: with LA + 1 stages or more that is never the one PV(i) has yet to free.
-  static_assert(NS >= LA + 1 && NS >= 2, "tile i + LA needs a V stage of its own");
   static_assert(PD * NPAD >= 8 * RQ, "the P images hold 128 dims of the parked accumulator of one softmax group");
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t* pimg = smem + L::pimg;
@@ -294,11 +294,10 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         tc::mbar_init(&bars[B::s_free + 2 * b + k], kGroupThreads);
       }
       tc::mbar_init(&bars[B::o_ready + b], 1);
-      tc::mbar_init(&bars[B::o_free + b], kGroupThreads);
       tc::mbar_init(&bars[B::p_ready + b], kGroupThreads);
     }
     for (int s = 0; s < kRawStages; ++s) {
-      tc::mbar_init(&bars[B::raw_full + s], kUnitKeys >> p.copy_shift);  // page copies of a unit
+      tc::mbar_init(&bars[B::raw_full + s], 2);                           // the loaders, each with the bytes of its copies
       tc::mbar_init(&bars[B::raw_free + s], kProducerThreads / RU);       // the threads whose keys are in the unit
     }
     for (int s = 0; s < kItemSlots; ++s) {
@@ -337,6 +336,19 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     else if (warp < kMmaWarp) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kProducerRegs));
     else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
   }
+  const DescWords vd = desc_words(vstage0, 128, kImgChunk);
+  const DescWords pd = desc_words(tc::smem_u32(pimg), 128, kDigitChunk);
+  // PV of the tile with running count i, by one thread: needs the group's P image and its O^T folded; frees the V stage.
+  auto issue_pv = [&](int i) {
+    const int g = i & 1;
+    tc::fence_after_sync();
+    DescWords vi = vd, pi = pd;
+    vi.lo += (uint32_t)(i % NS) * (kVStageHD >> 4);
+    pi.lo += (uint32_t)g * ((PD * NPAD * kKeys) >> 4);
+    issue_pv_i8_words<NPAD, PD, HD>(tmem_base + L::s_total + g * L::o_cols, vi, pi);
+    tc::mma_commit(&bars[B::o_ready + g]);
+    tc::mma_commit(&bars[B::empty + i % NS]);
+  };
   if (warp == kSchedWarp) {
     // =========================== scheduler ====================================
     // Walks the requests in blocks of 32 (lane l holds request base + l and the items of the
@@ -647,70 +659,69 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     //   raw_mode 2 (cells of a page contiguous and 16-byte aligned: HND, or one KV head): a
     //     plain bulk copy of the page run.
     // TMA writes shared memory directly (no L1 staging) and a handful of 4 KB copies per tile
-    // keeps tens of KB in flight per SM.  The block id of the next tile's page is fetched
-    // before waiting for the raw stage, so the block-table latency is off the refill path.
+    // keeps tens of KB in flight per SM.  A copy's page and slot are looked up a unit ahead of the wait for the raw
+    // stage, so the block-table latency is off the refill path.
     const int pages_per_unit = kUnitKeys >> p.copy_shift;  // page copies of a raw unit (a tile, or half of one)
     const int bs = p.copy_slots;                            // slots of one copy
-    // (copies are issued one lane after another: with eight of 16 slots a tile, one warp took as long as the tile)
+    // Two warps, a copy per lane: a warp issues its lanes' copies one after another, at 120 to 150 cycles each, so eight of
+    // 16 slots took one warp as long as a tile of 128 dims and longer than one of 64.  (One elected lane for all eight
+    // took twice as long.)  One lane announces the bytes of a warp's copies.
     const int copy = 2 * lane + (warp - kLoadWarp);         // this lane's copy of every unit
-    const uint32_t raw_s = tc::smem_u32(smem + L::raw);
-    int g0 = 0;  // running tile count at the start of the item
+    const uint32_t raw_s = tc::smem_u32(smem + L::raw) + copy * bs * kRawRowHD;
+    const uint32_t copy_bytes = bs * (p.raw_mode == 1 ? kRawRowHD : G::cell);  // a multiple of 16, like a run's address
+    int rs = 0;                  // ring slot of the next unit
+    uint32_t free_parity = 1;    // of the wait for its previous occupant, which the first round does without
+    bool waits = false;
 #pragma unroll 1
     for (int item = 0;; ++item) {
       const int slot = item % kItemSlots;
       ok &= wait_or_abort(&bars[B::item_desc + slot], (item / kItemSlots) & 1, abort_flag);
-      if (!ok) break;
+      if (!__all_sync(0xffffffffu, ok)) break;
       const int n_tiles = descs[slot].n_tiles;
       if (n_tiles == 0) break;
-      if (copy < pages_per_unit) {
-        const int tile_begin = descs[slot].tile_begin, range_begin = descs[slot].range_begin,
-                  range_end = descs[slot].range_end;
-        const int n_units = n_tiles * RU;
-        const int32_t* bt = p.block_table + (int64_t)descs[slot].req * p.block_table_row_stride;
-        const uint8_t* kb = p.k.data + (int64_t)descs[slot].kvh * p.k.stride_head;
-        const uint32_t delta = (uint32_t)(reinterpret_cast<uintptr_t>(kb) & 15);
-        // inner coordinate (4-byte elements) of this head's box: the tensor map starts at the
-        // 16-byte boundary below head 0's first cell
-        const int tma_x = (int)((reinterpret_cast<uintptr_t>(kb) - delta -
-                                 (reinterpret_cast<uintptr_t>(p.k.data) & ~(uintptr_t)15)) >> 2);
-        // block id of this lane's copy of unit v of the item, -1 if no key of the copy is in range
-        auto page_block = [&](int v) -> int {
-          const int pos0 = tile_begin * kKeys + v * kUnitKeys + copy * bs;
-          if (v >= n_units || pos0 >= range_end || pos0 + bs <= range_begin) return -1;
-          int page, slot;
-          page_and_slot(p, pos0, &page, &slot);
-          return __ldg(bt + page);
-        };
-        // first slot, inside its page, of this lane's copy of unit v
-        auto first_slot = [&](int v) -> int {
-          int page, slot;
-          page_and_slot(p, tile_begin * kKeys + v * kUnitKeys + copy * bs, &page, &slot);
-          return slot;
-        };
-        int blk = page_block(0);
+      const int tile_begin = descs[slot].tile_begin, range_begin = descs[slot].range_begin,
+                range_end = descs[slot].range_end;
+      const int n_units = n_tiles * RU;
+      const int32_t* bt = p.block_table + (int64_t)descs[slot].req * p.block_table_row_stride;
+      const uint8_t* kb = p.k.data + (int64_t)descs[slot].kvh * p.k.stride_head;
+      const uint32_t delta = (uint32_t)(reinterpret_cast<uintptr_t>(kb) & 15);
+      // inner coordinate (4-byte elements) of this head's box: the tensor map starts at the
+      // 16-byte boundary below head 0's first cell
+      const int tma_x = (int)((reinterpret_cast<uintptr_t>(kb) - delta -
+                               (reinterpret_cast<uintptr_t>(p.k.data) & ~(uintptr_t)15)) >> 2);
+      // block id and first slot of this lane's copy of unit v of the item; -1 if no key of the copy is in range
+      int pos0 = tile_begin * kKeys + copy * bs;
+      auto look_up = [&](int v, int* first) -> int {
+        if (copy >= pages_per_unit || v >= n_units || pos0 >= range_end || pos0 + bs <= range_begin) return -1;
+        int page;
+        page_and_slot(p, pos0, &page, first);
+        return __ldg(bt + page);
+      };
+      int first = 0, blk = look_up(0, &first);
 #pragma unroll 1
-        for (int v = 0; v < n_units; ++v) {
-          const int blk_next = page_block(v + 1);
-          const int u = g0 * RU + v, rs = u % kRawStages;  // running unit count, ring slot
-          if (u >= kRawStages) ok &= wait_raw_free(&bars[B::raw_free + rs], ((u / kRawStages) - 1) & 1, abort_flag);
-          uint64_t* bar = &bars[B::raw_full + rs];
-          if (blk >= 0 && ok) {
-            const uint32_t dst = raw_s + rs * kRawStageHD + copy * bs * kRawRowHD;
-            if (p.raw_mode == 1) {
-              mbar_arrive_expect_tx(bar, bs * kRawRowHD);
-              tma_load_3d(dst, &tmap, tma_x, first_slot(v), blk, bar);
-            } else {
-              const uint32_t bytes = bs * G::cell;  // a multiple of 16, like the run's address
-              mbar_arrive_expect_tx(bar, bytes);
-              bulk_copy_g2s(dst, kb + (int64_t)blk * p.k.stride_block + (int64_t)first_slot(v) * G::cell, bytes, bar);
-            }
-          } else {
-            mbar_arrive(bar);
-          }
-          blk = blk_next;
+      for (int v = 0; v < n_units; ++v) {
+        pos0 += kUnitKeys;
+        int first_next = 0;
+        const int blk_next = look_up(v + 1, &first_next);
+        uint64_t* bar = &bars[B::raw_full + rs];
+        if (waits) ok &= wait_raw_free(&bars[B::raw_free + rs], free_parity, abort_flag);
+        const uint32_t live = __ballot_sync(0xffffffffu, blk >= 0 && ok);
+        if (lane == 0) mbar_arrive_expect_tx(bar, __popc(live) * copy_bytes);
+        __syncwarp();
+        if (blk >= 0 && ok) {
+          const uint32_t dst = raw_s + rs * kRawStageHD;
+          if (p.raw_mode == 1) tma_load_3d(dst, &tmap, tma_x, first, blk, bar);
+          else bulk_copy_g2s(dst, kb + (int64_t)blk * p.k.stride_block + (int64_t)first * G::cell, copy_bytes, bar);
+        }
+        __syncwarp();
+        blk = blk_next;
+        first = first_next;
+        if (++rs == kRawStages) {
+          rs = 0;
+          waits = true;
+          free_parity ^= 1u;
         }
       }
-      g0 += n_tiles;
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars[B::item_empty + slot]);
     }
@@ -846,32 +857,17 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     }
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===================================
-    // ONE thread (the lane elect.sync picks) issues every tcgen05.mma of the CTA, item after item, inside an item
-    // in a fixed order (two issuing threads, one for QK and one for PV, produced rare
-    // run-to-run differences):
-    //   QK(0), QK(1), then for i = 0, 1, ...: QK(i + 2), PV(i)
-    // (with only two V stages - the 256-dim instances - QK runs one tile ahead instead of two).
-    // With g = running tile count of tile i:
-    //   QK(i): the tile belongs to softmax group g & 1, is that group's k-th tile (k = g >> 1)
-    //          and lands in its S^T buffer k % SB; needs the tile's images (full) and that
-    //          buffer read by the softmax (s_free);
-    //   PV(i): needs the group's P image (p_ready) and its O^T buffer folded (o_free); its
-    //          completion frees the V stage.
-    // Every condition of a step depends only on MMAs issued earlier in this order, so the
-    // order cannot deadlock, and QK runs two tiles ahead of PV, which is as far as the S^T
-    // buffers allow.  The next item's first QK follows the last PV of this item at once: its
-    // images have long been filled, so S^T of the next item is ready while the softmax groups
-    // still merge and write this one.  The two barriers of a step are waited for by lanes 0
-    // and 1 in the same instruction: a look at an mbarrier costs 100-200 cycles on the busy
-    // shared-memory pipe, and four looks in a row per tile made this thread the bottleneck.
-    // This thread's own instruction stream is the narrowest part of the CTA (a few hundred
-    // dependent instructions per tile took as long as the tile), so everything it needs is
-    // kept in registers: barrier addresses as shared-memory offsets, operand descriptors as
-    // word pairs that move by one addition per MMA.
+    // One elected lane issues every QK of the CTA in the order of the tiles.  With g = running tile count, the tile
+    // belongs to softmax group g & 1, is that group's k-th tile (k = g >> 1) and lands in its S^T buffer k % SB: it
+    // needs the tile's images (full) and that buffer read by the softmax (s_free), so QK runs SB tiles of a group ahead
+    // of the softmax, from one item into the next.  Where the softmax does not issue PV, the order inside an item is
+    // QK(0), QK(1), then for i = 0, 1, ...: QK(i + 2), PV(i): every condition depends only on MMAs issued earlier
+    // in this order (with two V stages QK runs one tile ahead instead of two).  The two barriers of a step
+    // are waited for by lanes 0 and 1 in the same instruction: a look at an mbarrier costs 100-200 cycles on the busy
+    // shared-memory pipe.  Everything the issuing thread needs is kept in registers: barrier addresses as
+    // shared-memory offsets, operand descriptors as word pairs that move by one addition per MMA.
     const uint32_t bars_s = tc::smem_u32(bars);
     const DescWords kd = desc_words(kstage0, kImgChunk, 128);
-    const DescWords vd = desc_words(vstage0, 128, kImgChunk);
-    const DescWords pd = desc_words(tc::smem_u32(pimg), 128, kDigitChunk);
     // lane 0 waits for barrier i0 (parity par0); lane 1 for barrier i1 if need1; true when both are complete
     auto wait_pair = [&](int i0, uint32_t par0, int i1, uint32_t par1, bool need1) -> bool {
       const uint32_t mine = bars_s + 8u * (uint32_t)(lane == 0 ? i0 : i1);
@@ -880,12 +876,12 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
       const bool done = !need || wait_or_abort_s(mine, par, abort_flag);
       return __all_sync(0xffffffffu, done);
     };
-    int g0 = 0;
+    int g0 = 0;  // running tile count at the start of the item
     bool go = true;
 #pragma unroll 1
     for (int item = 0; go; ++item) {
       const int slot = item % kItemSlots;
-      go = wait_or_abort(&bars[B::item_full + slot], (item / kItemSlots) & 1, abort_flag);
+      go = __all_sync(0xffffffffu, wait_or_abort(&bars[B::item_full + slot], (item / kItemSlots) & 1, abort_flag));
       if (!go) break;
       const int n_tiles = descs[slot].n_tiles;
       if (n_tiles == 0) break;
@@ -903,27 +899,24 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         }
         return ready;
       };
-      auto pv_step = [&](int i) -> bool {
-        const int g = i & 1;
-        const bool ready = wait_pair(B::p_ready + g, (i >> 1) & 1, B::o_free + g, ((i >> 1) - 1) & 1, i >= 2);
-        if (ready && elect_one()) {
-          tc::fence_after_sync();
-          DescWords vi = vd, pi = pd;
-          vi.lo += (uint32_t)(i % NS) * (kVStageHD >> 4);
-          pi.lo += (uint32_t)g * ((PD * NPAD * kKeys) >> 4);
-          issue_pv_i8_words<NPAD, PD, HD>(tmem_base + L::s_total + g * L::o_cols, vi, pi);
-          tc::mma_commit_s(bars_s + 8u * (B::o_ready + g));
-          tc::mma_commit_s(bars_s + 8u * (B::empty + i % NS));
-        }
-        return ready;
-      };
-#pragma unroll
-      for (int a = 0; a < LA; ++a)
-        if (go && a < n_tiles) go = qk_step(g0 + a);
+      if constexpr (kSoftmaxIssuesPV) {
 #pragma unroll 1
-      for (int i = 0; i < n_tiles && go; ++i) {
-        if (i + LA < n_tiles) go = qk_step(g0 + i + LA);
-        if (go) go = pv_step(g0 + i);
+        for (int i = 0; i < n_tiles && go; ++i) go = qk_step(g0 + i);
+      } else {
+        constexpr int LA = NS >= 3 ? 2 : 1;  // tiles QK runs ahead of PV: two when there is a V stage for it
+        // QK(i + LA) is issued before PV(i): with LA + 1 stages or more its V stage is never the one PV(i) has yet to free
+        static_assert(NS >= LA + 1, "tile i + LA needs a V stage of its own");
+#pragma unroll
+        for (int a = 0; a < LA; ++a)
+          if (go && a < n_tiles) go = qk_step(g0 + a);
+#pragma unroll 1
+        for (int i = 0; i < n_tiles && go; ++i) {
+          if (i + LA < n_tiles) go = qk_step(g0 + i + LA);
+          if (!go) break;
+          const int q = g0 + i;
+          go = wait_pair(B::p_ready + (q & 1), (q >> 1) & 1, 0, 0, false);
+          if (go && elect_one()) issue_pv(q);
+        }
       }
       g0 += n_tiles;
       __syncwarp();
@@ -1031,7 +1024,6 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
           }
         }
         tc::fence_before_sync();
-        mbar_arrive(&bars[B::o_free + g]);
       };
 
       int lit = 0;                // tiles of this item this group has started
@@ -1152,8 +1144,15 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
                   make_uint4(dig[k][0], dig[k][1], dig[k][2], dig[k][3]);
           }
         }
+        // P image of the tile complete, and O^T of the previous one folded by every thread of the group
         tc::fence_async_smem();
-        mbar_arrive(&bars[B::p_ready + g]);  // P image of the tile complete
+        if constexpr (kSoftmaxIssuesPV) {
+          named_barrier(1 + g, kGroupThreads);
+          if (gw == (it & 3) && elect_one()) issue_pv(q);
+          __syncwarp();
+        } else {
+          mbar_arrive(&bars[B::p_ready + g]);
+        }
       }
       if (lit > 0) fold_o(g0 + j - 2);  // the group's last tile of the item
 
