@@ -234,6 +234,7 @@ int32_t attention_impl(const PthAttnArgs* a, const PthB200Options* opt, void* st
     err = launch_umma_i8_attention(ps, static_cast<cudaStream_t>(stream));
     if (err == cudaSuccess) {
       ps.row_class = 2;
+      ps.late_wait = 1;
       err = launch_umma_rows_attention(ps, static_cast<cudaStream_t>(stream));
     }
   } else if (family == PTHB200_KERNEL_UMMA) {

@@ -62,6 +62,9 @@ struct KernelParams {
   int32_t num_sms;     // SMs of the device (set by the launchers whose kernels choose splits on the device)
   int32_t row_class;   // 0 = every request; 1 = only requests with q_len * group <= class_rows; 2 = only the others
   int32_t class_rows;
+  // Row-major kernels behind the integer kernel of the same call, with whose requests they share nothing: they start
+  // beside it and wait for it only before they end (pdl.cuh).
+  int32_t late_wait = 0;
 };
 
 // Re-tiles a launch to `bq` query tokens per row tile.  The caller's promise behind

@@ -68,6 +68,7 @@
 #include "sched.cuh"
 #include "umma_i8.cuh"
 #include "page_copy.cuh"
+#include "pdl.cuh"
 
 namespace pthb200 {
 
@@ -261,6 +262,42 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   // atomic sum, and the copies waiting for the queries' digits, the first copy of a launch of 8 x U[1, 4096] keys left
   // 14,000 cycles after the kernel's start, now 6,300: 26.7 and 22.9 us.)
   if (warp == kLoadWarp && lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
+  auto set_up = [&] {
+    if (warp == kMmaWarp && lane == 0) {
+      for (int s = 0; s < NS; ++s) {
+        tc::mbar_init(&bars[B::full + s], kProducerThreads);
+        tc::mbar_init(&bars[B::empty + s], 1);
+      }
+      for (int b = 0; b < 2; ++b) {
+        for (int k = 0; k < 2; ++k) {
+          tc::mbar_init(&bars[B::s_ready + 2 * b + k], 1);
+          tc::mbar_init(&bars[B::s_free + 2 * b + k], kGroupThreads);
+        }
+        tc::mbar_init(&bars[B::o_ready + b], 1);
+        tc::mbar_init(&bars[B::p_ready + b], kGroupThreads);
+      }
+      for (int s = 0; s < kRawStages; ++s) {
+        tc::mbar_init(&bars[B::raw_full + s], 2);                           // the loaders, each with the bytes of its copies
+        tc::mbar_init(&bars[B::raw_free + s], kProducerThreads / RU);       // the threads whose keys are in the unit
+      }
+      for (int s = 0; s < kItemSlots; ++s) {
+        tc::mbar_init(&bars[B::item_full + s], 32);
+        tc::mbar_init(&bars[B::item_desc + s], 1);
+        tc::mbar_init(&bars[B::item_empty + s], kItemReaders);
+      }
+      *abort_flag = 0;
+      tc::mbar_init_fence();
+    }
+    if (warp == kLoadWarp + 1) {
+      tc::tmem_alloc(tslot, L::tmem_alloc);
+      tc::tmem_relinquish();
+    }
+  };
+  if (p.row_class != 1) set_up();
+  pdl_wait();  // (the set-up may overlap the kernel in front; the lengths are the first thing that it or others wrote)
+  // A row-major kernel of the same call may start beside this one.  (A combine that waits on the SMs costs more than
+  // it gains: 64 x 8,192 keys 198 -> 210 us with its CTAs let in early.)
+  if (p.row_class == 1) pdl_trigger();
   // (the scheduler's first 32 requests)
   int pre_q0 = 0, pre_q1 = 0, pre_len = 0;
   if (warp == kSchedWarp && lane < p.num_reqs) {
@@ -282,35 +319,9 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     served |= row_tiles > 0;
   }
   // A prefill launch whose requests are all tall has nothing for this kernel: its CTAs leave before any set-up.
-  if (p.row_class == 1 && !__syncthreads_or(served)) return;
-  if (warp == kMmaWarp && lane == 0) {
-    for (int s = 0; s < NS; ++s) {
-      tc::mbar_init(&bars[B::full + s], kProducerThreads);
-      tc::mbar_init(&bars[B::empty + s], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      for (int k = 0; k < 2; ++k) {
-        tc::mbar_init(&bars[B::s_ready + 2 * b + k], 1);
-        tc::mbar_init(&bars[B::s_free + 2 * b + k], kGroupThreads);
-      }
-      tc::mbar_init(&bars[B::o_ready + b], 1);
-      tc::mbar_init(&bars[B::p_ready + b], kGroupThreads);
-    }
-    for (int s = 0; s < kRawStages; ++s) {
-      tc::mbar_init(&bars[B::raw_full + s], 2);                           // the loaders, each with the bytes of its copies
-      tc::mbar_init(&bars[B::raw_free + s], kProducerThreads / RU);       // the threads whose keys are in the unit
-    }
-    for (int s = 0; s < kItemSlots; ++s) {
-      tc::mbar_init(&bars[B::item_full + s], 32);
-      tc::mbar_init(&bars[B::item_desc + s], 1);
-      tc::mbar_init(&bars[B::item_empty + s], kItemReaders);
-    }
-    *abort_flag = 0;
-    tc::mbar_init_fence();
-  }
-  if (warp == kLoadWarp + 1) {
-    tc::tmem_alloc(tslot, L::tmem_alloc);
-    tc::tmem_relinquish();
+  if (p.row_class == 1) {
+    if (!__syncthreads_or(served)) return;
+    set_up();
   }
   {
     unsigned long long w = work;
@@ -1293,8 +1304,7 @@ cudaError_t launch_cfg(const KernelParams& p, const CUtensorMap& map, int num_ct
     if (err != cudaSuccess) return err;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  umma_i8_attention_kernel<HD, NPAD, PD, NS, NK, NR, SB, RQ, NP><<<num_ctas, threads_for(NP), smem, stream>>>(p, map);
-  return cudaGetLastError();
+  return pdl_launch(umma_i8_attention_kernel<HD, NPAD, PD, NS, NK, NR, SB, RQ, NP>, num_ctas, threads_for(NP), smem, stream, p, map);
 }
 
 }  // namespace

@@ -28,6 +28,7 @@
 #include "sched.cuh"
 #include "umma_rows.cuh"
 #include "page_copy.cuh"
+#include "pdl.cuh"
 
 namespace pthb200 {
 
@@ -123,6 +124,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
   rows_cta(p, &kvh, &tile_index);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (!p.late_wait) pdl_wait();
   // Row tile of this CTA: bisect a shared-memory copy of query_start_loc when it fits.
   constexpr int kQslCache = 4096;
   static_assert(kWNR * kWRawUnit >= 2 * kQslCache * 4, "the raw ring holds the copies of query_start_loc and seq_lens");
@@ -141,7 +143,10 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
   } else {
     t = resolve_row_tile(p, tile_index);
   }
-  if (t.req < 0) return;
+  if (t.req < 0) {
+    if (p.late_wait) pdl_wait();
+    return;
+  }
   const int rows = t.ntok * p.group;  // <= 128 by construction of bq
   // num_splits is a bound: the pieces a request is cut into are chosen here, from the lengths,
   // by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the
@@ -173,7 +178,10 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     __syncthreads();
     const int t_star = item_tiles(*total_s * (unsigned long long)p.num_kv_heads, p.num_sms);
     nsplits = req_splits(req_kv_tiles(shape, t.q_len, t.seq_len), t_star, p.num_splits);
-    if (split >= nsplits) return;
+    if (split >= nsplits) {
+      if (p.late_wait) pdl_wait();
+      return;
+    }
     if (split == 0) {
       for (int i = tid; i < rows * (p.num_splits - nsplits); i += kWThreads) {
         int token, head;
@@ -211,6 +219,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
                                   (int64_t)head * p.lse_stride_head) = -INFINITY;
       }
     }
+    if (p.late_wait) pdl_wait();
     return;
   }
 
@@ -590,6 +599,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     }
   }
 
+  if (p.late_wait) pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
@@ -625,8 +635,7 @@ cudaError_t launch_umma_rows256_attention(const KernelParams& p_in, cudaStream_t
   const int64_t ctas = (int64_t)p.num_q_tiles * p.num_kv_heads;
   if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
   const dim3 grid((unsigned)ctas, p.num_splits);
-  umma_rows256_attention_kernel<<<grid, kWThreads, WLayout::total, stream>>>(p, *mapp);
-  return cudaGetLastError();
+  return pdl_launch(umma_rows256_attention_kernel, grid, kWThreads, WLayout::total, stream, p, *mapp);
 }
 
 // Reads and clears this kernel's status word (device must be idle).

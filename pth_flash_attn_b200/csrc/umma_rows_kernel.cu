@@ -35,6 +35,7 @@
 #include "sched.cuh"
 #include "umma_rows.cuh"
 #include "page_copy.cuh"
+#include "pdl.cuh"
 
 namespace pthb200 {
 
@@ -114,6 +115,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   rows_cta(p, &kvh, &tile_index);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (!p.late_wait) pdl_wait();
   // Row tile of this CTA: bisect a shared-memory copy of query_start_loc when it fits.
   constexpr int kQslCache = 4096;
   static_assert(kRNR * kRawHalfBytes >= 2 * kQslCache * 4, "the raw ring holds the copies of query_start_loc and seq_lens");
@@ -132,7 +134,10 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   } else {
     t = resolve_row_tile(p, tile_index);
   }
-  if (t.req < 0) return;
+  if (t.req < 0) {
+    if (p.late_wait) pdl_wait();
+    return;
+  }
   const int rows = t.ntok * p.group;  // <= 128 by construction of bq
   // num_splits is a bound: the pieces a request is cut into are chosen here, from the lengths,
   // by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the
@@ -164,7 +169,10 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     __syncthreads();
     const int t_star = item_tiles(*total_s * (unsigned long long)p.num_kv_heads, p.num_sms);
     nsplits = req_splits(req_kv_tiles(shape, t.q_len, t.seq_len), t_star, p.num_splits);
-    if (split >= nsplits) return;
+    if (split >= nsplits) {
+      if (p.late_wait) pdl_wait();
+      return;
+    }
     if (split == 0) {
       for (int i = tid; i < rows * (p.num_splits - nsplits); i += kRThreads) {
         int token, head;
@@ -202,6 +210,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
                                   (int64_t)head * p.lse_stride_head) = -INFINITY;
       }
     }
+    if (p.late_wait) pdl_wait();
     return;
   }
 
@@ -644,6 +653,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     }
   }
 
+  if (p.late_wait) pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
@@ -674,8 +684,7 @@ cudaError_t launch_rows(const KernelParams& p, const CUtensorMap& map, dim3 grid
     if (err != cudaSuccess) return err;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  umma_rows_attention_kernel<NK, NR><<<grid, kRThreads, RLayout<NK, NR>::total, stream>>>(p, map);
-  return cudaGetLastError();
+  return pdl_launch(umma_rows_attention_kernel<NK, NR>, grid, kRThreads, RLayout<NK, NR>::total, stream, p, map);
 }
 }  // namespace
 
