@@ -85,6 +85,23 @@ struct RowTile {
   int32_t first_idx;  // index of tok0 inside the request
 };
 
+// Row tile x of the grid, which lies in the tiles of request `req` or behind them.
+__device__ __forceinline__ RowTile finish_row_tile(const KernelParams& p, int x, int req, int q0, int q1, int seq_len) {
+  RowTile t;
+  t.req = -1;
+  const int j = p.tile_map == 1 ? 0 : x - (q0 / p.bq + req);
+  const int q_len = q1 - q0;
+  if (j < 0 || j * p.bq >= q_len) return t;
+  if (p.row_class != 0 && (((int64_t)q_len * p.group <= p.class_rows) != (p.row_class == 1))) return t;
+  t.req = req;
+  t.first_idx = j * p.bq;
+  t.tok0 = q0 + t.first_idx;
+  t.ntok = min(p.bq, q_len - t.first_idx);
+  t.q_len = q_len;
+  t.seq_len = seq_len;
+  return t;
+}
+
 // Row tile x of the grid: request r owns tiles [qsl[r]/bq + r, ... + ceil(q_len/bq)).
 // The start index is strictly increasing in r, so the owner is found by
 // bisection; tiles that fall between two requests are surplus (req = -1).
@@ -108,20 +125,8 @@ __device__ __forceinline__ RowTile resolve_row_tile_with(const KernelParams& p, 
       if (first <= x) lo = mid; else hi = mid - 1;
     }
   }
-  const int q0 = qsl(lo);
-  const int q1 = qsl(lo + 1);
-  const int seq_len = len(lo);  // issued with the two loads above, not after the checks below
-  const int j = p.tile_map == 1 ? 0 : x - (q0 / p.bq + lo);
-  const int q_len = q1 - q0;
-  if (j < 0 || j * p.bq >= q_len) return t;
-  if (p.row_class != 0 && (((int64_t)q_len * p.group <= p.class_rows) != (p.row_class == 1))) return t;
-  t.req = lo;
-  t.first_idx = j * p.bq;
-  t.tok0 = q0 + t.first_idx;
-  t.ntok = min(p.bq, q_len - t.first_idx);
-  t.q_len = q_len;
-  t.seq_len = seq_len;
-  return t;
+  // (the length is loaded with the two others, not after the checks)
+  return finish_row_tile(p, x, lo, qsl(lo), qsl(lo + 1), len(lo));
 }
 
 __device__ __forceinline__ RowTile resolve_row_tile(const KernelParams& p, int x) {
@@ -164,6 +169,11 @@ __device__ __forceinline__ void split_tiles(const KernelParams& p, const RowTile
   }
   const int t0 = rb / kKvTile;
   const int t1 = (re + kKvTile - 1) / kKvTile;
+  if (num_splits == 1) {
+    *tile_begin = t0;
+    *tile_end = t1;
+    return;
+  }
   const int64_t n = t1 - t0;
   *tile_begin = t0 + (int)((int64_t)split * n / num_splits);
   *tile_end = t0 + (int)((int64_t)(split + 1) * n / num_splits);

@@ -39,6 +39,8 @@
 #include <cuda_fp16.h>
 
 #include "params.cuh"
+#include "pdl.cuh"
+#include "sched.cuh"
 #include "umma_tile.cuh"
 
 namespace pthb200 {
@@ -171,6 +173,142 @@ __device__ __forceinline__ void rows_cta(const KernelParams& p, int* kvh, int* t
   const uint32_t t = blockIdx.x / (uint32_t)p.num_kv_heads;
   *kvh = (int)(blockIdx.x - t * (uint32_t)p.num_kv_heads);
   *tile_index = p.num_q_tiles - 1 - (int)t;
+}
+
+// Row tile x of a padded tile grid (tile_map 0), found by one warp among up to kWarpRequests requests, 32 at a
+// time, while others set barriers and TMEM up; its result goes to all threads through shared memory behind the barrier
+// that ends the set-up.  (Not from every warp's own shuffles: the compiler then takes the length of the tile loops
+// for one per lane, which costs them 4 %.)  *work: the launch's KV tiles per head, if they are wanted.
+// (What a CTA does once costs by its instructions, which come from beyond the instruction caches at about ten cycles
+// each: so loops stay rolled here, in stage_queries and in write_rows32.  Twelve new prompts of 37 to 2,500 tokens, CTAs of
+// a handful of tiles: 425 us with all requests copied to shared memory and bisected by everybody behind two barriers, every
+// thread loading and storing its own row of queries and results, 350 with these; with the same unrolled 498.)
+constexpr int kWarpRequests = 96;
+__device__ __forceinline__ RowTile warp_row_tile(const KernelParams& p, int x, bool want_work, const SchedShape& shape, unsigned long long* work) {
+  const int lane = threadIdx.x & 31;
+  int owner = 0, q0 = 0, q1 = 0, len = 0;  // the last request whose first tile is not behind x
+#pragma unroll 1
+  for (int base = 0; base < p.num_reqs; base += 32) {
+    const int r = base + lane;
+    int a = 0, b = 0, c = 0;
+    if (r < p.num_reqs) {
+      a = __ldg(p.query_start_loc + r);
+      b = __ldg(p.query_start_loc + r + 1);
+      c = __ldg(p.seq_lens + r);
+    }
+    const uint32_t before = __ballot_sync(0xffffffffu, r < p.num_reqs && a / p.bq + r <= x);
+    if (before != 0u) {  // (consecutive lanes from 0 on)
+      const int src = __popc(before) - 1;
+      owner = base + src;
+      q0 = __shfl_sync(0xffffffffu, a, src);
+      q1 = __shfl_sync(0xffffffffu, b, src);
+      len = __shfl_sync(0xffffffffu, c, src);
+    } else if (!want_work) {
+      break;
+    }
+    if (want_work && r < p.num_reqs)
+      *work += (unsigned long long)req_row_tiles(shape, b - a) * (unsigned long long)req_kv_tiles(shape, b - a, c);
+  }
+  if (want_work) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) *work += __shfl_xor_sync(0xffffffffu, *work, o);
+  }
+  return finish_row_tile(p, x, owner, q0, q1, len);
+}
+__device__ __forceinline__ SchedShape sched_shape(const KernelParams& p) {
+  SchedShape shape;
+  shape.group = p.group;
+  shape.num_kv_heads = p.num_kv_heads;
+  shape.bq = p.bq;
+  shape.num_splits = p.num_splits;
+  shape.window = p.window;
+  shape.causal = p.causal;
+  shape.row_class = p.row_class;
+  shape.class_rows = p.class_rows;
+  return shape;
+}
+
+// What a CTA computes: the keys of one piece of a row tile.
+struct RowsItem {
+  RowTile t;
+  int rows, nsplits;
+  int tile_begin, tile_end, range_begin, range_end;
+  int state;  // 0: nothing, 1: keys, 2: rows without keys
+};
+constexpr int kRowsItemInts = sizeof(RowsItem) / 4;
+static_assert(sizeof(RowTile) == 24 && kRowsItemInts == 13, "as the broadcast copies it");
+// num_splits is a bound: the pieces a request is cut into are chosen here, from the lengths and the launch's KV tiles
+// per head, by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the
+// whole launch, so a prefill chunk among long decode requests is not cut at all.
+__device__ __forceinline__ RowsItem rows_item(const KernelParams& p, const RowTile& t, int split, unsigned long long work) {
+  RowsItem it;
+  it.t = t;
+  it.state = 0;
+  it.rows = it.nsplits = it.tile_begin = it.tile_end = it.range_begin = it.range_end = 0;
+  if (t.req < 0) return it;
+  it.rows = t.ntok * p.group;
+  it.nsplits = p.num_splits;
+  if (p.num_splits > 1) {
+    const int t_star = item_tiles(work * (unsigned long long)p.num_kv_heads, p.num_sms);
+    it.nsplits = req_splits(req_kv_tiles(sched_shape(p), t.q_len, t.seq_len), t_star, p.num_splits);
+    if (split >= it.nsplits) return it;
+  }
+  split_tiles(p, t, split, it.nsplits, &it.tile_begin, &it.tile_end, &it.range_begin, &it.range_end);
+  it.state = it.tile_begin < it.tile_end ? 1 : 2;
+  return it;
+}
+// The launch's KV tiles per head, summed over the CTA (`scratch`: 8 idle bytes).
+template <int kThreads>
+__device__ __forceinline__ unsigned long long cta_work(const KernelParams& p, uint8_t* scratch) {
+  const SchedShape shape = sched_shape(p);
+  unsigned long long* total_s = reinterpret_cast<unsigned long long*>(scratch);
+  unsigned long long w = 0;
+  for (int r = threadIdx.x; r < p.num_reqs; r += kThreads) {
+    const int a = __ldg(p.query_start_loc + r), b = __ldg(p.query_start_loc + r + 1);
+    w += (unsigned long long)req_row_tiles(shape, b - a) * (unsigned long long)req_kv_tiles(shape, b - a, __ldg(p.seq_lens + r));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+  if (threadIdx.x == 0) *total_s = 0ull;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0 && w != 0) atomicAdd(total_s, w);
+  __syncthreads();
+  return *total_s;
+}
+// By all threads of the CTA: the CTA of piece 0 marks the pieces that the request does not use as holding no keys; rows
+// without keys get a zero output and a log-sum-exp of -inf.
+template <int kThreads, int kDim>
+__device__ __forceinline__ void write_empty(const KernelParams& p, const RowsItem& it, int kvh, int split) {
+  const int tid = threadIdx.x;
+  const RowTile& t = it.t;
+  if (it.state != 0 && split == 0 && p.num_splits > it.nsplits) {
+    for (int i = tid; i < it.rows * (p.num_splits - it.nsplits); i += kThreads) {
+      const int token = t.tok0 + (i % it.rows) / p.group, head = kvh * p.group + (i % it.rows) % p.group;
+      *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)(it.nsplits + i / it.rows) * p.ws_lse_stride_split +
+                                (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = -INFINITY;
+    }
+  }
+  if (it.state != 2) return;
+  for (int idx = tid; idx < it.rows * kDim; idx += kThreads) {
+    const int n = idx / kDim, d = idx % kDim;
+    const int token = t.tok0 + n / p.group, head = kvh * p.group + n % p.group;
+    if (p.num_splits == 1) {
+      store_out_elem(p.out + (int64_t)token * p.out_stride_token + (int64_t)head * p.out_stride_head, d, p.out_dtype, 0.f);
+    } else {
+      reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
+                               (int64_t)token * p.ws_o_stride_token + (int64_t)head * p.ws_o_stride_head)[d] = 0.f;
+    }
+  }
+  if (tid < it.rows) {
+    const int token = t.tok0 + tid / p.group, head = kvh * p.group + tid % p.group;
+    if (p.num_splits > 1) {
+      *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
+                                (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = -INFINITY;
+    } else if (p.lse_out != nullptr) {
+      *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) + (int64_t)token * p.lse_stride_token +
+                                (int64_t)head * p.lse_stride_head) = -INFINITY;
+    }
+  }
 }
 
 // ---- queries ----
@@ -313,21 +451,132 @@ __device__ __forceinline__ float sum_pairs(const f32x2 (&ls)[2]) {
   return (a + b) + (c + d);
 }
 
-// 32 consecutive dims of an output row (16-byte aligned) in the caller's type, as 16-byte stores.
-__device__ __forceinline__ void store_out32(uint8_t* dst, int dtype, const float (&o)[32]) {
-  if (dtype == PTH_ATTN_F32) {
+// Byte offset of row n of an item in a [token][head] array (rows are token-major).  (n is below 256 and the group at most
+// 64: n + 1/2 keeps a distance of 1 / 128 from every multiple of the group.)
+__device__ __forceinline__ int64_t row_offset(const RowTile& t, int kvh, int group, float inv_group, int n, int64_t stride_token,
+                                              int64_t stride_head) {
+  const int tok = (int)(((float)n + 0.5f) * inv_group);
+  return (int64_t)(t.tok0 + tok) * stride_token + (int64_t)(kvh * group + (n - tok * group)) * stride_head;
+}
+
+__device__ __forceinline__ const uint8_t* shfl_ptr(const uint8_t* ptr, int lane) {
+  return reinterpret_cast<const uint8_t*>((uintptr_t)__shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)ptr, lane));
+}
+
+// Queries of kCount rows (row0 .. of the CTA) by one warp: as many lanes per row as it has 16-byte blocks, so that a
+// load covers whole rows.  Rows past the live ones are zeros.  Calls
+// put(row, block, fp16 block) for every block, and fixed(row, fix) in one lane for every row (QueryScale).
+template <int HD, int kCount, class Put, class Fixed>
+__device__ __forceinline__ void stage_queries(const KernelParams& p, const RowTile& t, int kvh, int rows, int row0, Put put, Fixed fixed) {
+  constexpr int kLanes = HD / 8, kAtOnce = 32 / kLanes, kSteps = kCount / kAtOnce, kBatch = 4;
+  static_assert(kLanes <= 32 && kCount <= 32 && kSteps % kBatch == 0, "a warp covers whole rows");
+  const int lane = threadIdx.x & 31, block = lane % kLanes, sub = lane / kLanes;
+  // (lane l looks row row0 + l up)
+  const uint8_t* mine = p.q + row_offset(t, kvh, p.group, 1.0f / (float)p.group, min(row0 + lane, rows - 1), p.q_stride_token, p.q_stride_head);
+  const bool bf16 = p.q_dtype == PTH_ATTN_BF16;
+  uint4 next[kBatch];
+  auto load = [&](int k0) {
 #pragma unroll
-    for (int n = 0; n < 32; n += 4) *reinterpret_cast<float4*>(dst + n * 4) = make_float4(o[n], o[n + 1], o[n + 2], o[n + 3]);
-  } else if (dtype == PTH_ATTN_BF16) {
+    for (int k = 0; k < kBatch; ++k) {
+      const int r = (k0 + k) * kAtOnce + sub;
+      const uint8_t* src = shfl_ptr(mine, r);
+      next[k] = row0 + r < rows ? __ldg(reinterpret_cast<const uint4*>(src) + block) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  load(0);
+#pragma unroll 1
+  for (int k0 = 0; k0 < kSteps; k0 += kBatch) {
+    uint4 q[kBatch];
 #pragma unroll
-    for (int n = 0; n < 32; n += 8)
-      *reinterpret_cast<uint4*>(dst + n * 2) = make_uint4(pack_bf16(o[n], o[n + 1]), pack_bf16(o[n + 2], o[n + 3]),
-                                                          pack_bf16(o[n + 4], o[n + 5]), pack_bf16(o[n + 6], o[n + 7]));
+    for (int k = 0; k < kBatch; ++k) q[k] = next[k];
+    if (k0 + kBatch < kSteps) load(k0 + kBatch);
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const int n = row0 + (k0 + k) * kAtOnce + sub;
+      float fix = 1.0f;
+      if (bf16) {
+        const uint4 one[1] = {q[k]};
+        uint32_t amax = finite_amax_bf16(one);
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1) amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        const QueryScale qs = query_scale(amax);
+        fix = qs.fix;
+        q[k] = queries_to_f16(q[k], qs.scale);
+      }
+      put(n, block, q[k]);
+      if (block == 0) fixed(n, fix);
+    }
+  }
+}
+
+// Where a row's results go (from dim 0 on), and in which type.
+struct RowsOut {
+  uint8_t* row;   // of this lane's row
+  uint32_t live;  // lanes with live rows
+  int dtype;
+};
+__device__ __forceinline__ RowsOut rows_out(const KernelParams& p, const RowTile& t, int kvh, int rows, int row, int split) {
+  RowsOut o;
+  const float inv_group = 1.0f / (float)p.group;
+  o.live = __ballot_sync(0xffffffffu, row < rows);
+  if (p.num_splits > 1) {
+    o.row = reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
+            row_offset(t, kvh, p.group, inv_group, row, p.ws_o_stride_token, p.ws_o_stride_head);
+    o.dtype = PTH_ATTN_F32;
   } else {
+    o.row = p.out + row_offset(t, kvh, p.group, inv_group, row, p.out_stride_token, p.out_stride_head);
+    o.dtype = p.out_dtype;
+  }
+  return o;
+}
+// 32 dims (from d0) of the results of a warp's 32 rows, a row per lane in o: through 4 KB of shared
+// memory of the warp's own, so that a store covers whole sectors of a few rows (each thread storing its own row 16 bytes
+// at a time, a store touches 32 lines).
+__device__ __forceinline__ void write_rows32(const RowsOut& out, int d0, uint8_t* stage, const float (&o)[32]) {
+  const int lane = threadIdx.x & 31;
+  if (out.dtype == PTH_ATTN_F32) {
 #pragma unroll
-    for (int n = 0; n < 32; n += 8)
-      *reinterpret_cast<uint4*>(dst + n * 2) = make_uint4(pack_f16(o[n], o[n + 1]), pack_f16(o[n + 2], o[n + 3]),
-                                                          pack_f16(o[n + 4], o[n + 5]), pack_f16(o[n + 6], o[n + 7]));
+    for (int c = 0; c < 8; ++c)
+      *reinterpret_cast<float4*>(stage + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+    __syncwarp();
+    const int c = lane & 7;
+#pragma unroll 2
+    for (int k = 0; k < 8; ++k) {
+      const int r = 4 * k + (lane >> 3);
+      uint8_t* dst = const_cast<uint8_t*>(shfl_ptr(out.row, r)) + d0 * 4 + c * 16;
+      const float4 v = *reinterpret_cast<const float4*>(stage + r * 128 + ((c ^ (r & 7)) << 4));
+      if (out.live >> r & 1u) *reinterpret_cast<float4*>(dst) = v;
+    }
+  } else {
+    const bool bf16 = out.dtype == PTH_ATTN_BF16;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[e] = bf16 ? pack_bf16(o[8 * c + 2 * e], o[8 * c + 2 * e + 1]) : pack_f16(o[8 * c + 2 * e], o[8 * c + 2 * e + 1]);
+      *reinterpret_cast<uint4*>(stage + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    __syncwarp();
+    const int c = lane & 3;
+#pragma unroll 2
+    for (int k = 0; k < 4; ++k) {
+      const int r = 8 * k + (lane >> 2);
+      uint8_t* dst = const_cast<uint8_t*>(shfl_ptr(out.row, r)) + d0 * 2 + c * 16;
+      const uint4 v = *reinterpret_cast<const uint4*>(stage + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+      if (out.live >> r & 1u) *reinterpret_cast<uint4*>(dst) = v;
+    }
+  }
+  __syncwarp();  // (the stage is written again)
+}
+// A row's log-sum-exp (log2 units) where the caller wants it.
+__device__ __forceinline__ void write_lse(const KernelParams& p, const RowTile& t, int kvh, int row, int split, float lse2) {
+  const float inv_group = 1.0f / (float)p.group;
+  if (p.num_splits > 1) {
+    *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
+                              row_offset(t, kvh, p.group, inv_group, row, p.ws_lse_stride_token, p.ws_lse_stride_head)) = lse2;
+  } else if (p.lse_out != nullptr) {
+    *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) +
+                              row_offset(t, kvh, p.group, inv_group, row, p.lse_stride_token, p.lse_stride_head)) = lse2 * kLn2;
   }
 }
 

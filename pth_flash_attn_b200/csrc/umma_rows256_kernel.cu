@@ -65,10 +65,11 @@ struct WLayout {
   static constexpr int ksc = raw + kWNR * kWRawUnit;                 // KeyScales<64> [kWKsRing]
   static constexpr int tile_max = ksc + kWKsRing * (int)sizeof(KeyScales<kWKeys>);  // float [2 tiles][2 groups][128 rows]
   static constexpr int half_sum = tile_max + 2 * 2 * kWGroup * 4;    // float [2 groups][128 rows]
-  static constexpr int bars = half_sum + 2 * kWGroup * 4;            // uint64 [...]
+  static constexpr int qstage = half_sum + 2 * kWGroup * 4;          // [8 warps] 32 dims of 32 rows of Q
+  static constexpr int bars = qstage + 8 * 2048;                     // uint64 [...]
   static constexpr int n_bars = kWNS * 2 + 2 * kWNK + 6 + 2 * kWNR;
   static constexpr int misc = bars + n_bars * 8;
-  static constexpr int total = misc + 32;
+  static constexpr int total = misc + 32 + 4 * kRowsItemInts;
 };
 
 struct WBars {
@@ -124,111 +125,13 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
   rows_cta(p, &kvh, &tile_index);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (!p.late_wait) pdl_wait();
-  // Row tile of this CTA: bisect a shared-memory copy of query_start_loc when it fits.
-  constexpr int kQslCache = 4096;
-  static_assert(kWNR * kWRawUnit >= 2 * kQslCache * 4, "the raw ring holds the copies of query_start_loc and seq_lens");
-  RowTile t;
-  if (p.tile_map == 0 && p.num_reqs + 1 <= kQslCache) {
-    int* qsl_s = reinterpret_cast<int*>(smem + L::raw);
-    int* len_s = qsl_s + kQslCache;
-    for (int i = tid; i <= p.num_reqs; i += kWThreads) {
-      qsl_s[i] = __ldg(p.query_start_loc + i);
-      if (i < p.num_reqs) len_s[i] = __ldg(p.seq_lens + i);
-    }
-    __syncthreads();
-    t = resolve_row_tile_with(p, tile_index, [&](int i) { return qsl_s[i]; }, [&](int r) { return len_s[r]; });
-    tc::fence_async_smem();  // (page copies write here next, through the other proxy)
-    __syncthreads();
-  } else {
-    t = resolve_row_tile(p, tile_index);
+  // Barriers and TMEM are set up by the warps that wait for nothing else.
+  if (warp == kWLoadWarp) {
+    if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
+    tc::tmem_alloc(tslot, 512);
+    tc::tmem_relinquish();
   }
-  if (t.req < 0) {
-    if (p.late_wait) pdl_wait();
-    return;
-  }
-  const int rows = t.ntok * p.group;  // <= 128 by construction of bq
-  // num_splits is a bound: the pieces a request is cut into are chosen here, from the lengths,
-  // by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the
-  // whole launch, so a prefill chunk among long decode requests is not cut at all.  CTAs of
-  // unused pieces leave at once; the CTA of piece 0 marks them as holding no keys.
-  int nsplits = p.num_splits;
-  if (p.num_splits > 1) {
-    unsigned long long* total_s = reinterpret_cast<unsigned long long*>(smem + L::misc + 16);
-    if (tid == 0) *total_s = 0ull;
-    __syncthreads();
-    SchedShape shape;
-    shape.group = p.group;
-    shape.num_kv_heads = p.num_kv_heads;
-    shape.bq = p.bq;
-    shape.num_splits = p.num_splits;
-    shape.window = p.window;
-    shape.causal = p.causal;
-    shape.row_class = p.row_class;
-    shape.class_rows = p.class_rows;
-    unsigned long long w = 0;
-    for (int r = tid; r < p.num_reqs; r += kWThreads) {
-      const int q0 = __ldg(p.query_start_loc + r), q1 = __ldg(p.query_start_loc + r + 1);
-      w += (unsigned long long)req_row_tiles(shape, q1 - q0) *
-           (unsigned long long)req_kv_tiles(shape, q1 - q0, __ldg(p.seq_lens + r));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-    if (lane == 0 && w != 0) atomicAdd(total_s, w);
-    __syncthreads();
-    const int t_star = item_tiles(*total_s * (unsigned long long)p.num_kv_heads, p.num_sms);
-    nsplits = req_splits(req_kv_tiles(shape, t.q_len, t.seq_len), t_star, p.num_splits);
-    if (split >= nsplits) {
-      if (p.late_wait) pdl_wait();
-      return;
-    }
-    if (split == 0) {
-      for (int i = tid; i < rows * (p.num_splits - nsplits); i += kWThreads) {
-        int token, head;
-        row_target(p, t, kvh, i % rows, &token, &head);
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)(nsplits + i / rows) * p.ws_lse_stride_split +
-                                  (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = -INFINITY;
-      }
-    }
-    __syncthreads();  // the scratch word is part of a region the barriers are initialised in next
-  }
-  int tile_begin, tile_end, range_begin, range_end;
-  split_tiles(p, t, split, nsplits, &tile_begin, &tile_end, &range_begin, &range_end);
-
-  if (tile_begin >= tile_end) {
-    // No keys for this work item: zero output, log-sum-exp -inf.
-    for (int idx = tid; idx < rows * kWDim; idx += kWThreads) {
-      const int n = idx / kWDim, d = idx % kWDim;
-      int token, head;
-      row_target(p, t, kvh, n, &token, &head);
-      if (p.num_splits == 1) {
-        store_out_elem(p.out + (int64_t)token * p.out_stride_token + (int64_t)head * p.out_stride_head, d, p.out_dtype, 0.f);
-      } else {
-        reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
-                                 (int64_t)token * p.ws_o_stride_token + (int64_t)head * p.ws_o_stride_head)[d] = 0.f;
-      }
-    }
-    if (tid < rows) {
-      int token, head;
-      row_target(p, t, kvh, tid, &token, &head);
-      if (p.num_splits > 1) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
-                                  (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = -INFINITY;
-      } else if (p.lse_out != nullptr) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) + (int64_t)token * p.lse_stride_token +
-                                  (int64_t)head * p.lse_stride_head) = -INFINITY;
-      }
-    }
-    if (p.late_wait) pdl_wait();
-    return;
-  }
-
-  // the CTA walks its keys in tiles of 64: from the first 128-key tile of its piece to the end
-  // of the keys its rows see (or of the piece)
-  const int key_begin = tile_begin * 128;
-  const int key_end = min(tile_end * 128, range_end);
-  const int n_tiles = (key_end - key_begin + kWKeys - 1) / kWKeys;
-  if (tid == 0) {
+  if (warp == kWMmaWarp && lane == 0) {
     for (int s = 0; s < kWNS; ++s) {
       tc::mbar_init(&bars[B::vfull + s], kWProducers / 2);
       tc::mbar_init(&bars[B::vempty + s], 1);
@@ -249,14 +152,61 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     *abort_flag = 0;
     tc::mbar_init_fence();
   }
-  if (warp == 0) {
-    tc::tmem_alloc(tslot, 512);
-    tc::tmem_relinquish();
+  if (!p.late_wait) pdl_wait();
+  // Row tile of this CTA: warp 0 finds it; for longer lists of requests all threads bisect a shared-memory copy of
+  // query_start_loc when it fits.
+  constexpr int kQslCache = 4096;
+  static_assert(kWNR * kWRawUnit >= 2 * kQslCache * 4, "the raw ring holds the copies of query_start_loc and seq_lens");
+  RowsItem item;
+  int* item_s = reinterpret_cast<int*>(smem + L::misc + 32);
+  const bool by_warp = p.num_reqs <= kWarpRequests && p.tile_map == 0;
+  if (by_warp) {
+    if (warp == 0) {
+      unsigned long long work = 0;
+      const RowTile found = warp_row_tile(p, tile_index, p.num_splits > 1, sched_shape(p), &work);
+      item = rows_item(p, found, split, work);
+      if (lane == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
+    }
+  } else {
+    RowTile t;
+    if (p.tile_map == 0 && p.num_reqs + 1 <= kQslCache) {
+      int* qsl_s = reinterpret_cast<int*>(smem + L::raw);
+      int* len_s = qsl_s + kQslCache;
+      for (int i = tid; i <= p.num_reqs; i += kWThreads) {
+        qsl_s[i] = __ldg(p.query_start_loc + i);
+        if (i < p.num_reqs) len_s[i] = __ldg(p.seq_lens + i);
+      }
+      __syncthreads();
+      t = resolve_row_tile_with(p, tile_index, [&](int i) { return qsl_s[i]; }, [&](int r) { return len_s[r]; });
+      tc::fence_async_smem();  // (page copies write here next, through the other proxy)
+      __syncthreads();
+    } else {
+      t = resolve_row_tile(p, tile_index);
+    }
+    const unsigned long long work = p.num_splits > 1 ? cta_work<kWThreads>(p, smem + L::misc + 16) : 0ull;
+    item = rows_item(p, t, split, work);
+    if (tid == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
   }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tslot;
+  item = *reinterpret_cast<const RowsItem*>(item_s);
+  if (item.state != 1 || (split == 0 && item.nsplits < p.num_splits)) write_empty<kWThreads, kWDim>(p, item, kvh, split);
+  if (item.state != 1) {
+    if (warp == kWLoadWarp) tc::tmem_dealloc(tmem_base, 512);
+    if (p.late_wait) pdl_wait();
+    return;
+  }
+  const RowTile& t = item.t;
+  const int rows = item.rows;  // <= 128 by construction of bq
+  const int tile_begin = item.tile_begin, tile_end = item.tile_end, range_begin = item.range_begin, range_end = item.range_end;
+
+  // the CTA walks its keys in tiles of 64: from the first 128-key tile of its piece to the end
+  // of the keys its rows see (or of the piece)
+  const int key_begin = tile_begin * 128;
+  const int key_end = min(tile_end * 128, range_end);
+  const int n_tiles = (key_end - key_begin + kWKeys - 1) / kWKeys;
   const uint32_t kimg_s = tc::smem_u32(smem + L::kimg), vst_s = tc::smem_u32(smem + L::vst);
   bool ok = true;
 
@@ -446,38 +396,61 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     const uint32_t s_part = tmem_base + kWSCol + g * kWGroupKeys + lane_addr;   // this group's columns of S buffer 0
     const uint32_t o_part = tmem_base + kWOCol + g * kWGroupDims + lane_addr;   // this group's columns of O
 
-    // ---- Q into TMEM: thread (row, g) stores dims 128 g .. 128 g + 127 of its row, two fp16 per column ----
+    // ---- Q into TMEM: dims 128 g .. 128 g + 127 of a row through the thread of the row, two fp16 per column.  A warp
+    // loads its 32 rows 64 bytes at a time, four lanes a row, and hands them to their threads 32 dims after 32 dims
+    // through 2 KB of shared memory.  (Each thread loading its own row: see stage_queries.) ----
     float q_fix = 1.0f;  // what the row's scores are multiplied by (QueryScale)
     {
-      int token, head;
-      row_target(p, t, kvh, row, &token, &head);
-      const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
-                                                        (int64_t)head * p.q_stride_head) + g * (kWGroupDims / 8);
-      uint4 qv[16];
+      const int row0 = row & ~31, c = lane & 3;
+      const uint8_t* mine = p.q + row_offset(t, kvh, p.group, 1.0f / (float)p.group, min(row, rows - 1), p.q_stride_token, p.q_stride_head);
+      uint8_t* stage = smem + L::qstage + warp * 2048;
+      uint4 qv[4][4];  // [32 dims][8 rows]
 #pragma unroll
-      for (int c = 0; c < 16; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
+      for (int k = 0; k < 4; ++k) {
+        const int n = row0 + 8 * k + (lane >> 2);
+        const uint4* src = reinterpret_cast<const uint4*>(shfl_ptr(mine, 8 * k + (lane >> 2))) + g * (kWGroupDims / 8) + c;
+#pragma unroll
+        for (int d = 0; d < 4; ++d) qv[d][k] = n < rows ? __ldg(src + 4 * d) : make_uint4(0u, 0u, 0u, 0u);
+      }
       if (p.q_dtype == PTH_ATTN_BF16) {
         uint32_t* part = reinterpret_cast<uint32_t*>(tile_max);  // [2 groups][128 rows] (idle until the first tile)
-        const uint32_t mine = finite_amax_bf16(qv);
-        part[g * kWGroup + row] = mine;
-        named_barrier(4, kWSoftmax);
-        const QueryScale qs = query_scale(max(mine, part[(g ^ 1) * kWGroup + row]));
-        q_fix = qs.fix;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) qv[c] = queries_to_f16(qv[c], qs.scale);
+        for (int k = 0; k < 4; ++k) {
+          const uint4 mine[4] = {qv[0][k], qv[1][k], qv[2][k], qv[3][k]};
+          uint32_t amax = finite_amax_bf16(mine);
+          amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+          amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+          if (c == 0) part[g * kWGroup + row0 + 8 * k + (lane >> 2)] = amax;
+        }
+        named_barrier(4, kWSoftmax);
+        q_fix = query_scale(max(part[row], part[kWGroup + row])).fix;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int n = row0 + 8 * k + (lane >> 2);
+          const float scale = query_scale(max(part[n], part[kWGroup + n])).scale;
+#pragma unroll
+          for (int d = 0; d < 4; ++d) qv[d][k] = queries_to_f16(qv[d][k], scale);
+        }
       }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t qw[32];
+      for (int d = 0; d < 4; ++d) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const uint4 v = qv[h * 8 + c];
-          qw[4 * c] = v.x;
-          qw[4 * c + 1] = v.y;
-          qw[4 * c + 2] = v.z;
-          qw[4 * c + 3] = v.w;
+        for (int k = 0; k < 4; ++k) {
+          const int r = 8 * k + (lane >> 2);
+          *reinterpret_cast<uint4*>(stage + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) = qv[d][k];
         }
-        tc::tmem_st32(tmem_base + kWQCol + g * (kWGroupDims / 2) + h * 32 + lane_addr, qw);
+        __syncwarp();
+        uint32_t qw[16];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint4 v = *reinterpret_cast<const uint4*>(stage + lane * 64 + ((e ^ ((lane >> 1) & 3)) << 4));
+          qw[4 * e] = v.x;
+          qw[4 * e + 1] = v.y;
+          qw[4 * e + 2] = v.z;
+          qw[4 * e + 3] = v.w;
+        }
+        tc::tmem_st16(tmem_base + kWQCol + g * (kWGroupDims / 2) + d * 16 + lane_addr, qw);
+        __syncwarp();
       }
       tc::tmem_st_wait();
     }
@@ -565,44 +538,29 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     named_barrier(4, kWSoftmax);
     const float lsum = half_sum[row] + half_sum[kWGroup + row];  // the same order in both threads
     const float inv = lsum > 0.f ? 1.0f / lsum : 0.f;
-    int token, head;
-    row_target(p, t, kvh, row, &token, &head);
-    uint8_t* out_row = p.out + (int64_t)token * p.out_stride_token + (int64_t)head * p.out_stride_head;
-    float* ws_row = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
-                                             (int64_t)token * p.ws_o_stride_token + (int64_t)head * p.ws_o_stride_head);
+    // (the K images are idle: every QK has completed)
+    uint8_t* stage = smem + L::kimg + warp * 4096;
+    static_assert(8 * 4096 <= kWNK * kWImage, "room for every warp's rows");
+    const RowsOut dst = rows_out(p, t, kvh, rows, row, split);
+    if ((row & ~31) < rows) {
 #pragma unroll 1
-    for (int j = 0; j < kWGroupDims / 32; ++j) {
-      uint32_t r[32];
-      tc::tmem_ld32(o_part + j * 32, r);
-      tc::tmem_ld_wait<32>(r);
-      float o[32];
+      for (int j = 0; j < kWGroupDims / 32; ++j) {
+        uint32_t r[32];
+        tc::tmem_ld32(o_part + j * 32, r);
+        tc::tmem_ld_wait<32>(r);
+        float o[32];
 #pragma unroll
-      for (int n = 0; n < 32; ++n) o[n] = __uint_as_float(r[n]) * inv;
-      const int d0 = g * kWGroupDims + j * 32;
-      if (row < rows) {
-        if (p.num_splits > 1) {
-          store_out32(reinterpret_cast<uint8_t*>(ws_row + d0), PTH_ATTN_F32, o);
-        } else {
-          store_out32(out_row + d0 * (p.out_dtype == PTH_ATTN_F32 ? 4 : 2), p.out_dtype, o);
-        }
+        for (int n = 0; n < 32; ++n) o[n] = __uint_as_float(r[n]) * inv;
+        write_rows32(dst, g * kWGroupDims + j * 32, stage, o);
       }
     }
-    if (g == 0 && row < rows) {
-      const float lse2 = lsum > 0.f ? m_ref - kPGain + log2f(lsum) : -INFINITY;
-      if (p.num_splits > 1) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
-                                  (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = lse2;
-      } else if (p.lse_out != nullptr) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) + (int64_t)token * p.lse_stride_token +
-                                  (int64_t)head * p.lse_stride_head) = lse2 * kLn2;
-      }
-    }
+    if (g == 0 && row < rows && (p.num_splits > 1 || p.lse_out != nullptr)) write_lse(p, t, kvh, row, split, lsum > 0.f ? m_ref - kPGain + log2f(lsum) : -INFINITY);
   }
 
   if (p.late_wait) pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
+  if (warp == kWLoadWarp) tc::tmem_dealloc(tmem_base, 512);
   if (tid == 0 && *abort_flag) atomicOr(&g_rows256_status, 4u);
   (void)ok;
 }

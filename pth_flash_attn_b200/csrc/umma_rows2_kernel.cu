@@ -76,10 +76,11 @@ struct XLayout {
   static constexpr int qimg = vst + kXNS * G::image;                 // [2 row tiles] Q images
   static constexpr int raw = (qimg + 2 * G::qimage + 127) / 128 * 128;
   static constexpr int ksc = raw + kXNR * G::raw_unit;               // KeyScales<64> [kXKsRing]
-  static constexpr int bars = ksc + kXKsRing * (int)sizeof(KeyScales<kXKeys>);  // uint64 [...]
+  static constexpr int fix = ksc + kXKsRing * (int)sizeof(KeyScales<kXKeys>);   // float [256 rows], see QueryScale
+  static constexpr int bars = fix + kXRows * 4;                                  // uint64 [...]
   static constexpr int n_bars = 2 * kXNS + 2 * kXNK + 12 + 2 * kXNR;
   static constexpr int misc = bars + n_bars * 8;
-  static constexpr int total = misc + 32;
+  static constexpr int total = misc + 32 + 4 * kRowsItemInts;
 };
 
 struct XBars {
@@ -137,120 +138,19 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
   rows_cta(p, &kvh, &tile_index);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (!p.late_wait) pdl_wait();
-  // Row tile of this CTA: bisect a shared-memory copy of query_start_loc when it fits.
-  constexpr int kQslCache = 4096;
-  static_assert(kXNR * kXRawUnit >= 2 * kQslCache * 4, "the raw ring holds the copies of query_start_loc and seq_lens");
-  RowTile t;
-  if (p.tile_map == 0 && p.num_reqs + 1 <= kQslCache) {
-    int* qsl_s = reinterpret_cast<int*>(smem + L::raw);
-    int* len_s = qsl_s + kQslCache;
-    for (int i = tid; i <= p.num_reqs; i += kXThreads) {
-      qsl_s[i] = __ldg(p.query_start_loc + i);
-      if (i < p.num_reqs) len_s[i] = __ldg(p.seq_lens + i);
-    }
-    __syncthreads();
-    t = resolve_row_tile_with(p, tile_index, [&](int i) { return qsl_s[i]; }, [&](int r) { return len_s[r]; });
-    tc::fence_async_smem();  // (page copies write here next, through the other proxy)
-    __syncthreads();
-  } else {
-    t = resolve_row_tile(p, tile_index);
+  // Barriers and TMEM are set up by the warps that wait for nothing else.
+  if (warp == kXLoadWarp) {
+    if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
+    tc::tmem_alloc(tslot, 512);
+    tc::tmem_relinquish();
   }
-  if (t.req < 0) {
-    if (p.late_wait) pdl_wait();
-    return;
-  }
-  const int rows = t.ntok * p.group;  // <= 256 by construction of bq
-  // num_splits is a bound: the pieces a request is cut into are chosen here, from the lengths,
-  // by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the
-  // whole launch, so a prefill chunk among long decode requests is not cut at all.  CTAs of
-  // unused pieces leave at once; the CTA of piece 0 marks them as holding no keys.
-  int nsplits = p.num_splits;
-  if (p.num_splits > 1) {
-    unsigned long long* total_s = reinterpret_cast<unsigned long long*>(smem + L::misc + 16);
-    if (tid == 0) *total_s = 0ull;
-    __syncthreads();
-    SchedShape shape;
-    shape.group = p.group;
-    shape.num_kv_heads = p.num_kv_heads;
-    shape.bq = p.bq;
-    shape.num_splits = p.num_splits;
-    shape.window = p.window;
-    shape.causal = p.causal;
-    shape.row_class = p.row_class;
-    shape.class_rows = p.class_rows;
-    unsigned long long w = 0;
-    for (int r = tid; r < p.num_reqs; r += kXThreads) {
-      const int q0 = __ldg(p.query_start_loc + r), q1 = __ldg(p.query_start_loc + r + 1);
-      w += (unsigned long long)req_row_tiles(shape, q1 - q0) *
-           (unsigned long long)req_kv_tiles(shape, q1 - q0, __ldg(p.seq_lens + r));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-    if (lane == 0 && w != 0) atomicAdd(total_s, w);
-    __syncthreads();
-    const int t_star = item_tiles(*total_s * (unsigned long long)p.num_kv_heads, p.num_sms);
-    nsplits = req_splits(req_kv_tiles(shape, t.q_len, t.seq_len), t_star, p.num_splits);
-    if (split >= nsplits) {
-      if (p.late_wait) pdl_wait();
-      return;
-    }
-    if (split == 0) {
-      for (int i = tid; i < rows * (p.num_splits - nsplits); i += kXThreads) {
-        int token, head;
-        row_target(p, t, kvh, i % rows, &token, &head);
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)(nsplits + i / rows) * p.ws_lse_stride_split +
-                                  (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = -INFINITY;
-      }
-    }
-    __syncthreads();  // the scratch word is part of a region the barriers are initialised in next
-  }
-  int tile_begin, tile_end, range_begin, range_end;
-  split_tiles(p, t, split, nsplits, &tile_begin, &tile_end, &range_begin, &range_end);
-
-  if (tile_begin >= tile_end) {
-    // No keys for this work item: zero output, log-sum-exp -inf.
-    for (int idx = tid; idx < rows * kXDim; idx += kXThreads) {
-      const int n = idx / kXDim, d = idx % kXDim;
-      int token, head;
-      row_target(p, t, kvh, n, &token, &head);
-      if (p.num_splits == 1) {
-        store_out_elem(p.out + (int64_t)token * p.out_stride_token + (int64_t)head * p.out_stride_head, d, p.out_dtype, 0.f);
-      } else {
-        reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
-                                 (int64_t)token * p.ws_o_stride_token + (int64_t)head * p.ws_o_stride_head)[d] = 0.f;
-      }
-    }
-    if (tid < rows) {
-      int token, head;
-      row_target(p, t, kvh, tid, &token, &head);
-      if (p.num_splits > 1) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
-                                  (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = -INFINITY;
-      } else if (p.lse_out != nullptr) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) + (int64_t)token * p.lse_stride_token +
-                                  (int64_t)head * p.lse_stride_head) = -INFINITY;
-      }
-    }
-    if (p.late_wait) pdl_wait();
-    return;
-  }
-
-  // the CTA walks its keys in tiles of 64: from the first 128-key tile of its piece to the end
-  // of the keys its rows see (or of the piece)
-  const int key_begin = tile_begin * 128;
-  const int key_end = min(tile_end * 128, range_end);
-  const int n_tiles = (key_end - key_begin + kXKeys - 1) / kXKeys;
-  // Row tiles with live rows: a CTA of at most 128 rows (the end of a chunk, a short request
-  // inside a prefill launch) issues no MMA for its second row tile, whose softmax warps idle.
-  const int n_rt = rows > 128 ? 2 : 1;
-  if (tid == 0) {
+  if (warp == kXMmaWarp && lane == 0) {
     for (int s = 0; s < kXNS; ++s) {
       tc::mbar_init(&bars[B::vfull + s], kXProducers / 2);
-      tc::mbar_init(&bars[B::vempty + s], n_rt);  // one commit per row tile's PV
+      tc::mbar_init(&bars[B::vempty + s], 2);  // one commit per row tile's PV
     }
     for (int s = 0; s < kXNK; ++s) {
-      tc::mbar_init(&bars[B::kempty + s], n_rt);  // one commit per row tile's QK
+      tc::mbar_init(&bars[B::kempty + s], 2);  // one commit per row tile's QK
       tc::mbar_init(&bars[B::kfull + s], kXProducers / 2);
     }
     for (int g = 0; g < 4; ++g) {
@@ -265,14 +165,64 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     *abort_flag = 0;
     tc::mbar_init_fence();
   }
-  if (warp == 0) {
-    tc::tmem_alloc(tslot, 512);
-    tc::tmem_relinquish();
+  if (!p.late_wait) pdl_wait();
+  // Row tile of this CTA: warp 0 finds it; for longer lists of requests all threads bisect a shared-memory copy of
+  // query_start_loc when it fits.
+  constexpr int kQslCache = 4096;
+  static_assert(kXNR * kXRawUnit >= 2 * kQslCache * 4, "the raw ring holds the copies of query_start_loc and seq_lens");
+  RowsItem item;
+  int* item_s = reinterpret_cast<int*>(smem + L::misc + 32);
+  const bool by_warp = p.num_reqs <= kWarpRequests && p.tile_map == 0;
+  if (by_warp) {
+    if (warp == 0) {
+      unsigned long long work = 0;
+      const RowTile found = warp_row_tile(p, tile_index, p.num_splits > 1, sched_shape(p), &work);
+      item = rows_item(p, found, split, work);
+      if (lane == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
+    }
+  } else {
+    RowTile t;
+    if (p.tile_map == 0 && p.num_reqs + 1 <= kQslCache) {
+      int* qsl_s = reinterpret_cast<int*>(smem + L::raw);
+      int* len_s = qsl_s + kQslCache;
+      for (int i = tid; i <= p.num_reqs; i += kXThreads) {
+        qsl_s[i] = __ldg(p.query_start_loc + i);
+        if (i < p.num_reqs) len_s[i] = __ldg(p.seq_lens + i);
+      }
+      __syncthreads();
+      t = resolve_row_tile_with(p, tile_index, [&](int i) { return qsl_s[i]; }, [&](int r) { return len_s[r]; });
+      tc::fence_async_smem();  // (page copies write here next, through the other proxy)
+      __syncthreads();
+    } else {
+      t = resolve_row_tile(p, tile_index);
+    }
+    const unsigned long long work = p.num_splits > 1 ? cta_work<kXThreads>(p, smem + L::misc + 16) : 0ull;
+    item = rows_item(p, t, split, work);
+    if (tid == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
   }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tslot;
+  item = *reinterpret_cast<const RowsItem*>(item_s);
+  if (item.state != 1 || (split == 0 && item.nsplits < p.num_splits)) write_empty<kXThreads, HD>(p, item, kvh, split);
+  if (item.state != 1) {
+    if (warp == kXLoadWarp) tc::tmem_dealloc(tmem_base, 512);
+    if (p.late_wait) pdl_wait();
+    return;
+  }
+  const RowTile& t = item.t;
+  const int rows = item.rows;  // <= 256 by construction of bq
+  const int tile_begin = item.tile_begin, tile_end = item.tile_end, range_begin = item.range_begin, range_end = item.range_end;
+
+  // the CTA walks its keys in tiles of 64: from the first 128-key tile of its piece to the end
+  // of the keys its rows see (or of the piece)
+  const int key_begin = tile_begin * 128;
+  const int key_end = min(tile_end * 128, range_end);
+  const int n_tiles = (key_end - key_begin + kXKeys - 1) / kXKeys;
+  // Row tiles with live rows: a CTA of at most 128 rows (the end of a chunk, a short request
+  // inside a prefill launch) issues no MMA for its second row tile, whose softmax warps idle.
+  const int n_rt = rows > 128 ? 2 : 1;
   const uint32_t kimg_s = tc::smem_u32(smem + L::kimg), vst_s = tc::smem_u32(smem + L::vst);
   bool ok = true;
 
@@ -436,6 +386,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
             issue_qk_x<HD>(tmem_base + (2 * rt + b) * kXKeys, qq, k);
             tc::mma_commit(&bars[B::s_ready + 2 * rt + b]);
             tc::mma_commit(&bars[B::kempty + q % kXNK]);  // (free once both row tiles' QK have read the K image)
+            if constexpr (kRowTiles == 1) tc::mma_commit(&bars[B::kempty + q % kXNK]);
           }
           __syncwarp();
         }
@@ -456,6 +407,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
             issue_pv_x<HD>(tmem_base + kXOCol + rt * kXDim, tmem_base + (2 * rt + b) * kXKeys, v, i > 0);
             tc::mma_commit(&bars[B::pv_done + 2 * rt + b]);
             tc::mma_commit(&bars[B::vempty + i % kXNS]);  // (free once both row tiles' PV have read the V stage)
+            if constexpr (kRowTiles == 1) tc::mma_commit(&bars[B::vempty + i % kXNS]);
           }
           __syncwarp();
         }
@@ -472,28 +424,17 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     const uint32_t s_rt = tmem_base + 2 * rt * kXKeys + lane_addr;          // S(rt, 0)
     const uint32_t o_tmem = tmem_base + kXOCol + rt * kXDim + lane_addr;    // O(rt)
 
-    // ---- Q image of this row tile: thread converts its row, 16 column blocks of 8 dims ----
-    float q_fix = 1.0f;  // what the row's scores are multiplied by (QueryScale)
+    // ---- Q image of this row tile: a warp converts the 32 rows of its threads ----
+    float* fix_s = reinterpret_cast<float*>(smem + L::fix);
     {
-      int token, head;
-      row_target(p, t, kvh, row, &token, &head);
-      const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
-                                                        (int64_t)head * p.q_stride_head);
-      uint8_t* qrow = smem + L::qimg + rt * kXQImage + (tid & 127) * 16;
-      uint4 qv[kXChunks];
-#pragma unroll
-      for (int c = 0; c < kXChunks; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
-      if (p.q_dtype == PTH_ATTN_BF16) {
-        const QueryScale qs = query_scale(finite_amax_bf16(qv));
-        q_fix = qs.fix;
-#pragma unroll
-        for (int c = 0; c < kXChunks; ++c) qv[c] = queries_to_f16(qv[c], qs.scale);
-      }
-#pragma unroll
-      for (int c = 0; c < kXChunks; ++c) *reinterpret_cast<uint4*>(qrow + c * kXQStride) = qv[c];
+      uint8_t* qimg = smem + L::qimg + rt * kXQImage;
+      stage_queries<HD, 32>(p, t, kvh, rows, row & ~31,
+          [&](int n, int block, const uint4& v) { *reinterpret_cast<uint4*>(qimg + block * kXQStride + (n & 127) * 16) = v; },
+          [&](int n, float fix) { fix_s[n] = fix; });
     }
     tc::fence_async_smem();
     named_barrier(5, kXQBarrier);  // Q images complete; the QK issuer may start
+    const float q_fix = fix_s[row];  // what the row's scores are multiplied by (QueryScale)
 
     int rlo = 0, rhi = -1;  // visible keys of this row (none for a padding row)
     if (row < rows) visible_range(p, t, t.first_idx + row / p.group, &rlo, &rhi);
@@ -592,44 +533,28 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     if (rt < n_rt) ok &= wait_or_abort(&bars[B::pv_done + 2 * rt + ((n_tiles - 1) & 1)], ((n_tiles - 1) >> 1) & 1, abort_flag);
     tc::fence_after_sync();
     const float inv = l > 0.f ? 1.0f / l : 0.f;
-    int token, head;
-    row_target(p, t, kvh, row, &token, &head);
-    uint8_t* out_row = p.out + (int64_t)token * p.out_stride_token + (int64_t)head * p.out_stride_head;
-    float* ws_row = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
-                                             (int64_t)token * p.ws_o_stride_token + (int64_t)head * p.ws_o_stride_head);
+    // (the Q image of this row tile is idle: every QK that reads it has completed)
+    uint8_t* stage = smem + L::qimg + rt * kXQImage + (warp & 3) * 4096;
+    const RowsOut dst = rows_out(p, t, kvh, rows, row, split);
+    if ((row & ~31) < rows) {
 #pragma unroll 1
-    for (int j = 0; j < kXDim / 32; ++j) {
-      uint32_t r[32];
-      tc::tmem_ld32(o_tmem + j * 32, r);
-      tc::tmem_ld_wait<32>(r);
-      float o[32];
+      for (int j = 0; j < kXDim / 32; ++j) {
+        uint32_t r[32];
+        tc::tmem_ld32(o_tmem + j * 32, r);
+        tc::tmem_ld_wait<32>(r);
+        float o[32];
 #pragma unroll
-      for (int n = 0; n < 32; ++n) o[n] = __uint_as_float(r[n]) * inv;
-      const int d0 = j * 32;
-      if (row < rows) {
-        if (p.num_splits > 1) {
-          store_out32(reinterpret_cast<uint8_t*>(ws_row + d0), PTH_ATTN_F32, o);
-        } else {
-          store_out32(out_row + d0 * (p.out_dtype == PTH_ATTN_F32 ? 4 : 2), p.out_dtype, o);
-        }
+        for (int n = 0; n < 32; ++n) o[n] = __uint_as_float(r[n]) * inv;
+        write_rows32(dst, j * 32, stage, o);
       }
     }
-    if (row < rows) {
-      const float lse2 = l > 0.f ? m_ref - kPGain + log2f(l) : -INFINITY;
-      if (p.num_splits > 1) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
-                                  (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = lse2;
-      } else if (p.lse_out != nullptr) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) + (int64_t)token * p.lse_stride_token +
-                                  (int64_t)head * p.lse_stride_head) = lse2 * kLn2;
-      }
-    }
+    if (row < rows && (p.num_splits > 1 || p.lse_out != nullptr)) write_lse(p, t, kvh, row, split, l > 0.f ? m_ref - kPGain + log2f(l) : -INFINITY);
   }
 
   if (p.late_wait) pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
+  if (warp == kXLoadWarp) tc::tmem_dealloc(tmem_base, 512);
   if (tid == 0 && *abort_flag) atomicOr(&g_rows2_status, 4u);
   (void)ok;
 }

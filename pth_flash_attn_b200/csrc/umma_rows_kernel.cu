@@ -68,12 +68,13 @@ struct RLayout {
   static constexpr int qimg = vst + kRNS * kRVStage;
   static constexpr int raw = qimg + kQImageBytes;
   static constexpr int ksc = raw + kRNR * kRawHalfBytes;       // KeyScales<128> [kRKsRing]
-  static constexpr int park_m = ksc + kRKsRing * (int)sizeof(KeyScales<kTileKeys>); // float [128]
-  static constexpr int park_l = park_m + kRGroup * 4;          // float [128]
-  static constexpr int bars = park_l + kRGroup * 4;            // uint64 [...]
+  static constexpr int park_m = ksc + kRKsRing * (int)sizeof(KeyScales<kTileKeys>); // float [2 groups][128]
+  static constexpr int park_l = park_m + 2 * kRGroup * 4;      // float [2 groups][128]
+  static constexpr int fix = park_l + 2 * kRGroup * 4;         // float [128], see QueryScale
+  static constexpr int bars = fix + kRGroup * 4;               // uint64 [...]
   static constexpr int n_bars = kRNS * 2 + 2 * kRNK + 6 + 2 * kRNR;
   static constexpr int misc = bars + n_bars * 8;
-  static constexpr int total = misc + 32;
+  static constexpr int total = misc + 32 + 4 * kRowsItemInts;
 };
 
 template <int kRNK, int kRNR>
@@ -115,107 +116,13 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   rows_cta(p, &kvh, &tile_index);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (!p.late_wait) pdl_wait();
-  // Row tile of this CTA: bisect a shared-memory copy of query_start_loc when it fits.
-  constexpr int kQslCache = 4096;
-  static_assert(kRNR * kRawHalfBytes >= 2 * kQslCache * 4, "the raw ring holds the copies of query_start_loc and seq_lens");
-  RowTile t;
-  if (p.tile_map == 0 && p.num_reqs + 1 <= kQslCache) {
-    int* qsl_s = reinterpret_cast<int*>(smem + L::raw);
-    int* len_s = qsl_s + kQslCache;
-    for (int i = tid; i <= p.num_reqs; i += kRThreads) {
-      qsl_s[i] = __ldg(p.query_start_loc + i);
-      if (i < p.num_reqs) len_s[i] = __ldg(p.seq_lens + i);
-    }
-    __syncthreads();
-    t = resolve_row_tile_with(p, tile_index, [&](int i) { return qsl_s[i]; }, [&](int r) { return len_s[r]; });
-    tc::fence_async_smem();  // (page copies write here next, through the other proxy)
-    __syncthreads();
-  } else {
-    t = resolve_row_tile(p, tile_index);
+  // Barriers and TMEM are set up by the warps that wait for nothing else.
+  if (warp == kRLoadWarp) {
+    if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
+    tc::tmem_alloc(tslot, 512);
+    tc::tmem_relinquish();
   }
-  if (t.req < 0) {
-    if (p.late_wait) pdl_wait();
-    return;
-  }
-  const int rows = t.ntok * p.group;  // <= 128 by construction of bq
-  // num_splits is a bound: the pieces a request is cut into are chosen here, from the lengths,
-  // by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the
-  // whole launch, so a prefill chunk among long decode requests is not cut at all.  CTAs of
-  // unused pieces leave at once; the CTA of piece 0 marks them as holding no keys.
-  int nsplits = p.num_splits;
-  if (p.num_splits > 1) {
-    unsigned long long* total_s = reinterpret_cast<unsigned long long*>(smem + L::misc + 16);
-    if (tid == 0) *total_s = 0ull;
-    __syncthreads();
-    SchedShape shape;
-    shape.group = p.group;
-    shape.num_kv_heads = p.num_kv_heads;
-    shape.bq = p.bq;
-    shape.num_splits = p.num_splits;
-    shape.window = p.window;
-    shape.causal = p.causal;
-    shape.row_class = p.row_class;
-    shape.class_rows = p.class_rows;
-    unsigned long long w = 0;
-    for (int r = tid; r < p.num_reqs; r += kRThreads) {
-      const int q0 = __ldg(p.query_start_loc + r), q1 = __ldg(p.query_start_loc + r + 1);
-      w += (unsigned long long)req_row_tiles(shape, q1 - q0) *
-           (unsigned long long)req_kv_tiles(shape, q1 - q0, __ldg(p.seq_lens + r));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-    if (lane == 0 && w != 0) atomicAdd(total_s, w);
-    __syncthreads();
-    const int t_star = item_tiles(*total_s * (unsigned long long)p.num_kv_heads, p.num_sms);
-    nsplits = req_splits(req_kv_tiles(shape, t.q_len, t.seq_len), t_star, p.num_splits);
-    if (split >= nsplits) {
-      if (p.late_wait) pdl_wait();
-      return;
-    }
-    if (split == 0) {
-      for (int i = tid; i < rows * (p.num_splits - nsplits); i += kRThreads) {
-        int token, head;
-        row_target(p, t, kvh, i % rows, &token, &head);
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)(nsplits + i / rows) * p.ws_lse_stride_split +
-                                  (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = -INFINITY;
-      }
-    }
-    __syncthreads();  // the scratch word is part of a region the barriers are initialised in next
-  }
-  int tile_begin, tile_end, range_begin, range_end;
-  split_tiles(p, t, split, nsplits, &tile_begin, &tile_end, &range_begin, &range_end);
-
-  if (tile_begin >= tile_end) {
-    // No keys for this work item: zero output, log-sum-exp -inf.
-    for (int idx = tid; idx < rows * kHeadDim; idx += kRThreads) {
-      const int n = idx >> 7, d = idx & 127;
-      int token, head;
-      row_target(p, t, kvh, n, &token, &head);
-      if (p.num_splits == 1) {
-        store_out_elem(p.out + (int64_t)token * p.out_stride_token + (int64_t)head * p.out_stride_head, d, p.out_dtype, 0.f);
-      } else {
-        reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
-                                 (int64_t)token * p.ws_o_stride_token + (int64_t)head * p.ws_o_stride_head)[d] = 0.f;
-      }
-    }
-    if (tid < rows) {
-      int token, head;
-      row_target(p, t, kvh, tid, &token, &head);
-      if (p.num_splits > 1) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
-                                  (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = -INFINITY;
-      } else if (p.lse_out != nullptr) {
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) + (int64_t)token * p.lse_stride_token +
-                                  (int64_t)head * p.lse_stride_head) = -INFINITY;
-      }
-    }
-    if (p.late_wait) pdl_wait();
-    return;
-  }
-
-  const int n_tiles = tile_end - tile_begin;
-  if (tid == 0) {
+  if (warp == kRMmaWarp && lane == 0) {
     for (int s = 0; s < kRNS; ++s) {
       tc::mbar_init(&bars[B::vfull + s], kRProducers / 2);
       tc::mbar_init(&bars[B::vempty + s], 1);
@@ -236,14 +143,57 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     *abort_flag = 0;
     tc::mbar_init_fence();
   }
-  if (warp == 0) {
-    tc::tmem_alloc(tslot, 512);
-    tc::tmem_relinquish();
+  if (!p.late_wait) pdl_wait();
+  // Row tile of this CTA: warp 0 finds it; for longer lists of requests all threads bisect a shared-memory copy of
+  // query_start_loc when it fits.
+  constexpr int kQslCache = 4096;
+  static_assert(kRNR * kRawHalfBytes >= 2 * kQslCache * 4, "the raw ring holds the copies of query_start_loc and seq_lens");
+  RowsItem item;
+  int* item_s = reinterpret_cast<int*>(smem + L::misc + 32);
+  const bool by_warp = p.num_reqs <= kWarpRequests && p.tile_map == 0;
+  if (by_warp) {
+    if (warp == 0) {
+      unsigned long long work = 0;
+      const RowTile found = warp_row_tile(p, tile_index, p.num_splits > 1, sched_shape(p), &work);
+      item = rows_item(p, found, split, work);
+      if (lane == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
+    }
+  } else {
+    RowTile t;
+    if (p.tile_map == 0 && p.num_reqs + 1 <= kQslCache) {
+      int* qsl_s = reinterpret_cast<int*>(smem + L::raw);
+      int* len_s = qsl_s + kQslCache;
+      for (int i = tid; i <= p.num_reqs; i += kRThreads) {
+        qsl_s[i] = __ldg(p.query_start_loc + i);
+        if (i < p.num_reqs) len_s[i] = __ldg(p.seq_lens + i);
+      }
+      __syncthreads();
+      t = resolve_row_tile_with(p, tile_index, [&](int i) { return qsl_s[i]; }, [&](int r) { return len_s[r]; });
+      tc::fence_async_smem();  // (page copies write here next, through the other proxy)
+      __syncthreads();
+    } else {
+      t = resolve_row_tile(p, tile_index);
+    }
+    const unsigned long long work = p.num_splits > 1 ? cta_work<kRThreads>(p, smem + L::misc + 16) : 0ull;
+    item = rows_item(p, t, split, work);
+    if (tid == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
   }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tslot;
+  item = *reinterpret_cast<const RowsItem*>(item_s);
+  if (item.state != 1 || (split == 0 && item.nsplits < p.num_splits)) write_empty<kRThreads, kHeadDim>(p, item, kvh, split);
+  if (item.state != 1) {
+    if (warp == kRLoadWarp) tc::tmem_dealloc(tmem_base, 512);
+    if (p.late_wait) pdl_wait();
+    return;
+  }
+  const RowTile& t = item.t;
+  const int rows = item.rows;  // <= 128 by construction of bq
+  const int tile_begin = item.tile_begin, tile_end = item.tile_end, range_begin = item.range_begin, range_end = item.range_end;
+
+  const int n_tiles = tile_end - tile_begin;
   const uint32_t kimg_s = tc::smem_u32(smem + L::kimg), vst_s = tc::smem_u32(smem + L::vst);
   bool ok = true;
 
@@ -463,32 +413,14 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     const uint32_t s_half = tmem_base + g * 64 + lane_addr;         // this group's columns of S buffer 0
     const uint32_t o_tmem = tmem_base + 256 + g * 128 + lane_addr;  // O(g)
 
-    // ---- Q image: thread (row, half) converts 8 of the 16 d-chunks of its row ----
-    float q_fix = 1.0f;  // what the row's scores are multiplied by (QueryScale)
-    {
-      const int half = tid >> 7;
-      int token, head;
-      row_target(p, t, kvh, row, &token, &head);
-      const uint4* src = reinterpret_cast<const uint4*>(p.q + (int64_t)token * p.q_stride_token +
-                                                        (int64_t)head * p.q_stride_head) + half * 8;
-      uint4 qv[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) qv[c] = row < rows ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
-      if (p.q_dtype == PTH_ATTN_BF16) {
-        uint32_t* part = reinterpret_cast<uint32_t*>(half == 0 ? park_m : park_l);  // (idle until the epilogue)
-        const uint32_t mine = finite_amax_bf16(qv);
-        part[row] = mine;
-        named_barrier(4, kRSoftmax);
-        const QueryScale qs = query_scale(max(mine, reinterpret_cast<const uint32_t*>(half == 0 ? park_l : park_m)[row]));
-        q_fix = qs.fix;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) qv[c] = queries_to_f16(qv[c], qs.scale);
-      }
-#pragma unroll
-      for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(qimg + (half * 8 + c) * kChunkStride + row * 16) = qv[c];
-    }
+    // ---- Q image: a warp converts 16 rows ----
+    float* fix_s = reinterpret_cast<float*>(smem + L::fix);
+    stage_queries<kHeadDim, 16>(p, t, kvh, rows, 16 * warp,
+        [&](int n, int block, const uint4& v) { *reinterpret_cast<uint4*>(qimg + block * kChunkStride + n * 16) = v; },
+        [&](int n, float fix) { fix_s[n] = fix; });
     tc::fence_async_smem();
     named_barrier(5, kRQBarrier);  // Q image complete; the QK issuer may start
+    const float q_fix = fix_s[row];  // what the row's scores are multiplied by (QueryScale)
 
     int rlo = 0, rhi = -1;  // visible keys of this row (none for a padding row)
     if (row < rows) visible_range(p, t, t.first_idx + row / p.group, &rlo, &rhi);
@@ -582,81 +514,45 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     // (the commit after the last PV covers every MMA issued before it)
     ok &= wait_or_abort(&bars[B::pv_done + ((n_tiles - 1) & 1)], ((n_tiles - 1) >> 1) & 1, abort_flag);
     tc::fence_after_sync();
-    // Group 1 hands its state to group 0 through 64 KB of shared memory that is idle by
-    // now: the K images if they are large enough (every QK has completed once the last
-    // tile's K image has been released), else the raw ring (every producer has read it
-    // once the last tile's images are full).
-    constexpr int kParkBytes = kRGroup * kHeadDim * 4;
-    constexpr bool kParkInK = kRNK * kWideBytes >= kParkBytes;
-    static_assert(kParkInK || kRNR * kRawHalfBytes >= kParkBytes, "no idle region holds the parked accumulator");
-    float* park = reinterpret_cast<float*>(smem + (kParkInK ? L::kimg : L::raw));  // [d][row] fp32
-    if (g == 1) {
-      if constexpr (kParkInK) {
-        ok &= wait_or_abort(&bars[B::kempty + (n_tiles - 1) % kRNK], ((n_tiles - 1) / kRNK) & 1, abort_flag);
-      } else {
-        ok &= wait_or_abort(&bars[B::vfull + (n_tiles - 1) % kRNS], ((n_tiles - 1) / kRNS) & 1, abort_flag);
-        ok &= wait_or_abort(&bars[B::kfull + (n_tiles - 1) % kRNK], ((n_tiles - 1) / kRNK) & 1, abort_flag);
-      }
-      park_m[row] = m_ref;
-      park_l[row] = l;
-#pragma unroll 1
-      for (int j = 0; j < 4; ++j) {
-        uint32_t r[32];
-        tc::tmem_ld32(o_tmem + j * 32, r);
-        tc::tmem_ld_wait<32>(r);
-#pragma unroll
-        for (int n = 0; n < 32; ++n) park[(j * 32 + n) * kRGroup + row] = __uint_as_float(r[n]);
-      }
-    }
+    // A row's two accumulators are in the same TMEM lane: either group reads both for its half of the columns, and
+    // only maximum and sum go through shared memory.
+    park_m[g * kRGroup + row] = m_ref;
+    park_l[g * kRGroup + row] = l;
     named_barrier(4, kRSoftmax);
-    if (g == 0) {
-      const float m1 = park_m[row], l1 = park_l[row];
-      const float m = fmaxf(m_ref, m1);
-      const float c0 = m_ref == -INFINITY ? 0.f : ex2f(m_ref - m);
-      const float c1 = m1 == -INFINITY ? 0.f : ex2f(m1 - m);
-      const float lsum = l * c0 + l1 * c1;
-      const float inv = lsum > 0.f ? 1.0f / lsum : 0.f;
-      int token, head;
-      row_target(p, t, kvh, row, &token, &head);
-      uint8_t* out_row = p.out + (int64_t)token * p.out_stride_token + (int64_t)head * p.out_stride_head;
-      float* ws_row = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_o) + (int64_t)split * p.ws_o_stride_split +
-                                               (int64_t)token * p.ws_o_stride_token + (int64_t)head * p.ws_o_stride_head);
+    const float m0 = park_m[row], m1 = park_m[kRGroup + row], l0 = park_l[row], l1 = park_l[kRGroup + row];
+    const float m = fmaxf(m0, m1);
+    const float c0 = m0 == -INFINITY ? 0.f : ex2f(m0 - m);
+    const float c1 = m1 == -INFINITY ? 0.f : ex2f(m1 - m);
+    const float lsum = l0 * c0 + l1 * c1;
+    const float inv = lsum > 0.f ? 1.0f / lsum : 0.f;
+    // (the Q image is idle: every QK has completed)
+    uint8_t* stage = qimg + warp * 4096;
+    static_assert(8 * 4096 <= kQImageBytes, "room for every warp's rows");
+    const RowsOut dst = rows_out(p, t, kvh, rows, row, split);
+    if ((row & ~31) < rows) {
 #pragma unroll 1
-      for (int j = 0; j < 4; ++j) {
-        uint32_t r[32];
-        tc::tmem_ld32(o_tmem + j * 32, r);
-        tc::tmem_ld_wait<32>(r);
+      for (int j = 2 * g; j < 2 * g + 2; ++j) {
+        uint32_t r0[32], r1[32];
+        tc::tmem_ld32(tmem_base + 256 + lane_addr + j * 32, r0);
+        tc::tmem_ld32(tmem_base + 384 + lane_addr + j * 32, r1);
+        tc::tmem_ld_wait<32>(r0);
+        tc::tmem_landed<32>(r1);
         float o[32];
 #pragma unroll
         for (int n = 0; n < 32; ++n) {
-          const float o1 = c1 > 0.f ? park[(j * 32 + n) * kRGroup + row] * c1 : 0.f;
-          o[n] = (__uint_as_float(r[n]) * c0 + o1) * inv;
+          const float o1 = c1 > 0.f ? __uint_as_float(r1[n]) * c1 : 0.f;
+          o[n] = (__uint_as_float(r0[n]) * c0 + o1) * inv;
         }
-        if (row < rows) {
-          if (p.num_splits > 1) {
-            store_out32(reinterpret_cast<uint8_t*>(ws_row + j * 32), PTH_ATTN_F32, o);
-          } else {
-            store_out32(out_row + (j * 32) * (p.out_dtype == PTH_ATTN_F32 ? 4 : 2), p.out_dtype, o);
-          }
-        }
-      }
-      if (row < rows) {
-        const float lse2 = lsum > 0.f ? m - kPGain + log2f(lsum) : -INFINITY;
-        if (p.num_splits > 1) {
-          *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.ws_lse) + (int64_t)split * p.ws_lse_stride_split +
-                                    (int64_t)token * p.ws_lse_stride_token + (int64_t)head * p.ws_lse_stride_head) = lse2;
-        } else if (p.lse_out != nullptr) {
-          *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) + (int64_t)token * p.lse_stride_token +
-                                    (int64_t)head * p.lse_stride_head) = lse2 * kLn2;
-        }
+        write_rows32(dst, j * 32, stage, o);
       }
     }
+    if (g == 0 && row < rows && (p.num_splits > 1 || p.lse_out != nullptr)) write_lse(p, t, kvh, row, split, lsum > 0.f ? m - kPGain + log2f(lsum) : -INFINITY);
   }
 
   if (p.late_wait) pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
+  if (warp == kRLoadWarp) tc::tmem_dealloc(tmem_base, 512);
   if (tid == 0 && *abort_flag) atomicOr(&g_rows_status, 4u);
   (void)ok;
 }
