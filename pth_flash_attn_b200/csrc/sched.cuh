@@ -79,7 +79,7 @@ PTHB_HD void visible_bounds(int window, int causal, int seq_len, int q_len, int 
 PTHB_HD int req_row_tiles(const SchedShape& s, int q_len) {
   if (q_len <= 0) return 0;
   if (s.row_class != 0 && (((int64_t)q_len * s.group <= s.class_rows) != (s.row_class == 1))) return 0;
-  return (q_len + s.bq - 1) / s.bq;
+  return q_len <= s.bq ? 1 : (q_len + s.bq - 1) / s.bq;
 }
 
 // KV tiles the rows of a request touch together.
@@ -123,10 +123,11 @@ struct ItemCoord {
 };
 PTHB_HD ItemCoord item_coord(int local, int num_kv_heads, int splits) {
   ItemCoord c;
-  c.kvh = local % num_kv_heads;
-  const int rest = local / num_kv_heads;
-  c.split = rest % splits;
-  c.row_tile = rest / splits;
+  // (unsigned, and no division for the one row tile that most requests have: the first item waits for it)
+  const unsigned rest = (unsigned)local / (unsigned)num_kv_heads;
+  c.kvh = (int)((unsigned)local - rest * (unsigned)num_kv_heads);
+  c.row_tile = rest < (unsigned)splits ? 0 : (int)(rest / (unsigned)splits);
+  c.split = (int)rest - c.row_tile * splits;
   return c;
 }
 
@@ -150,10 +151,11 @@ PTHB_HD void split_tile_span(int range_begin, int range_end, int split, int spli
 }
 
 // ---- ranges ----
-// KV tiles per CTA from which a launch is dealt out in ranges.  Below, a CTA's share is a few short pieces, whose ends
-// cost more than the balance gives: 8 x 8,192 keys of 8 heads (27 tiles per CTA) 46.1 us in ranges, 45.1 in equal
-// pieces; 60 x U[1, 988] (14 tiles) 55.3 and 51.3; 64 x U[1, 4096] (60 tiles) 89.7 and 96.8.
-constexpr int kRangeTilesMin = 32;
+// KV tiles per CTA from which a launch is dealt out in ranges.  Below, a CTA's share is one or two pieces, and cuts that
+// ignore the ends of requests make them three.  Equal pieces against ranges: 16 x U[1, 4096] keys of 8 heads (16 tiles
+// per CTA) 31.7 and 24.1 us, 16 x U[1, 8192] at 64 dims 48.1 and 34.4, 69 x U[1, 951] at 256 dims (15 tiles) 48.4 and 42.5,
+// 8 x 8,192 34.2 and 34.7, 60 x U[1, 988] at 8 rows (14 tiles) 31.9 and 34.1; 8 x U[1, 4096] (8 tiles) 17.7 and 18.5.
+constexpr int kRangeTilesMin = 12;
 constexpr int kRangeGroupsMax = 160;   // groups a scheduler warp holds the cuts of
 
 struct RangeSched {

@@ -241,9 +241,9 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::misc + 8);
   // (each warp's part of the launch's work and its longest row tile, in the softmax's scratch until the roles begin)
-  unsigned long long* work_s = reinterpret_cast<unsigned long long*>(smem + L::wred);
-  int* longest_s = reinterpret_cast<int*>(smem + L::wred + 8 * 32);
-  static_assert(2 * 2 * 4 * L::wred_row * 4 >= 12 * 32, "room for the parts of every warp");
+  uint32_t* work_s = reinterpret_cast<uint32_t*>(smem + L::wred);
+  int* longest_s = reinterpret_cast<int*>(smem + L::wred + 4 * 32);
+  static_assert(2 * 2 * 4 * L::wred_row * 4 >= 8 * 32, "room for the parts of every warp");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   SchedShape shape;
@@ -305,17 +305,22 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     pre_q1 = __ldg(p.query_start_loc + lane + 1);
     pre_len = __ldg(p.seq_lens + lane);
   }
-  unsigned long long work = 0;
+  // KV tiles of the launch per head, in 32 bits: a thread's part is capped where 268 million keys of one head would be,
+  // and a launch that meets the cap is not dealt out in ranges, which need the exact sum.
+  constexpr uint32_t kWorkCap = 1u << 21;
+  uint32_t work = 0;
   int longest = 0;
   bool served = false;
+#pragma unroll 1
   for (int r = tid; r < p.num_reqs; r += kThreads) {
     const int q0 = __ldg(p.query_start_loc + r), q1 = __ldg(p.query_start_loc + r + 1);
     const int len = __ldg(p.seq_lens + r);
     const int row_tiles = req_row_tiles(shape, q1 - q0);
     const int kv_tiles = req_kv_tiles(shape, q1 - q0, len);
-    work += (unsigned long long)row_tiles * (unsigned long long)kv_tiles;
+    const unsigned long long all = (unsigned long long)row_tiles * (unsigned long long)kv_tiles + work;
+    work = all < kWorkCap ? (uint32_t)all : kWorkCap;
     // (a request without keys has a result but no tiles: such a launch is not dealt out in ranges)
-    if (row_tiles > 0) longest = max(longest, kv_tiles > 0 ? kv_tiles : 0x7fffffff);
+    if (row_tiles > 0) longest = max(longest, kv_tiles > 0 && work < kWorkCap ? kv_tiles : 0x7fffffff);
     served |= row_tiles > 0;
   }
   // A prefill launch whose requests are all tall has nothing for this kernel: its CTAs leave before any set-up.
@@ -324,9 +329,7 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     set_up();
   }
   {
-    unsigned long long w = work;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    const uint32_t w = __reduce_add_sync(0xffffffffu, work);
     const int n = __reduce_max_sync(0xffffffffu, longest);
     if (lane == 0) {
       work_s[warp] = w;
@@ -365,9 +368,8 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
     // Walks the requests in blocks of 32 (lane l holds request base + l and the items of the
     // requests before it), so this CTA's items c, c + CTAs, ... are found in one pass.
     const int S = p.num_splits, hkv = p.num_kv_heads;
-    unsigned long long total = lane < kThreads / 32 ? work_s[lane] : 0ull;  // (every CTA computes the same number)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    // (every CTA computes the same number; at most 20 warps x 32 threads x 2^21)
+    const unsigned long long total = __reduce_add_sync(0xffffffffu, lane < kThreads / 32 ? work_s[lane] : 0u);
     const int row_tile_max = __reduce_max_sync(0xffffffffu, lane < kThreads / 32 ? longest_s[lane] : 0);
     const RangeSched ranges = range_sched(total, row_tile_max, hkv, (int)gridDim.x, S);
     const bool ranged = ranges.work != 0;
@@ -454,11 +456,12 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
             blk_first = 0;
             load_block(0);
           }
-          while (at >= blk_first + blk_total) {  // (the sequence does not end before run_hi)
+          while (at >= blk_first + blk_total && base < p.num_reqs) {
             blk_first += blk_total;
             base += 32;
             load_block(base);
           }
+          if (base >= p.num_reqs) break;  // (never: the sequence does not end before run_hi)
           const int rel = (int)(at - blk_first);
           const bool mine = rel >= my_excl && rel < my_excl + my_n;
           const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
