@@ -15,11 +15,13 @@
 // cell, and the row maximum is a reduction over 16 lanes.  A warp issues the loads of two to four cells before it
 // uses any, which leaves the quantisation's instructions as the bound (2 T Hkv D source elements in, T Hkv (2 D + 8)
 // bytes out, at 0.56 of the rate of a copy).
-// 8,192 tokens of 8 KV heads x 128 dims in bf16 (51 MB): 14 us in a graph, 3.7 TB/s; 19 us a call, of which the
-// caller's side is 11 (one warp per row with 2-byte loads, fourteen rows after another: 43 us a call).
+// 8,192 tokens of 8 KV heads x 128 dims in bf16 (51 MB): 12.0 us a call back to back, 4.2 TB/s.  (One warp per row with
+// 2-byte loads, fourteen rows after another: 43 us; with this shape, but maxima and scaling one element at a time, at 77
+// registers and as an ordinary launch: 14.5, of which 1.4 were the launch; 40 registers spill: 15.3.)
 #include <type_traits>
 
 #include "params.cuh"
+#include "pdl.cuh"
 
 namespace pthb200 {
 namespace {
@@ -66,8 +68,46 @@ struct Four {
   }
 };
 
+// Two fp32 lanes per instruction; each rounds as the instruction for one does.
+__device__ __forceinline__ unsigned long long pair(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void mul2(float& a, float& b, float by) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair(a, b)), "l"(pair(by, by)));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ void add2(float& a, float& b, float x, float y) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair(a, b)), "l"(pair(x, y)));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+
+// Four elements to int8: scaled, rounded half away from zero.  kFinite: all of the row are finite, and with the scale of
+// their own maximum none reaches 127.5 by more than its rounding (inv <= 127 (1 + 2^-22) / amax), so nothing clamps
+// them; an infinite row has inv = 0 and its infinities turn NaN, which the clamp makes -128 as a NaN is anywhere.
+template <bool kFinite, Source kSource>
+__device__ __forceinline__ uint32_t quantised(const Four<kSource>& x, float inv, int dtype) {
+  int q[4];
+#pragma unroll
+  for (int e = 0; e < 4; e += 2) {
+    float a = x.get(e, dtype), b = x.get(e + 1, dtype);
+    mul2(a, b, inv);
+    add2(a, b, copysignf(0.5f, a), copysignf(0.5f, b));
+    if constexpr (!kFinite) {
+      a = fminf(fmaxf(a, -128.0f), 127.0f);
+      b = fminf(fmaxf(b, -128.0f), 127.0f);
+    }
+    q[e] = __float2int_rz(a);
+    q[e + 1] = __float2int_rz(b);
+  }
+  return __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+}
+
 template <int D, Source kSource>
-__global__ void __launch_bounds__(kWriterThreads) kv_writer_kernel(const WriterParams p) {
+__global__ void __launch_bounds__(kWriterThreads, kSource == kAny ? 1 : 5) kv_writer_kernel(const WriterParams p) {
   constexpr int kCells = cells_in_flight(D);
   constexpr int kRuns = D / (4 * kRowLanes);  // runs of 64 elements per row
   const int lane = threadIdx.x & 31, rl = lane & (kRowLanes - 1);
@@ -75,6 +115,7 @@ __global__ void __launch_bounds__(kWriterThreads) kv_writer_kernel(const WriterP
   const int64_t warp = ((int64_t)blockIdx.x * kWriterThreads + threadIdx.x) >> 5;
   const int64_t warps = ((int64_t)gridDim.x * kWriterThreads) >> 5;
   const int64_t cells = (int64_t)p.num_tokens * p.num_kv_heads;
+  pdl_wait();
   const uint8_t* src0 = is_v ? p.value : p.key;
   const int64_t src_token = is_v ? p.value_stride_token : p.key_stride_token;
   const int64_t src_head = is_v ? p.value_stride_head : p.key_stride_head;
@@ -112,17 +153,42 @@ __global__ void __launch_bounds__(kWriterThreads) kv_writer_kernel(const WriterP
     }
     const int64_t dst_off = block * rows.stride_block + pos * rows.stride_slot + head * rows.stride_head;
     const uint32_t skipped = __ballot_sync(0xffffffffu, slot < 0);  // bit c: cell c
+    // Largest magnitude of each cell's row.  Of 16-bit values as whole numbers, two at a time; an infinity or a NaN, which
+    // does not count here, sends the warp's cells the long way.
     float amax_mine = 0.f;
+    bool finite = kSource != kAny;
+    if constexpr (kSource != kAny) {
+      uint32_t bits_mine = 0u, top = 0u;
 #pragma unroll
-    for (int c = 0; c < kCells; ++c) {
-      float amax = 0.f;
+      for (int c = 0; c < kCells; ++c) {
+        uint32_t m = 0u;
 #pragma unroll
-      for (int r = 0; r < kRuns; ++r)
+        for (int r = 0; r < kRuns; ++r) m = __vimax3_u16x2(m, x[c][r].w[0] & 0x7fff7fffu, x[c][r].w[1] & 0x7fff7fffu);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) amax = fmaxf(amax, fabsf(x[c][r].get(e, p.src_dtype)));
+        for (int o = kRowLanes / 2; o > 0; o >>= 1) m = __vmaxu2(m, __shfl_xor_sync(0xffffffffu, m, o));
+        m = max(m & 0xffffu, m >> 16);
+        top = max(top, m);
+        if (c_mine == c) bits_mine = m;
+      }
+      finite = !__any_sync(0xffffffffu, top >= (kSource == kBf16 ? 0x7f80u : 0x7c00u));
+      amax_mine = kSource == kBf16 ? __uint_as_float(bits_mine << 16) : __half2float(__ushort_as_half((unsigned short)bits_mine));
+    }
+    if (!finite) {
+#pragma unroll 1
+      for (int c = 0; c < kCells; ++c) {
+        float amax = 0.f;
 #pragma unroll
-      for (int o = kRowLanes / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      if (c_mine == c) amax_mine = amax;
+        for (int k = 0; k < kCells; ++k) {
+          if (k != c) continue;
+#pragma unroll
+          for (int r = 0; r < kRuns; ++r)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) amax = fmaxf(amax, fabsf(x[k][r].get(e, p.src_dtype)));
+        }
+#pragma unroll
+        for (int o = kRowLanes / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if (c_mine == c) amax_mine = amax;
+      }
     }
     const float scale_mine = fmaxf(__fdiv_rn(amax_mine, 127.0f), 1e-6f);
     const float inv_mine = __fdiv_rn(1.0f, scale_mine);
@@ -136,17 +202,9 @@ __global__ void __launch_bounds__(kWriterThreads) kv_writer_kernel(const WriterP
       uint8_t* dst = const_cast<uint8_t*>(rows.data) + __shfl_sync(0xffffffffu, dst_off, c, kRowLanes);
       if (skipped >> c & 1u) continue;  // (the same for all lanes)
 #pragma unroll
-      for (int r = 0; r < kRuns; ++r) {
-        uint32_t word = 0;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float v = __fmul_rn(x[c][r].get(e, p.src_dtype), inv);
-          v = __fadd_rn(v, copysignf(0.5f, v));
-          v = fminf(fmaxf(v, -128.0f), 127.0f);
-          word |= (uint32_t)(uint8_t)(int8_t)__float2int_rz(v) << (8 * e);
-        }
-        reinterpret_cast<uint32_t*>(dst)[r * kRowLanes + rl] = word;
-      }
+      for (int r = 0; r < kRuns; ++r)
+        reinterpret_cast<uint32_t*>(dst)[r * kRowLanes + rl] =
+            finite ? quantised<true>(x[c][r], inv, p.src_dtype) : quantised<false>(x[c][r], inv, p.src_dtype);
     }
   }
 }
@@ -182,22 +240,18 @@ cudaError_t launch_kv_writer(const PthB200WriteArgs& a, cudaStream_t stream) {
                       on8(a.value, a.value_stride_token, a.value_stride_head);
   auto launch = [&](auto head_size) {
     constexpr int D = decltype(head_size)::value;
-    if (vector && a.src_dtype == PTH_ATTN_BF16) kv_writer_kernel<D, kBf16><<<grid, kWriterThreads, 0, stream>>>(p);
-    else if (vector) kv_writer_kernel<D, kF16><<<grid, kWriterThreads, 0, stream>>>(p);
-    else kv_writer_kernel<D, kAny><<<grid, kWriterThreads, 0, stream>>>(p);
+    if (vector && a.src_dtype == PTH_ATTN_BF16) return pdl_launch(kv_writer_kernel<D, kBf16>, grid, kWriterThreads, 0, stream, p);
+    if (vector) return pdl_launch(kv_writer_kernel<D, kF16>, grid, kWriterThreads, 0, stream, p);
+    return pdl_launch(kv_writer_kernel<D, kAny>, grid, kWriterThreads, 0, stream, p);
   };
   switch (a.head_size) {
     case 64:
-      launch(std::integral_constant<int, 64>{});
-      break;
+      return launch(std::integral_constant<int, 64>{});
     case 128:
-      launch(std::integral_constant<int, 128>{});
-      break;
+      return launch(std::integral_constant<int, 128>{});
     default:
-      launch(std::integral_constant<int, 256>{});
-      break;
+      return launch(std::integral_constant<int, 256>{});
   }
-  return cudaGetLastError();
 }
 
 }  // namespace pthb200
