@@ -65,6 +65,8 @@ struct KernelParams {
   // Row-major kernels behind the integer kernel of the same call, with whose requests they share nothing: they start
   // beside it and wait for it only before they end (pdl.cuh).
   int32_t late_wait = 0;
+  // Row-major kernels: CTAs of a cluster that share the keys of one row tile among them (1, 2, 4 or 8).
+  int32_t cluster = 1;
 };
 
 // Re-tiles a launch to `bq` query tokens per row tile.  The caller's promise behind

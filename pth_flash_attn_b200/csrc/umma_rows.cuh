@@ -38,6 +38,10 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <atomic>
+#include <type_traits>
+
 #include "params.cuh"
 #include "pdl.cuh"
 #include "sched.cuh"
@@ -169,9 +173,11 @@ __device__ __forceinline__ float ex2f(float x) {
 // another: under a causal mask those are then the first tiles of the first request, its shortest.  (Row tiles
 // in ascending order, head by head: twelve new prompts of 37 to 2,500 tokens ended on the longest tiles of the
 // last of them.)
+template <bool kClusters>
 __device__ __forceinline__ void rows_cta(const KernelParams& p, int* kvh, int* tile_index) {
-  const uint32_t t = blockIdx.x / (uint32_t)p.num_kv_heads;
-  *kvh = (int)(blockIdx.x - t * (uint32_t)p.num_kv_heads);
+  const uint32_t x = kClusters ? blockIdx.x / (uint32_t)p.cluster : blockIdx.x;
+  const uint32_t t = x / (uint32_t)p.num_kv_heads;
+  *kvh = (int)(x - t * (uint32_t)p.num_kv_heads);
   *tile_index = p.num_q_tiles - 1 - (int)t;
 }
 
@@ -228,22 +234,130 @@ __device__ __forceinline__ SchedShape sched_shape(const KernelParams& p) {
   return shape;
 }
 
+// ---- clusters ----
+// A launch of few row tiles (a chunk or a prompt, few KV heads) leaves SMs idle, and its caller need not have reserved a
+// workspace for pieces.  Then the CTAs of a cluster take a row tile together: each walks a run of its keys, leaves maximum,
+// sum and accumulator of every row in its shared memory, and then merges and writes a slice of the columns, reading the
+// others' through distributed shared memory.  The host takes the largest cluster with which the launch still is one round
+// of the SMs (instances of their own: the cluster's code in the others cost twelve short prompts 1.5 %); the CTAs share a
+// row tile of 8 tiles of 128 keys or more, at least two tiles each, and those that are not needed leave.
+// What bounds it: the walk of a piece, then 3 to 4 us for the merge, which reads 128 KB per CTA (at pieces of one tile it
+// cost more than it gave: 200 tokens without a cache 17.7 us in two pieces, 13.4 in one).  One CTA per row tile / clusters:
+// 200 tokens over 30,000 keys, 1 KV head 569 / 58 us, 8 KV heads over 8,000 162 / 57; 300 over 3,000 at 256 dims 65 / 35,
+// two of them at 64 dims, 2 KV heads 68 / 31; 2,000 over 2,000, 1 KV head 86 / 54; 16 over 1,000 17.5 / 14.2.
+constexpr int kClusterMax = 16;
+__host__ __device__ constexpr int cluster_pieces(int tiles, int cluster) {
+  int n = 1;
+  while (tiles >= 8 && 2 * n <= cluster && 4 * n <= tiles) n *= 2;
+  return n;
+}
+// (An SM takes one CTA, and the SMs of a cluster come from one group of them: how many clusters of 8 fit at once is asked.)
+template <auto kKernel>
+int clusters_at_once(int size, int threads, int smem) {
+  static std::atomic<int> known[64][5];  // by device and log2(size): clusters + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::atomic<int>* slot = dev >= 0 && dev < 64 ? &known[dev][size == 2 ? 1 : size == 4 ? 2 : size == 8 ? 3 : 4] : nullptr;
+  if (slot != nullptr && slot->load(std::memory_order_relaxed) != 0) return slot->load(std::memory_order_relaxed) - 1;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)size;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)size);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if ((size > 8 && cudaFuncSetAttribute(kKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&n, kKernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  if (slot != nullptr) slot->store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+template <auto kKernel>
+int cluster_for(const KernelParams& p, int threads, int smem) {
+  if (p.num_splits > 1) return 1;
+  // Tiles of a row tile, as far as the host knows: a row of the block table and the window bound them.  (A row that is
+  // longer than the stride says, or a stride of 0, which says nothing: the CTAs go by the lengths, this only by the time.)
+  int64_t tiles = p.block_table_row_stride > 0 ? (p.block_table_row_stride * p.block_size + 127) / 128 : 0x7fffffff;
+  if (p.window > 0) tiles = std::min(tiles, (int64_t)(p.window + p.bq) / 128 + 2);
+  const int64_t row_tiles = (int64_t)p.num_q_tiles * p.num_kv_heads;
+  const int most = cluster_pieces((int)std::min(tiles, (int64_t)0x7fffffff), kClusterMax);
+  int c = 1;
+  while (2 * c <= most && 2 * c * row_tiles <= p.num_sms && row_tiles <= clusters_at_once<kKernel>(2 * c, threads, smem)) c *= 2;
+  return c;
+}
+// One CTA (kKernel) or one cluster of CTAs (kClustered) per row tile, KV head and piece.
+template <auto kKernel, auto kClustered>
+cudaError_t launch_row_tiles(const KernelParams& p_in, const CUtensorMap& map, int threads, int smem, cudaStream_t stream) {
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    err = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(kClustered, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (err != cudaSuccess) return err;
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+  }
+  KernelParams p = p_in;
+  p.cluster = cluster_for<kClustered>(p, threads, smem);
+  const int64_t ctas = (int64_t)p.num_q_tiles * p.num_kv_heads * p.cluster;
+  if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
+  const dim3 grid((unsigned)ctas, p.num_splits);
+  if (p.cluster > 1) return pdl_launch_clusters(p.cluster, kClustered, grid, threads, smem, stream, p, map);
+  return pdl_launch(kKernel, grid, threads, smem, stream, p, map);
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_address(uint32_t saddr, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+// (between two cluster_sync: nobody writes what is read, so these may be moved among one another)
+__device__ __forceinline__ float peer_load(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ float4 peer_load4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+// Columns d0 .. d0 + 31 of row `tile_row` of an accumulator into park: [dim / 4][kRows][4] fp32.
+template <int kRows>
+__device__ __forceinline__ void park_row32(float* park, int d0, int tile_row, const float (&o)[32]) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    *reinterpret_cast<float4*>(park + ((d0 / 4 + c) * kRows + tile_row) * 4) = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+}
+
 // What a CTA computes: the keys of one piece of a row tile.
 struct RowsItem {
   RowTile t;
   int rows, nsplits;
   int tile_begin, tile_end, range_begin, range_end;
-  int state;  // 0: nothing, 1: keys, 2: rows without keys
+  int state;   // 0: nothing, 1: keys, 2: rows without keys
+  int pieces;  // CTAs of the cluster that share the row tile's keys: this one has piece (rank in the cluster)
 };
 constexpr int kRowsItemInts = sizeof(RowsItem) / 4;
-static_assert(sizeof(RowTile) == 24 && kRowsItemInts == 13, "as the broadcast copies it");
+static_assert(sizeof(RowTile) == 24 && kRowsItemInts == 14, "as the broadcast copies it");
 // num_splits is a bound: the pieces a request is cut into are chosen here, from the lengths and the launch's KV tiles
 // per head, by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the
 // whole launch, so a prefill chunk among long decode requests is not cut at all.
+template <bool kClusters>
 __device__ __forceinline__ RowsItem rows_item(const KernelParams& p, const RowTile& t, int split, unsigned long long work) {
   RowsItem it;
   it.t = t;
   it.state = 0;
+  it.pieces = 1;
   it.rows = it.nsplits = it.tile_begin = it.tile_end = it.range_begin = it.range_end = 0;
   if (t.req < 0) return it;
   it.rows = t.ntok * p.group;
@@ -255,6 +369,16 @@ __device__ __forceinline__ RowsItem rows_item(const KernelParams& p, const RowTi
   }
   split_tiles(p, t, split, it.nsplits, &it.tile_begin, &it.tile_end, &it.range_begin, &it.range_end);
   it.state = it.tile_begin < it.tile_end ? 1 : 2;
+  if constexpr (kClusters) {
+    const int rank = (int)(blockIdx.x & (uint32_t)(p.cluster - 1)), n = it.tile_end - it.tile_begin, first = it.tile_begin;
+    it.pieces = cluster_pieces(n, p.cluster);
+    if (rank >= it.pieces) {
+      it.state = 0;
+    } else if (it.state == 1) {
+      it.tile_begin = first + (int)((int64_t)rank * n / it.pieces);
+      it.tile_end = first + (int)((int64_t)(rank + 1) * n / it.pieces);
+    }
+  }
   return it;
 }
 // The launch's KV tiles per head, summed over the CTA (`scratch`: 8 idle bytes).
@@ -578,6 +702,91 @@ __device__ __forceinline__ void write_lse(const KernelParams& p, const RowTile& 
     *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.lse_out) +
                               row_offset(t, kvh, p.group, inv_group, row, p.lse_stride_token, p.lse_stride_head)) = lse2 * kLn2;
   }
+}
+
+// By the kRows * kParts threads of the softmax (`row`, `part`): the rows of a row tile whose keys `pieces` CTAs of the
+// cluster have walked (a power of two).  This CTA (`rank`) merges and writes the rank-th run of columns from every CTA's
+// parked accumulator (park_row32, relative to the row's maximum there), maxima and sums (stats: [2][kRows]); `weights`:
+// idle shared memory, [kClusterMax][kRows].  Each starts with its own piece, so no CTA is read by all at once, and a
+// thread has four to eight loads under way: a remote load takes many hundred cycles.
+template <int kRows, int kParts, int kDim>
+__device__ __forceinline__ void merge_pieces(const KernelParams& p, const RowTile& t, int kvh, int row, int part, int rank, int pieces,
+                                             const float* park_own, const float* stats_own, float* weights) {
+  const uint32_t park = tc::smem_u32(park_own) + row * 16, stats = tc::smem_u32(stats_own) + row * 4;
+  auto peer = [&](int k) { return (rank + k) & (pieces - 1); };
+  float m = -INFINITY, l = 0.f;
+#pragma unroll 1
+  for (int k0 = 0; k0 < pieces; k0 += 2) {
+    const float a = peer_load(peer_address(stats, peer(k0))), b = peer_load(peer_address(stats, peer(k0 + 1)));
+    m = fmaxf(m, fmaxf(a, b));
+  }
+#pragma unroll 2
+  for (int k = 0; k < pieces; ++k) {
+    const uint32_t from = peer_address(stats, peer(k));
+    const float v = peer_load(from), sum = peer_load(from + kRows * 4);
+    float w = v == -INFINITY ? 0.f : ex2f(v - m);
+    if (sum != sum) w = sum;  // (a NaN among a piece's scores makes the row NaN, whatever its weight)
+    if (w != 0.f) l = fmaf(w, sum, l);
+    weights[k * kRows + row] = w;  // (the same value from every part; read by this thread)
+  }
+  const float inv = l > 0.f ? 1.0f / l : 0.f;
+  uint8_t* dst = p.out + row_offset(t, kvh, p.group, 1.0f / (float)p.group, row, p.out_stride_token, p.out_stride_head);
+  const int blocks = kDim / 4 / pieces, first = rank * blocks;  // 4 columns each
+  // N blocks of columns from K pieces at once
+  auto merge = [&](auto pieces_at_once, auto blocks_at_once) {
+    constexpr int K = decltype(pieces_at_once)::value, N = decltype(blocks_at_once)::value;
+#pragma unroll 1
+    for (int b = part * N; b < blocks; b += kParts * N) {
+      float o[N][4] = {};
+#pragma unroll 1
+      for (int k0 = 0; k0 < pieces; k0 += K) {
+        float4 v[K][N];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const uint32_t from = peer_address(park, peer(k0 + k));
+#pragma unroll
+          for (int n = 0; n < N; ++n) v[k][n] = peer_load4(from + (first + min(b + n, blocks - 1)) * kRows * 16);
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const float w = weights[(k0 + k) * kRows + row];
+          if (w != 0.f) {  // (a NaN counts)
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+              o[n][0] = fmaf(w, v[k][n].x, o[n][0]);
+              o[n][1] = fmaf(w, v[k][n].y, o[n][1]);
+              o[n][2] = fmaf(w, v[k][n].z, o[n][2]);
+              o[n][3] = fmaf(w, v[k][n].w, o[n][3]);
+            }
+          }
+        }
+      }
+      const int d = (first + b) * 4;
+#pragma unroll
+      for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[n][e] *= inv;
+      if (p.out_dtype == PTH_ATTN_F32) {
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+          if (b + n < blocks) *reinterpret_cast<float4*>(dst + (d + 4 * n) * 4) = make_float4(o[n][0], o[n][1], o[n][2], o[n][3]);
+      } else {
+        const bool bf16 = p.out_dtype == PTH_ATTN_BF16;
+#pragma unroll
+        for (int n = 0; n < N; n += 2) {
+          auto two = [&](float x, float y) { return bf16 ? pack_bf16(x, y) : pack_f16(x, y); };
+          const uint2 x = make_uint2(two(o[n][0], o[n][1]), two(o[n][2], o[n][3]));
+          if (b + n + 1 < blocks)  // (then d is a multiple of 8)
+            *reinterpret_cast<uint4*>(dst + (d + 4 * n) * 2) = make_uint4(x.x, x.y, two(o[n + 1][0], o[n + 1][1]), two(o[n + 1][2], o[n + 1][3]));
+          else if (b + n < blocks)
+            *reinterpret_cast<uint2*>(dst + (d + 4 * n) * 2) = x;
+        }
+      }
+    }
+  };
+  if (pieces == 2) merge(std::integral_constant<int, 2>{}, std::integral_constant<int, 2>{});
+  else merge(std::integral_constant<int, 4>{}, std::integral_constant<int, 2>{});
+  if (rank == 0 && part == 0) write_lse(p, t, kvh, row, 0, l > 0.f ? m - kPGain + log2f(l) : -INFINITY);
 }
 
 }  // namespace pthb200

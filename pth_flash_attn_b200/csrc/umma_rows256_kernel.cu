@@ -66,7 +66,10 @@ struct WLayout {
   static constexpr int tile_max = ksc + kWKsRing * (int)sizeof(KeyScales<kWKeys>);  // float [2 tiles][2 groups][128 rows]
   static constexpr int half_sum = tile_max + 2 * 2 * kWGroup * 4;    // float [2 groups][128 rows]
   static constexpr int qstage = half_sum + 2 * kWGroup * 4;          // [8 warps] 32 dims of 32 rows of Q
-  static constexpr int bars = qstage + 8 * 2048;                     // uint64 [...]
+  static constexpr int stats = qstage + 8 * 2048;                    // float [2][128 rows], see merge_pieces
+  static constexpr int bars = stats + 2 * kWGroup * 4;               // uint64 [...]
+  static constexpr int park = kimg;                                  // the images, idle at the end: [256][128 rows] fp32
+  static_assert(kWDim * kWGroup * 4 <= raw, "room for a parked accumulator");
   static constexpr int n_bars = kWNS * 2 + 2 * kWNK + 6 + 2 * kWNR;
   static constexpr int misc = bars + n_bars * 8;
   static constexpr int total = misc + 32 + 4 * kRowsItemInts;
@@ -106,6 +109,7 @@ __device__ __forceinline__ void issue_pv_w(uint32_t o_tmem, uint32_t s_tmem, Row
                    accumulate || g > 0 || kk > 0);
 }
 
+template <bool kClusters>
 __global__ void __launch_bounds__(kWThreads, 1)
 umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __grid_constant__ CUtensorMap tmap) {
   using L = WLayout;
@@ -122,7 +126,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
   KeyScales<kWKeys>* key_scales = reinterpret_cast<KeyScales<kWKeys>*>(smem + L::ksc);
 
   int kvh, tile_index;
-  rows_cta(p, &kvh, &tile_index);
+  rows_cta<kClusters>(p, &kvh, &tile_index);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // Barriers and TMEM are set up by the warps that wait for nothing else.
@@ -164,7 +168,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     if (warp == 0) {
       unsigned long long work = 0;
       const RowTile found = warp_row_tile(p, tile_index, p.num_splits > 1, sched_shape(p), &work);
-      item = rows_item(p, found, split, work);
+      item = rows_item<kClusters>(p, found, split, work);
       if (lane == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
     }
   } else {
@@ -184,7 +188,7 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       t = resolve_row_tile(p, tile_index);
     }
     const unsigned long long work = p.num_splits > 1 ? cta_work<kWThreads>(p, smem + L::misc + 16) : 0ull;
-    item = rows_item(p, t, split, work);
+    item = rows_item<kClusters>(p, t, split, work);
     if (tid == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
   }
   tc::fence_before_sync();
@@ -541,6 +545,24 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
     // (the K images are idle: every QK has completed)
     uint8_t* stage = smem + L::kimg + warp * 4096;
     static_assert(8 * 4096 <= kWNK * kWImage, "room for every warp's rows");
+    if (kClusters && item.pieces > 1) {
+      // (both groups are behind the barrier of the sums, so every MMA is done with the images)
+      float* stats = reinterpret_cast<float*>(smem + L::stats);
+      float* park = reinterpret_cast<float*>(smem + L::park);
+      if (g == 0) {
+        stats[row] = m_ref;
+        stats[kWGroup + row] = lsum;
+      }
+      if ((row & ~31) < rows) {
+#pragma unroll 1
+        for (int j = 0; j < kWGroupDims / 32; ++j) {
+          float o[32];
+          tc::tmem_ld32(o_part + j * 32, reinterpret_cast<uint32_t*>(o));
+          tc::tmem_ld_wait<32>(reinterpret_cast<uint32_t*>(o));
+          park_row32<kWGroup>(park, g * kWGroupDims + j * 32, row, o);
+        }
+      }
+    } else {
     const RowsOut dst = rows_out(p, t, kvh, rows, row, split);
     if ((row & ~31) < rows) {
 #pragma unroll 1
@@ -555,8 +577,17 @@ umma_rows256_attention_kernel(const __grid_constant__ KernelParams p, const __gr
       }
     }
     if (g == 0 && row < rows && (p.num_splits > 1 || p.lse_out != nullptr)) write_lse(p, t, kvh, row, split, lsum > 0.f ? m_ref - kPGain + log2f(lsum) : -INFINITY);
+    }
   }
 
+  if (kClusters && item.pieces > 1) {
+    cluster_sync();
+    if (warp < 8 && (tid & 127) < rows)
+      merge_pieces<kWGroup, 2, kWDim>(p, t, kvh, tid & 127, tid >> 7, (int)(blockIdx.x & (uint32_t)(p.cluster - 1)), item.pieces,
+                                      reinterpret_cast<const float*>(smem + L::park), reinterpret_cast<const float*>(smem + L::stats),
+                                      reinterpret_cast<float*>(smem + L::raw));
+    cluster_sync();  // (the others still read this CTA's rows)
+  }
   if (p.late_wait) pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
@@ -581,19 +612,7 @@ cudaError_t launch_umma_rows256_attention(const KernelParams& p_in, cudaStream_t
     mapp = cached_page_map(p);
     if (mapp == nullptr) return cudaErrorInvalidValue;
   }
-  static bool configured[64] = {};
-  int dev = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err != cudaSuccess) return err;
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    err = cudaFuncSetAttribute(umma_rows256_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WLayout::total);
-    if (err != cudaSuccess) return err;
-    if (dev >= 0 && dev < 64) configured[dev] = true;
-  }
-  const int64_t ctas = (int64_t)p.num_q_tiles * p.num_kv_heads;
-  if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
-  const dim3 grid((unsigned)ctas, p.num_splits);
-  return pdl_launch(umma_rows256_attention_kernel, grid, kWThreads, WLayout::total, stream, p, *mapp);
+  return launch_row_tiles<umma_rows256_attention_kernel<false>, umma_rows256_attention_kernel<true>>(p, *mapp, kWThreads, WLayout::total, stream);
 }
 
 // Reads and clears this kernel's status word (device must be idle).

@@ -77,7 +77,11 @@ struct XLayout {
   static constexpr int raw = (qimg + 2 * G::qimage + 127) / 128 * 128;
   static constexpr int ksc = raw + kXNR * G::raw_unit;               // KeyScales<64> [kXKsRing]
   static constexpr int fix = ksc + kXKsRing * (int)sizeof(KeyScales<kXKeys>);   // float [256 rows], see QueryScale
-  static constexpr int bars = fix + kXRows * 4;                                  // uint64 [...]
+  static constexpr int stats = fix + kXRows * 4;                                 // float [2][256 rows], see merge_pieces
+  static constexpr int bars = stats + 2 * kXRows * 4;                            // uint64 [...]
+  static constexpr int park = kimg;                                              // the images, idle at the end: [HD][256 rows] fp32
+  static_assert(HD * kXRows * 4 <= raw, "room for a parked accumulator");
+  static_assert(kClusterMax * kXRows * 4 <= kXNR * G::raw_unit, "room for the weights of the pieces, in the idle ring");
   static constexpr int n_bars = 2 * kXNS + 2 * kXNK + 12 + 2 * kXNR;
   static constexpr int misc = bars + n_bars * 8;
   static constexpr int total = misc + 32 + 4 * kRowsItemInts;
@@ -115,7 +119,7 @@ __device__ __forceinline__ void issue_pv_x(uint32_t o_tmem, uint32_t p_tmem, Row
   for (int kk = 0; kk < kXKeys / 16; ++kk) mma_ts_words(o_tmem, p_tmem + kk * 8, v.lo + kk * (256 >> 4), v.hi, idesc, accumulate || kk > 0);
 }
 
-template <int HD>
+template <int HD, bool kClusters>
 __global__ void __launch_bounds__(kXThreads, 1)
 umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid_constant__ CUtensorMap tmap) {
   using L = XLayout<HD>;
@@ -135,7 +139,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
   KeyScales<kXKeys>* key_scales = reinterpret_cast<KeyScales<kXKeys>*>(smem + L::ksc);
 
   int kvh, tile_index;
-  rows_cta(p, &kvh, &tile_index);
+  rows_cta<kClusters>(p, &kvh, &tile_index);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // Barriers and TMEM are set up by the warps that wait for nothing else.
@@ -177,7 +181,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     if (warp == 0) {
       unsigned long long work = 0;
       const RowTile found = warp_row_tile(p, tile_index, p.num_splits > 1, sched_shape(p), &work);
-      item = rows_item(p, found, split, work);
+      item = rows_item<kClusters>(p, found, split, work);
       if (lane == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
     }
   } else {
@@ -197,7 +201,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       t = resolve_row_tile(p, tile_index);
     }
     const unsigned long long work = p.num_splits > 1 ? cta_work<kXThreads>(p, smem + L::misc + 16) : 0ull;
-    item = rows_item(p, t, split, work);
+    item = rows_item<kClusters>(p, t, split, work);
     if (tid == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
   }
   tc::fence_before_sync();
@@ -535,6 +539,22 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
     const float inv = l > 0.f ? 1.0f / l : 0.f;
     // (the Q image of this row tile is idle: every QK that reads it has completed)
     uint8_t* stage = smem + L::qimg + rt * kXQImage + (warp & 3) * 4096;
+    if (kClusters && item.pieces > 1) {
+      float* stats = reinterpret_cast<float*>(smem + L::stats);
+      float* park = reinterpret_cast<float*>(smem + L::park);
+      named_barrier(4, kXSoftmax);  // (both row tiles' MMAs are done with the images)
+      stats[row] = m_ref;
+      stats[kXRows + row] = l;
+      if ((row & ~31) < rows) {
+#pragma unroll 1
+        for (int j = 0; j < kXDim / 32; ++j) {
+          float o[32];
+          tc::tmem_ld32(o_tmem + j * 32, reinterpret_cast<uint32_t*>(o));
+          tc::tmem_ld_wait<32>(reinterpret_cast<uint32_t*>(o));
+          park_row32<kXRows>(park, j * 32, row, o);
+        }
+      }
+    } else {
     const RowsOut dst = rows_out(p, t, kvh, rows, row, split);
     if ((row & ~31) < rows) {
 #pragma unroll 1
@@ -549,8 +569,17 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
       }
     }
     if (row < rows && (p.num_splits > 1 || p.lse_out != nullptr)) write_lse(p, t, kvh, row, split, l > 0.f ? m_ref - kPGain + log2f(l) : -INFINITY);
+    }
   }
 
+  if (kClusters && item.pieces > 1) {
+    cluster_sync();
+    if (warp < 8 && tid < rows)
+      merge_pieces<kXRows, 1, HD>(p, t, kvh, tid, 0, (int)(blockIdx.x & (uint32_t)(p.cluster - 1)), item.pieces,
+                                  reinterpret_cast<const float*>(smem + L::park), reinterpret_cast<const float*>(smem + L::stats),
+                                  reinterpret_cast<float*>(smem + L::raw));
+    cluster_sync();  // (the others still read this CTA's rows)
+  }
   if (p.late_wait) pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
@@ -564,19 +593,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
 namespace {
 template <int HD>
 cudaError_t launch_rows2(const KernelParams& p, const CUtensorMap& map, cudaStream_t stream) {
-  static bool configured[64] = {};
-  int dev = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err != cudaSuccess) return err;
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    err = cudaFuncSetAttribute(umma_rows2_attention_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, XLayout<HD>::total);
-    if (err != cudaSuccess) return err;
-    if (dev >= 0 && dev < 64) configured[dev] = true;
-  }
-  const int64_t ctas = (int64_t)p.num_q_tiles * p.num_kv_heads;
-  if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
-  const dim3 grid((unsigned)ctas, p.num_splits);
-  return pdl_launch(umma_rows2_attention_kernel<HD>, grid, kXThreads, XLayout<HD>::total, stream, p, map);
+  return launch_row_tiles<umma_rows2_attention_kernel<HD, false>, umma_rows2_attention_kernel<HD, true>>(p, map, kXThreads, XLayout<HD>::total, stream);
 }
 }  // namespace
 

@@ -71,7 +71,10 @@ struct RLayout {
   static constexpr int park_m = ksc + kRKsRing * (int)sizeof(KeyScales<kTileKeys>); // float [2 groups][128]
   static constexpr int park_l = park_m + 2 * kRGroup * 4;      // float [2 groups][128]
   static constexpr int fix = park_l + 2 * kRGroup * 4;         // float [128], see QueryScale
-  static constexpr int bars = fix + kRGroup * 4;               // uint64 [...]
+  static constexpr int stats = fix + kRGroup * 4;              // float [2][128], see merge_pieces
+  static constexpr int bars = stats + 2 * kRGroup * 4;         // uint64 [...]
+  static constexpr int park = kimg;                            // the K images, idle at the end: [128][128 rows] fp32
+  static_assert(kHeadDim * kRGroup * 4 <= kRNK * kWideBytes, "room for a parked accumulator");
   static constexpr int n_bars = kRNS * 2 + 2 * kRNK + 6 + 2 * kRNR;
   static constexpr int misc = bars + n_bars * 8;
   static constexpr int total = misc + 32 + 4 * kRowsItemInts;
@@ -96,7 +99,7 @@ __device__ __forceinline__ int tile_key_rows(int raw_mode, int r) {
   return raw_mode == 2 ? (r & 64) + 2 * (r & 31) + ((r >> 5) & 1) : r;
 }
 
-template <int kRNK, int kRNR>
+template <int kRNK, int kRNR, bool kClusters>
 __global__ void __launch_bounds__(kRThreads, 1)
 umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_constant__ CUtensorMap tmap) {
   using L = RLayout<kRNK, kRNR>;
@@ -113,7 +116,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   KeyScales<kTileKeys>* key_scales = reinterpret_cast<KeyScales<kTileKeys>*>(smem + L::ksc);
 
   int kvh, tile_index;
-  rows_cta(p, &kvh, &tile_index);
+  rows_cta<kClusters>(p, &kvh, &tile_index);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // Barriers and TMEM are set up by the warps that wait for nothing else.
@@ -155,7 +158,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     if (warp == 0) {
       unsigned long long work = 0;
       const RowTile found = warp_row_tile(p, tile_index, p.num_splits > 1, sched_shape(p), &work);
-      item = rows_item(p, found, split, work);
+      item = rows_item<kClusters>(p, found, split, work);
       if (lane == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
     }
   } else {
@@ -175,7 +178,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
       t = resolve_row_tile(p, tile_index);
     }
     const unsigned long long work = p.num_splits > 1 ? cta_work<kRThreads>(p, smem + L::misc + 16) : 0ull;
-    item = rows_item(p, t, split, work);
+    item = rows_item<kClusters>(p, t, split, work);
     if (tid == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
   }
   tc::fence_before_sync();
@@ -524,7 +527,12 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     const float c0 = m0 == -INFINITY ? 0.f : ex2f(m0 - m);
     const float c1 = m1 == -INFINITY ? 0.f : ex2f(m1 - m);
     const float lsum = l0 * c0 + l1 * c1;
-    const float inv = lsum > 0.f ? 1.0f / lsum : 0.f;
+    const float inv = kClusters && item.pieces > 1 ? 1.0f : lsum > 0.f ? 1.0f / lsum : 0.f;  // (pieces are merged as they are)
+    if (kClusters && item.pieces > 1 && g == 0) {
+      float* stats = reinterpret_cast<float*>(smem + L::stats);
+      stats[row] = m;
+      stats[kRGroup + row] = lsum;
+    }
     // (the Q image is idle: every QK has completed)
     uint8_t* stage = qimg + warp * 4096;
     static_assert(8 * 4096 <= kQImageBytes, "room for every warp's rows");
@@ -543,12 +551,24 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
           const float o1 = c1 > 0.f ? __uint_as_float(r1[n]) * c1 : 0.f;
           o[n] = (__uint_as_float(r0[n]) * c0 + o1) * inv;
         }
-        write_rows32(dst, j * 32, stage, o);
+        if (kClusters && item.pieces > 1) {
+          park_row32<kRGroup>(reinterpret_cast<float*>(smem + L::park), j * 32, row, o);
+        } else {
+          write_rows32(dst, j * 32, stage, o);
+        }
       }
     }
-    if (g == 0 && row < rows && (p.num_splits > 1 || p.lse_out != nullptr)) write_lse(p, t, kvh, row, split, lsum > 0.f ? m - kPGain + log2f(lsum) : -INFINITY);
+    if (g == 0 && row < rows && (!kClusters || item.pieces == 1) && (p.num_splits > 1 || p.lse_out != nullptr)) write_lse(p, t, kvh, row, split, lsum > 0.f ? m - kPGain + log2f(lsum) : -INFINITY);
   }
 
+  if (kClusters && item.pieces > 1) {
+    cluster_sync();
+    if (warp < 8 && (tid & 127) < rows)
+      merge_pieces<kRGroup, 2, kHeadDim>(p, t, kvh, tid & 127, tid >> 7, (int)(blockIdx.x & (uint32_t)(p.cluster - 1)), item.pieces,
+                                         reinterpret_cast<const float*>(smem + L::park), reinterpret_cast<const float*>(smem + L::stats),
+                                         reinterpret_cast<float*>(smem + L::raw));
+    cluster_sync();  // (the others still read this CTA's rows)
+  }
   if (p.late_wait) pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
@@ -569,18 +589,9 @@ bool umma_rows_supports(const KernelParams& p, const char** why) {
 
 namespace {
 template <int NK, int NR>
-cudaError_t launch_rows(const KernelParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t stream) {
-  static bool configured[64] = {};
-  int dev = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err != cudaSuccess) return err;
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    err = cudaFuncSetAttribute(umma_rows_attention_kernel<NK, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               RLayout<NK, NR>::total);
-    if (err != cudaSuccess) return err;
-    if (dev >= 0 && dev < 64) configured[dev] = true;
-  }
-  return pdl_launch(umma_rows_attention_kernel<NK, NR>, grid, kRThreads, RLayout<NK, NR>::total, stream, p, map);
+cudaError_t launch_rows(const KernelParams& p, const CUtensorMap& map, cudaStream_t stream) {
+  return launch_row_tiles<umma_rows_attention_kernel<NK, NR, false>, umma_rows_attention_kernel<NK, NR, true>>(p, map, kRThreads,
+                                                                                                              RLayout<NK, NR>::total, stream);
 }
 }  // namespace
 
@@ -610,10 +621,7 @@ cudaError_t launch_umma_rows_attention(const KernelParams& p_in, cudaStream_t st
   // their K operand from the same shared-memory addresses: with a single K image that the
   // producers rewrote between two QKs, results varied from run to run although every
   // producer / consumer edge was ordered by an mbarrier and a proxy fence.
-  const int64_t ctas = (int64_t)p.num_q_tiles * p.num_kv_heads;
-  if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
-  const dim3 grid((unsigned)ctas, p.num_splits);
-  return launch_rows<2, 3>(p, map, grid, stream);
+  return launch_rows<2, 3>(p, map, stream);
 }
 
 // Reads and clears this file's status word (device must be idle).
