@@ -67,3 +67,20 @@ def test_rows_that_are_nan(D):
         nan = np.isnan(res["out"][:40])
         assert (nan.all(-1) == want).all() and (nan.any(-1) == want).all()
         assert (np.isneginf(res["lse"][:40]) == want).all()
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("lens", [[30, 9, 40, 120], [1500, 9, 700, 2000]])
+def test_bound_on_pieces_above_what_the_lengths_allow(D, lens):
+    """Pieces that a row of the block table is too short for get no CTA; they read as holding no keys all the same."""
+    qlens, rng = [30, 9, 0, 25], np.random.default_rng(D)
+    c = orc.make_paged_cache(lens, 2, D, 16, seed=D)
+    q = orc.round_to_bf16(rng.standard_normal((sum(qlens), 8, D), dtype=np.float32))
+    qsl = np.concatenate([[0], np.cumsum(qlens)]).astype(np.int64)
+    ref = orc.ref_attention_paged(q, c, qsl, D ** -0.5)
+    res = run_case(c, q, qsl, D ** -0.5, bq=16, num_splits=24, kernel=capi.KERNEL_UMMA_ROWS)
+    assert capi.load_library().device_status() == 0
+    check_out(res["out"], ref.out, what=f"D{D} {lens}")
+    check_lse(res["lse"], ref.lse, what=f"D{D} {lens}")
+    most = (-(-max(lens) // 128) + 2) // 4
+    assert np.isneginf(res["ws_lse"][max(1, most):]).all()
