@@ -66,3 +66,16 @@ def test_the_scratch_copies_in_the_raw_ring_are_fenced(name):
     scratch = code[code.index("int* qsl_s = reinterpret_cast<int*>(smem + L::raw)"):code.index("resolve_row_tile(p, tile_index)")]
     last = scratch.rindex("__syncthreads();")
     assert scratch.index("resolve_row_tile_with(") < scratch.index("fence_async_smem();") < last
+
+
+@pytest.mark.parametrize("name", KERNELS + ["umma_i8_kernel.cu"])
+def test_no_mma_is_issued_behind_a_wait_that_gave_up(name):
+    """Its operands are not what it needs, and nobody would wait for it before TMEM is freed."""
+    code = _code(name)
+    calls = [m.start() for m in re.finditer(r"\bif \([^;{}]*\belect_one\(\)\)\s*(?:\{|issue_pv\()", code)]
+    assert len(calls) >= 2
+    for at in calls:
+        condition = code[at:code.index("elect_one()", at)]
+        assert re.search(r"(\bok|\bgo|\bready|__all_sync\(0xffffffffu, sound\)) &&", condition), f"{name}: {condition}"
+    if "sound" in code:
+        assert "const bool sound = ok && *abort_flag == 0;" in code
