@@ -63,7 +63,8 @@ struct KernelParams {
   int32_t row_class;   // 0 = every request; 1 = only requests with q_len * group <= class_rows; 2 = only the others
   int32_t class_rows;
   // Row-major kernels behind the integer kernel of the same call, with whose requests they share nothing: they start
-  // beside it and wait for it only before they end (pdl.cuh).
+  // beside it and wait for it only before they end (pdl.cuh).  They hold no TMEM while they wait: the integer kernel lets them
+  // start before it has its own, and a CTA of it on the same SM would wait for theirs.
   int32_t late_wait = 0;
   // Row-major kernels: CTAs of a cluster that share the keys of one row tile among them (1, 2, 4 or 8).
   int32_t cluster = 1;

@@ -569,11 +569,11 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
                                          reinterpret_cast<float*>(smem + L::raw));
     cluster_sync();  // (the others still read this CTA's rows)
   }
-  if (p.late_wait) pdl_wait();
   tc::fence_before_sync();
   __syncthreads();
   if (warp == kRLoadWarp) tc::tmem_dealloc(tmem_base, 512);
   if (tid == 0 && *abort_flag) atomicOr(&g_rows_status, 4u);
+  if (p.late_wait) pdl_wait();  // (TMEM is free by now: see late_wait)
   (void)ok;
 }
 

@@ -79,3 +79,14 @@ def test_no_mma_is_issued_behind_a_wait_that_gave_up(name):
         assert re.search(r"(\bok|\bgo|\bready|__all_sync\(0xffffffffu, sound\)) &&", condition), f"{name}: {condition}"
     if "sound" in code:
         assert "const bool sound = ok && *abort_flag == 0;" in code
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_tmem_is_freed_before_the_wait_for_the_integer_kernel(name):
+    """That kernel lets this one start before it allocates: a CTA that waited for it and held TMEM would hold it up for good."""
+    code = _code(name)
+    code = code[code.index("if (!p.late_wait) pdl_wait();"):]
+    waits = [m.start() for m in re.finditer(r"if \(p\.late_wait\) pdl_wait\(\);", code)]
+    frees = [m.start() for m in re.finditer(r"tmem_dealloc\(tmem_base, 512\);", code)]
+    assert len(waits) == len(frees) == 2        # without work, and at the end
+    assert frees[0] < waits[0] < frees[1] < waits[1]
