@@ -159,6 +159,7 @@ EXPORTED_SYMBOLS = (
     "pthb200_launch_count",
     "pthb200_test_schedule",
     "pthb200_test_range_schedule",
+    "pthb200_test_row_bounds",
     "pthb200_test_tile",
     "pthb200_test_tile_i8",
     "pthb200_test_tile_rows",
@@ -217,6 +218,8 @@ class B200Lib:
         for fn in (lib.pthb200_test_schedule, lib.pthb200_test_range_schedule):
             fn.restype = ctypes.c_int32
             fn.argtypes = [ctypes.c_void_p] * 2 + [ctypes.c_int32] * 10 + [ctypes.c_void_p, ctypes.c_int32]
+        lib.pthb200_test_row_bounds.restype = ctypes.c_int32
+        lib.pthb200_test_row_bounds.argtypes = [ctypes.c_int64] + [ctypes.c_int32] * 5 + [ctypes.POINTER(ctypes.c_int32)]
         lib.pthb200_test_tile.restype = ctypes.c_int32
         lib.pthb200_test_tile.argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_int32, ctypes.c_void_p]
         lib.pthb200_test_tile_i8.restype = ctypes.c_int32
@@ -304,6 +307,16 @@ class B200Lib:
         out = np.zeros((max(n, 1), 8), dtype=np.int32)
         fn(*args, out.ctypes.data, n)
         return out[:n]
+
+    def row_bounds(self, *, block_table_row_stride: int, block_size: int, bq: int, num_splits: int, window: int = 0,
+                   causal: bool = True) -> tuple[int, int]:
+        """KV tiles that a row tile of a row-major launch can touch, and the most pieces it is cut into (no device access)."""
+        pieces = ctypes.c_int32(0)
+        tiles = int(self.lib.pthb200_test_row_bounds(block_table_row_stride, block_size, window, int(causal), bq, num_splits,
+                                                     ctypes.byref(pieces)))
+        if tiles < 0:
+            raise RuntimeError(self.last_error())
+        return tiles, pieces.value
 
     def launch_count(self, args: PthAttnArgs) -> tuple[int, int]:
         a, c = ctypes.c_int32(0), ctypes.c_int32(0)

@@ -528,6 +528,17 @@ int32_t pthb200_test_range_schedule(const int32_t* query_start_loc, const int32_
   return count;
 }
 
+// What the row-major launch takes for the KV tiles of a row tile and for the pieces that it is cut into at most.
+int32_t pthb200_test_row_bounds(int64_t block_table_row_stride, int32_t block_size, int32_t window, int32_t causal, int32_t bq,
+                                int32_t num_splits, int32_t* pieces) {
+  using namespace pthb200;
+  g_last_error.clear();
+  PTHB_REQUIRE(pieces != nullptr && block_size >= 1 && window >= 0 && bq >= 1 && num_splits >= 1, "counts must be >= 1");
+  const int64_t tiles = row_tile_bound(block_table_row_stride, block_size, window, causal, bq);
+  *pieces = pieces_bound(tiles, num_splits);
+  return (int32_t)tiles;
+}
+
 }  // extern "C"
 
 // ---- split attention without a caller workspace ---------------------------------

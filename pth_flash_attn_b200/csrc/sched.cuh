@@ -114,6 +114,24 @@ PTHB_HD int req_splits(int kv_tiles, int t_star, int num_splits) {
   return s < 1 ? 1 : (s > (unsigned)num_splits ? num_splits : (int)s);
 }
 
+// KV tiles of a row tile of bq query tokens, as far as the host knows: a row of the block table and the window bound
+// them, the window on both sides of a token where the mask is not causal.  (A row that is longer than the stride says, or
+// a stride of 0, which says nothing: the CTAs go by the lengths, this only by the time.)
+inline int64_t row_tile_bound(int64_t block_table_row_stride, int block_size, int window, int causal, int bq) {
+  constexpr int64_t most = 0x7fffffff;
+  int64_t tiles = block_table_row_stride > 0 && block_table_row_stride < (1 << 30) ? (block_table_row_stride * block_size + 127) / 128 : most;
+  if (window > 0) {
+    const int64_t in_window = ((int64_t)window * (causal ? 1 : 2) + bq) / 128 + 2;
+    tiles = tiles < in_window ? tiles : in_window;
+  }
+  return tiles < most ? tiles : most;
+}
+// Pieces that row tiles of at most `tiles` KV tiles are cut into at most.
+inline int pieces_bound(int64_t tiles, int num_splits) {
+  const int64_t pieces = (tiles + kItemTilesMin / 2) / kItemTilesMin;
+  return pieces < 1 ? 1 : pieces < num_splits ? (int)pieces : num_splits;
+}
+
 // Items of a request, and the coordinates of its item `local`.
 PTHB_HD int64_t req_items(int row_tiles, int splits, int num_kv_heads) {
   return (int64_t)row_tiles * splits * num_kv_heads;

@@ -278,12 +278,8 @@ int clusters_at_once(int size, int threads, int smem) {
   if (slot != nullptr) slot->store(n + 1, std::memory_order_relaxed);
   return n;
 }
-// KV tiles of a row tile, as far as the host knows: a row of the block table and the window bound them.  (A row that is
-// longer than the stride says, or a stride of 0, which says nothing: the CTAs go by the lengths, this only by the time.)
 inline int64_t tiles_bound(const KernelParams& p) {
-  int64_t tiles = p.block_table_row_stride > 0 && p.block_table_row_stride < (1 << 30) ? (p.block_table_row_stride * p.block_size + 127) / 128 : 0x7fffffff;
-  if (p.window > 0) tiles = std::min(tiles, (int64_t)(p.window + p.bq) / 128 + 2);
-  return std::min(tiles, (int64_t)0x7fffffff);
+  return row_tile_bound(p.block_table_row_stride, p.block_size, p.window, p.causal, p.bq);
 }
 template <auto kKernel>
 int cluster_for(const KernelParams& p, int threads, int smem) {
@@ -313,8 +309,7 @@ cudaError_t launch_row_tiles(const KernelParams& p_in, const CUtensorMap& map, i
   if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
   // Pieces that no request of these lengths is cut into get no CTA (one that finds nothing to do still takes an SM for 5 us:
   // 14 requests of 8 tokens over 2,000 keys at 64 dims, 43 pieces at most, 220 us with all of them, 67 with 4).
-  const int64_t pieces = (tiles_bound(p) + kItemTilesMin / 2) / kItemTilesMin;
-  const dim3 grid((unsigned)ctas, (unsigned)std::max((int64_t)1, std::min(pieces, (int64_t)p.num_splits)));
+  const dim3 grid((unsigned)ctas, (unsigned)pieces_bound(tiles_bound(p), p.num_splits));
   if (p.cluster > 1) return pdl_launch_clusters(p.cluster, kClustered, grid, threads, smem, stream, p, map);
   return pdl_launch(kKernel, grid, threads, smem, stream, p, map);
 }
