@@ -1259,7 +1259,9 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
           if (n < rows && d < HD) {  // (a head of 64 dims uses half of the group's threads)
             const float mine = g ? acc[h][2 * n2 + 1] : acc[h][2 * n2], other = park[n * kKeys + gt];
             const float a0 = g ? other : mine, a1 = g ? mine : other;
-            const float val = fmaf(a0, x0, x1 > 0.f ? a1 * x1 : 0.f);
+            // (neither group has a share of a row without keys, which is zero whatever is in its accumulators: an infinite
+            // v_scale beside it makes them NaN)
+            const float val = x0 > 0.f || x1 > 0.f ? fmaf(a0, x0, x1 > 0.f ? a1 * x1 : 0.f) : 0.f;
             const uint32_t id = rowid[n];
             uint8_t* const row = o_item + (int64_t)(id & 255u) * o_token + (int64_t)(id >> 8) * o_head;
             if (!S1) reinterpret_cast<float*>(row)[d] = val;

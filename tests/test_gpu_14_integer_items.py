@@ -94,3 +94,16 @@ def test_ranges(Hkv, D, G, qlen, hnd, S, lens):
         ref = torch.einsum("tgrn,ngd->tgrd", s.softmax(-1), v).reshape(qlen, Hq, D)
         check_out(out[rows].float().cpu().numpy(), ref.cpu().numpy(), what=f"request {r}")
         check_lse(lse[rows].cpu().numpy(), s.logsumexp(-1).reshape(qlen, Hq).cpu().numpy(), what=f"request {r}")
+
+
+@pytest.mark.parametrize("D, G, bq", [(128, 2, 2), (128, 2, 4), (64, 4, 4), (256, 1, 4)])
+@pytest.mark.parametrize("S", [1, 2])
+def test_rows_without_keys_beside_an_infinite_scale(D, G, bq, S):
+    """More query tokens than keys: the first see none and are zero, whatever the cells hold that the others see."""
+    c = orc.make_paged_cache([bq - 1, 300], 1, D, 16, seed=D)
+    c.v_scale[c.block_table[0, 0], 0] = np.inf                # (what the writer makes of a row with an infinity)
+    q = orc.round_to_bf16(np.random.default_rng(D).standard_normal((bq + 1, G, D), dtype=np.float32))
+    res = run_case(c, q, [0, bq, bq + 1], D ** -0.5, bq=bq, num_splits=S, kernel=capi.KERNEL_UMMA)
+    assert capi.load_library().device_status() == 0
+    assert (res["out"][0] == 0).all() and np.isneginf(res["lse"][0]).all()
+    assert not np.isfinite(res["out"][1:bq]).any() and np.isfinite(res["out"][bq]).all()
