@@ -307,8 +307,10 @@ cudaError_t launch_row_tiles(const KernelParams& p_in, const CUtensorMap& map, i
   p.cluster = cluster_for<kClustered>(p, threads, smem);
   const int64_t ctas = (int64_t)p.num_q_tiles * p.num_kv_heads * p.cluster;
   if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
-  // Pieces that no request of these lengths is cut into get no CTA (one that finds nothing to do still takes an SM for 5 us:
-  // 14 requests of 8 tokens over 2,000 keys at 64 dims, 43 pieces at most, 220 us with all of them, 67 with 4).
+  // Pieces that no request of these lengths is cut into get no CTA (one that finds nothing to do still takes an SM for 2.7 us).
+  // That holds as far as the block table is cut to the lengths; an engine's table of the longest context says less.  14 requests
+  // of 8 tokens over 2,000 keys at 64 dims, 85 pieces at most: 67 us with a table of 2,000 keys a row, 213 with one of 131,072;
+  // 20 of 6 over 1,000, 2 KV heads 19 and 51.  (With TMEM taken by every CTA before it looks for work 220 and 53.4.)
   const dim3 grid((unsigned)ctas, (unsigned)pieces_bound(tiles_bound(p), p.num_splits));
   if (p.cluster > 1) return pdl_launch_clusters(p.cluster, kClustered, grid, threads, smem, stream, p, map);
   return pdl_launch(kKernel, grid, threads, smem, stream, p, map);

@@ -119,11 +119,15 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   rows_cta<kClusters>(p, &kvh, &tile_index);
   const int split = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // Barriers and TMEM are set up by the warps that wait for nothing else.
+  // Barriers and TMEM are set up by the warps that wait for nothing else.  The CTA of a further piece of the bound, which
+  // mostly finds that its request is not cut that often, takes TMEM when it has found work (see launch_row_tiles).
+  const bool tmem_ahead = split == 0;
   if (warp == kRLoadWarp) {
     if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
-    tc::tmem_alloc(tslot, 512);
-    tc::tmem_relinquish();
+    if (tmem_ahead) {
+      tc::tmem_alloc(tslot, 512);
+      tc::tmem_relinquish();
+    }
   }
   if (warp == kRMmaWarp && lane == 0) {
     for (int s = 0; s < kRNS; ++s) {
@@ -184,14 +188,23 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem_base = *tslot;
   item = *reinterpret_cast<const RowsItem*>(item_s);
   if (item.state != 1 || (split == 0 && item.nsplits < p.num_splits)) write_empty<kRThreads, kHeadDim>(p, item, kvh, split);
   if (item.state != 1) {
-    if (warp == kRLoadWarp) tc::tmem_dealloc(tmem_base, 512);
+    if (tmem_ahead && warp == kRLoadWarp) tc::tmem_dealloc(*tslot, 512);
     if (p.late_wait) pdl_wait();
     return;
   }
+  if (!tmem_ahead) {
+    if (warp == kRLoadWarp) {
+      tc::tmem_alloc(tslot, 512);
+      tc::tmem_relinquish();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+  }
+  const uint32_t tmem_base = *tslot;
   const RowTile& t = item.t;
   const int rows = item.rows;  // <= 128 by construction of bq
   const int tile_begin = item.tile_begin, tile_end = item.tile_end, range_begin = item.range_begin, range_end = item.range_end;

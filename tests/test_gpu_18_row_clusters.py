@@ -84,3 +84,22 @@ def test_bound_on_pieces_above_what_the_lengths_allow(D, lens):
     check_lse(res["lse"], ref.lse, what=f"D{D} {lens}")
     most = (-(-max(lens) // 128) + 2) // 4
     assert np.isneginf(res["ws_lse"][max(1, most):]).all()
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("lens", [[30, 9, 40, 120], [1500, 9, 700, 2000], [9000, 20, 30, 40]])
+def test_pieces_that_find_nothing(D, lens):
+    """A block table as wide as the longest context an engine allows: every piece of the bound gets a CTA, few find keys."""
+    qlens, rng = [30, 9, 0, 25], np.random.default_rng(D + 1)
+    c = orc.make_paged_cache(lens, 2, D, 16, seed=D + 1)
+    q = orc.round_to_bf16(rng.standard_normal((sum(qlens), 8, D), dtype=np.float32))
+    qsl = np.concatenate([[0], np.cumsum(qlens)]).astype(np.int64)
+    ref = orc.ref_attention_paged(q, c, qsl, D ** -0.5)
+    c.block_table = np.pad(c.block_table, ((0, 0), (0, 8192 - c.block_table.shape[1])))
+    res = run_case(c, q, qsl, D ** -0.5, bq=16, num_splits=24, kernel=capi.KERNEL_UMMA_ROWS)
+    assert capi.load_library().device_status() == 0
+    check_out(res["out"], ref.out, what=f"D{D} {lens}")
+    check_lse(res["lse"], ref.lse, what=f"D{D} {lens}")
+    tiles = sum(-(-n // 128) * -(-4 * t // (128 if D == 256 else 256)) for n, t in zip(lens, qlens))
+    used = int((~np.isneginf(res["ws_lse"])).any(axis=(1, 2)).sum())
+    assert 1 <= used <= max(1, -(-max(lens) // 128) // 4 + 1) and (tiles < 16 or used > 1)

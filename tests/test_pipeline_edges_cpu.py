@@ -87,6 +87,23 @@ def test_tmem_is_freed_before_the_wait_for_the_integer_kernel(name):
     code = _code(name)
     code = code[code.index("if (!p.late_wait) pdl_wait();"):]
     waits = [m.start() for m in re.finditer(r"if \(p\.late_wait\) pdl_wait\(\);", code)]
-    frees = [m.start() for m in re.finditer(r"tmem_dealloc\(tmem_base, 512\);", code)]
+    frees = [m.start() for m in re.finditer(r"tmem_dealloc\(", code)]
     assert len(waits) == len(frees) == 2        # without work, and at the end
     assert frees[0] < waits[0] < frees[1] < waits[1]
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_a_cta_of_an_unused_piece_leaves_without_tmem(name):
+    """Most pieces of a generous bound are not used, and taking TMEM for them cost small launches 5 %."""
+    code = _code(name)
+    assert code.count("const bool tmem_ahead = split == 0;") == 1
+    allocs = [m.start() for m in re.finditer(r"tmem_alloc\(tslot, 512\)", code)]
+    frees = [m.start() for m in re.finditer(r"tmem_dealloc\(", code)]
+    found = code.index("item = *reinterpret_cast<const RowsItem*>(item_s);")
+    later = code.index("if (!tmem_ahead) {")
+    assert len(allocs) == len(frees) == 2
+    assert "if (tmem_ahead) {" in code[:allocs[0]] and allocs[0] < found < frees[0] < later < allocs[1] < frees[1]
+    assert re.search(r"if \(tmem_ahead && warp == k\wLoadWarp\) tc::tmem_dealloc\(", code[found:later])
+    # its address is read by everybody: a barrier of the CTA behind the allocation, between the two TMEM fences
+    behind = code[allocs[1]:code.rindex("tmem_base = *tslot;")]
+    assert behind.index("fence_before_sync();") < behind.index("__syncthreads();") < behind.index("fence_after_sync();")
