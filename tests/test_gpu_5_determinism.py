@@ -1,9 +1,10 @@
 """Run-to-run determinism: the same launch repeated must give the same bytes.
 
 The kernels' reductions have a fixed order (their atomics add whole numbers or take maxima), so any
-difference between two runs is a synchronisation bug (two were found this way: two threads issuing
-tcgen05.mma concurrently in the row-major kernel, and page copies without a proxy fence behind the
-reads of the stage they overwrite)."""
+difference between two runs is a synchronisation bug (two were found this way: one with two threads issuing
+tcgen05.mma concurrently in an early row-major kernel, and page copies without a proxy fence behind the
+reads of the stage they overwrite).  In the integer kernel two threads issue up to 8 rows, on operands and accumulators
+that an mbarrier chain orders."""
 import numpy as np
 import pytest
 import torch
@@ -28,6 +29,19 @@ LONG_CASES = [
     (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 2, 1], 12, 2, 2, 3, 5000, 256),
     (capi.KERNEL_UMMA_ROWS, [4096, 700], [1024, 40], 16, 4, 16, 1, 5000, 64),
     (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 4, 1], 16, 4, 4, 3, 5000, 64),
+    # PV issued by the softmax warps beside the thread that issues QK: row tiles of up to 4 and up to 8 rows
+    (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 1, 1], 16, 4, 1, 4, 5000, 64),
+    (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 1, 1], 16, 2, 1, 4, 5000, 64),
+    (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 1, 1], 16, 2, 1, 4, 5000, 128),
+    (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 1, 1], 8, 2, 1, 4, 5000, 256),
+    (capi.KERNEL_UMMA, [20000, 9000, 300], [1, 1, 1], 12, 2, 1, 4, 5000, 256),
+    # the same dealt out in ranges, items of several requests behind one another in a CTA
+    (capi.KERNEL_UMMA, [60000, 700, 50000, 300, 8000, 100], [1] * 6, 8, 2, 1, 74, 5000, 128),
+    (capi.KERNEL_UMMA, [60000, 700, 50000, 300, 8000, 100], [1] * 6, 16, 2, 1, 74, 5000, 64),
+    # clusters: the keys of a row tile shared by 16, 8 and 4 CTAs
+    (capi.KERNEL_UMMA_ROWS, [5000], [30], 4, 1, 32, 1, 5000, 128),
+    (capi.KERNEL_UMMA_ROWS, [3000, 2500], [30, 50], 12, 2, 10, 1, 5000, 256),
+    (capi.KERNEL_UMMA_ROWS, [2000, 2500], [60, 30], 16, 4, 16, 1, 5000, 64),
 ]
 
 CASES = [
