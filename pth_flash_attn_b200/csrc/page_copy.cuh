@@ -103,20 +103,6 @@ __device__ __forceinline__ bool wait_or_abort_s(uint32_t bar_s, uint32_t parity,
   return false;
 }
 
-// The same wait for a thread that others wait for (the MMA-issuing thread): it polls without
-// a suspend hint, so it sees the phase complete as early as possible.
-__device__ __forceinline__ bool wait_or_abort_spin_s(uint32_t bar_s, uint32_t parity, volatile int* abort_flag) {
-  if (tc::mbar_try_wait_s(bar_s, parity)) return true;
-  const long long deadline = clock64() + (1ll << 32);
-  for (;;) {
-    if (tc::mbar_try_wait_s(bar_s, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() > deadline) break;
-  }
-  *abort_flag = 1;
-  return false;
-}
-
 // What a lane of a loader waits for before it copies into a raw stage again: every reader's arrive on
 // raw_free.  The readers' loads go through the generic proxy and the copy's writes through the async proxy, and an
 // mbarrier alone does not keep the one in front of the other: that takes a proxy fence between the wait and the copy.
@@ -142,11 +128,6 @@ __device__ __forceinline__ bool elect_one() {
       "}\n"
       : "=r"(pred));
   return pred != 0;
-}
-
-__device__ __forceinline__ void row_target(const KernelParams& p, const RowTile& t, int kvh, int n, int* token, int* head) {
-  *token = t.tok0 + n / p.group;
-  *head = kvh * p.group + n % p.group;
 }
 
 // cuTensorMapEncodeTiled, looked up once through the runtime (no link against libcuda).

@@ -84,21 +84,6 @@ __device__ __forceinline__ bool mbar_try_wait_hint_s(uint32_t bar_s, uint32_t pa
   return ok != 0;
 }
 
-// Non-blocking test of a phase (never suspends the thread).
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // try_wait with a suspend-time hint (nanoseconds): the hardware may park the thread until
 // the phase completes or the time has passed, instead of returning at once.  A waiting warp
 // that spins on plain try_wait takes issue slots from the warps that do the work.

@@ -833,7 +833,6 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
         uint8_t* stage = smem + L::vstages + st * kVStageHD;  // V image, then the scales
         uint8_t* krow = smem + L::kstages + (g % NK) * kImgHD + pt * 16;
         uint8_t* vrow = stage + pt * 16;
-        const int ko = odd ? 2 : 0, vo = odd ? 3 : 1;  // first word of K / V inside their sets of pieces
         if (!odd) {
 #pragma unroll
           for (int b = 0; b < NCH; ++b)
@@ -845,7 +844,6 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
                 make_uint4(kw[2 + 4 * b], kw[3 + 4 * b], kw[4 + 4 * b], kw[5 + 4 * b]);
         }
         const uint32_t k_scale_bits = odd ? kw[HD / 4 + 2] : kw[HD / 4];
-        (void)ko;
         if constexpr (kTwoPhase) {
           load_part(row + NCH, vw);
           mbar_arrive(&bars[B::raw_free + rs]);
@@ -861,7 +859,6 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
             *reinterpret_cast<uint4*>(vrow + b * kImgChunk) =
                 make_uint4(vw[3 + 4 * b], vw[4 + 4 * b], vw[5 + 4 * b], vw[6 + 4 * b]);
         }
-        (void)vo;
         *reinterpret_cast<uint32_t*>(stage + kImgHD + pt * 4) = k_scale_bits;
         *reinterpret_cast<uint32_t*>(stage + kImgHD + kKeys * 4 + pt * 4) = odd ? vw[HD / 4 + 3] : vw[HD / 4 + 1];
         tc::fence_async_smem();

@@ -125,7 +125,7 @@ umma_rows2_attention_kernel(const __grid_constant__ KernelParams p, const __grid
   using L = XLayout<HD>;
   using B = XBars;
   using G = XG<HD>;
-  constexpr int kXDim = HD, kXChunks = G::chunks, kXImage = G::image, kXVStage = G::image, kXQImage = G::qimage;
+  constexpr int kXDim = HD, kXImage = G::image, kXVStage = G::image, kXQImage = G::qimage;
   constexpr int kXRawRow = G::raw_row, kXRawUnit = G::raw_unit;
   static_assert(L::raw % 128 == 0 && kXRawUnit % 128 == 0 && (16 * kXRawRow) % 128 == 0, "TMA destinations");
   static_assert(L::vst % 16 == 0 && kXVStage % 16 == 0 && kXImage % 16 == 0 && L::qimg % 16 == 0 && kXQImage % 16 == 0,
