@@ -330,6 +330,9 @@ int32_t pthb200_test_range_schedule(const int32_t* query_start_loc, const int32_
                                     int32_t group, int32_t num_kv_heads, int32_t bq, int32_t num_splits,
                                     int32_t window, int32_t causal, int32_t row_class, int32_t class_rows,
                                     int32_t num_ctas, int32_t* out, int32_t max_items);
+/* CTAs per cluster of the calling thread's latest row-major launch: 1 where row tiles are not shared, 0 before the
+ * first such launch. */
+int32_t pthb200_test_row_cluster(void);
 /* The bounds that a row-major launch takes from its arguments: the KV tiles that a row tile of bq query
  * tokens can touch (returned), and the pieces that it is cut into at most. */
 int32_t pthb200_test_row_bounds(int64_t block_table_row_stride, int32_t block_size, int32_t window, int32_t causal, int32_t bq,

@@ -160,6 +160,7 @@ EXPORTED_SYMBOLS = (
     "pthb200_test_schedule",
     "pthb200_test_range_schedule",
     "pthb200_test_row_bounds",
+    "pthb200_test_row_cluster",
     "pthb200_test_tile",
     "pthb200_test_tile_i8",
     "pthb200_test_tile_rows",
@@ -218,6 +219,8 @@ class B200Lib:
         for fn in (lib.pthb200_test_schedule, lib.pthb200_test_range_schedule):
             fn.restype = ctypes.c_int32
             fn.argtypes = [ctypes.c_void_p] * 2 + [ctypes.c_int32] * 10 + [ctypes.c_void_p, ctypes.c_int32]
+        lib.pthb200_test_row_cluster.restype = ctypes.c_int32
+        lib.pthb200_test_row_cluster.argtypes = []
         lib.pthb200_test_row_bounds.restype = ctypes.c_int32
         lib.pthb200_test_row_bounds.argtypes = [ctypes.c_int64] + [ctypes.c_int32] * 5 + [ctypes.POINTER(ctypes.c_int32)]
         lib.pthb200_test_tile.restype = ctypes.c_int32

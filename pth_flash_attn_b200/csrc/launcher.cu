@@ -528,6 +528,9 @@ int32_t pthb200_test_range_schedule(const int32_t* query_start_loc, const int32_
   return count;
 }
 
+// CTAs per cluster of the calling thread's latest row-major launch (0: there was none).
+int32_t pthb200_test_row_cluster(void) { return pthb200::last_row_cluster; }
+
 // What the row-major launch takes for the KV tiles of a row tile and for the pieces that it is cut into at most.
 int32_t pthb200_test_row_bounds(int64_t block_table_row_stride, int32_t block_size, int32_t window, int32_t causal, int32_t bq,
                                 int32_t num_splits, int32_t* pieces) {

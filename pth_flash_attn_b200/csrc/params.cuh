@@ -66,9 +66,11 @@ struct KernelParams {
   // beside it and wait for it only before they end (pdl.cuh).  They hold no TMEM while they wait: the integer kernel lets them
   // start before it has its own, and a CTA of it on the same SM would wait for theirs.
   int32_t late_wait = 0;
-  // Row-major kernels: CTAs of a cluster that share the keys of one row tile among them (1, 2, 4 or 8).
+  // Row-major kernels: CTAs of a cluster that share the keys of one row tile among them (1, 2, 4, 8 or 16).
   int32_t cluster = 1;
 };
+// CTAs per cluster of the calling thread's latest row-major launch, for the tests.
+inline thread_local int32_t last_row_cluster = 0;
 
 // Re-tiles a launch to `bq` query tokens per row tile.  The caller's promise behind
 // tile_map = 1 (no request longer than its bq) survives only while bq does not shrink.

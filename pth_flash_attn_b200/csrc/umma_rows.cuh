@@ -304,7 +304,7 @@ cudaError_t launch_row_tiles(const KernelParams& p_in, const CUtensorMap& map, i
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   KernelParams p = p_in;
-  p.cluster = cluster_for<kClustered>(p, threads, smem);
+  p.cluster = last_row_cluster = cluster_for<kClustered>(p, threads, smem);
   const int64_t ctas = (int64_t)p.num_q_tiles * p.num_kv_heads * p.cluster;
   if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
   // Pieces that no request of these lengths is cut into get no CTA (one that finds nothing to do still takes an SM for 2.7 us).

@@ -96,6 +96,47 @@ def test_ranges(Hkv, D, G, qlen, hnd, S, lens):
         check_lse(lse[rows].cpu().numpy(), s.logsumexp(-1).reshape(qlen, Hq).cpu().numpy(), what=f"request {r}")
 
 
+@pytest.mark.parametrize("Hkv, G, bq, S, window, kernel, qlens, lens", [
+    (8, 4, 4, 37, 0, "UMMA", [10, 3, 4, 1, 9], [20000, 130, 33000, 127, 9000]),           # two or three row tiles a request
+    (2, 4, 2, 60, 0, "UMMA", [7, 1, 8], [60000, 900, 50000]),
+    (8, 2, 4, 37, 3000, "UMMA", [20, 3, 16, 17], [20000, 130, 33000, 4000]),              # row tiles of different first tiles
+    (2, 4, 2, 20, 900, "UMMA", [40, 64, 33] * 3, [9000, 200, 4000] * 3),
+    (8, 4, 16, 37, 0, "AUTO", [1, 200, 1, 4, 70, 2], [40000, 2000, 300, 20000, 90, 9000]),    # the short requests of a pair launch
+    (2, 4, 16, 60, 0, "AUTO", [100, 1, 1, 3], [1500, 90000, 4000, 50000]),
+])
+def test_ranges_of_several_row_tiles_and_of_pair_launches(Hkv, G, bq, S, window, kernel, qlens, lens):
+    D, qsl = 128, np.concatenate([[0], np.cumsum(qlens)])
+    pair = dict(bq=16 // G, row_class=1, class_rows=16) if kernel == "AUTO" else dict(bq=bq)
+    planned = capi.load_library().schedule(qsl, lens, group=G, num_kv_heads=Hkv, num_splits=S, num_ctas=148, window=window,
+                                           ranges=True, **pair)
+    assert len(planned) > 0 and planned[:, 5].max() > 1
+    if kernel == "UMMA":
+        assert planned[:, 2].max() > 0
+    gen = torch.Generator(device="cuda").manual_seed(Hkv + G + window)
+    storage, views, table, dense = _device_cache(lens, Hkv, D, False, gen)
+    T, Hq = sum(qlens), Hkv * G
+    q = torch.randn((T, Hq, D), generator=gen, device="cuda").to(torch.bfloat16)
+    out = torch.full_like(q, float("nan"))
+    lse = torch.full((T, Hq), float("nan"), device="cuda")
+    ws_o = torch.full((S, T, Hq, D), float("nan"), device="cuda")
+    ws_lse = torch.full((S, T, Hq), float("nan"), device="cuda")
+    host.attention_forward(q, out, views, table, torch.tensor(lens, dtype=torch.int32, device="cuda"),
+                           torch.tensor(qsl, dtype=torch.int32, device="cuda"), bq=bq, num_splits=S, softmax_scale=D ** -0.5,
+                           ws_o=ws_o, ws_lse=ws_lse, lse_out=lse, window=window, kernel=getattr(capi, f"KERNEL_{kernel}"))
+    torch.cuda.synchronize()
+    assert capi.load_library().device_status() == 0
+    for r, (k, v) in enumerate(dense):
+        n, rows = lens[r], slice(int(qsl[r]), int(qsl[r + 1]))
+        pos, at = torch.arange(n, device="cuda"), torch.arange(n - qlens[r], n, device="cuda")[:, None]
+        hidden = (pos > at) | (pos <= at - window if window else pos < 0)
+        for h in range(Hkv):
+            s = torch.einsum("trd,nd->trn", q[rows, h * G:(h + 1) * G].double(), k[:, h]) * D ** -0.5
+            s = s.masked_fill(hidden[:, None], float("-inf"))
+            ref = torch.einsum("trn,nd->trd", s.softmax(-1), v[:, h])
+            check_out(out[rows, h * G:(h + 1) * G].float().cpu().numpy(), ref.cpu().numpy(), what=f"request {r} head {h}")
+            check_lse(lse[rows, h * G:(h + 1) * G].cpu().numpy(), s.logsumexp(-1).cpu().numpy(), what=f"request {r} head {h}")
+
+
 @pytest.mark.parametrize("D, G, bq", [(128, 2, 2), (128, 2, 4), (64, 4, 4), (256, 1, 4)])
 @pytest.mark.parametrize("S", [1, 2])
 def test_rows_without_keys_beside_an_infinite_scale(D, G, bq, S):

@@ -38,6 +38,15 @@ def test_lengths(D, prior):
     check_lse(res["lse"], ref.lse, what=f"D{D} prior {prior}")
 
 
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("requests, prior, ctas", [(1, 400, 1), (1, 900, 4), (1, 1930, 8), (1, 5000, 16), (160, 5000, 1)])
+def test_how_many_ctas_share_a_row_tile(D, requests, prior, ctas):
+    """From 8 tiles on a power of two with two tiles each, on SMs that the launch leaves idle (none beside 160 requests)."""
+    res, ref = _run([37] + [1] * (requests - 1), [prior] + [5] * (requests - 1), D, 4, 1, seed=D + ctas)
+    assert capi.load_library().lib.pthb200_test_row_cluster() == ctas
+    check_out(res["out"], ref.out, what=f"D{D} prior {prior}")
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("D, G, Hkv, qlens, priors", [
     (128, 8, 1, [300], [0]), (128, 1, 2, [600], [700]), (128, 5, 2, [1, 130, 0, 40], [3000, 0, 500, 1290]),
