@@ -30,7 +30,10 @@
  * Units: every stride is in BYTES except block_table_row_stride (int32
  * ELEMENTS).  All pointers are device pointers.  No entry point allocates
  * device memory, copies to the host or synchronises; a launch only enqueues
- * kernels on `stream`, so it can be captured in a CUDA graph.
+ * kernels on `stream`, so it can be captured in a CUDA graph.  The kernels are launched as
+ * programmatic dependents: they may begin to set up while the kernel in front of them on the
+ * stream ends, and read or write device memory only when all work in front of the call is complete.
+ * For the caller the order on the stream is the ordinary one.
  *
  * Semantics (identical to the reference, attn_args.h:20-51): query token i of
  * request r (q_len = qsl[r+1]-qsl[r], L = seq_lens[r], both read on the device)

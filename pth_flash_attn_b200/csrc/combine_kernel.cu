@@ -16,8 +16,8 @@
 // The order of a row's sums depends on its log-sum-exps and the number of splits alone, never on the
 // number of rows or on timing.  What bounds it: two round trips to memory, one after the other, then bandwidth.
 // (One warp per row reading all of its splits' log-sum-exps twice, one after the other with the token count in front, and
-// launched behind the attention kernel's end: mixed batch, 136,000 rows of up to 8 pieces, 97 us, now 49; 768 rows of
-// 256 dims and up to 37 pieces 10.2 and 5.1; 8 x U[1, 4096] keys 22.6 us a call, now 17.7.)
+// launched behind the attention kernel's end: mixed batch, 136,000 rows of up to 8 pieces, 97 us, now 46; 768 rows of
+// 256 dims and up to 37 pieces 7.6 and 4.0; 8 x U[1, 4096] keys 22.6 us a call, now 17.7.)
 //
 // A split with lse = -inf is skipped BEFORE its ws_o row is read, so garbage
 // (NaN included) in the partial of an empty split never reaches the output.

@@ -57,7 +57,7 @@
 // redux.f32, the two integer accumulators joined before their conversion and the digits cut out of
 // two rows at once brought verification of 4 tokens (32 requests x 16 to 32 K keys) from 495 to
 // 406 us, decode at 64 dims from 199 to 193, at 256 dims from 151 to 146 (with ranges, a shorter item end and the steps noted
-// below 357, 145 and 104).
+// below 360 - 381, 149 - 156 and 104 - 110, by box).
 // Every mbarrier wait is bounded: a wait that gives up raises a CTA-wide abort
 // flag (all later waits return at once), sets bit 2 of the status word, and the
 // CTA still finishes and frees its TMEM.
@@ -225,6 +225,9 @@ umma_i8_attention_kernel(const __grid_constant__ KernelParams p, const __grid_co
   // cycles (decode at 64 dims 159.8 -> 156.4 us, 256 dims 118.9 -> 116.5, 8 x 8,192 keys 40.9 -> 39.6).  At 16 rows the
   // softmax is the longest of a tile's stages (verification of 4 tokens 373.8 -> 377 us, 48 decode requests of 4 to
   // 128 K keys in a 16-row launch 1,320 -> 1,371).
+  // Two threads issue MMAs then, on accumulators of their own.  What PV reads is in order without the issuer: P and the folded
+  // O^T by the barrier of the group, the V image by way of `full`, the commit of the tile's QK and s_ready; and `empty`,
+  // which frees the V stage, is committed by the thread that issued the PV.
   constexpr bool kSoftmaxIssuesPV = RQ <= 2;
   constexpr int kMmaWarp = 8 + 4 * NP;     // issues QK, and PV where the softmax does not
   constexpr int kLoadWarp = kMmaWarp + 1;  // this warp and the next issue the page copies

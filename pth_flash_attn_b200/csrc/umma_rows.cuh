@@ -240,7 +240,9 @@ __device__ __forceinline__ SchedShape sched_shape(const KernelParams& p) {
 // sum and accumulator of every row in its shared memory, and then merges and writes a slice of the columns, reading the
 // others' through distributed shared memory.  The host takes the largest cluster with which the launch still is one round
 // of the SMs (instances of their own: the cluster's code in the others cost twelve short prompts 1.5 %); the CTAs share a
-// row tile of 8 tiles of 128 keys or more, at least two tiles each, and those that are not needed leave.
+// row tile of 8 tiles of 128 keys or more, at least two tiles each, and those that are not needed leave.  (The host knows the
+// lengths no better than the block table's rows: a prompt of 16 tokens takes 9.2 us with a table cut to it, 10.3 with one of
+// 131,072 keys a row, whose clusters then have nothing to share.)
 // What bounds it: the walk of a piece, then 3 to 4 us for the merge, which reads 128 KB per CTA (at pieces of one tile it
 // cost more than it gave: 200 tokens without a cache 17.7 us in two pieces, 13.4 in one).  One CTA per row tile / clusters:
 // 200 tokens over 30,000 keys, 1 KV head 569 / 58 us, 8 KV heads over 8,000 162 / 57; 300 over 3,000 at 256 dims 65 / 35,
@@ -251,7 +253,7 @@ __host__ __device__ constexpr int cluster_pieces(int tiles, int cluster) {
   while (tiles >= 8 && 2 * n <= cluster && 4 * n <= tiles) n *= 2;
   return n;
 }
-// (An SM takes one CTA, and the SMs of a cluster come from one group of them: how many clusters of 8 fit at once is asked.)
+// (An SM takes one CTA, and the SMs of a cluster come from one group of them: how many of a size fit at once is asked.)
 template <auto kKernel>
 int clusters_at_once(int size, int threads, int smem) {
   static std::atomic<int> known[64][5];  // by device and log2(size): clusters + 1
@@ -353,8 +355,9 @@ struct RowsItem {
 constexpr int kRowsItemInts = sizeof(RowsItem) / 4;
 static_assert(sizeof(RowTile) == 24 && kRowsItemInts == 14, "as the broadcast copies it");
 // num_splits is a bound: the pieces a request is cut into are chosen here, from the lengths and the launch's KV tiles
-// per head, by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the
-// whole launch, so a prefill chunk among long decode requests is not cut at all.
+// per head, by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the requests that this launch
+// serves.  In a pair launch those are the tall ones alone: two chunks of 136 tiles beside eight verification requests of 256 are
+// cut in two pieces each, those in four, whatever decode requests the integer kernel has.
 template <bool kClusters>
 __device__ __forceinline__ RowsItem rows_item(const KernelParams& p, const RowTile& t, int split, unsigned long long work) {
   RowsItem it;

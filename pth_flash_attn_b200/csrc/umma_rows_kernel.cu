@@ -55,7 +55,7 @@ constexpr int kRVStage = kWideBytes;                 // V image
 constexpr int kRKsRing = 4;                          // tiles of key scales kept
 constexpr int kRQBarrier = kRSoftmax + 32;  // Q image complete: softmax, MMA issuer
 // Registers: the CTA starts with 96 per thread (18 warps: five on two of the SM's four schedulers, whose
-// 16,384 registers that fills).  The two producer warpgroups hand 16 per thread to the two softmax
+// 16,384 registers that fills).  The two producer warpgroups hand 32 per thread to the two softmax
 // warpgroups, which keep the 64 scores of a row and half tile in registers between the two passes;
 // every scheduler has two warps of either kind.
 constexpr int kRProducerRegs = 64, kRSoftmaxRegs = 128;
@@ -372,9 +372,9 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     // overwrites that buffer, waits for PV(i) to have finished reading them - one whole tile
     // of softmax later than it is issued, so the wait is not on the critical path.  PV(i) is
     // two chains: keys 0-63 of the tile into O(0), keys 64-127 into O(1), the accumulators of
-    // the two softmax groups.  (A version with one issuing thread for QK and another for PV
-    // produced results that varied from run to run; a version that polled the barriers and
-    // issued whatever was ready first was slower.)  Operand descriptors are kept as register
+    // the two softmax groups.  (Another issuing warp
+    // for PV cost the two-row-tile kernel 3 %; polling the barriers and
+    // issuing whatever was ready first was slower, too.)  Operand descriptors are kept as register
     // word pairs.
     named_barrier(5, kRQBarrier);  // wait for the Q image
     {
@@ -630,10 +630,8 @@ cudaError_t launch_umma_rows_attention(const KernelParams& p_in, cudaStream_t st
     if (mapp == nullptr) return cudaErrorInvalidValue;
   }
   const CUtensorMap& map = *mapp;
-  // Two K images and three raw half stages (64 keys each).  Consecutive QK MMAs must not read
-  // their K operand from the same shared-memory addresses: with a single K image that the
-  // producers rewrote between two QKs, results varied from run to run although every
-  // producer / consumer edge was ordered by an mbarrier and a proxy fence.
+  // Two K images, so that a tile's keys are widened while the QK of the one in front reads its own, and three raw half
+  // stages (64 keys each): all that fits beside them.
   return launch_rows<2, 3>(p, map, stream);
 }
 

@@ -15,7 +15,8 @@
 // cell, and the row maximum is a reduction over 16 lanes.  A warp issues the loads of two to four cells before it
 // uses any, which leaves the quantisation's instructions as the bound (2 T Hkv D source elements in, T Hkv (2 D + 8)
 // bytes out, at 0.56 of the rate of a copy).
-// 8,192 tokens of 8 KV heads x 128 dims in bf16 (51 MB): 12.0 us a call back to back, 4.2 TB/s.  (One warp per row with
+// 8,192 tokens of 8 KV heads x 128 dims in bf16 (51 MB, which the L2 cache holds from call to call): 12.0 us a call back to
+// back, 4.2 TB/s.  (One warp per row with
 // 2-byte loads, fourteen rows after another: 43 us; with this shape, but maxima and scaling one element at a time, at 77
 // registers and as an ordinary launch: 14.5, of which 1.4 were the launch; 40 registers spill: 15.3.)
 #include <type_traits>

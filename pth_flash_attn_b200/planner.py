@@ -11,10 +11,13 @@ so one plan is valid for every replay of a CUDA graph captured for its descripto
 What is planned differs, because the kernels differ:
 
 * The attention kernel for short row tiles is persistent: it is launched with one CTA per
-  SM, cuts every request into pieces of about equal length ON THE DEVICE (where the
-  lengths are) and deals the pieces out to its CTAs.  The host's ``num_splits`` is
-  therefore only a bound - the most pieces a request may be cut into, which is what sizes
-  the workspace - and the planner's job is to make that bound generous enough:
+  SM and shares the work out among them ON THE DEVICE (where the lengths are): a small
+  launch in pieces of about equal length per request, one with 12 KV tiles per CTA or more
+  in equal runs of the sequence of all KV tiles, which cut a request where a run ends.
+  The host's ``num_splits`` is therefore only a bound - the most pieces a request may be
+  cut into, which is what sizes the workspace (and where too few are allowed for equal
+  runs, the launch keeps equal pieces) - and the planner's job is to make that bound
+  generous enough:
 
       unsplit = Hkv * row tiles of the launch        work items without any split
       S = ceil(ITEMS_PER_SM * SMs / unsplit)         room for the device's choice (it aims at 8 items per SM)
@@ -27,9 +30,11 @@ What is planned differs, because the kernels differ:
   op's frozen schema; rows per tile are 16, 32 or 64 and the kernels pad to those.
 * A sliding window caps the pieces at the number of 128-key tiles a row tile can touch.
 * Tall row tiles (more than 16 rows) run on the row-major kernels, which launch one CTA per
-  (row tile, KV head, piece of the bound): there a generous bound does cost time - CTAs of
-  unused pieces that start only to leave, fp32 partials and a combine for requests the
-  device left whole (a drafter step of 32 requests: 183 us at a bound of 10, 146 us at 1).
+  (row tile, KV head, piece of the bound), as far as a row of the block table or the window
+  is long enough for that many pieces: there a generous bound does cost time - CTAs of
+  unused pieces that start only to leave (2.7 us of an SM each), fp32 partials and a combine
+  for requests the device left whole (a drafter step of 32 requests: 183 us at a bound of
+  10, 146 us at 1).
   Under a sliding window every request longer than the window holds the same work per row
   tile, so pieces only serve to fill the SMs: the bound of a tall windowed launch is
   ``ceil(SMs / unsplit)``.  Without a window the lengths may differ by orders of magnitude
@@ -217,7 +222,8 @@ def plan_launch(
         # Chunks of any length: full 64-row tiles over all tokens.  The bound on the pieces
         # counts REQUESTS, not row tiles: a prefill launch may hold long decode requests of
         # very different lengths (a mixed batch in one launch), which only balance when they
-        # may be cut.  The kernels cut on the device and leave the prefill chunks whole, and
+        # may be cut.  The kernels cut on the device, each by the work of the requests that it
+        # serves (a chunk as often as the other tall requests' work asks for), and
         # the bound only matters to a caller that reserved S * T token-splits for such launches.
         wm = max(WM_CHOICES)
         row_tiles = _ceil_div(requests, 2)
