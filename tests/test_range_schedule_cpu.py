@@ -15,7 +15,7 @@ def _tiles(seq_len, q_len, row_tile, bq, window):
     return (lo // KV_TILE, -(-end // KV_TILE)) if end > lo else (lo // KV_TILE, lo // KV_TILE)
 
 
-def _check(items, qlens, lens, *, bq, S, Hkv, window=0):
+def _check(items, qlens, lens, *, Hkv, bq, S, ctas, window=0):
     """Every row tile and KV head once, its pieces in order and none too many."""
     by_key = {}
     for cta, r, rt, kvh, split, splits, tb, te in items.tolist():
@@ -30,28 +30,37 @@ def _check(items, qlens, lens, *, bq, S, Hkv, window=0):
         assert all(a[3] == b[2] for a, b in zip(pieces, pieces[1:]))
 
 
-def _random_launch(rng, several):
+@pytest.mark.parametrize("seed", range(40))
+def test_random_launches_are_covered_exactly_once(seed):
+    rng = np.random.default_rng(seed)
     R, Hkv = int(rng.integers(1, 70)), int(rng.choice([1, 2, 3, 5, 8, 16]))
     bq, ctas = int(rng.choice([1, 2, 4])), int(rng.choice([7, 148, 148, 160]))
-    qlens = rng.integers(0, 3 * bq + 1 if several else bq + 1, size=R).tolist()
+    qlens = rng.integers(0, bq + 1 if seed % 2 else 3 * bq + 1, size=R).tolist()
     lens = [int(q + rng.integers(1, int(rng.choice([300, 9000, 70000])))) for q in qlens]
     window = int(rng.choice([0, 0, 3000]))
     S = int(rng.choice([2, 5, 37, 296]))
-    return qlens, lens, dict(Hkv=Hkv, bq=bq, S=S, window=window), ctas
+    items = capi.load_library().schedule(np.concatenate([[0], np.cumsum(qlens)]), lens, group=4, num_kv_heads=Hkv, bq=bq,
+                                         num_splits=S, num_ctas=ctas, window=window, ranges=True)
+    if len(items):
+        _check(items, qlens, lens, Hkv=Hkv, bq=bq, S=S, ctas=ctas, window=window)
 
 
 @pytest.mark.parametrize("seed", range(40))
-def test_random_launches_are_covered_exactly_once(seed):
-    """Launches drawn until one is dealt out in ranges (about every second is)."""
-    rng = np.random.default_rng(seed)
+def test_random_launches_that_are_dealt_out(seed):
+    """Launches drawn until one is dealt out in ranges (about every second is): one row tile a request and several."""
+    rng = np.random.default_rng(1000 + seed)
     for _ in range(40):
-        qlens, lens, kw, ctas = _random_launch(rng, seed % 2 == 0)
-        items = capi.load_library().schedule(np.concatenate([[0], np.cumsum(qlens)]), lens, group=4, num_kv_heads=kw["Hkv"],
-                                             bq=kw["bq"], num_splits=kw["S"], num_ctas=ctas, window=kw["window"], ranges=True)
+        R, Hkv = int(rng.integers(1, 70)), int(rng.choice([1, 2, 3, 5, 8, 16]))
+        bq, ctas = int(rng.choice([1, 2, 4])), int(rng.choice([7, 148, 148, 160]))
+        qlens = rng.integers(0, bq + 1 if seed % 2 else 3 * bq + 1, size=R).tolist()
+        lens = [int(q + rng.integers(1, int(rng.choice([300, 9000, 70000])))) for q in qlens]
+        window, S = int(rng.choice([0, 0, 3000])), int(rng.choice([2, 5, 37, 296]))
+        items = capi.load_library().schedule(np.concatenate([[0], np.cumsum(qlens)]), lens, group=4, num_kv_heads=Hkv, bq=bq,
+                                             num_splits=S, num_ctas=ctas, window=window, ranges=True)
         if len(items):
             break
     assert len(items)
-    _check(items, qlens, lens, **kw)
+    _check(items, qlens, lens, Hkv=Hkv, bq=bq, S=S, ctas=ctas, window=window)
 
 
 @pytest.mark.parametrize("lens, Hkv, S, least", [
@@ -66,7 +75,7 @@ def test_ctas_get_equal_loads(lens, Hkv, S, least):
                                          num_ctas=148, ranges=True)
     load = np.bincount(items[:, 0], weights=items[:, 7] - items[:, 6], minlength=148)
     assert load.mean() >= least * load.max()
-    _check(items, [1] * len(lens), lens, Hkv=Hkv, bq=1, S=S)
+    _check(items, [1] * len(lens), lens, Hkv=Hkv, bq=1, S=S, ctas=148)
 
 
 def test_launches_that_keep_equal_pieces():
