@@ -175,7 +175,7 @@ __device__ __forceinline__ float ex2f(float x) {
 // last of them.)
 template <bool kClusters>
 __device__ __forceinline__ void rows_cta(const KernelParams& p, int* kvh, int* tile_index) {
-  const uint32_t x = kClusters ? blockIdx.x / (uint32_t)p.cluster : blockIdx.x;
+  const uint32_t x = kClusters ? blockIdx.x >> (__ffs(p.cluster) - 1) : blockIdx.x;
   const uint32_t t = x / (uint32_t)p.num_kv_heads;
   *kvh = (int)(x - t * (uint32_t)p.num_kv_heads);
   *tile_index = p.num_q_tiles - 1 - (int)t;
@@ -184,7 +184,7 @@ __device__ __forceinline__ void rows_cta(const KernelParams& p, int* kvh, int* t
 // Row tile x of a padded tile grid (tile_map 0), found by one warp among up to kWarpRequests requests, 32 at a
 // time, while others set barriers and TMEM up; its result goes to all threads through shared memory behind the barrier
 // that ends the set-up.  (Not from every warp's own shuffles: the compiler then takes the length of the tile loops
-// for one per lane, which costs them 4 %.)  *work: the launch's KV tiles per head, if they are wanted.
+// for one per lane, which costs them 4 %.)  *work: the lane's part of the launch's KV tiles per head, if they are wanted.
 // (What a CTA does once costs by its instructions, which come from beyond the instruction caches at about ten cycles
 // each: so loops stay rolled here, in stage_queries and in write_rows32.  Twelve new prompts of 37 to 2,500 tokens, CTAs of
 // a handful of tiles: 425 us with all requests copied to shared memory and bisected by everybody behind two barriers, every
@@ -214,10 +214,6 @@ __device__ __forceinline__ RowTile warp_row_tile(const KernelParams& p, int x, b
     }
     if (want_work && r < p.num_reqs)
       *work += (unsigned long long)req_row_tiles(shape, b - a) * (unsigned long long)req_kv_tiles(shape, b - a, c);
-  }
-  if (want_work) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) *work += __shfl_xor_sync(0xffffffffu, *work, o);
   }
   return finish_row_tile(p, x, owner, q0, q1, len);
 }
@@ -309,10 +305,11 @@ cudaError_t launch_row_tiles(const KernelParams& p_in, const CUtensorMap& map, i
   p.cluster = last_row_cluster = cluster_for<kClustered>(p, threads, smem);
   const int64_t ctas = (int64_t)p.num_q_tiles * p.num_kv_heads * p.cluster;
   if (ctas > 0x7fffffff) return cudaErrorInvalidConfiguration;
-  // Pieces that no request of these lengths is cut into get no CTA (one that finds nothing to do still takes an SM for 2.7 us).
+  // Pieces that no request of these lengths is cut into get no CTA (one that finds nothing to do still takes an SM for 1.4 us).
   // That holds as far as the block table is cut to the lengths; an engine's table of the longest context says less.  14 requests
-  // of 8 tokens over 2,000 keys at 64 dims, 85 pieces at most: 67 us with a table of 2,000 keys a row, 213 with one of 131,072;
-  // 20 of 6 over 1,000, 2 KV heads 19 and 51.  (With TMEM taken by every CTA before it looks for work 220 and 53.4.)
+  // of 8 tokens over 2,000 keys at 64 dims, 85 pieces at most: 68 us with a table of 2,000 keys a row, 158 with one of 131,072;
+  // 20 of 6 over 1,000, 2 KV heads 19 and 37.  (Those with the wide table while every CTA summed the launch's work up before it
+  // asked whether its request has that many pieces 213 and 51, with TMEM taken by every CTA besides 220 and 53.)
   const dim3 grid((unsigned)ctas, (unsigned)pieces_bound(tiles_bound(p), p.num_splits));
   if (p.cluster > 1) return pdl_launch_clusters(p.cluster, kClustered, grid, threads, smem, stream, p, map);
   return pdl_launch(kKernel, grid, threads, smem, stream, p, map);
@@ -358,8 +355,11 @@ static_assert(sizeof(RowTile) == 24 && kRowsItemInts == 14, "as the broadcast co
 // per head, by the rule of the integer kernel (sched.cuh) - pieces of about equal length over the requests that this launch
 // serves.  In a pair launch those are the tall ones alone: two chunks of 136 tiles beside eight verification requests of 256 are
 // cut in two pieces each, those in four, whatever decode requests the integer kernel has.
-template <bool kClusters>
-__device__ __forceinline__ RowsItem rows_item(const KernelParams& p, const RowTile& t, int split, unsigned long long work) {
+// work(): those tiles, by all threads that call this.  It is asked for only if the request's own tiles allow this piece and more
+// than one, whatever the others' are (a piece holds kItemTilesMin tiles on the average at least): most pieces of a generous
+// bound are told empty without it, which takes 1.4 us of an SM instead of 2.2.
+template <bool kClusters, class Work>
+__device__ __forceinline__ RowsItem rows_item(const KernelParams& p, const RowTile& t, int split, Work work) {
   RowsItem it;
   it.t = t;
   it.state = 0;
@@ -369,8 +369,10 @@ __device__ __forceinline__ RowsItem rows_item(const KernelParams& p, const RowTi
   it.rows = t.ntok * p.group;
   it.nsplits = p.num_splits;
   if (p.num_splits > 1) {
-    const int t_star = item_tiles(work * (unsigned long long)p.num_kv_heads, p.num_sms);
-    it.nsplits = req_splits(req_kv_tiles(sched_shape(p), t.q_len, t.seq_len), t_star, (int)gridDim.y);
+    const int kv_tiles = req_kv_tiles(sched_shape(p), t.q_len, t.seq_len);
+    const int most = req_splits(kv_tiles, kItemTilesMin, (int)gridDim.y);
+    if (split >= most) return it;
+    it.nsplits = most == 1 ? 1 : req_splits(kv_tiles, item_tiles(work() * (unsigned long long)p.num_kv_heads, p.num_sms), (int)gridDim.y);
     if (split >= it.nsplits) return it;
   }
   split_tiles(p, t, split, it.nsplits, &it.tile_begin, &it.tile_end, &it.range_begin, &it.range_end);
@@ -381,11 +383,17 @@ __device__ __forceinline__ RowsItem rows_item(const KernelParams& p, const RowTi
     if (rank >= it.pieces) {
       it.state = 0;
     } else if (it.state == 1) {
-      it.tile_begin = first + (int)((int64_t)rank * n / it.pieces);
-      it.tile_end = first + (int)((int64_t)(rank + 1) * n / it.pieces);
+      const int log2_pieces = __ffs(it.pieces) - 1;  // (two divisions of 64-bit numbers here: 0.4 us)
+      it.tile_begin = first + (int)((int64_t)rank * n >> log2_pieces);
+      it.tile_end = first + (int)((int64_t)(rank + 1) * n >> log2_pieces);
     }
   }
   return it;
+}
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long w) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+  return w;
 }
 // The launch's KV tiles per head, summed over the CTA (`scratch`: 8 idle bytes).
 template <int kThreads>
@@ -397,8 +405,7 @@ __device__ __forceinline__ unsigned long long cta_work(const KernelParams& p, ui
     const int a = __ldg(p.query_start_loc + r), b = __ldg(p.query_start_loc + r + 1);
     w += (unsigned long long)req_row_tiles(shape, b - a) * (unsigned long long)req_kv_tiles(shape, b - a, __ldg(p.seq_lens + r));
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+  w = warp_sum(w);
   if (threadIdx.x == 0) *total_s = 0ull;
   __syncthreads();
   if ((threadIdx.x & 31) == 0 && w != 0) atomicAdd(total_s, w);

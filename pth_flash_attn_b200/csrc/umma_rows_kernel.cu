@@ -162,7 +162,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     if (warp == 0) {
       unsigned long long work = 0;
       const RowTile found = warp_row_tile(p, tile_index, p.num_splits > 1, sched_shape(p), &work);
-      item = rows_item<kClusters>(p, found, split, work);
+      item = rows_item<kClusters>(p, found, split, [&] { return warp_sum(work); });
       if (lane == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
     }
   } else {
@@ -181,8 +181,7 @@ umma_rows_attention_kernel(const __grid_constant__ KernelParams p, const __grid_
     } else {
       t = resolve_row_tile(p, tile_index);
     }
-    const unsigned long long work = p.num_splits > 1 ? cta_work<kRThreads>(p, smem + L::misc + 16) : 0ull;
-    item = rows_item<kClusters>(p, t, split, work);
+    item = rows_item<kClusters>(p, t, split, [&] { return cta_work<kRThreads>(p, smem + L::misc + 16); });
     if (tid == 0) *reinterpret_cast<RowsItem*>(item_s) = item;
   }
   tc::fence_before_sync();

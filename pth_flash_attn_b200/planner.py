@@ -32,7 +32,7 @@ What is planned differs, because the kernels differ:
 * Tall row tiles (more than 16 rows) run on the row-major kernels, which launch one CTA per
   (row tile, KV head, piece of the bound), as far as a row of the block table or the window
   is long enough for that many pieces: there a generous bound does cost time - CTAs of
-  unused pieces that start only to leave (2.7 us of an SM each), fp32 partials and a combine
+  unused pieces that start only to leave (1.4 us of an SM each), fp32 partials and a combine
   for requests the device left whole (a drafter step of 32 requests: 183 us at a bound of
   10, 146 us at 1).
   Under a sliding window every request longer than the window holds the same work per row
