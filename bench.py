@@ -764,7 +764,7 @@ def main():
                                  f"rotation over {wl.num_sets} cache sets (>= 4x L2)"),
                    "cuda_graph": True,
                    "arithmetic": "int8 cache bytes and int8 digits of Q / P on tcgen05 kind::i8 with int32 accumulators "
-                                 "(short row tiles); int8 cache widened exactly to bf16, tcgen05 kind::f16 with fp32 "
+                                 "(short row tiles); int8 cache widened exactly to fp16, tcgen05 kind::f16 with fp32 "
                                  "accumulators (tall row tiles); fp32 softmax",
                    "kv_bytes_per_pass": wl.bytes_total, "flops_per_pass": wl.flops_total},
         "tflops": wl.flops_total / (ms_pass * 1e-3) / 1e12,
